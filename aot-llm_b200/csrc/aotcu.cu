@@ -18,8 +18,8 @@
 
 #include "../../include/aot_cuda.h"
 #include "gemv.cuh"
-#include "gemm.cuh"
 #include "gemm_tc.cuh"
+#include "kmma.cuh"
 #include "mega.cuh"
 #include "q80stream.cuh"
 #include "floatstream.cuh"
@@ -64,7 +64,7 @@ struct aotcu_ctx {
   uint64_t launches = 0;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   std::vector<struct aotcu_gpu*> gpus;  // live Gpus of this context (freed with it)
-  uint8_t* ximg = nullptr;              // Q8_0 activation images made from reference-layout blocks (launch_q80_stream)
+  uint8_t* ximg = nullptr;              // activations converted from reference-layout blocks (ctx_workspace)
   size_t ximg_bytes = 0;
 };
 
@@ -108,7 +108,7 @@ struct GemvCall {
   int pair = 0;
   size_t cols = 0;
   const void* x = nullptr;
-  int x_mode = 0;  // 0 reference-layout blocks (or f32 for float kinds), 1 block images
+  int x_mode = 0;  // 0 reference-layout blocks (or f32 for float kinds), 1 block images, 2 fragments (Q8_K, kmma.cuh)
   size_t m = 1;
   int epilogue = EPI_STORE;
   const uint8_t* prep[3] = {nullptr, nullptr, nullptr};  // prepared tensor-core operands of each matrix, if any
@@ -119,19 +119,6 @@ static int check_weight_alignment(int kind, const void* w) {
   uintptr_t need = (kind == Q4_K || kind == Q5_K) ? 16 : (kind == F32 ? 4 : 2);
   ARG_CHECK((a % need) == 0, "weights of kind %d must be %zu-byte aligned", kind, (size_t)need);
   return 0;
-}
-
-// m = 8..64 activation rows against K-quant matrices: int8 tensor-core tiles (gemm.cuh).
-// Arguments were checked by launch_gemv.
-template <bool PAIR>
-static int launch_gemm_t(aotcu_ctx* c, const GemmParams& P, int grid, size_t smem) {
-  static bool attr_set[64] = {};
-  int dev = c->device;
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    CU_TRY(cudaFuncSetAttribute(gemm_q8k_mma_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
-    attr_set[dev] = true;
-  }
-  return launch(c, gemm_q8k_mma_kernel<PAIR>, dim3(grid), dim3(GEMM_WARPS * 32), smem, P);
 }
 
 // Q4_K / Q5_K matrices: the tcgen05 kernel (gemm_tc.cuh). A gate/up pair runs as two
@@ -189,59 +176,15 @@ static int launch_gemm_tc(aotcu_ctx* c, const GemvCall& call) {
   return 0;
 }
 
-// 0: choose by size (the tcgen05 kernel works on tiles of 128 rows, one CTA each: it wins
-// once a launch has enough tiles to occupy the GPU, measured 32 us against 45 us for the
-// gate/up pair of the TinyLlama shape, and loses on 16..20 tiles); 1: always; -1: never.
+// 1: prompt chunks of Q4_K / Q5_K matrices go to the tcgen05 kernels (option "tc_gemm" 2). Not the
+// default: their tiles of 128 rows pay about 1.6 K cycles of mbarrier hand-overs per super-block
+// and up to 2.7 K instructions per 64-weight chunk for the digits; kmma.cuh is 1.6x (14336 x
+// 4096 x 64: 48 against 77 us) to 5x (4096 x 14336 x 64: 43 against 230 us) faster.
 static int g_tc_force = 0;
-// Does a prompt chunk go to a tcgen05 kernel? Q4_K / Q5_K only, and (128-row tiles, one CTA
-// each) only with enough tiles to occupy the GPU.
-static bool takes_tc(const aotcu_ctx* c, const GemvCall& call) {
-  bool k4 = g_use_tc && g_tc_force >= 0;
-  int tc_tiles = 0;
-  for (int s = 0; s < call.nseg; s++) {
-    k4 = k4 && (call.seg[s].kind == Q4_K || call.seg[s].kind == Q5_K);
-    tc_tiles += (call.seg[s].rows + TC_ROWS - 1) / TC_ROWS;
-  }
-  return k4 && (g_tc_force > 0 || tc_tiles >= c->n_sm / 2);
-}
-static int launch_gemm(aotcu_ctx* c, const GemvCall& call) {
-  if (takes_tc(c, call)) return launch_gemm_tc(c, call);
-  GemmParams P = {};
-  int tiles = 0;
-  for (int s = 0; s < call.nseg; s++) {
-    P.seg[s] = call.seg[s];
-    P.tiles_before[s] = tiles;
-    if (!call.pair || s == 0) tiles += (call.seg[s].rows + 15) / 16;
-  }
-  if (call.pair) P.tiles_before[1] = 0;
-  P.nseg = call.nseg;
-  P.pair = call.pair;
-  P.cols = (int)call.cols;
-  P.m = (int)call.m;
-  P.epilogue = call.epilogue;
-  P.x = reinterpret_cast<const uint8_t*>(call.x);
-  P.x_image = call.x_mode == 1;
-  P.n_tiles = tiles;
-  P.n_groups = (P.m + GEMM_TOK - 1) / GEMM_TOK;
-  const int nb = (int)(call.cols / 256), n_mat = call.pair ? 2 : 1;
-  // The warps of a tile split its super-blocks four ways when there are enough of them.
-  P.ks = nb >= 4 ? 4 : (nb >= 2 ? 2 : 1);
-  const int tpc = GEMM_WARPS / P.ks;
-  // Super-blocks staged at a time: all of them if images + terms fit, else as many as fit
-  // beside a second resident CTA.
-  const size_t per_block = (size_t)GEMM_TOK * XK_STRIDE + (size_t)tpc * n_mat * 32 * GEMM_NT * 4 * sizeof(float);
-  const size_t budget = c->max_smem / 2 - 2048;
-  int kc = nb;
-  if ((size_t)kc * per_block > budget) kc = (int)(budget / per_block);
-  ARG_CHECK(kc >= 1, "one super-block column does not fit in shared memory");
-  kc = (kc / P.ks) * P.ks > 0 ? (kc / P.ks) * P.ks : kc;  // whole strides of the k-split
-  P.kc = kc;
-  const size_t smem = (size_t)kc * per_block;
-  int ctas_per_group = (tiles + tpc - 1) / tpc;
-  const int cap = (c->n_sm * 2) / P.n_groups;
-  if (ctas_per_group > cap) ctas_per_group = cap < 1 ? 1 : cap;
-  const int grid = ctas_per_group * P.n_groups;
-  return call.pair ? launch_gemm_t<true>(c, P, grid, smem) : launch_gemm_t<false>(c, P, grid, smem);
+static bool takes_tc(const GemvCall& call) {
+  bool k4 = g_use_tc && g_tc_force > 0 && call.m >= 8 && call.m <= (size_t)TC_TOK;
+  for (int s = 0; s < call.nseg; s++) k4 = k4 && (call.seg[s].kind == Q4_K || call.seg[s].kind == Q5_K);
+  return k4;
 }
 
 // Fields of a MegaOp the kernels would otherwise derive with integer divisions.
@@ -326,6 +269,107 @@ static int launch_gemv_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
     const size_t smem = (size_t)n_stages * STREAM_STAGE_BYTES + fixed;
     auto kernel = P.q80 ? gemv_stream_kernel<0> : (P.wide ? gemv_stream_kernel<1> : gemv_stream_kernel<2>);
     if (int rc = launch(c, kernel, dim3(grid), dim3(MEGA_THREADS), smem, P)) return rc;
+  }
+  return 0;
+}
+
+// The context's conversion buffer, at least `need` bytes: kept from call to call, grown on demand
+// (not during a stream capture: 1 then, and the caller takes a path without it).
+static int ctx_workspace(aotcu_ctx* c, size_t need) {
+  if (need <= c->ximg_bytes) return 0;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CU_TRY(cudaStreamIsCapturing(c->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return 1;
+  CU_TRY(cudaStreamSynchronize(c->stream));
+  if (c->ximg) cudaFree(c->ximg);
+  c->ximg = nullptr;
+  c->ximg_bytes = 0;
+  CU_TRY(cudaMalloc(&c->ximg, need));
+  c->ximg_bytes = need;
+  return 0;
+}
+
+// K-quant products of several activation rows on the int8 tensor-core kernel of kmma.cuh.
+// Activations that are not in its fragment order are converted first. Returns 1 when the call
+// does not fit.
+template <int KIND, int RT, bool PAIR, int WK>
+static int launch_kmma_t(aotcu_ctx* c, KmmaParams& P, int grid) {
+  using S = KmmaShape<KIND, RT, PAIR, WK>;
+  static bool attr_set[64] = {};
+  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(kmma_kernel<KIND, RT, PAIR, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    attr_set[c->device] = true;
+  }
+  P.n_stages = (int)std::min<size_t>(8, (c->max_smem - S::FIXED) / (KM_WARPS * S::A_SLOT));
+  return launch(c, kmma_kernel<KIND, RT, PAIR, WK>, dim3(grid), dim3(KM_WARPS * 32), (size_t)S::FIXED + (size_t)P.n_stages * KM_WARPS * S::A_SLOT, P);
+}
+template <int KIND>
+static int launch_kmma_k(aotcu_ctx* c, KmmaParams& P, int rt, bool pair, int wk, int grid) {
+  if (pair) return wk == 8 ? launch_kmma_t<KIND, 2, true, 8>(c, P, grid) : launch_kmma_t<KIND, 2, true, 4>(c, P, grid);
+  if (rt == 2) return wk == 8 ? launch_kmma_t<KIND, 2, false, 8>(c, P, grid) : launch_kmma_t<KIND, 2, false, 4>(c, P, grid);
+  return wk == 8 ? launch_kmma_t<KIND, 1, false, 8>(c, P, grid) : launch_kmma_t<KIND, 1, false, 4>(c, P, grid);
+}
+// The matrices of one kind of `call` (all of them have it), activations in fragment order.
+static int launch_kmma_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xf, int xf_nt) {
+  const int nb = (int)(call.cols / 256), kind = call.seg[0].kind;
+  // Shape: a CTA's tile costs ceil(nb / WK) stages; two row tiles per warp instead of one cost
+  // about 1.5 times as much.
+  int rt = 2, wk = 8;
+  double best = 1e30;
+  for (int k : {8, 4})
+    for (int r = call.pair ? 2 : 1; r <= 2; r++) {
+      const int rows = 16 * (call.pair ? 1 : r) * (KM_WARPS / k);
+      int tiles = 0;
+      for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) tiles += (call.seg[s].rows + rows - 1) / rows;
+      const double t = (double)((tiles + c->n_sm - 1) / c->n_sm) * ((nb + k - 1) / k) * (r == 2 ? 1.5 : 1.0);
+      if (t < best * 0.999) {
+        best = t;
+        rt = r;
+        wk = k;
+      }
+    }
+  const int rows = 16 * (call.pair ? 1 : rt) * (KM_WARPS / wk);
+  KmmaParams P = {};
+  int tiles = 0;
+  for (int s = 0; s < call.nseg; s++) {
+    P.seg[s] = call.seg[s];
+    P.tiles_before[s] = call.pair ? 0 : tiles;
+    if (!call.pair || s == 0) tiles += (call.seg[s].rows + rows - 1) / rows;
+  }
+  P.nseg = call.nseg;
+  P.cols = (int)call.cols;
+  P.epilogue = call.epilogue;
+  P.n_tiles = tiles;
+  P.xf_nt = xf_nt;
+  const int grid = tiles < c->n_sm ? tiles : c->n_sm;
+  for (size_t t0 = 0; t0 < call.m; t0 += KM_MAX_M) {
+    P.m = (int)std::min<size_t>(KM_MAX_M, call.m - t0);
+    P.nt = (P.m + 7) / 8;
+    P.xf = xf + (t0 / 8) * XF_BLOCK;
+    for (int s = 0; s < call.nseg; s++) P.seg[s].out = call.seg[s].out + t0 * (size_t)call.seg[s].rows;
+    const bool pair = call.pair != 0;
+    const int rc = kind == Q4_K ? launch_kmma_k<Q4_K>(c, P, rt, pair, wk, grid)
+                   : kind == Q5_K ? launch_kmma_k<Q5_K>(c, P, rt, pair, wk, grid) : launch_kmma_k<Q6_K>(c, P, rt, pair, wk, grid);
+    if (rc) return rc;
+  }
+  return 0;
+}
+static int launch_kmma(aotcu_ctx* c, const GemvCall& call) {
+  const int nb = (int)(call.cols / 256), nt = (int)((call.m + 7) / 8);
+  const uint8_t* xf = reinterpret_cast<const uint8_t*>(call.x);
+  if (call.x_mode != 2) {
+    if (const int rc = ctx_workspace(c, (size_t)nt * nb * XF_BLOCK)) return rc;
+    if (int rc = launch(c, xf_kernel, dim3((unsigned)nt * nb), dim3(256), 0, xf, call.x_mode, c->ximg, (int)call.m, nb)) return rc;
+    xf = c->ximg;
+  }
+  if (call.pair) return launch_kmma_one(c, call, xf, nt);
+  for (int kind : {Q4_K, Q5_K, Q6_K}) {
+    GemvCall one = call;
+    one.nseg = 0;
+    for (int s = 0; s < call.nseg; s++)
+      if (call.seg[s].kind == kind) one.seg[one.nseg++] = call.seg[s];
+    if (one.nseg)
+      if (int rc = launch_kmma_one(c, one, xf, nt)) return rc;
   }
   return 0;
 }
@@ -451,18 +495,7 @@ static int launch_q80_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   // converted into a buffer of the context first (grown here: not during a stream capture).
   const uint8_t* ximg = reinterpret_cast<const uint8_t*>(call.x);
   if (!P.x_image) {
-    const size_t need = call.m * x_image_bytes;
-    if (need > c->ximg_bytes) {
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      CU_TRY(cudaStreamIsCapturing(c->stream, &cs));
-      if (cs != cudaStreamCaptureStatusNone) return 1;
-      CU_TRY(cudaStreamSynchronize(c->stream));
-      if (c->ximg) cudaFree(c->ximg);
-      c->ximg = nullptr;
-      c->ximg_bytes = 0;
-      CU_TRY(cudaMalloc(&c->ximg, need));
-      c->ximg_bytes = need;
-    }
+    if (const int rc = ctx_workspace(c, call.m * x_image_bytes)) return rc;
     const int n_blocks = (int)(call.m * nb);
     if (int rc = launch(c, q80_to_image_kernel, dim3(grid_for(c, (size_t)n_blocks * 9, 256)), dim3(256), 0,
                         reinterpret_cast<const uint8_t*>(call.x), c->ximg, n_blocks))
@@ -570,11 +603,11 @@ static int launch_float_stream(aotcu_ctx* c, const GemvCall& call, size_t span) 
   return 0;
 }
 
-// K-quant products of a short batch of activation rows (2..7, and up to a few dozen on small
-// matrices: see launch_gemv): gemv_stream_kernel<3>, one lane per super-block, grid = (row
+// K-quant products of the smallest batches (see launch_gemv): gemv_stream_kernel<3>, one lane per super-block, grid = (row
 // ranges) x (groups of activation rows). Returns 1 when the call does not fit.
-static int g_wide_multi = 1;  // option "wide_multi": 0 keeps these launches on gemm_q8k_mma_kernel / the per-row loop
-static int g_wide_multi_work = 57344;  // option "wide_multi_work": weight rows x activation rows up to which 8..64 rows take it
+static int g_wide_multi = 1;          // option "wide_multi": 0 sends these products to kmma.cuh as well
+static int g_wide_multi_work = 8192;  // option "wide_multi_work": weight rows x activation rows up to which three rows or more take it
+static bool takes_kmma(size_t m, size_t work) { return !g_wide_multi || (m > 2 && work > (size_t)g_wide_multi_work); }
 static int launch_gemv_stream_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
   if (call.pair || g_dbg_sumi || call.cols % 256) return 1;
   StreamGemvParams P = {};
@@ -680,18 +713,18 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
   }
   ARG_CHECK(((uintptr_t)call.x % (P.x_image ? 16 : 4)) == 0, "activation blocks are misaligned");
 
-  // Prompt chunks of K-quant matrices go to the tensor-core kernel, single rows to the
-  // streaming kernel (whole rows per warp, no barrier per tile).
-  // Short batches of K-quant products: one lane per super-block against every activation row
-  // (time grows with rows x batch: 2048 x 2048 8.5 us at 8 rows, 17 us at 32), where the
-  // tile kernels' time hardly depends on the batch (14-17 us). Measured break-even: about
-  // 57 K (weight rows x activation rows); below 8 rows the alternative is a loop over rows.
-  if (act == ACT_Q8_K && call.m >= 2 && call.m <= (size_t)GEMM_MAX_M && g_wide_multi &&
-      (call.m < 8 || (!takes_tc(c, call) && call.m * span <= (size_t)g_wide_multi_work))) {
-    const int rc = launch_gemv_stream_multi(c, call, span);
-    if (rc <= 0) return rc;  // 1: a pair or a very long row, the tile kernels take it
+  // K-quant products of several activation rows: the tensor-core kernel of kmma.cuh, but for two
+  // rows and the smallest products one lane per super-block against every row, whose time grows
+  // with rows x batch (2048 x 2048: 4.1 us at 2 rows and 8.3 at 8 against 6.8 at either).
+  if (act == ACT_Q8_K && call.m >= 2) {
+    if (takes_tc(call)) return launch_gemm_tc(c, call);
+    if (!takes_kmma(call.m, call.m * span) && call.x_mode != 2) {
+      const int rc = launch_gemv_stream_multi(c, call, span);
+      if (rc <= 0) return rc;  // 1: a pair or a very long row
+    }
+    const int rc = launch_kmma(c, call);
+    if (rc <= 0) return rc;  // 1: a conversion buffer would have to grow during a stream capture
   }
-  if (act == ACT_Q8_K && call.m >= 8 && call.m <= (size_t)GEMM_MAX_M) return launch_gemm(c, call);
   if (act == ACT_Q8_0 && g_q80_chunks) {
     const int rc = launch_q80_stream(c, call, span);
     if (rc <= 0) return rc;  // 1: mixed kinds or a very long activation row, the whole-row kernels take it
@@ -843,6 +876,7 @@ struct aotcu_gpu {
     const float* ptr = nullptr;
     size_t n = 0, m = 0;
     bool q8k = false, q80 = false;
+    bool xf = false;  // q8k: in fragment order
   } qsrc;
   bool use_graph = true;
   // Persistent one-kernel decode step (mega.cuh), when the model qualifies.
@@ -899,6 +933,9 @@ static void note_write(aotcu_gpu* g, const float* p) {
 }
 
 // Make sure the block images of `src` (m rows of n floats) exist for `act`.
+// Q8_K activations of several rows are kept in the fragment order of kmma.cuh, those of a single
+// row (and of chunks sent to the tcgen05 kernels) as block images.
+static bool xf_rows(size_t m) { return m >= 2 && g_tc_force <= 0; }
 static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, int act) {
   if (act == ACT_F32) return 0;
   aotcu_ctx* c = g->c;
@@ -909,11 +946,16 @@ static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, 
     g->qsrc.n = n;
     g->qsrc.m = m;
   }
-  if (act == ACT_Q8_K && !g->qsrc.q8k) {
+  if (act == ACT_Q8_K && (!g->qsrc.q8k || g->qsrc.xf != xf_rows(m))) {
     ARG_CHECK(n % 256 == 0, "row length %zu is not a multiple of 256", n);
     int nblk = (int)(n * m / 256);
-    if (int rc = launch(c, quantize_q8k_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, nblk, 1)) return rc;
+    if (xf_rows(m)) {
+      if (int rc = launch(c, quantize_xf_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, (int)m, (int)(n / 256))) return rc;
+    } else {
+      if (int rc = launch(c, quantize_q8k_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, nblk, 1)) return rc;
+    }
     g->qsrc.q8k = true;
+    g->qsrc.xf = xf_rows(m);
   }
   if (act == ACT_Q8_0 && !g->qsrc.q80) {
     ARG_CHECK(n % 32 == 0, "row length %zu is not a multiple of 32", n);
@@ -924,6 +966,7 @@ static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, 
   return 0;
 }
 
+static int act_mode(int act, size_t m) { return act == ACT_Q8_K && xf_rows(m) ? 2 : 1; }
 static const void* act_images(const aotcu_gpu* g, int act, const float* src) {
   return act == ACT_Q8_K ? (const void*)g->aqk : act == ACT_Q8_0 ? (const void*)g->aq0 : (const void*)src;
 }
@@ -943,6 +986,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   bool q = quantize && !accumulate && dst_stride == n;
   P.q8k_out = (q && g->need_q8k && n % 256 == 0) ? g->aqk : nullptr;
   P.q80_out = (q && g->need_q80 && n % 32 == 0) ? g->aq0 : nullptr;
+  P.xf_nt = P.q8k_out && xf_rows(m) ? (int)((m + 7) / 8) : 0;
   size_t smem = (2 * n + 4) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "rmsnorm row of %zu floats does not fit shared memory", n);
   note_write(g, dst);
@@ -953,6 +997,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
     g->qsrc.n = n;
     g->qsrc.m = m;
     g->qsrc.q8k = P.q8k_out != nullptr;
+    g->qsrc.xf = P.xf_nt > 0;
     g->qsrc.q80 = P.q80_out != nullptr;
   }
   return 0;
@@ -961,7 +1006,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
 // dst (+)= W . src for m rows (Gpu::mv / Gpu::matmul).
 // Prepared operands of tensor t for a batch of m rows, or null.
 static const uint8_t* prep_of(const aotcu_gpu* g, const aotcu_tensor& t, size_t m) {
-  if (g->prep_state != 1 || m < 8 || m > (size_t)TC_TOK) return nullptr;
+  if (g->prep_state != 1 || g_tc_force <= 0 || m < 8 || m > (size_t)TC_TOK) return nullptr;
   auto it = g->prep.find(t.off);
   return it == g->prep.end() ? nullptr : it->second;
 }
@@ -970,35 +1015,16 @@ static const uint8_t* prep_of(const aotcu_gpu* g, const aotcu_tensor& t, size_t 
 // only when they take at most half of the memory that is free, so that a model sized for
 // the device keeps fitting; otherwise prompt chunks keep unpacking weights per launch.
 static int ensure_prepared(aotcu_gpu* g) {
-  if (g->prep_state != 0) return 0;
+  if (g->prep_state != 0 || !g_use_tc || g_tc_force <= 0) return 0;
   g->prep_state = -1;
-  if (!g_use_tc || g_tc_force < 0) return 0;
   std::vector<const aotcu_tensor*> ts;
   size_t total = 0;
-  // only matrices whose launches reach the tensor-core kernel (launch_gemm: at least n_sm / 2
-  // tiles of 128 rows per launch): q/k/v go out as one launch, gate/up as one, wo and down alone
-  auto k4 = [](const aotcu_tensor* t) { return (t->kind == Q4_K || t->kind == Q5_K) && t->cols % 256 == 0; };
-  auto tiles = [](const aotcu_tensor* t) { return (int)((t->rows + TC_ROWS - 1) / TC_ROWS); };
-  const int need = g_tc_force > 0 ? 1 : g->c->n_sm / 2;
-  auto want = [&](std::initializer_list<const aotcu_tensor*> group) {
-    int n = 0;
-    for (auto t : group) {
-      if (!k4(t) || t->cols != (*group.begin())->cols) return;
-      n += tiles(t);
-    }
-    if (n < need) return;
-    for (auto t : group)
-      if (!g->prep.count(t->off) && std::find(ts.begin(), ts.end(), t) == ts.end()) {
+  for (const auto& l : g->layers)
+    for (auto t : {&l.wq, &l.wk, &l.wv, &l.gate, &l.up, &l.wo, &l.down})
+      if ((t->kind == Q4_K || t->kind == Q5_K) && t->cols % 256 == 0 && std::find(ts.begin(), ts.end(), t) == ts.end()) {
         ts.push_back(t);
         total += tc_prep_bytes(t->rows, t->cols);
       }
-  };
-  for (const auto& l : g->layers) {
-    want({&l.wq, &l.wk, &l.wv});
-    want({&l.gate, &l.up});
-    want({&l.wo});
-    want({&l.down});
-  }
   if (ts.empty()) return 0;
   size_t free_b = 0, total_b = 0;
   CU_TRY(cudaMemGetInfo(&free_b, &total_b));
@@ -1024,7 +1050,7 @@ static int gpu_matmul(aotcu_gpu* g, float* dst, const aotcu_tensor& t, const flo
   call.nseg = 1;
   call.cols = t.cols;
   call.x = act_images(g, act, src);
-  call.x_mode = 1;
+  call.x_mode = act_mode(act, m);
   call.m = m;
   call.epilogue = accumulate ? EPI_ACCUM : EPI_STORE;
   call.prep[0] = prep_of(g, t, m);
@@ -1054,7 +1080,7 @@ static int gpu_mv3(aotcu_gpu* g, float* const dst[3], const aotcu_tensor* const 
     if (int rc = ensure_quantized(g, src, t[a]->cols, m, act)) return rc;
     call.cols = t[a]->cols;
     call.x = act_images(g, act, src);
-    call.x_mode = 1;
+    call.x_mode = act_mode(act, m);
     call.m = m;
     if (int rc = launch_gemv(g->c, call)) return rc;
   }
@@ -1075,7 +1101,7 @@ static int gpu_gate_up(aotcu_gpu* g, float* hb, float* hb2, const aotcu_tensor& 
     call.pair = 1;
     call.cols = gate.cols;
     call.x = act_images(g, act, src);
-    call.x_mode = 1;
+    call.x_mode = act_mode(act, m);
     call.m = m;
     call.epilogue = gelu ? EPI_STORE : EPI_SILU_MUL;
     call.prep[0] = prep_of(g, gate, m);
@@ -2059,7 +2085,8 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   {
     size_t widest = xbw > (size_t)d.hidden ? xbw : (size_t)d.hidden;
     size_t rows = g->max_batch;
-    G_TRY(cudaMalloc(&g->aqk, rows * (widest / 256 + 1) * XIMG_K));
+    G_TRY(cudaMalloc(&g->aqk, ((rows + 7) / 8) * (widest / 256 + 1) * 8 * XIMG_K));  // whole groups of 8 rows (XF_BLOCK <= 8 * XIMG_K)
+    G_TRY(cudaMemsetAsync(g->aqk, 0, ((rows + 7) / 8) * (widest / 256 + 1) * 8 * XIMG_K, c->stream));
     G_TRY(cudaMalloc(&g->aq0, rows * (widest / 32 + 1) * XIMG_0));
   }
   // Attention scores: shared memory when the context fits, else a global scratch.
@@ -2615,8 +2642,7 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
     return 0;
   }
   if (!strcmp(name, "tc_gemm")) {
-    // process-wide: prompt chunks of Q4_K / Q5_K matrices on tcgen05 (2: always, 1: when the
-    // launch has enough 128-row tiles to occupy the GPU) or on mma.sync tiles (0)
+    // process-wide: prompt chunks of Q4_K / Q5_K matrices on tcgen05 (2) or on kmma.cuh (1, 0)
     g_use_tc = value != 0;
     g_tc_force = value >= 2 ? 1 : 0;
     return 0;

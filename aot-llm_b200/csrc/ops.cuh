@@ -8,6 +8,8 @@
 // reference's order with unfused round-to-nearest operations; order-free
 // reductions (max, argmax, integer sums) run in parallel.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "blockmath.cuh"
 #include "device_utils.cuh"
 #include "expf_exact.cuh"
@@ -48,7 +50,12 @@ __device__ __forceinline__ float block_seq_sum(const float* p, int n, float* slo
 // the reference's BlockQ8_K layout (image == 0) or as the 304-byte image the GEMV
 // kernels read (image == 1).
 // Core: lane holds elements 8*lane .. 8*lane+7 of the block in v[].
-__device__ __forceinline__ void warp_quantize_q8k_vals(const float (&v)[8], uint8_t* dst, int image) {
+struct Q8kLane {
+  uint32_t w0, w1;  // the lane's eight quants
+  int s;            // their sum
+  float d;          // the block's scale
+};
+__device__ __forceinline__ Q8kLane warp_q8k_lane(const float (&v)[8]) {
   const int lane = threadIdx.x & 31;
   // signed extreme: the first element with strictly larger |v|. |v| orders like its bit
   // pattern; a NaN never compares larger in the reference and counts as zero here. Two
@@ -70,29 +77,58 @@ __device__ __forceinline__ void warp_quantize_q8k_vals(const float (&v)[8], uint
   const uint32_t widx = __reduce_min_sync(0xffffffffu, best == wmax ? (uint32_t)idx : 256u);
   mx = __shfl_sync(0xffffffffu, mx, (int)(widx >> 3));
   const float amax = __uint_as_float(wmax);
-  int8_t* qs = reinterpret_cast<int8_t*>(dst + (image ? 0 : 4));
-  int16_t* bs = reinterpret_cast<int16_t*>(dst + (image ? 256 : 260));
-  float* dptr = reinterpret_cast<float*>(dst + (image ? 288 : 0));
-  uint32_t w0 = 0, w1 = 0;
-  int s = 0;
-  float d = 0.0f;
+  Q8kLane r{0u, 0u, 0, 0.0f};
   if (amax != 0.0f) {
     float iscale = fdiv(-127.0f, mx);
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       int q = (int)roundf(fmul(iscale, v[i]));
       q = q > 127 ? 127 : q;
-      s += q;
+      r.s += q;
       uint32_t b = (uint32_t)(q & 0xFF);
-      if (i < 4) w0 |= b << (8 * i); else w1 |= b << (8 * (i - 4));
+      if (i < 4) r.w0 |= b << (8 * i); else r.w1 |= b << (8 * (i - 4));
     }
-    d = fdiv(1.0f, iscale);
+    r.d = fdiv(1.0f, iscale);
   }
-  reinterpret_cast<uint32_t*>(qs)[2 * lane] = w0;
-  reinterpret_cast<uint32_t*>(qs)[2 * lane + 1] = w1;
-  int s2 = s + __shfl_xor_sync(0xffffffffu, s, 1);
+  return r;
+}
+__device__ __forceinline__ void warp_quantize_q8k_vals(const float (&v)[8], uint8_t* dst, int image) {
+  const int lane = threadIdx.x & 31;
+  const Q8kLane r = warp_q8k_lane(v);
+  int8_t* qs = reinterpret_cast<int8_t*>(dst + (image ? 0 : 4));
+  int16_t* bs = reinterpret_cast<int16_t*>(dst + (image ? 256 : 260));
+  float* dptr = reinterpret_cast<float*>(dst + (image ? 288 : 0));
+  reinterpret_cast<uint32_t*>(qs)[2 * lane] = r.w0;
+  reinterpret_cast<uint32_t*>(qs)[2 * lane + 1] = r.w1;
+  int s2 = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
   if ((lane & 1) == 0) bs[lane >> 1] = (int16_t)s2;
-  if (lane == 0) *dptr = d;
+  if (lane == 0) *dptr = r.d;
+}
+
+// Activations of several rows in the order the tensor-core products read them ("XF", see
+// kmma.cuh): [super-block][token group of 8], XF_BLOCK bytes each. Lane l of the warp holds the
+// quants 8l .. 8l+7 of token `g` of the group; lanes 0..15 the sums of the 16-element groups.
+constexpr int XF_BLOCK = 2336;
+constexpr int XF_BSUMS = 2048;
+constexpr int XF_D = 2304;
+__device__ __forceinline__ void xf_store(uint8_t* o, int g, int lane, uint32_t w0, uint32_t w1, int bsum, float d) {
+  const int s = lane >> 1, h = lane & 1;
+  uint32_t* q = reinterpret_cast<uint32_t*>(o + ((s >> 2) * 32 + g * 4 + 2 * h) * 16 + (s & 3) * 4);
+  q[0] = w0;
+  q[4] = w1;
+  if (lane < 16)
+    reinterpret_cast<__half*>(o + XF_BSUMS + (g * 4 + ((lane & 7) >> 1)) * 8)[(lane >> 3) * 2 + (lane & 1)] = __int2half_rn(bsum);
+  if (lane == 0) *reinterpret_cast<float*>(o + XF_D + 4 * g) = d;
+}
+// Block b of row `tok` (of nt groups of 8 rows), quantized straight into that order.
+__device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, int tok, int b, int nt) {
+  const int lane = threadIdx.x & 31;
+  const float4 a = reinterpret_cast<const float4*>(src)[2 * lane], c = reinterpret_cast<const float4*>(src)[2 * lane + 1];
+  const float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+  const Q8kLane r = warp_q8k_lane(v);
+  const int s2 = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
+  const int bs = __shfl_sync(0xffffffffu, s2, (2 * lane) & 31);
+  xf_store(xf + ((size_t)b * nt + (tok >> 3)) * XF_BLOCK, tok & 7, lane, r.w0, r.w1, bs, r.d);
 }
 
 template <bool CG = false>
@@ -136,6 +172,13 @@ __global__ void quantize_q8k_kernel(const float* __restrict__ x, uint8_t* __rest
   int nw = (gridDim.x * blockDim.x) >> 5;
   for (int b = wid; b < n_blocks; b += nw) warp_quantize_q8k(x + (size_t)b * 256, out + (size_t)b * (image ? XIMG_K : 292), image);
 }
+// m rows of nb blocks into the fragment order.
+__global__ void quantize_xf_kernel(const float* __restrict__ x, uint8_t* __restrict__ xf, int m, int nb) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5, nt = (m + 7) >> 3;
+  for (int i = wid; i < m * nb; i += nw) warp_quantize_xf(x + (size_t)i * 256, xf, i / nb, i % nb, nt);
+}
 __global__ void quantize_q80_kernel(const float* __restrict__ x, uint8_t* __restrict__ out, int n_blocks, int image) {
   pdl_launch_dependents();
   pdl_wait();
@@ -176,6 +219,7 @@ struct RmsnormParams {
   float eps;
   int accumulate;    // out[i] = out[i] + y[i] (Gemma post-norm residual join)
   uint8_t* q8k_out;  // images, n/256 per row
+  int xf_nt;         // > 0: q8k_out in fragment order instead, this many groups of 8 rows
   uint8_t* q80_out;  // images, n/32 per row
 };
 
@@ -205,8 +249,10 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   if (P.q8k_out) {
     int nb = P.n / 256;
-    for (int b = warp; b < nb; b += nwarps)
-      warp_quantize_q8k(row + b * 256, P.q8k_out + ((size_t)blockIdx.x * nb + b) * XIMG_K, 1);
+    for (int b = warp; b < nb; b += nwarps) {
+      if (P.xf_nt) warp_quantize_xf(row + b * 256, P.q8k_out, blockIdx.x, b, P.xf_nt);
+      else warp_quantize_q8k(row + b * 256, P.q8k_out + ((size_t)blockIdx.x * nb + b) * XIMG_K, 1);
+    }
   }
   if (P.q80_out) {
     int nb = P.n / 32;

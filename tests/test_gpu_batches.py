@@ -1,0 +1,44 @@
+"""Products of several activation rows at the sizes where their kernels change path: edges of row
+tiles and token groups, super-block counts around the number a CTA splits, and integers at the
+ends of their range. Bit-exact against the CPU oracle (batched == per-token,
+crates/aot-kernels/tests/dots.rs:205-266)."""
+import numpy as np
+import pytest
+
+from conftest import assert_bits_equal, make_weights
+
+pytestmark = pytest.mark.gpu
+
+Q4_K, Q5_K, Q6_K = 6, 7, 8
+
+
+def _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, what):
+    q = ob.quantize_act(kind, xs)
+    want = ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols)
+    dout = ctx.alloc(m * rows * 4)
+    ctx.matmul(kind, dout, ctx.to_device(w), ctx.to_device(q.view(np.uint8)), m, rows, cols)
+    assert_bits_equal(dout.download(np.float32, m * rows).reshape(m, rows), want, what)
+    ctx.device_status()
+
+
+@pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (17, 768), (2400, 2304), (4735, 1280)])
+def test_k_quant_tile_edges(pkg, ob, ctx, kind, rows, cols):
+    w = make_weights(pkg, kind, rows, cols, 21 + kind + rows, "uniform")
+    for m in (3, 8, 9, 17, 64, 65):
+        xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+        _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+
+
+@pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
+def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, kind):
+    rows, cols, m = 48, 1024, 12
+    w = make_weights(pkg, kind, rows, cols, 5, "uniform").reshape(rows * cols // 256, -1)
+    w[:, 4:] = 0xFF                                   # largest quants, scales and mins (Q4_K, Q5_K)
+    if kind == Q6_K:
+        w[:, :192] = np.where(np.arange(w.shape[0])[:, None] % 2, 0xFF, 0x00)   # 31 or -32 ...
+        w[:, 192:208] = 0x80                                                    # ... times -128
+        w[:, 208:210] = np.frombuffer(np.float16(0.01).tobytes(), dtype=np.uint8)
+    xs = np.ones(m * cols, dtype=np.float32)
+    xs[cols:2 * cols] = -1.0                          # every quant -127, or 127
+    _run(pkg, ob, ctx, kind, w.reshape(-1), xs, m, rows, cols, f"kind {kind} at the bounds")
