@@ -987,7 +987,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   P.q8k_out = (q && g->need_q8k && n % 256 == 0) ? g->aqk : nullptr;
   P.q80_out = (q && g->need_q80 && n % 32 == 0) ? g->aq0 : nullptr;
   P.xf_nt = P.q8k_out && xf_rows(m) ? (int)((m + 7) / 8) : 0;
-  size_t smem = (2 * n + 4) * sizeof(float);
+  size_t smem = (2 * n + 12) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "rmsnorm row of %zu floats does not fit shared memory", n);
   note_write(g, dst);
   if (int rc = launch(c, rmsnorm_kernel, dim3((unsigned)m), dim3(512), smem, P)) return rc;
@@ -1169,7 +1169,7 @@ static AttnShape attn_shape(const aotcu_ctx* c, int n_head, int n_kv_head, int h
   int rmax = ATTN_MAX_WARPS / a.hpc;
   if ((size_t)rmax > m) rmax = (int)m;
   if (rmax < 1) rmax = 1;
-  max_len = (max_len + 3) & ~(size_t)3;
+  max_len = (max_len + 7) & ~(size_t)7;
   const size_t budget = attn_smem_budget(c);
   if (want_smem_scores)
     for (int r = rmax; r >= 1; r--)
@@ -1208,14 +1208,14 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
   P.n_head = n_head;
   P.n_kv_head = n_kv_head;
   P.head_dim = head_dim;
-  P.ctx = (int)((n_ctx + 3) & ~(size_t)3);  // row stride of the score scratch, 16-byte aligned rows
+  P.ctx = (int)((n_ctx + 7) & ~(size_t)7);  // row stride of the score scratch: aligned rows, room for the zero fill of a row's sum
   P.window = (int)window;
   P.scale = 1.0f / sqrtf((float)head_dim);
   ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim must be a multiple of 4, at most 256");
   const int gqa = n_head / n_kv_head;
   // Scores in shared memory when the longest row of this call fits, else in `scratch`.
   size_t max_len = pos_ptr ? n_ctx : std::min(n_ctx, pos0 + m);
-  max_len = (max_len + 3) & ~(size_t)3;
+  max_len = (max_len + 7) & ~(size_t)7;
   const AttnShape a = attn_shape(c, n_head, n_kv_head, head_dim, m, max_len, smem_scores != 0);
   P.heads_per_cta = a.hpc;
   P.rows_per_cta = a.rpc;
@@ -1383,7 +1383,7 @@ static int mega_setup(aotcu_gpu* g) {
   // Scratch: a head of norm rows (2 x dim) or attention vectors (q, k, v, squares, scores),
   // then the area that stages cached K and V rows. 72 KB of staging hold every cached row of
   // one head up to 140 positions at head_dim 64; longer contexts go through two chunk buffers.
-  const size_t small_floats = (std::max((size_t)2 * d.dim, (size_t)5 * d.head_dim + ((g->n_ctx + 3) & ~(size_t)3)) + 31) & ~(size_t)31;
+  const size_t small_floats = (std::max((size_t)2 * d.dim, (size_t)5 * d.head_dim + ((g->n_ctx + 7) & ~(size_t)7)) + 31) & ~(size_t)31;
   size_t stage_floats = 18432;
   const size_t table_bytes = (((size_t)d.n_layer + 1) * sizeof(StepLayer) + 15) & ~(size_t)15;
   size_t scratch = 0, fixed = 0;
@@ -1893,7 +1893,7 @@ int aotcu_rmsnorm(aotcu_ctx* c, float* out, const float* x, const float* w, size
   P.n = (int)n;
   P.x_stride = P.out_stride = (int)n;
   P.eps = eps;
-  size_t smem = (2 * n + 4) * sizeof(float);
+  size_t smem = (2 * n + 12) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "row of %zu floats does not fit shared memory", n);
   return launch(c, rmsnorm_kernel, dim3((unsigned)m), dim3(512), smem, P);
 }
@@ -2095,7 +2095,7 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
       g->smem_scores = (int)n_ctx;
     } else {
       g->smem_scores = 0;
-      G_TRY(cudaMalloc(&g->attn_scratch, g->max_batch * d.n_head * ((n_ctx + 3) & ~(size_t)3) * sizeof(float)));
+      G_TRY(cudaMalloc(&g->attn_scratch, g->max_batch * d.n_head * ((n_ctx + 7) & ~(size_t)7) * sizeof(float)));
     }
   }
   g->history_cap = n_ctx;

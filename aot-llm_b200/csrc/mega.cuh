@@ -161,9 +161,8 @@ __device__ __forceinline__ float ll_wait_sys(const LLWord* p, uint32_t tag, vola
 // the SM's instruction cache: everything large that is used from more than one place is
 // kept out of line.
 __device__ __noinline__ float silu_mul_call(float g, float u) { return fmul(fdiv(g, fadd(1.0f, expf_exact(-g))), u); }
-__device__ __noinline__ float group_seq_sum_call(const float* p, int n, SeqSumScratch* sc, int tid, int nthreads, int bar_id,
-                                                 unsigned long long* prof) {
-  return group_seq_sum(p, n, sc, CtaGroup{tid, nthreads, bar_id}, prof);
+__device__ __noinline__ float group_seq_sum_call(const float* p, int n, SeqSumScratch* sc, int tid, int nthreads, int bar_id) {
+  return group_seq_sum(p, n, sc, CtaGroup{tid, nthreads, bar_id});
 }
 __device__ __noinline__ float dequant_elem_call(int kind, const uint8_t* row, size_t e) { return dequant_elem(kind, row, e); }
 
@@ -608,6 +607,10 @@ __device__ __forceinline__ void phase_norm_quant(const LLWord* src, uint32_t tag
       } else {
         ll_wait8(src + e0, tag, v[k], M.abort, M.err);
       }
+      if (!src_in_scr) {
+        *reinterpret_cast<float4*>(row + e0) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+        *reinterpret_cast<float4*>(row + e0 + 4) = make_float4(v[k][4], v[k][5], v[k][6], v[k][7]);
+      }
       if (mirror) {
         *reinterpret_cast<float4*>(mirror + e0) = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
         *reinterpret_cast<float4*>(mirror + e0 + 4) = make_float4(v[k][4], v[k][5], v[k][6], v[k][7]);
@@ -632,7 +635,7 @@ __device__ __forceinline__ void phase_norm_quant(const LLWord* src, uint32_t tag
     g.sync();
     ss = red_sum(M.red, nw);
   } else {
-    ss = group_seq_sum_call(sq, n, M.ss, g.tid, g.nthreads, g.bar_id, walker_prof ? walker_prof : sp.prof);  // opens with a barrier
+    ss = group_seq_sum(sq, n, M.ss, g, walker_prof ? walker_prof : sp.prof);  // opens with a barrier
     sp.last = clock64();
   }
   sp.mark(17);
@@ -640,10 +643,15 @@ __device__ __forceinline__ void phase_norm_quant(const LLWord* src, uint32_t tag
 #pragma unroll
   for (int k = 0; k < 2; k++) {
     const int b = warp + k * nw;
-    if (b < nblk)
+    if (b < nblk) {
+      // the row's values wait in shared memory, not in registers, for the sum
+      const float4 a0 = *reinterpret_cast<const float4*>(row + b * 256 + 8 * lane), a1 = *reinterpret_cast<const float4*>(row + b * 256 + 8 * lane + 4);
+      v[k][0] = a0.x; v[k][1] = a0.y; v[k][2] = a0.z; v[k][3] = a0.w;
+      v[k][4] = a1.x; v[k][5] = a1.y; v[k][6] = a1.z; v[k][7] = a1.w;
       quantize_block_call(fmul(fmul(v[k][0], r), w0[k].x), fmul(fmul(v[k][1], r), w0[k].y), fmul(fmul(v[k][2], r), w0[k].z),
                           fmul(fmul(v[k][3], r), w0[k].w), fmul(fmul(v[k][4], r), w1[k].x), fmul(fmul(v[k][5], r), w1[k].y),
                           fmul(fmul(v[k][6], r), w1[k].z), fmul(fmul(v[k][7], r), w1[k].w), M.sx + b * XK_STRIDE);
+    }
   }
   g.sync();
   sp.mark(19);
@@ -675,36 +683,27 @@ __device__ __forceinline__ void stage_kv_rows(float* buf, int stride, const floa
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Sum of p[0..n) (shared memory, written by any thread of the group) returned to every
-// thread: in the reference's sequential order, or as a tree when `tree` is set. Longer
-// sequential sums go through the chunked algorithm of groupsum.cuh; up to SEQ_CHAIN_MAX
-// terms one thread's plain add chain (4 cycles per term) is quicker than its set-up.
-constexpr int SEQ_CHAIN_MAX = 256;
+// Sum of p[0..n) (shared memory, written by any thread of the group, zero-filled to a multiple of
+// eight) returned to every thread: in the reference's sequential order, or as a tree when `tree`
+// is set.
 __device__ __forceinline__ float cta_sum(const float* p, int n, bool tree, const MegaSmem& M, const CtaGroup& g) {
-  if (!tree && n > SEQ_CHAIN_MAX) return group_seq_sum_call(p, n, M.ss, g.tid, g.nthreads, g.bar_id, nullptr);
+  if (!tree && n > SEQ_CHAIN_MAX) return group_seq_sum_call(p, n, M.ss, g.tid, g.nthreads, g.bar_id);
   g.sync();
-  if (tree) {
-    float a = 0.0f;
-    for (int i = g.tid; i < n; i += g.nthreads) a = fadd(a, p[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a = fadd(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if ((g.tid & 31) == 0) M.red[g.tid >> 5] = a;
-    g.sync();
-    return red_sum(M.red, g.nthreads >> 5);
-  }
-  if (g.tid == 0) {
-    float s = 0.0f;
-    int i = 0;
-    for (; i + 8 <= n; i += 8) {
-      const float4 a = *reinterpret_cast<const float4*>(p + i), b = *reinterpret_cast<const float4*>(p + i + 4);
-      s = fadd(s, a.x); s = fadd(s, a.y); s = fadd(s, a.z); s = fadd(s, a.w);
-      s = fadd(s, b.x); s = fadd(s, b.y); s = fadd(s, b.z); s = fadd(s, b.w);
+  if (!tree) {
+    if (g.tid < 32) {
+      const float s = seq_chain(p, n);
+      if (g.tid == 0) M.red[40] = s;
     }
-    for (; i < n; i++) s = fadd(s, p[i]);
-    M.red[40] = s;
+    g.sync();
+    return M.red[40];
   }
+  float a = 0.0f;
+  for (int i = g.tid; i < n; i += g.nthreads) a = fadd(a, p[i]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a = fadd(a, __shfl_xor_sync(0xffffffffu, a, o));
+  if ((g.tid & 31) == 0) M.red[g.tid >> 5] = a;
   g.sync();
-  return M.red[40];
+  return red_sum(M.red, g.nthreads >> 5);
 }
 
 // Softmax over sc[0..n) in place (ops.rs:98-112): `lmax` is this thread's maximum of the
@@ -719,6 +718,7 @@ __device__ __forceinline__ void softmax_rows(float* sc, int n, float lmax, int f
   float mx = M.red[0];
   for (int w = 1; w < (T >> 5); w++) mx = fmaxf(mx, M.red[w]);
   for (int t = tid; t < n; t += T) sc[t] = expf_exact(fsub(sc[t], mx));
+  if (n + tid < ((n + 7) & ~7)) sc[n + tid] = 0.0f;
   const float sum = cta_sum(sc, n, (fast & FAST_SOFTMAX_SUM) != 0, M, g);  // opens with a barrier
   const float inv = fdiv(1.0f, sum);
   g.sync();

@@ -226,7 +226,7 @@ struct RmsnormParams {
 __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   extern __shared__ __align__(16) float sm_f[];
   float* row = sm_f;          // n
-  float* sq = sm_f + P.n;     // n
+  float* sq = sm_f + ((P.n + 3) & ~3);  // n, 16-byte aligned, zero-filled to a multiple of eight
   __shared__ SeqSumScratch ssc;
   pdl_launch_dependents();
   pdl_wait();
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
     row[i] = v;
     sq[i] = fmul(v, v);
   }
-  __syncthreads();
+  if (P.n + (int)threadIdx.x < ((P.n + 7) & ~7)) sq[P.n + threadIdx.x] = 0.0f;
   float ss = group_seq_sum(sq, P.n, &ssc, CtaGroup{(int)threadIdx.x, (int)blockDim.x, 0});
   float r = fdiv(1.0f, fsqrt(fadd(fdiv(ss, (float)P.n), P.eps)));
   for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
@@ -392,7 +392,7 @@ struct AttnParams {
 constexpr int ATTN_MAX_WARPS = 16;
 // Bytes of the warps' exact-sum scratch at the head of the kernel's shared memory, rounded so
 // that what follows stays 16-byte aligned for any warp count.
-__host__ __device__ inline size_t attn_ssc_bytes(size_t warps) { return (warps * sizeof(SeqSumScratch) + 15) & ~(size_t)15; }
+__host__ __device__ inline size_t attn_ssc_bytes(size_t warps) { return (warps * sizeof(SeqFastScratch) + 15) & ~(size_t)15; }
 constexpr int ATTN_CHUNK = 64;      // cached positions staged at a time ...
 constexpr int ATTN_CHUNK_BIG = 128;  // ... or this many when shared memory allows: half the staging rounds
 
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(ATTN_MAX_WARPS * 32) attention_kernel(const At
   const int T0 = (P.window > 0 && pos_a + 1 > P.window) ? pos_a + 1 - P.window : 0;
   const int LEN = pos_b + 1 - T0;
   const int kstride = hd + 4, CH = P.chunk;
-  SeqSumScratch* ssc = reinterpret_cast<SeqSumScratch*>(sm_f);
+  SeqFastScratch* ssc = reinterpret_cast<SeqFastScratch*>(sm_f);
   float* qs = sm_f + attn_ssc_bytes(nwarps) / sizeof(float);  // nwarps x hd, 16-byte aligned
   float* kv = qs + nwarps * hd;                       // two buffers of CH x (hd + 4)
   const int buf_floats = CH * kstride;
@@ -507,8 +507,9 @@ __global__ void __launch_bounds__(ATTN_MAX_WARPS * 32) attention_kernel(const At
     for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
     __syncwarp();
     for (int t = lane; t < len; t += 32) sc[t] = expf_exact(fsub(sc[t], lmax));
+    if (len + lane < ((len + 7) & ~7)) sc[len + lane] = 0.0f;
     __syncwarp();
-    const float sum = group_seq_sum(sc, len, &ssc[warp], CtaGroup{lane, 32, 1 + warp});
+    const float sum = warp_seq_sum(sc, len, &ssc[warp]);
     const float inv = fdiv(1.0f, sum);
     for (int t = lane; t < len; t += 32) sc[t] = fmul(sc[t], inv);
     __syncwarp();

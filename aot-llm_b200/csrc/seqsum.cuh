@@ -99,7 +99,7 @@ struct SeqItem {
   int count;  // terms
 };
 
-struct SeqSumScratch {
+struct alignas(16) SeqSumScratch {
   SeqItem item[SEQ_CHUNKS];        // group g's items start at item[32 g]
   int n_items[SEQ_CHUNKS / 32];
   float gtot[SEQ_CHUNKS / 32];     // inexact sum of each group
