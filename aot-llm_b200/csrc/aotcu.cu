@@ -19,6 +19,7 @@
 #include "../../include/aot_cuda.h"
 #include "gemv.cuh"
 #include "gemm_tc.cuh"
+#include "attention.cuh"
 #include "kmma.cuh"
 #include "mega.cuh"
 #include "q80stream.cuh"
@@ -905,7 +906,6 @@ struct aotcu_gpu {
   // the tensor's offset; built before the first prompt chunk of 8 tokens or more.
   std::unordered_map<uint64_t, uint8_t*> prep;
   int prep_state = 0;                           // 0 not built yet, 1 built, -1 off (option, memory, or nothing to prepare)
-  int smem_scores = 0;
 };
 
 static size_t xb_width(const aotcu_dims& d) {
@@ -1145,58 +1145,13 @@ static int gpu_qk_post(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos0,
   return launch(g->c, qk_post_kernel, dim3(d.n_head + d.n_kv_head, (unsigned)m), dim3(128), 0, P);
 }
 
-// Shared memory of the attention kernel with the scores of rows up to `max_len` positions
-// kept on chip, and what a CTA may use.
-// Shared memory of the attention kernel with the scores of rows up to `max_len` positions
-// kept on chip, and what a CTA may use. A CTA has heads_per_cta x rows_per_cta warps, each
-// with its exact-sum scratch, its query row and (when they fit) its scores.
-static size_t attn_smem_budget(const aotcu_ctx* c) { return c->max_smem - 1024; }
-struct AttnShape {
-  int hpc, rpc, chunk;
-  bool scores_in_smem;
-  size_t smem;
-};
-static size_t attn_smem_of(int warps, int head_dim, int chunk, size_t score_floats) {
-  return attn_ssc_bytes(warps) + ((size_t)warps * head_dim + (size_t)2 * chunk * (head_dim + 4) + (size_t)warps * score_floats) * sizeof(float);
-}
-// Warps per CTA and staging chunk for rows of up to `max_len` positions: scores stay in shared
-// memory if any shape allows it (fewer rows per CTA rather than scores in global memory),
-// and the larger chunk is taken when it still fits.
-static AttnShape attn_shape(const aotcu_ctx* c, int n_head, int n_kv_head, int head_dim, size_t m, size_t max_len, bool want_smem_scores) {
-  const int gqa = n_head / n_kv_head;
-  AttnShape a;
-  a.hpc = gqa < 8 ? gqa : 8;
-  int rmax = ATTN_MAX_WARPS / a.hpc;
-  if ((size_t)rmax > m) rmax = (int)m;
-  if (rmax < 1) rmax = 1;
-  max_len = (max_len + 7) & ~(size_t)7;
-  const size_t budget = attn_smem_budget(c);
-  if (want_smem_scores)
-    for (int r = rmax; r >= 1; r--)
-      for (int chunk : {ATTN_CHUNK_BIG, ATTN_CHUNK}) {
-        const size_t need = attn_smem_of(a.hpc * r, head_dim, chunk, max_len);
-        if (need <= budget) {
-          a.rpc = r;
-          a.chunk = chunk;
-          a.scores_in_smem = true;
-          a.smem = need;
-          return a;
-        }
-      }
-  a.rpc = rmax;
-  a.chunk = ATTN_CHUNK;
-  a.scores_in_smem = false;
-  a.smem = attn_smem_of(a.hpc * rmax, head_dim, ATTN_CHUNK, 0);
-  return a;
-}
-static size_t attn_smem_bytes(const aotcu_ctx* c, int n_head, int n_kv_head, int head_dim, size_t max_len, size_t m = 1) {
-  const AttnShape a = attn_shape(c, n_head, n_kv_head, head_dim, m, max_len, true);
-  return a.scores_in_smem ? a.smem : (size_t)-1;
-}
+// Positions whose scores fit shared memory: two CTAs per SM if that is enough, else one.
+static size_t attn_smem_bytes(int head_dim, size_t max_len) { return ((size_t)attn_fixed(head_dim) + max_len * ATTN_NQ) * sizeof(float); }
+static size_t attn_ctas(size_t m, int n_head, int n_kv_head) { return ((m * (n_head / n_kv_head) + ATTN_NQ - 1) / ATTN_NQ) * n_kv_head; }
 
 static int launch_attention(aotcu_ctx* c, float* out, const float* q, const float* kc, const float* vc, float* scratch,
                             const int* pos_ptr, size_t pos0, size_t m, int n_head, int n_kv_head, int head_dim,
-                            size_t n_ctx, size_t window, int smem_scores) {
+                            size_t n_ctx, size_t window) {
   AttnParams P = {};
   P.out = out;
   P.q = q;
@@ -1208,30 +1163,34 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
   P.n_head = n_head;
   P.n_kv_head = n_kv_head;
   P.head_dim = head_dim;
-  P.ctx = (int)((n_ctx + 7) & ~(size_t)7);  // row stride of the score scratch: aligned rows, room for the zero fill of a row's sum
+  P.ctx = (int)n_ctx;
   P.window = (int)window;
-  P.scale = 1.0f / sqrtf((float)head_dim);
-  ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim must be a multiple of 4, at most 256");
-  const int gqa = n_head / n_kv_head;
-  // Scores in shared memory when the longest row of this call fits, else in `scratch`.
-  size_t max_len = pos_ptr ? n_ctx : std::min(n_ctx, pos0 + m);
-  max_len = (max_len + 7) & ~(size_t)7;
-  const AttnShape a = attn_shape(c, n_head, n_kv_head, head_dim, m, max_len, smem_scores != 0);
-  P.heads_per_cta = a.hpc;
-  P.rows_per_cta = a.rpc;
-  P.chunk = a.chunk;
   P.m = (int)m;
-  const int splits = (gqa + P.heads_per_cta - 1) / P.heads_per_cta;
-  const size_t warps = (size_t)P.heads_per_cta * P.rows_per_cta;
-  const size_t smem = a.smem;
-  if (a.scores_in_smem) {
-    P.smem_scores = (int)max_len;
-  } else {
-    ARG_CHECK(scratch, "attention needs a score scratch buffer for this context length");
-    P.smem_scores = 0;
+  P.v_chunk = ATTN_STAGE / 2 / head_dim;
+  P.scale = 1.0f / sqrtf((float)head_dim);
+  P.neg_zero = -0.0f;
+  ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim must be a multiple of 4, at most 256");
+  // Scores in shared memory when the longest row of this call fits, else in `scratch`.
+  const size_t max_len = pos_ptr ? n_ctx : std::min(n_ctx, pos0 + m);
+  size_t smem = attn_smem_bytes(head_dim, max_len);
+  const bool in_smem = smem <= c->max_smem;
+  if (!in_smem) {
+    smem = attn_smem_bytes(head_dim, 0);
+    const size_t ctas = attn_ctas(m, n_head, n_kv_head);
+    if (!scratch) {  // the stand-alone entry point: scores in the context's conversion buffer
+      const int rc = ctx_workspace(c, ctas * n_ctx * ATTN_NQ * sizeof(float));
+      if (rc) return rc < 0 ? rc : fail(AOTCU_ERR_UNSUPPORTED, "attention over %zu positions needs a score buffer, which cannot grow during a stream capture", max_len);
+      P.scratch = reinterpret_cast<float*>(c->ximg);
+    }
   }
-  const unsigned row_groups = (unsigned)((m + P.rows_per_cta - 1) / P.rows_per_cta);
-  return launch(c, attention_kernel, dim3((unsigned)(n_kv_head * splits), row_groups), dim3((unsigned)warps * 32), smem, P);
+  static bool attr_set[64] = {};
+  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    attr_set[c->device] = true;
+  }
+  const unsigned groups = (unsigned)((m * (n_head / n_kv_head) + ATTN_NQ - 1) / ATTN_NQ);
+  return launch(c, in_smem ? attention_kernel<true> : attention_kernel<false>, dim3((unsigned)n_kv_head, groups), dim3(ATTN_THREADS), smem, P);
 }
 
 static int gpu_attention(aotcu_gpu* g, float* out, const float* q, size_t li, const int* pos_ptr, size_t pos0, size_t m,
@@ -1241,7 +1200,7 @@ static int gpu_attention(aotcu_gpu* g, float* out, const float* q, size_t li, co
   note_write(g, out);
   return launch_attention(g->c, out, q, g->bufs[AOTCU_BUF_KCACHE] + li * g->n_ctx * kvd,
                           g->bufs[AOTCU_BUF_VCACHE] + li * g->n_ctx * kvd, g->attn_scratch, pos_ptr, pos0, m, d.n_head,
-                          d.n_kv_head, d.head_dim, g->n_ctx, window, g->smem_scores);
+                          d.n_kv_head, d.head_dim, g->n_ctx, window);
 }
 
 // ---- the generated forward pass, interpreted (emit.rs) -----------------------------------------------
@@ -1641,10 +1600,9 @@ int aotcu_init(int device, aotcu_ctx** out) {
   CU_TRY(cudaMemset(c->d_err, 0, sizeof(int)));
   CU_TRY(cudaFuncSetAttribute(gemv_q8k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
   CU_TRY(cudaFuncSetAttribute(gemv_q80_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
-  // These two also hold the exact-sum scratch in static shared memory.
+  // This one also holds the exact-sum scratch in static shared memory.
   CU_TRY(cudaFuncSetAttribute(rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(c->max_smem - sizeof(SeqSumScratch) - 1024)));
-  CU_TRY(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem_budget(c)));
   *out = c;
   return 0;
 }
@@ -1953,10 +1911,8 @@ int aotcu_attention(aotcu_ctx* c, float* out, const float* q, const float* k_cac
   ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim %zu must be a multiple of 4, at most 256", head_dim);
   ARG_CHECK(pos0 + m <= ctx_len, "positions exceed the context");
   if (m == 0) return 0;
-  ARG_CHECK(attn_smem_bytes(c, (int)n_head, (int)n_kv_head, (int)head_dim, pos0 + m, m) <= attn_smem_budget(c),
-            "%zu positions are too many for the stand-alone attention entry point (scores are kept in shared memory)", pos0 + m);
   return launch_attention(c, out, q, k_cache, v_cache, nullptr, nullptr, pos0, m, (int)n_head, (int)n_kv_head,
-                          (int)head_dim, ctx_len, window, (int)ctx_len);
+                          (int)head_dim, ctx_len, window);
 }
 
 int aotcu_argmax(aotcu_ctx* c, const float* x, size_t n, int32_t* out_token) {
@@ -2091,12 +2047,8 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   }
   // Attention scores: shared memory when the context fits, else a global scratch.
   {
-    if (attn_smem_bytes(c, d.n_head, d.n_kv_head, d.head_dim, n_ctx, g->max_batch) <= attn_smem_budget(c)) {
-      g->smem_scores = (int)n_ctx;
-    } else {
-      g->smem_scores = 0;
-      G_TRY(cudaMalloc(&g->attn_scratch, g->max_batch * d.n_head * ((n_ctx + 7) & ~(size_t)7) * sizeof(float)));
-    }
+    if (attn_smem_bytes(d.head_dim, n_ctx) > c->max_smem)
+      G_TRY(cudaMalloc(&g->attn_scratch, attn_ctas(g->max_batch, d.n_head, d.n_kv_head) * n_ctx * ATTN_NQ * sizeof(float)));
   }
   g->history_cap = n_ctx;
   G_TRY(cudaMalloc(&g->d_step, 4 * sizeof(int)));

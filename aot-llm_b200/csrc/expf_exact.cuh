@@ -81,7 +81,10 @@ AOT_HD double u2d(uint64_t u) {
 #endif
 }
 
-AOT_HD float expf_exact(float x) {
+// `tab`: where the table is read. On the device lanes read different entries, which a constant
+// bank serves one address after the other (about 25 of them per warp): kernels that evaluate many
+// exponentials keep a copy in shared memory (exp_table_load) and pass that.
+AOT_HD float expf_exact(float x, const uint64_t* tab) {
   const double kInvLn2N = 0x1.71547652b82fep+0 * 32.0;
   const double kShift = 0x1.8p+52;
   const double kC0 = 0x1.c6af84b912394p-5 / 32.0 / 32.0 / 32.0;
@@ -101,11 +104,7 @@ AOT_HD float expf_exact(float x) {
   uint64_t ki = d2u(kd);
   kd = dadd(kd, -kShift);
   double r = dfma(kInvLn2N, xd, -kd);
-#if AOT_DEVICE_CODE
-  uint64_t t = c_exp2_tab[ki & 31u];
-#else
-  uint64_t t = h_exp2_tab[ki & 31u];
-#endif
+  uint64_t t = tab[ki & 31u];
   t += ki << 47;
   double s = u2d(t);
   double p = dfma(kC0, r, kC1);
@@ -115,5 +114,20 @@ AOT_HD float expf_exact(float x) {
   y = dmul(y, s);
   return (float)y;
 }
+AOT_HD float expf_exact(float x) {
+#if AOT_DEVICE_CODE
+  return expf_exact(x, c_exp2_tab);
+#else
+  return expf_exact(x, h_exp2_tab);
+#endif
+}
+
+#if defined(__CUDACC__)
+// The first 32 threads of a CTA copy the table into shared memory; a barrier before its use is the
+// caller's.
+__device__ __forceinline__ void exp_table_load(uint64_t* tab) {
+  if (threadIdx.x < 32) tab[threadIdx.x] = c_exp2_tab[threadIdx.x];
+}
+#endif
 
 }  // namespace aot

@@ -161,7 +161,7 @@ __device__ __noinline__ float group_seq_sum_items(const float* p, int n, SeqSumS
 // squares: 4.3 K cycles on its own (9.3 K with an item per run, crossing chunk and tie walked one
 // by one through shared memory; 11.2 K for a plain chain), 4.0 K inside the decode step (7.8 K).
 // A wrong prediction, a sum that goes down in the inexact prefix or more than SEQ_BINADES
-// binades are noticed and send the whole sum to group_seq_sum_items (warp_seq_sum: to a chain).
+// binades are noticed and send the whole sum to group_seq_sum_items.
 constexpr int SEQ_BINADES = 8;
 constexpr int SEQ_GROUPS = 16;  // groups per round: 4096 terms
 
@@ -320,42 +320,8 @@ __device__ __forceinline__ float seq_chain(const float* p, int n) {
   return s;
 }
 
-// One warp on its own (p 16-byte aligned and zero-filled to a multiple of SEQ_E terms); the result in every lane.
-__device__ __forceinline__ float warp_seq_sum(const float* p, int n, SeqFastScratch* sc) {
-  const int lane = threadIdx.x & 31;
-  if (n <= SEQ_CHAIN_MAX) return seq_chain(p, n);
-  float s = seq_chain(p, SEQ_HEAD), approx = 0.0f;
-#pragma unroll 1
-  for (int base = 0; base < n; base += SEQ_GROUPS * 32 * SEQ_E) {
-    const int len = min(n - base, SEQ_GROUPS * 32 * SEQ_E), ngr = (len + 32 * SEQ_E - 1) / (32 * SEQ_E);
-    __syncwarp();
-    seq_fast_clear(sc, lane, 32);
-    __syncwarp();
-    int e0 = seq_exp_field(base == 0 ? s : approx);
-#pragma unroll 1
-    for (int gr = 0; gr < ngr; gr++) {
-      float v[SEQ_E];
-      seq_chunk(p + base, len, gr * 32 + lane, v);
-      const float t = seq_chunk_sum(v), incl = seq_warp_scan(t), after = approx + __shfl_sync(0xffffffffu, incl, 31);
-      const int head = base == 0 && gr == 0 ? SEQ_HEAD / SEQ_E : 0;
-      const float before = approx + (incl - t);
-      if (gr == 0) e0 = seq_exp_field(__shfl_sync(0xffffffffu, before, head));
-      seq_group_fn(v, before, after, gr, len, head, e0, sc);
-      approx = after;
-    }
-    if (lane == 0) sc->e0 = e0;
-    __syncwarp();
-    float x = s;
-    if (sc->over || !seq_walk_binades(p + base, len, sc, x)) {  // the plain chain, from the start of the round
-      x = s;
-      for (int i = base == 0 ? SEQ_HEAD : 0; i < len; i++) x = fadd(x, p[base + i]);
-    }
-    s = x;
-  }
-  return s;
-}
-
-// A group of several warps (p as above). Opens with a barrier; the result in every thread.
+// Every thread of the group calls it (p 16-byte aligned and zero-filled to a multiple of SEQ_E
+// terms). Opens with a barrier; the result in every thread.
 __device__ __forceinline__ float group_seq_sum(const float* p, int n, SeqSumScratch* scratch, const CtaGroup& g, unsigned long long* prof = nullptr) {
   SubProf sp{prof, clock64()};
   SeqFastScratch* const sc = reinterpret_cast<SeqFastScratch*>(scratch);

@@ -89,19 +89,6 @@ __device__ __forceinline__ void mma_s8s8_k16(int (&c)[4], uint32_t a0, uint32_t 
                : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
-// Two f32 values in one register pair: one instruction for two round-to-nearest operations.
-typedef unsigned long long F2;
-__device__ __forceinline__ F2 f2_pack(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // Byte i of w, sign-extended: a permute whose upper selectors replicate the byte's sign.
 __device__ __forceinline__ int sext_byte(uint32_t w, int i) {
   int r;

@@ -365,194 +365,6 @@ __global__ void __launch_bounds__(128) rmsnorm_heads_kernel(float* x, const floa
   for (int i = threadIdx.x; i < head_dim; i += blockDim.x) v[i] = fmul(fmul(h[i], r), w[i]);
 }
 
-// ---- attention (ops.rs:185-218, 517-556) ------------------------------------------------------
-// One CTA per (group of up to 8 query heads that share a KV head, query row); one warp
-// per query head. Cached K and V rows are staged through shared memory once per CTA and
-// used by all its heads. Scores and the softmax live in shared memory (or in `scratch`
-// for contexts that do not fit). Order-sensitive reductions keep the reference's order:
-// each q.k dot is one sequential chain, the softmax denominator is the exact sequential
-// sum, the value mix runs over positions in order.
-struct AttnParams {
-  float* out;         // m x q_dim
-  const float* q;     // m x q_dim
-  const float* k_cache;  // layer base: ctx x kv_dim
-  const float* v_cache;
-  float* scratch;     // (m x n_head) x ctx floats, used when smem_scores == 0
-  const int* pos_ptr;
-  int pos0;
-  int n_head, n_kv_head, head_dim, ctx, window;
-  int smem_scores;    // capacity (floats per head) of the shared score buffer, 0 = use scratch
-  int heads_per_cta;  // query heads of one KV head handled by a CTA (<= 8)
-  int rows_per_cta;   // consecutive query rows handled by a CTA (heads_per_cta x rows_per_cta warps, <= 16)
-  int m;              // query rows
-  int chunk;          // cached positions per staging buffer
-  float scale;
-};
-
-constexpr int ATTN_MAX_WARPS = 16;
-// Bytes of the warps' exact-sum scratch at the head of the kernel's shared memory, rounded so
-// that what follows stays 16-byte aligned for any warp count.
-__host__ __device__ inline size_t attn_ssc_bytes(size_t warps) { return (warps * sizeof(SeqFastScratch) + 15) & ~(size_t)15; }
-constexpr int ATTN_CHUNK = 64;      // cached positions staged at a time ...
-constexpr int ATTN_CHUNK_BIG = 128;  // ... or this many when shared memory allows: half the staging rounds
-
-// o[j] += a[t] * v[t][lane + 32 j] for t in [ta, tb), positions in order (ops.rs:208-214), for
-// the NJ dims a lane owns; only the last of them can lie beyond the head width.
-template <int NJ>
-__device__ __forceinline__ void attn_value_mix(float (&o)[8], const float* a, const float* cur, int ta, int tb, int hd, int lane) {
-  const bool last = lane + 32 * (NJ - 1) < hd;
-#pragma unroll 4
-  for (int t = ta; t < tb; t++) {
-    const float at = a[t];
-    const float* v = cur + t * hd + lane;
-#pragma unroll
-    for (int j = 0; j < NJ - 1; j++) o[j] = fadd(o[j], fmul(at, v[32 * j]));
-    if (last) o[NJ - 1] = fadd(o[NJ - 1], fmul(at, v[32 * (NJ - 1)]));
-  }
-}
-
-// One CTA serves `rows_per_cta` consecutive query rows of one KV head: a warp per (row, query
-// head). The cached rows the CTA stages cover the union of its rows' ranges (rows differ by
-// one position each, and by their window start), so they are fetched once for all of them.
-__global__ void __launch_bounds__(ATTN_MAX_WARPS * 32) attention_kernel(const AttnParams P) {
-  extern __shared__ __align__(16) float sm_f[];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int hd = P.head_dim, hd4 = hd >> 2, kv_dim = P.n_kv_head * hd, q_dim = P.n_head * hd;
-  const int gqa = P.n_head / P.n_kv_head, hpc = P.heads_per_cta, rpc = P.rows_per_cta;
-  const int nthreads = blockDim.x, nwarps = nthreads >> 5;
-  const int splits = (gqa + hpc - 1) / hpc;
-  const int kvh = blockIdx.x / splits, part = blockIdx.x - kvh * splits;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rs = warp / hpc, wh = warp - rs * hpc;            // row slot and head slot of this warp
-  const int row = blockIdx.y * rpc + rs;
-  const int h_local = part * hpc + wh;                        // head inside the KV group
-  const bool has_head = rs < rpc && row < P.m && h_local < gqa;
-  const int h = kvh * gqa + (h_local < gqa ? h_local : 0);
-  const int base_pos = P.pos_ptr ? *P.pos_ptr : P.pos0;
-  const int pos = base_pos + row;
-  const int n = pos + 1;
-  const int t0 = (P.window > 0 && pos + 1 > P.window) ? pos + 1 - P.window : 0;
-  const int len = n - t0;
-  // the CTA's rows: first and last valid one, and the union [T0, N) of their ranges
-  const int row_a = blockIdx.y * rpc, row_b = min(row_a + rpc, P.m) - 1;
-  const int pos_a = base_pos + row_a, pos_b = base_pos + row_b;
-  const int T0 = (P.window > 0 && pos_a + 1 > P.window) ? pos_a + 1 - P.window : 0;
-  const int LEN = pos_b + 1 - T0;
-  const int kstride = hd + 4, CH = P.chunk;
-  SeqFastScratch* ssc = reinterpret_cast<SeqFastScratch*>(sm_f);
-  float* qs = sm_f + attn_ssc_bytes(nwarps) / sizeof(float);  // nwarps x hd, 16-byte aligned
-  float* kv = qs + nwarps * hd;                       // two buffers of CH x (hd + 4)
-  const int buf_floats = CH * kstride;
-  float* sc_all = kv + 2 * buf_floats;                // nwarps x smem_scores
-  float* sc = P.smem_scores ? sc_all + warp * P.smem_scores : P.scratch + ((size_t)(has_head ? row : 0) * P.n_head + h) * P.ctx;
-  for (int i = threadIdx.x; i < nwarps * hd; i += nthreads) {
-    const int w = i / hd, wr = w / hpc, hl = part * hpc + (w - wr * hpc), r = row_a + wr;
-    qs[i] = (wr < rpc && r < P.m && hl < gqa) ? P.q[(size_t)r * q_dim + (kvh * gqa + hl) * hd + (i - w * hd)] : 0.0f;
-  }
-  // Cached rows [c0, c0 + cn) of the union, of this KV head, into a chunk buffer with cp.async:
-  // the next chunk loads while the current one is consumed.
-  auto stage = [&](float* buf, const float* cache, int stride, int c0, int cn) {
-    for (int j = threadIdx.x; j < cn * hd4; j += nthreads) {
-      const int t = j / hd4, i4 = j - t * hd4;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(buf + t * stride + 4 * i4)),
-                   "l"(cache + (size_t)(T0 + c0 + t) * kv_dim + kvh * hd + 4 * i4)
-                   : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // scores: dot(q, k_t) * scale, each dot a sequential f32 loop (ops.rs:160-166)
-  float lmax = -INFINITY;
-  const float* qh = qs + warp * hd;
-  const int off = t0 - T0;                            // this row's first position inside the union
-  stage(kv, P.k_cache, kstride, 0, min(CH, LEN));
-  for (int c0 = 0, ci = 0; c0 < LEN; c0 += CH, ci++) {
-    const int cn = min(CH, LEN - c0);
-    const float* cur = kv + (ci & 1) * buf_floats;
-    if (c0 + CH < LEN) {
-      stage(kv + ((ci + 1) & 1) * buf_floats, P.k_cache, kstride, c0 + CH, min(CH, LEN - c0 - CH));
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    if (has_head) {
-      for (int t = lane; t < cn; t += 32) {
-        const int u = c0 + t - off;                   // position index inside this row's range
-        if (u < 0 || u >= len) continue;
-        const float4* kt = reinterpret_cast<const float4*>(cur + t * kstride);
-        float s = 0.0f;
-#pragma unroll 4
-        for (int i = 0; i < hd4; i++) {
-          const float4 kk = kt[i];
-          const float4 qq = reinterpret_cast<const float4*>(qh)[i];
-          s = fadd(s, fmul(qq.x, kk.x));
-          s = fadd(s, fmul(qq.y, kk.y));
-          s = fadd(s, fmul(qq.z, kk.z));
-          s = fadd(s, fmul(qq.w, kk.w));
-        }
-        s = fmul(s, P.scale);
-        sc[u] = s;
-        lmax = fmaxf(lmax, s);
-      }
-    }
-    __syncthreads();  // this buffer is refilled two chunks later
-  }
-  // the first chunk of V rows loads while the softmax runs
-  stage(kv, P.v_cache, hd, 0, min(CH, LEN));
-  if (has_head) {
-    // this head's softmax, by its own warp: max (order-free), exp, the denominator in
-    // position order (ops.rs:103-107)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
-    __syncwarp();
-    for (int t = lane; t < len; t += 32) sc[t] = expf_exact(fsub(sc[t], lmax));
-    if (len + lane < ((len + 7) & ~7)) sc[len + lane] = 0.0f;
-    __syncwarp();
-    const float sum = warp_seq_sum(sc, len, &ssc[warp]);
-    const float inv = fdiv(1.0f, sum);
-    for (int t = lane; t < len; t += 32) sc[t] = fmul(sc[t], inv);
-    __syncwarp();
-  }
-  // out[i] = sum_t a_t * v_t[i], t in order (ops.rs:208-214); lane owns dims lane, lane+32, ...
-  float o[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) o[j] = 0.0f;
-  for (int c0 = 0, ci = 0; c0 < LEN; c0 += CH, ci++) {
-    const int cn = min(CH, LEN - c0);
-    const float* cur = kv + (ci & 1) * buf_floats;
-    if (c0 + CH < LEN) {
-      stage(kv + ((ci + 1) & 1) * buf_floats, P.v_cache, hd, c0 + CH, min(CH, LEN - c0 - CH));
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    if (has_head) {
-      // this row's positions inside the chunk; the loop over a lane's dims is instantiated for
-      // the head width (predicated-off iterations of a fixed eight would still issue)
-      const int ta = max(0, off - c0), tb = min(cn, off + len - c0);
-      const float* a = sc + (c0 - off);
-      switch ((hd + 31) >> 5) {
-        case 1: attn_value_mix<1>(o, a, cur, ta, tb, hd, lane); break;
-        case 2: attn_value_mix<2>(o, a, cur, ta, tb, hd, lane); break;
-        case 3: attn_value_mix<3>(o, a, cur, ta, tb, hd, lane); break;
-        case 4: attn_value_mix<4>(o, a, cur, ta, tb, hd, lane); break;
-        case 5: attn_value_mix<5>(o, a, cur, ta, tb, hd, lane); break;
-        case 6: attn_value_mix<6>(o, a, cur, ta, tb, hd, lane); break;
-        case 7: attn_value_mix<7>(o, a, cur, ta, tb, hd, lane); break;
-        default: attn_value_mix<8>(o, a, cur, ta, tb, hd, lane); break;  // head_dim <= 256
-      }
-    }
-    __syncthreads();
-  }
-  if (has_head) {
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (lane + 32 * j < hd) P.out[(size_t)row * q_dim + h * hd + lane + 32 * j] = o[j];
-  }
-}
-
 // ---- element-wise ----------------------------------------------------------------------------------
 __global__ void silu_mul_kernel(float* h, const float* up, size_t n) {
   pdl_launch_dependents();

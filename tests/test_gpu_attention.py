@@ -1,0 +1,30 @@
+"""Attention at the sizes where its kernel changes path: query groups that span rows and are not
+full, head widths that are not whole pieces, windows, more positions than the scores' shared
+memory holds. Bit-exact against the CPU oracle (crates/aot-kernels/src/ops.rs:517-556)."""
+import numpy as np
+import pytest
+
+from conftest import assert_bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_head,n_kv,hd,ctxlen,calls", [
+    (6, 2, 20, 700, [(1, 699, 0), (11, 600, 0), (64, 300, 77)]),     # three heads per group, a partial piece
+    (1, 1, 256, 300, [(1, 0, 0), (9, 290, 33)]),                      # one query per row, widest heads
+    (24, 2, 64, 260, [(3, 0, 0), (5, 255, 0)]),                       # twelve heads per group: two CTAs a row
+    (4, 1, 32, 6200, [(1, 6100, 0), (3, 6190, 0), (2, 6000, 5900)]),  # scores in global memory
+])
+def test_attention_paths(pkg, ob, ctx, n_head, n_kv, hd, ctxlen, calls):
+    rng = np.random.default_rng(hd)
+    kc, vc = (rng.standard_normal(ctxlen * n_kv * hd).astype(np.float32) for _ in range(2))
+    d = ob.Dims()
+    d.n_head, d.n_kv_head, d.head_dim = n_head, n_kv, hd
+    dk, dv = ctx.to_device(kc), ctx.to_device(vc)
+    for m, pos0, window in calls:
+        q = rng.standard_normal(m * n_head * hd).astype(np.float32)
+        dout = ctx.alloc(q.nbytes)
+        ctx.attention(dout, ctx.to_device(q), dk, dv, n_head, n_kv, hd, ctxlen, pos0, m, window)
+        assert_bits_equal(dout.download(np.float32, q.size), ob.attention_rows(ob.Pool(4), q, kc, vc, d, ctxlen, 0, pos0, m, window),
+                          f"m {m} pos0 {pos0} window {window}")
+    ctx.device_status()
