@@ -23,6 +23,7 @@
 #include "kmma.cuh"
 #include "mega.cuh"
 #include "q80stream.cuh"
+#include "floatmulti.cuh"
 #include "floatstream.cuh"
 #include "ops.cuh"
 
@@ -526,34 +527,106 @@ static int launch_q80_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   return 0;
 }
 
-// F16 / BF16 / F32 products on the chunk-streaming kernel (floatstream.cuh): matrices of one
+// F16 / BF16 / F32 products of several activation rows on the packed kernel of floatmulti.cuh.
+// Returns 1 when the call does not fit.
+template <int KIND, int R, int T>
+static int launch_float_multi_t(aotcu_ctx* c, const FloatMultiParams& P, int grid) {
+  static bool attr_set[64] = {};
+  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(float_multi_kernel<KIND, R, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    attr_set[c->device] = true;
+  }
+  return launch(c, float_multi_kernel<KIND, R, T>, dim3(grid), dim3(32 * P.wt), (size_t)FM_STAGES * FmShape<KIND, R, T>::stage_bytes(P.wt), P);
+}
+template <int KIND, int R>
+static int launch_float_multi_r(aotcu_ctx* c, const FloatMultiParams& P, int t, int grid) {
+  if (t == 2) return launch_float_multi_t<KIND, R, 2>(c, P, grid);
+  if (t == 4) return launch_float_multi_t<KIND, R, 4>(c, P, grid);
+  if (t == 5) return launch_float_multi_t<KIND, R, 5>(c, P, grid);
+  return launch_float_multi_t<KIND, R, 8>(c, P, grid);
+}
+template <int KIND>
+static int launch_float_multi_k(aotcu_ctx* c, const FloatMultiParams& P, int r, int t, int grid) {
+  return r == 2 ? launch_float_multi_r<KIND, 2>(c, P, t, grid) : launch_float_multi_r<KIND, 4>(c, P, t, grid);
+}
+static int g_float_chunks = 1;  // 0: keep float-kind products on gemv_float_kernel (option "float_chunks")
+static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
+  const int kind = call.seg[0].kind;
+  if (call.cols % 8 || ((uintptr_t)call.x & 15)) return 1;
+  for (int s = 0; s < call.nseg; s++)
+    if (call.seg[s].kind != kind || ((uintptr_t)call.seg[s].w & 15)) return 1;
+  FloatMultiParams P = {};
+  P.nseg = call.nseg;
+  P.cols = (int)call.cols;
+  P.m = (int)call.m;
+  P.epilogue = call.pair ? EPI_STORE : call.epilogue;
+  P.x = reinterpret_cast<const float*>(call.x);
+  // Shape: R weight rows and T activation rows per lane, wt warps per CTA. Fitted to 116 timings
+  // over eight matrices and batches of 2 to 64: a step of eight columns takes a scheduler about
+  // 20 + 4 R T cycles per warp that it holds, and 50 + 8 R T if it holds few; the fullest
+  // scheduler's share (a CTA's warps go to schedulers in turn) counts for a quarter.
+  int r_best = 2, t_best = 2;
+  size_t grid = 0;
+  double best = 1e30;
+  for (int r : {2, 4}) {
+    size_t tiles = 0;
+    for (int s = 0; s < call.nseg; s++) tiles += (call.seg[s].rows + 8 * r - 1) / (8 * r);
+    for (int t : {2, 4, 5, 8}) {
+      const size_t nw = (call.m + t - 1) / t;
+      for (int k = FM_MAX_WARPS; k >= 1; k--) {
+        const size_t nc = (nw + k - 1) / k, wt = (nw + nc - 1) / nc, per_sm = (tiles * nc + c->n_sm - 1) / c->n_sm;
+        const double warps = 0.75 * (double)(tiles * nc * wt) / (4 * c->n_sm) + 0.25 * (double)(per_sm * ((wt + 3) / 4));
+        const double cost = std::max(warps * (20 + 4 * r * t), 50.0 + 8 * r * t);
+        if (cost < best * 0.999 && tiles * nc < (1u << 30)) {
+          best = cost;
+          r_best = r;
+          t_best = t;
+          P.n_tcta = (int)nc;
+          P.wt = (int)wt;
+          grid = tiles * nc;
+        }
+      }
+    }
+  }
+  if (!grid) return 1;
+  int tiles = 0;
+  for (int s = 0; s < call.nseg; s++) {
+    P.seg[s] = call.seg[s];
+    P.tiles_before[s] = tiles;
+    tiles += (call.seg[s].rows + 8 * r_best - 1) / (8 * r_best);
+  }
+  int rc;
+  if (kind == F16) rc = launch_float_multi_k<F16>(c, P, r_best, t_best, (int)grid);
+  else if (kind == BF16) rc = launch_float_multi_k<BF16>(c, P, r_best, t_best, (int)grid);
+  else rc = launch_float_multi_k<F32>(c, P, r_best, t_best, (int)grid);
+  if (rc || !call.pair || call.epilogue != EPI_SILU_MUL) return rc;
+  const size_t n = call.m * (size_t)call.seg[0].rows;
+  return launch(c, silu_mul_kernel, dim3(grid_for(c, n, 256)), dim3(256), 0, call.seg[0].out, (const float*)call.seg[1].out, n);
+}
+
+// F16 / BF16 / F32 products of one activation row on the chunk-streaming kernel (floatstream.cuh): matrices of one
 // kind, columns in eights, rows in fours, 16-byte aligned rows and activations. Returns 1
 // when the call does not fit.
-template <int KIND, int NR, int NT>
+template <int KIND, int NR>
 static int launch_float_stream_t(aotcu_ctx* c, const FloatStreamParams& P, int grid, size_t smem) {
   static bool attr_set[64] = {};
   if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
-    CU_TRY(cudaFuncSetAttribute(float_stream_kernel<KIND, NR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(float_stream_kernel<KIND, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
     attr_set[c->device] = true;
   }
-  return launch(c, float_stream_kernel<KIND, NR, NT>, dim3(grid), dim3(MEGA_THREADS), smem, P);
+  return launch(c, float_stream_kernel<KIND, NR>, dim3(grid), dim3(MEGA_THREADS), smem, P);
 }
 template <int KIND>
-static int launch_float_stream_k(aotcu_ctx* c, const FloatStreamParams& P, int nr, int nt, int grid, size_t smem) {
-  if (nr == 4) return launch_float_stream_t<KIND, 4, 8>(c, P, grid, smem);
-  if (nt == 16) return launch_float_stream_t<KIND, 2, 16>(c, P, grid, smem);
-  if (nt == 8) return nr == 2 ? launch_float_stream_t<KIND, 2, 8>(c, P, grid, smem) : launch_float_stream_t<KIND, 1, 8>(c, P, grid, smem);
-  return nr == 2 ? launch_float_stream_t<KIND, 2, 1>(c, P, grid, smem) : launch_float_stream_t<KIND, 1, 1>(c, P, grid, smem);
+static int launch_float_stream_k(aotcu_ctx* c, const FloatStreamParams& P, int nr, int grid, size_t smem) {
+  return nr == 2 ? launch_float_stream_t<KIND, 2>(c, P, grid, smem) : launch_float_stream_t<KIND, 1>(c, P, grid, smem);
 }
-static int g_float_chunks = 1;  // 0: keep float-kind products on gemv_float_kernel (option "float_chunks")
-static int g_float_rows4 = 1;   // several activation rows, many weight rows per CTA: four weight rows per lane (option "float_rows4")
 static int launch_float_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   const int kind = call.seg[0].kind;
   const size_t row_bytes = kind_row_bytes(kind, call.cols);
   if (call.cols % 8 || row_bytes % 16 || span % 4 || ((uintptr_t)call.x & 15)) return 1;
   for (int s = 0; s < call.nseg; s++)
     if (call.seg[s].kind != kind || call.seg[s].rows % 4 || ((uintptr_t)call.seg[s].w & 15)) return 1;
-  const int cb = fs_chunk_bytes(call.m);
+  const int cb = FS_CB;
   FloatStreamParams P = {};
   for (int s = 0; s < call.nseg; s++) {
     P.seg[s] = call.seg[s];
@@ -568,40 +641,21 @@ static int launch_float_stream(aotcu_ctx* c, const GemvCall& call, size_t span) 
   const int grid = quads < (size_t)c->n_sm ? (int)quads : c->n_sm;
   P.quad_base = (int)(quads / grid);
   P.quad_rem = (int)(quads % grid);
-  ChunkShape shape = chunk_shape(P.quad_base + (P.quad_rem ? 1 : 0), call.pair != 0, call.m, 0);
-  if (shape.nt == 16 && !call.pair && g_float_rows4) {
-    // 16 rows as two token groups of 8 with four weight rows per lane: 12 shared-memory loads
-    // per 32 fused multiply-adds instead of 18 (the load/store pipe is what bounds this kernel)
-    shape = ChunkShape{4, 8, MEGA_CONSUMER_WARPS / 2, 2};
-  }
-  if (shape.nt == 16 && call.m <= 8) shape = ChunkShape{2, 8, MEGA_CONSUMER_WARPS, 1};  // a short batch: one token group
-  if (shape.nr == 4 && call.m <= 8) shape = ChunkShape{2, 8, MEGA_CONSUMER_WARPS, 1};
+  const ChunkShape shape = chunk_shape(P.quad_base + (P.quad_rem ? 1 : 0), call.pair != 0, 1, 0);
   P.qw = shape.qw;
-  P.ts = shape.ts;
-  const int chunk_cols = cb / (kind == F32 ? 4 : 2), xrows = call.m == 1 ? 1 : FS_MAX_TOK;
+  const int chunk_cols = cb / (kind == F32 ? 4 : 2);
   const int x_copies = chunk_cols > 256 ? 2 : 1, xbox = chunk_cols / x_copies;  // a box row holds at most 256 elements
-  const size_t stage = (size_t)shape.qw * shape.nr * 4 * cb + x_copies * (((size_t)xrows * xbox * 4 + 127) & ~(size_t)127);
+  const size_t stage = (size_t)shape.qw * shape.nr * 4 * cb + x_copies * (((size_t)xbox * 4 + 127) & ~(size_t)127);
   const size_t tail = 128 + 16 + 128;
   int n_stages = (int)((c->max_smem - tail) / stage);
   n_stages = n_stages > 8 ? 8 : n_stages;
   if (n_stages < 2) return 1;
   P.n_stages = n_stages;
   const size_t smem = (size_t)n_stages * stage + tail;
-  const size_t group = (size_t)shape.ts * shape.nt;
-  const float* x = reinterpret_cast<const float*>(call.x);
-  for (size_t t0 = 0; t0 < call.m; t0 += group) {
-    const size_t mg = std::min(group, call.m - t0);
-    P.m = (int)mg;
-    if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x + t0 * call.cols, call.cols, mg, call.cols * 4, xbox, xrows))
-      return t0 == 0 ? 1 : fail(AOTCU_ERR_CUDA, "tensor map of the activation rows refused");
-    for (int s = 0; s < call.nseg; s++) P.seg[s].out = call.seg[s].out + t0 * (size_t)call.seg[s].rows;
-    int rc;
-    if (kind == F16) rc = launch_float_stream_k<F16>(c, P, shape.nr, shape.nt, grid, smem);
-    else if (kind == BF16) rc = launch_float_stream_k<BF16>(c, P, shape.nr, shape.nt, grid, smem);
-    else rc = launch_float_stream_k<F32>(c, P, shape.nr, shape.nt, grid, smem);
-    if (rc) return rc;
-  }
-  return 0;
+  if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, call.x, call.cols, 1, call.cols * 4, xbox, 1)) return 1;
+  if (kind == F16) return launch_float_stream_k<F16>(c, P, shape.nr, grid, smem);
+  if (kind == BF16) return launch_float_stream_k<BF16>(c, P, shape.nr, grid, smem);
+  return launch_float_stream_k<F32>(c, P, shape.nr, grid, smem);
 }
 
 // K-quant products of the smallest batches (see launch_gemv): gemv_stream_kernel<3>, one lane per super-block, grid = (row
@@ -703,8 +757,9 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
   if (act == ACT_F32) {
     ARG_CHECK(((uintptr_t)call.x % 4) == 0, "activations must be 4-byte aligned");
     if (g_float_chunks) {
-      const int rc = launch_float_stream(c, call, span);
-      if (rc <= 0) return rc;  // 1: a shape the tensor copies do not take, the plain kernel does
+      // 1: a shape that the 16-byte (tensor) copies do not take, the plain kernel does
+      const int rc = call.m >= 2 ? launch_float_multi(c, call) : launch_float_stream(c, call, span);
+      if (rc <= 0) return rc;
     }
     int rows_per_block = 32;
     int grid = (int)((span + rows_per_block - 1) / rows_per_block);
@@ -2578,10 +2633,6 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
   }
   if (!strcmp(name, "wide_multi")) {  // process-wide: K-quant prompt chunks of few tiles (and Q6_K) on gemv_stream_kernel<3> (1, default)
     g_wide_multi = value != 0;
-    return 0;
-  }
-  if (!strcmp(name, "float_rows4")) {  // process-wide: four weight rows per lane in the float chunk kernel at 9..16 activation rows (1, default)
-    g_float_rows4 = value != 0;
     return 0;
   }
   if (!strcmp(name, "float_chunks")) {  // process-wide: F16 / BF16 / F32 products on the chunk-streaming kernel (1, default)

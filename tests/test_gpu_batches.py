@@ -42,3 +42,12 @@ def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, kind):
     xs = np.ones(m * cols, dtype=np.float32)
     xs[cols:2 * cols] = -1.0                          # every quant -127, or 127
     _run(pkg, ob, ctx, kind, w.reshape(-1), xs, m, rows, cols, f"kind {kind} at the bounds")
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])           # F32, F16, BF16
+@pytest.mark.parametrize("rows,cols", [(1, 8), (33, 72), (600, 1016), (5000, 128)])
+def test_float_tile_edges(pkg, ob, ctx, kind, rows, cols):
+    w = make_weights(pkg, kind, rows, cols, 31 + kind + rows)
+    for m in (2, 3, 5, 9, 41, 64):                    # 41: a last warp with one row, two CTAs per row tile
+        xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+        _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
