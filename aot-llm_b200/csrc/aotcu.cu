@@ -951,6 +951,7 @@ struct aotcu_gpu {
   void* d_ll = nullptr;               // tagged activation vectors of the one-kernel step
   StepParams step_params = {};
   size_t mega_smem = 0;
+  bool mega_q80 = false;              // the step's layers are of the Q8_0 family
   // Captured decode steps: [want_logits + 2 * long-context variant of the one-kernel step]
   cudaGraphExec_t decode_graph[4] = {};
   cudaGraphExec_t gen_graph[2] = {};            // [long-context variant]
@@ -1363,7 +1364,7 @@ static int logits_from(aotcu_gpu* g, const float* xrow) {
 
 
 // Decide whether the one-kernel decode step can run this model and build its
-// description. It handles the plain Llama / Qwen3 block (K-quant matrices, optional
+// description. It handles the plain Llama / Qwen3 block (K-quant or Q8_0-family matrices, optional
 // per-head q/k norm, either RoPE layout); everything else keeps the per-operator path.
 static int mega_setup(aotcu_gpu* g) {
   aotcu_ctx* c = g->c;
@@ -1371,10 +1372,14 @@ static int mega_setup(aotcu_gpu* g) {
   const aotcu_tensor& out_t = g->head.output.present ? g->head.output : g->head.token_embd;
   const size_t qd = (size_t)d.n_head * d.head_dim;
   bool ok = !d.qkv_bias && !d.post_norms && !d.gelu && !d.embd_scale && d.swa_window == 0 && d.dim % 256 == 0 &&
-            d.hidden % 256 == 0 && qd % 256 == 0 && d.head_dim % 16 == 0 && kind_act(out_t.kind) == ACT_Q8_K;
+            d.hidden % 256 == 0 && qd % 256 == 0 && d.head_dim % 16 == 0;
+  // all layers K-quants, or all of them of the Q8_0 family with a head of either sort
+  const int act = g->layers.empty() ? ACT_Q8_K : kind_act(g->layers[0].wq.kind);
+  const bool q80 = act == ACT_Q8_0;
+  ok = ok && (act == ACT_Q8_K || q80) && (kind_act(out_t.kind) == ACT_Q8_K || (q80 && kind_act(out_t.kind) == ACT_Q8_0));
   for (const auto& l : g->layers) {
     const aotcu_tensor* ts[7] = {&l.wq, &l.wk, &l.wv, &l.wo, &l.gate, &l.up, &l.down};
-    for (auto t : ts) ok = ok && kind_act(t->kind) == ACT_Q8_K;
+    for (auto t : ts) ok = ok && kind_act(t->kind) == act;
     ok = ok && l.gate.kind == l.up.kind && l.gate.rows == l.up.rows && !l.local_attn;
   }
   // Every CTA must own a row of every product (the tagged hand-over between phases relies
@@ -1404,7 +1409,7 @@ static int mega_setup(aotcu_gpu* g) {
   int stage_bytes = 0, n_stages = 0;
   for (;;) {
     scratch = ((small_floats + stage_floats) * sizeof(float) + 127) & ~(size_t)127;
-    fixed = nb_max * XK_STRIDE + scratch + MEGA_TAIL_BYTES + table_bytes;
+    fixed = nb_max * (q80 ? 8 * X0_STRIDE : XK_STRIDE) + scratch + MEGA_TAIL_BYTES + table_bytes;
     // ring: the stage size that leaves the least shared memory unused
     size_t best = 0;
     for (int sb : {16384, 24576, 32768, 12288}) {
@@ -1427,7 +1432,10 @@ static int mega_setup(aotcu_gpu* g) {
   CU_TRY(cudaFuncSetAttribute(decode_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
   CU_TRY(cudaFuncSetAttribute(decode_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
   CU_TRY(cudaFuncSetAttribute(decode_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+  CU_TRY(cudaFuncSetAttribute(decode_step_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+  CU_TRY(cudaFuncSetAttribute(decode_step_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
   g->mega_smem = (size_t)n_stages * stage_bytes + fixed;
+  g->mega_q80 = q80;
   int per_sm = 0;
   CU_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_step_kernel<true, true>, MEGA_THREADS, g->mega_smem));
   if (per_sm < 1) return 0;
@@ -1559,7 +1567,9 @@ static int enqueue_mega(aotcu_gpu* g, int want_logits, bool with_argmax, unsigne
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cudaError_t e;
-  if (g->split_now)
+  if (g->mega_q80)
+    e = g->split_now ? cudaLaunchKernelEx(&cfg, decode_step_kernel<false, true, true>, P) : cudaLaunchKernelEx(&cfg, decode_step_kernel<false, false, true>, P);
+  else if (g->split_now)
     e = P.tp.world > 1 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<true, true>, P) : cudaLaunchKernelEx(&cfg, decode_step_kernel<false, true>, P);
   else
     e = P.tp.world > 1 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<true, false>, P) : cudaLaunchKernelEx(&cfg, decode_step_kernel<false, false>, P);
@@ -2524,7 +2534,7 @@ int aotcu_tp_attach(aotcu_gpu* g, const char* nccl_library, int rank, int world,
   }
   // Peers' inboxes first, the (blocking, collective) communicator second: once any rank is
   // back from this call, every rank has mapped every inbox.
-  const bool fused = world > 1 && peer_handles && g->tp_inbox && g->mega_ok;
+  const bool fused = world > 1 && peer_handles && g->tp_inbox && g->mega_ok && !g->mega_q80;
   if (fused) {
     TpExchange& x = g->step_params.tp;
     x.world = world;

@@ -508,6 +508,113 @@ __device__ __forceinline__ void consume_op(const MegaOp& op, const Ring& R, Ring
   sp.mark(30);
 }
 
+// ---- Q4_0 / Q5_0 / Q8_0 rows from the ring --------------------------------------------------
+// The reference's AVX2 kernels keep eight f32 lane accumulators per row; lane k adds
+// fma(d_w*d_x, float(p_k), acc_k) per 32-weight block, in block order, and the row ends
+// with a fixed 8-lane tree (simd_avx2.rs:29-34, 61-72). Here eight threads own the eight
+// lane chains of a row (four rows per warp pass).
+__device__ __forceinline__ uint32_t lds32_a2s(uint32_t a) {  // 32-bit word at a 2-byte aligned shared address
+  uint32_t lo, hi;
+  asm("ld.shared.u16 %0, [%1];" : "=r"(lo) : "r"(a));
+  asm("ld.shared.u16 %0, [%1];" : "=r"(hi) : "r"(a + 2));
+  return lo | (hi << 16);
+}
+
+template <int KIND>
+__device__ __forceinline__ float row_chain_q80(uint32_t row, uint32_t sx, int nb, int k) {
+  constexpr int BS = KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34);
+  float acc = 0.0f;
+#pragma unroll 4
+  for (int b = 0; b < nb; b++) {
+    const uint32_t wb = row + (uint32_t)b * BS, xb = sx + (uint32_t)b * X0_STRIDE;
+    uint32_t hd;
+    asm("ld.shared.u16 %0, [%1];" : "=r"(hd) : "r"(wb));
+    const float d = fmul(half_bits_hw(hd), __uint_as_float(rd_lds32(xb + X0_D)));
+    const uint32_t y = rd_lds32(xb + 4 * k);
+    int p;
+    if (KIND == Q8_0) p = q8_0_lane(lds32_a2s(wb + 2 + 4 * k), y);
+    else if (KIND == Q4_0) p = q4_0_lane(lds32_a2s(wb + 2 + 4 * (k & 3)), k, y);
+    else p = q5_0_lane(lds32_a2s(wb + 6 + 4 * (k & 3)), lds32_a2s(wb + 2), k, y);
+    acc = ffma(d, i2f(p), acc);
+  }
+  return acc;
+}
+
+// The one-kernel step's consumer side for matrices of the Q8_0 family: a warp takes four units
+// (rows, or gate/up row pairs) at a time, eight lanes each; a pair's two chains run side by side.
+// What bounds it: the chains' nb dependent steps, of which a CTA has (its rows) x 8 only; the
+// launches that the per-operator path put around every product cost more (TinyLlama shape in
+// Q4_0 at position 160: 1.34 ms a token by operators, 0.95 in one kernel).
+template <int KIND, int NM>
+__device__ __forceinline__ void rows_chain_q80(const uint32_t (&row)[2], uint32_t sx, int nb, int k, float (&acc)[2]) {
+  constexpr int BS = KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34);
+  acc[0] = acc[1] = 0.0f;
+#pragma unroll 4
+  for (int b = 0; b < nb; b++) {
+    const uint32_t xb = sx + (uint32_t)b * X0_STRIDE, y = rd_lds32(xb + 4 * k);
+    const float dx = __uint_as_float(rd_lds32(xb + X0_D));
+#pragma unroll
+    for (int i = 0; i < NM; i++) {
+      const uint32_t wb = row[i] + (uint32_t)b * BS;
+      uint32_t hd;
+      asm("ld.shared.u16 %0, [%1];" : "=r"(hd) : "r"(wb));
+      int p;
+      if (KIND == Q8_0) p = q8_0_lane(lds32_a2s(wb + 2 + 4 * k), y);
+      else if (KIND == Q4_0) p = q4_0_lane(lds32_a2s(wb + 2 + 4 * (k & 3)), k, y);
+      else p = q5_0_lane(lds32_a2s(wb + 6 + 4 * (k & 3)), lds32_a2s(wb + 2), k, y);
+      acc[i] = ffma(fmul(half_bits_hw(hd), dx), i2f(p), acc[i]);
+    }
+  }
+}
+__device__ __forceinline__ void consume_step_q80(const MegaOp& op, const Ring& R, RingPos& cp, const uint8_t* sx, int warp, int n_warps,
+                                                 uint32_t tag) {
+  const int nb = op.cols >> 5, lane = threadIdx.x & 31, k = lane & 7;
+  const uint32_t sxa = smem_addr(sx);
+  const int n_tiles = (int)blockIdx.x < op.cta_rem ? op.n_tiles_hi : op.n_tiles_lo;
+  int next = warp;  // this warp's next pass, counted over the passes of all tiles
+#pragma unroll 1
+  for (int tile = 0; tile < n_tiles; tile++) {
+    if (!ring_wait(R, &R.full[cp.st], cp.parity)) return;
+    const TileDesc& D = R.desc[cp.st];
+    const int n_units = D.n_units, n_pass = (n_units + 3) >> 2;
+#pragma unroll 1
+    for (; next < n_pass; next += n_warps) {
+      const int u = next * 4 + (lane >> 3);
+      const TileUnit U = D.unit[min(u, n_units - 1)];  // lanes past the end repeat the last unit
+      const uint32_t row[2] = {U.row[0] & 0xFFFFFFu, U.row[1] & 0xFFFFFFu};
+      const int kind = (int)(U.row[0] >> 24);
+      LLWord* const ll = reinterpret_cast<LLWord*>(U.out);
+      const bool writer = k == 0 && u < n_units, accum = op.epilogue == EPI_ACCUM;
+      float old = 0.0f, v[2];
+      if (writer && accum && op.ll) old = ll_value(ll);
+      if (op.pair) {
+        if (kind == Q4_0) rows_chain_q80<Q4_0, 2>(row, sxa, nb, k, v);
+        else if (kind == Q5_0) rows_chain_q80<Q5_0, 2>(row, sxa, nb, k, v);
+        else rows_chain_q80<Q8_0, 2>(row, sxa, nb, k, v);
+      } else {
+        if (kind == Q4_0) rows_chain_q80<Q4_0, 1>(row, sxa, nb, k, v);
+        else if (kind == Q5_0) rows_chain_q80<Q5_0, 1>(row, sxa, nb, k, v);
+        else rows_chain_q80<Q8_0, 1>(row, sxa, nb, k, v);
+      }
+      __syncwarp();  // units of two matrices may be of two kinds
+      // ((a0+a4)+(a2+a6)) + ((a1+a5)+(a3+a7)) over the row's eight lanes
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v[i] = fadd(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
+      if (writer) {
+        const float r = op.pair ? silu_mul_call(v[0], v[1]) : accum ? fadd(old, v[0]) : v[0];
+        if (op.ll) ll_store(ll, r, tag);
+        else *U.out = r;  // the output head
+      }
+    }
+    next -= n_pass;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&R.empty[cp.st]);
+    cp.advance(R.n_stages);
+  }
+}
+
 // ---- grid-wide barrier for the consumer warps ---------------------------------------------
 // Arrival counter in global memory, zero at launch, never reset: barrier number k
 // completes when it reaches k * gridDim.x. The spin is bounded; when it gives up the
@@ -563,20 +670,35 @@ __device__ __forceinline__ float red_sum(const float* red, int nw) {
   return s;
 }
 
-// quant.rs:248-283 for the 256 values a warp holds (lane l: elements 8l..8l+7), written as
-// a block image.
-__device__ __forceinline__ void quantize_block_call(float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7,
-                                                    uint8_t* dst) {
-  const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
-  warp_quantize_q8k_vals(v, dst, 1);
+// The 256 values a warp holds (lane l: elements 8l..8l+7) as eight Q8_0 block images
+// (quant.rs:231-245): four lanes per block.
+__device__ __forceinline__ void quantize_q80_blocks(const float (&v)[8], uint8_t* dst) {
+  const int lane = threadIdx.x & 31;
+  float amax = fabsf(v[0]);
+#pragma unroll
+  for (int i = 1; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  const float d = fdiv(amax, 127.0f), id = d != 0.0f ? fdiv(1.0f, d) : 0.0f;
+  uint32_t w[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    int q = (int)roundf(fmul(v[i], id));
+    q = q < -127 ? -127 : (q > 127 ? 127 : q);
+    w[i >> 2] |= (uint32_t)(q & 0xFF) << (8 * (i & 3));
+  }
+  uint8_t* const o = dst + (lane >> 2) * X0_STRIDE;
+  *reinterpret_cast<uint2*>(o + 8 * (lane & 3)) = make_uint2(w[0], w[1]);
+  if ((lane & 3) == 0) *reinterpret_cast<float*>(o + X0_D) = d;
 }
 
-// x -> rmsnorm -> Q8_K images in shared memory (ops.rs:7-18 then quant.rs:248-283).
+// x -> rmsnorm -> Q8_K images (Q8_0 images for `q80`) in shared memory (ops.rs:7-18 then quant.rs:248-283).
 // `src` holds tagged words other CTAs publish under `tag`; for the embedding the row is
 // already in scr[0..n). `mirror`, when given, receives a plain copy of the row. The warp
 // that owns a super-block keeps its 256 values in registers from the load to the quantized
 // image (at most two super-blocks per warp: n <= 512 * warps).
-__device__ __forceinline__ void phase_norm_quant(const LLWord* src, uint32_t tag, bool src_in_scr, float* mirror, const float* w,
+template <bool Q80>
+__device__ __forceinline__ void phase_norm_quant(bool q80, const LLWord* src, uint32_t tag, bool src_in_scr, float* mirror, const float* w,
                                                  int n, float eps, int fast, const MegaSmem& M, const CtaGroup& g,
                                                  SubProf sp = SubProf{nullptr, 0}, unsigned long long* walker_prof = nullptr) {
   sp.last = clock64();
@@ -648,22 +770,26 @@ __device__ __forceinline__ void phase_norm_quant(const LLWord* src, uint32_t tag
       const float4 a0 = *reinterpret_cast<const float4*>(row + b * 256 + 8 * lane), a1 = *reinterpret_cast<const float4*>(row + b * 256 + 8 * lane + 4);
       v[k][0] = a0.x; v[k][1] = a0.y; v[k][2] = a0.z; v[k][3] = a0.w;
       v[k][4] = a1.x; v[k][5] = a1.y; v[k][6] = a1.z; v[k][7] = a1.w;
-      quantize_block_call(fmul(fmul(v[k][0], r), w0[k].x), fmul(fmul(v[k][1], r), w0[k].y), fmul(fmul(v[k][2], r), w0[k].z),
+      const float y[8] = {fmul(fmul(v[k][0], r), w0[k].x), fmul(fmul(v[k][1], r), w0[k].y), fmul(fmul(v[k][2], r), w0[k].z),
                           fmul(fmul(v[k][3], r), w0[k].w), fmul(fmul(v[k][4], r), w1[k].x), fmul(fmul(v[k][5], r), w1[k].y),
-                          fmul(fmul(v[k][6], r), w1[k].z), fmul(fmul(v[k][7], r), w1[k].w), M.sx + b * XK_STRIDE);
+                          fmul(fmul(v[k][6], r), w1[k].z), fmul(fmul(v[k][7], r), w1[k].w)};
+      if (Q80 && q80) quantize_q80_blocks(y, M.sx + b * (8 * X0_STRIDE));
+      else warp_quantize_q8k_vals(y, M.sx + b * XK_STRIDE, 1);
     }
   }
   g.sync();
   sp.mark(19);
 }
 
-// A vector other CTAs publish under `tag` -> Q8_K images.
+// A vector other CTAs publish under `tag` -> Q8_K (Q80: Q8_0) images.
+template <bool Q80>
 __device__ __forceinline__ void phase_quant(const LLWord* src, uint32_t tag, int n, const MegaSmem& M, const CtaGroup& g) {
   const int warp = g.tid >> 5, nw = g.nthreads >> 5, lane = g.tid & 31;
   for (int b = warp; b < n / 256; b += nw) {
     float v[8];
     ll_wait8(src + b * 256 + 8 * lane, tag, v, M.abort, M.err);
-    quantize_block_call(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], M.sx + b * XK_STRIDE);
+    if (Q80) quantize_q80_blocks(v, M.sx + b * (8 * X0_STRIDE));
+    else warp_quantize_q8k_vals(v, M.sx + b * XK_STRIDE, 1);
   }
   g.sync();
 }
@@ -1210,14 +1336,15 @@ constexpr int MEGA_TAIL_BYTES = MEGA_BAR_BYTES + 64 * 4 + 16 + MEGA_TERMS_BYTES;
 // TP: this GPU holds one shard of a row-sharded model and exchanges partial rows with its peers.
 // SPLIT: the long-context variant, in which several CTAs share each head's attention (the
 // host picks the variant from the position; see attention_split).
-template <bool TP, bool SPLIT>
+// Q80: the layers' matrices are of the Q8_0 family (the output head may be a K-quant).
+template <bool TP, bool SPLIT, bool Q80 = false>
 __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const StepParams P) {
   extern __shared__ __align__(128) uint8_t smem[];
   // [stages][sx images][scratch][barriers 128 B][red 64 floats][abort][term strips | SeqSumScratch][table]
   const int nb_max = (max(max(P.dim, P.hidden), P.n_head * P.head_dim)) / 256;
   uint8_t* stages = smem;
   uint8_t* sx = stages + (size_t)P.n_stages * P.stage_bytes;
-  uint8_t* cur = sx + (size_t)nb_max * XK_STRIDE;  // 16-byte aligned: 304 = 19 * 16
+  uint8_t* cur = sx + (size_t)nb_max * (Q80 ? 8 * X0_STRIDE : XK_STRIDE);  // 16-byte aligned: 304 = 19 * 16, 384
   float* scr = reinterpret_cast<float*>(cur);
   cur += P.scratch_bytes;                          // a multiple of 128
   uint64_t* bars = reinterpret_cast<uint64_t*>(cur);
@@ -1333,6 +1460,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
   // that each phase's code exists once. Phases hand their vectors on as tagged words;
   // the only grid-wide barrier left is the one in front of the argmax.
   const int n_stage = 4 * P.n_layer + (P.want_logits ? 1 : 0);
+  const bool head_q80 = Q80 && table[P.n_layer].qkv.seg[0].kind < Q4_K;
 #pragma unroll 1
   for (int st = 0; st < n_stage; st++) {
     const int li = st >> 2, ph = st & 3;
@@ -1366,13 +1494,13 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
       // attention norm -> q/k/v, ffn norm -> gate/up + SiLU, output norm -> logits
       const float* w = head ? P.output_norm : (ph == 0 ? L.attn_norm : L.ffn_norm);
       const uint32_t tin = ph == 0 ? tl : tl + 3u;  // residual after the previous layer's down / this layer's wo
-      phase_norm_quant(P.xl, tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
+      phase_norm_quant<Q80>(!head || head_q80, P.xl, tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
                        SubProf{prof_on && ph == 0 && !head ? P.prof : nullptr, 0},
                        P.prof && (int)blockIdx.x == P.prof_cta && ph == 0 && !head && g.tid == (MEGA_CONSUMER_WARPS - 1) * 32 ? P.prof : nullptr);
     } else {
       // attention output -> wo, activated hidden -> down; both join the residual stream
-      if (ph == 1) phase_quant(P.attl, tl + 2u, qd, M, g);
-      else phase_quant(P.hbl, tl + 4u, P.hidden, M, g);
+      if (ph == 1) phase_quant<Q80>(P.attl, tl + 2u, qd, M, g);
+      else phase_quant<Q80>(P.hbl, tl + 4u, P.hidden, M, g);
     }
     if (!head) MEGA_PROF(slot);
     // q/k/v: tl+1, wo: tl+3, gate/up: tl+4, down: tl+5 (the head writes plain floats)
@@ -1380,8 +1508,9 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
     const bool exchange = TP && (ph & 1) && !head;
     int xr0 = 0, xr1 = 0;  // rows of the residual stream this CTA owns (the rows of wo / down it computes)
     if (TP && exchange) cta_rows(P.dim, xr0, xr1);
-    consume_op<TP>(op, R, cp, sx, wterms, warp, MEGA_CONSUMER_WARPS, tag_out, exchange ? &P.tp : nullptr, ph >> 1,
-                   SubProf{nullptr, 0}, M.red, xr0);
+    if (Q80 && (!head || head_q80)) consume_step_q80(op, R, cp, sx, warp, MEGA_CONSUMER_WARPS, tag_out);
+    else consume_op<TP>(op, R, cp, sx, wterms, warp, MEGA_CONSUMER_WARPS, tag_out, exchange ? &P.tp : nullptr, ph >> 1,
+                        SubProf{nullptr, 0}, M.red, xr0);
     if (head) break;
     // The next phase rewrites the activation images and the scratch rows; warps that are
     // done must also not start polling while others still compute.
@@ -1450,38 +1579,6 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
   if (blockIdx.x == 0 && g.tid == 0) *P.epoch = *P.epoch + 1u;
   MEGA_PROF(15);
 #undef MEGA_PROF
-}
-
-// ---- Q4_0 / Q5_0 / Q8_0 rows from the ring --------------------------------------------------
-// The reference's AVX2 kernels keep eight f32 lane accumulators per row; lane k adds
-// fma(d_w*d_x, float(p_k), acc_k) per 32-weight block, in block order, and the row ends
-// with a fixed 8-lane tree (simd_avx2.rs:29-34, 61-72). Here eight threads own the eight
-// lane chains of a row (four rows per warp pass).
-__device__ __forceinline__ uint32_t lds32_a2s(uint32_t a) {  // 32-bit word at a 2-byte aligned shared address
-  uint32_t lo, hi;
-  asm("ld.shared.u16 %0, [%1];" : "=r"(lo) : "r"(a));
-  asm("ld.shared.u16 %0, [%1];" : "=r"(hi) : "r"(a + 2));
-  return lo | (hi << 16);
-}
-
-template <int KIND>
-__device__ __forceinline__ float row_chain_q80(uint32_t row, uint32_t sx, int nb, int k) {
-  constexpr int BS = KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34);
-  float acc = 0.0f;
-#pragma unroll 4
-  for (int b = 0; b < nb; b++) {
-    const uint32_t wb = row + (uint32_t)b * BS, xb = sx + (uint32_t)b * X0_STRIDE;
-    uint32_t hd;
-    asm("ld.shared.u16 %0, [%1];" : "=r"(hd) : "r"(wb));
-    const float d = fmul(half_bits_hw(hd), __uint_as_float(rd_lds32(xb + X0_D)));
-    const uint32_t y = rd_lds32(xb + 4 * k);
-    int p;
-    if (KIND == Q8_0) p = q8_0_lane(lds32_a2s(wb + 2 + 4 * k), y);
-    else if (KIND == Q4_0) p = q4_0_lane(lds32_a2s(wb + 2 + 4 * (k & 3)), k, y);
-    else p = q5_0_lane(lds32_a2s(wb + 6 + 4 * (k & 3)), lds32_a2s(wb + 2), k, y);
-    acc = ffma(d, i2f(p), acc);
-  }
-  return acc;
 }
 
 // Consumer side for matrices of the Q8_0 family; `sx` holds the 48-byte Q8_0 images.
