@@ -1376,10 +1376,11 @@ static int mega_setup(aotcu_gpu* g) {
   // all layers K-quants, or all of them of the Q8_0 family with a head of either sort
   const int act = g->layers.empty() ? ACT_Q8_K : kind_act(g->layers[0].wq.kind);
   const bool q80 = act == ACT_Q8_0;
-  ok = ok && (act == ACT_Q8_K || q80) && (kind_act(out_t.kind) == ACT_Q8_K || (q80 && kind_act(out_t.kind) == ACT_Q8_0));
+  ok = ok && (act == ACT_Q8_K || q80) && (kind_act(out_t.kind) == ACT_Q8_K || (q80 && kind_act(out_t.kind) == ACT_Q8_0 && !((uintptr_t)wptr(g, out_t) & 3)));
   for (const auto& l : g->layers) {
     const aotcu_tensor* ts[7] = {&l.wq, &l.wk, &l.wv, &l.wo, &l.gate, &l.up, &l.down};
-    for (auto t : ts) ok = ok && kind_act(t->kind) == act;
+    // Q8_0-family rows are read as 32-bit words
+    for (auto t : ts) ok = ok && kind_act(t->kind) == act && !(q80 && ((uintptr_t)wptr(g, *t) & 3));
     ok = ok && l.gate.kind == l.up.kind && l.gate.rows == l.up.rows && !l.local_attn;
   }
   // Every CTA must own a row of every product (the tagged hand-over between phases relies
@@ -1409,7 +1410,7 @@ static int mega_setup(aotcu_gpu* g) {
   int stage_bytes = 0, n_stages = 0;
   for (;;) {
     scratch = ((small_floats + stage_floats) * sizeof(float) + 127) & ~(size_t)127;
-    fixed = nb_max * (q80 ? 8 * X0_STRIDE : XK_STRIDE) + scratch + MEGA_TAIL_BYTES + table_bytes;
+    fixed = nb_max * XK_STRIDE + scratch + MEGA_TAIL_BYTES + table_bytes;
     // ring: the stage size that leaves the least shared memory unused
     size_t best = 0;
     for (int sb : {16384, 24576, 32768, 12288}) {

@@ -542,35 +542,87 @@ __device__ __forceinline__ float row_chain_q80(uint32_t row, uint32_t sx, int nb
 
 // The one-kernel step's consumer side for matrices of the Q8_0 family: a warp takes four units
 // (rows, or gate/up row pairs) at a time, eight lanes each; a pair's two chains run side by side.
-// What bounds it: the chains' nb dependent steps, of which a CTA has (its rows) x 8 only; the
-// launches that the per-operator path put around every product cost more (TinyLlama shape in
-// Q4_0 at position 160: 1.34 ms a token by operators, 0.95 in one kernel).
+// What bounds it: a lone warp's instructions where a CTA has few rows (its chains are all the
+// parallelism there is), the loads where it has many. So blocks go in twos, whose 32-bit words lie
+// at fixed places of an aligned run, and activations are stored for this order (StepImage): 25
+// instructions for two blocks of Q4_0, 38 with one block at a time. Splitting a row's blocks over
+// more lanes loses: the shuffles that bring the factors to the chain cost more than they save
+// (down 9900 cycles a layer with 8 lanes a row, 11800 with 32).
+//
+// TinyLlama shape in Q4_0 at position 160: 1.34 ms a token by operators, 0.92 in one kernel with one
+// block at a time, 0.80 in pairs.
+//
+// StepImage of n activations: 64 bytes per block pair, lane k's four quants of either block at
+// 8 k and 8 k + 4; then the n / 32 block scales.
+__device__ __forceinline__ void rd_lds64(uint32_t a, uint32_t& x, uint32_t& y) {
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x), "=r"(y) : "r"(a));  // stays behind the barrier that published the activations
+}
+template <int KIND>
+__device__ __forceinline__ void q80_pair(uint32_t w, int k, uint32_t y0, uint32_t y1, float& d0, float& d1, float& p0, float& p1) {
+  // the second block starts in the middle of word W, so that its quants are whole words
+  constexpr int W = (KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34)) / 4;
+  const uint32_t first = rd_lds32(w), mid = rd_lds32(w + 4 * W);
+  const int j = KIND == Q8_0 ? k : (k & 3), o = KIND == Q5_0 ? 1 : 0;
+  const uint32_t wj = w + 4 * j;
+  uint32_t v0 = funnel_r(rd_lds32(wj + 4 * o), rd_lds32(wj + 4 * o + 4), 16), v1 = rd_lds32(wj + 4 * (W + 1 + o));
+  int c0 = 0, c1 = 0;
+  if (KIND != Q8_0) {
+    // unsigned nibbles (and fifth bits); the offset of 8 (16) times the activations' sum starts the dot
+    v0 = (v0 >> (k & 4)) & 0x0F0F0F0Fu;
+    v1 = (v1 >> (k & 4)) & 0x0F0F0F0Fu;
+    const int off = KIND == Q4_0 ? (int)0xF8F8F8F8u : (int)0xF0F0F0F0u;
+    c0 = __dp4a(off, (int)y0, 0);
+    c1 = __dp4a(off, (int)y1, 0);
+  }
+  if (KIND == Q5_0) {
+    const uint32_t h0 = funnel_r(first, rd_lds32(w + 4), 16) >> (4 * k), h1 = rd_lds32(w + 4 * (W + 1)) >> (4 * k);
+    v0 |= ((h0 & 1u) << 4) | ((h0 & 2u) << 11) | ((h0 & 4u) << 18) | ((h0 & 8u) << 25);
+    v1 |= ((h1 & 1u) << 4) | ((h1 & 2u) << 11) | ((h1 & 4u) << 18) | ((h1 & 8u) << 25);
+  }
+  p0 = i2f(__dp4a((int)v0, (int)y0, c0));
+  p1 = i2f(__dp4a((int)v1, (int)y1, c1));
+  d0 = half_bits_hw(first & 0xFFFFu);
+  d1 = half_bits_hw(mid >> 16);
+}
+// Where the rows of a warp lie a multiple of 64 bytes apart, row q runs q block pairs behind row 0,
+// so that their words fall on different banks (gate/up of 2048 columns: 19000 -> 11100 cycles).
 template <int KIND, int NM>
-__device__ __forceinline__ void rows_chain_q80(const uint32_t (&row)[2], uint32_t sx, int nb, int k, float (&acc)[2]) {
-  constexpr int BS = KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34);
+__device__ __forceinline__ void rows_chain_q80(const uint32_t (&row)[2], uint32_t sx, int nb, bool skewed, float (&acc)[2]) {
+  constexpr int PB = 2 * (KIND == Q4_0 ? 18 : (KIND == Q5_0 ? 22 : 34));
+  const int lane = threadIdx.x & 31, k = lane & 7, q = skewed ? lane >> 3 : 0, np = nb >> 1;
   acc[0] = acc[1] = 0.0f;
-#pragma unroll 4
-  for (int b = 0; b < nb; b++) {
-    const uint32_t xb = sx + (uint32_t)b * X0_STRIDE, y = rd_lds32(xb + 4 * k);
-    const float dx = __uint_as_float(rd_lds32(xb + X0_D));
+  auto step = [&](int b, bool on) {
+    uint32_t y0, y1, x0, x1;
+    rd_lds64(sx + (uint32_t)(b * 64 + 8 * k), y0, y1);
+    rd_lds64(sx + (uint32_t)(nb * 32 + b * 8), x0, x1);
 #pragma unroll
     for (int i = 0; i < NM; i++) {
-      const uint32_t wb = row[i] + (uint32_t)b * BS;
-      uint32_t hd;
-      asm("ld.shared.u16 %0, [%1];" : "=r"(hd) : "r"(wb));
-      int p;
-      if (KIND == Q8_0) p = q8_0_lane(lds32_a2s(wb + 2 + 4 * k), y);
-      else if (KIND == Q4_0) p = q4_0_lane(lds32_a2s(wb + 2 + 4 * (k & 3)), k, y);
-      else p = q5_0_lane(lds32_a2s(wb + 6 + 4 * (k & 3)), lds32_a2s(wb + 2), k, y);
-      acc[i] = ffma(fmul(half_bits_hw(hd), dx), i2f(p), acc[i]);
+      float d0, d1, p0, p1;
+      q80_pair<KIND>(row[i] + (uint32_t)(b * PB), k, y0, y1, d0, d1, p0, p1);
+      const float n = ffma(fmul(d1, __uint_as_float(x1)), p1, ffma(fmul(d0, __uint_as_float(x0)), p0, acc[i]));
+      acc[i] = on ? n : acc[i];
     }
-  }
+  };
+  const int lag = skewed ? 3 : 0;
+#pragma unroll 1
+  for (int b = 0; b < lag; b++) step(max(b - q, 0), b >= q);
+#pragma unroll 4
+  for (int b = lag; b < np; b++) step(b - q, true);
+#pragma unroll 1
+  for (int b = np; b < np + lag; b++) step(min(b - q, np - 1), b - q < np);
+}
+template <int NM>
+__device__ __forceinline__ void unit_chain_q80(int kind, const uint32_t (&row)[2], uint32_t sx, int nb, bool skewed, float (&acc)[2]) {
+  if (kind == Q4_0) rows_chain_q80<Q4_0, NM>(row, sx, nb, skewed, acc);
+  else if (kind == Q5_0) rows_chain_q80<Q5_0, NM>(row, sx, nb, skewed, acc);
+  else rows_chain_q80<Q8_0, NM>(row, sx, nb, skewed, acc);
 }
 __device__ __forceinline__ void consume_step_q80(const MegaOp& op, const Ring& R, RingPos& cp, const uint8_t* sx, int warp, int n_warps,
                                                  uint32_t tag) {
-  const int nb = op.cols >> 5, lane = threadIdx.x & 31, k = lane & 7;
+  const int nb = op.cols >> 5, lane = threadIdx.x & 31;
   const uint32_t sxa = smem_addr(sx);
   const int n_tiles = (int)blockIdx.x < op.cta_rem ? op.n_tiles_hi : op.n_tiles_lo;
+  const bool skewed = (op.row_bytes[0] & 63u) == 0;
   int next = warp;  // this warp's next pass, counted over the passes of all tiles
 #pragma unroll 1
   for (int tile = 0; tile < n_tiles; tile++) {
@@ -584,18 +636,11 @@ __device__ __forceinline__ void consume_step_q80(const MegaOp& op, const Ring& R
       const uint32_t row[2] = {U.row[0] & 0xFFFFFFu, U.row[1] & 0xFFFFFFu};
       const int kind = (int)(U.row[0] >> 24);
       LLWord* const ll = reinterpret_cast<LLWord*>(U.out);
-      const bool writer = k == 0 && u < n_units, accum = op.epilogue == EPI_ACCUM;
+      const bool writer = (lane & 7) == 0 && u < n_units, accum = op.epilogue == EPI_ACCUM;
       float old = 0.0f, v[2];
       if (writer && accum && op.ll) old = ll_value(ll);
-      if (op.pair) {
-        if (kind == Q4_0) rows_chain_q80<Q4_0, 2>(row, sxa, nb, k, v);
-        else if (kind == Q5_0) rows_chain_q80<Q5_0, 2>(row, sxa, nb, k, v);
-        else rows_chain_q80<Q8_0, 2>(row, sxa, nb, k, v);
-      } else {
-        if (kind == Q4_0) rows_chain_q80<Q4_0, 1>(row, sxa, nb, k, v);
-        else if (kind == Q5_0) rows_chain_q80<Q5_0, 1>(row, sxa, nb, k, v);
-        else rows_chain_q80<Q8_0, 1>(row, sxa, nb, k, v);
-      }
+      if (op.pair) unit_chain_q80<2>(kind, row, sxa, nb, skewed, v);
+      else unit_chain_q80<1>(kind, row, sxa, nb, skewed, v);
       __syncwarp();  // units of two matrices may be of two kinds
       // ((a0+a4)+(a2+a6)) + ((a1+a5)+(a3+a7)) over the row's eight lanes
 #pragma unroll
@@ -670,9 +715,10 @@ __device__ __forceinline__ float red_sum(const float* red, int nw) {
   return s;
 }
 
-// The 256 values a warp holds (lane l: elements 8l..8l+7) as eight Q8_0 block images
-// (quant.rs:231-245): four lanes per block.
-__device__ __forceinline__ void quantize_q80_blocks(const float (&v)[8], uint8_t* dst) {
+// The 256 values a warp holds (lane l: elements 8l..8l+7) as eight Q8_0 blocks
+// (quant.rs:231-245), four lanes per block, in the order of consume_step_q80; `b`: their number in a
+// vector of n.
+__device__ __forceinline__ void quantize_q80_blocks(const float (&v)[8], uint8_t* sx, int n, int b) {
   const int lane = threadIdx.x & 31;
   float amax = fabsf(v[0]);
 #pragma unroll
@@ -687,9 +733,11 @@ __device__ __forceinline__ void quantize_q80_blocks(const float (&v)[8], uint8_t
     q = q < -127 ? -127 : (q > 127 ? 127 : q);
     w[i >> 2] |= (uint32_t)(q & 0xFF) << (8 * (i & 3));
   }
-  uint8_t* const o = dst + (lane >> 2) * X0_STRIDE;
-  *reinterpret_cast<uint2*>(o + 8 * (lane & 3)) = make_uint2(w[0], w[1]);
-  if ((lane & 3) == 0) *reinterpret_cast<float*>(o + X0_D) = d;
+  const int blk = 8 * b + (lane >> 2);
+  uint32_t* const o = reinterpret_cast<uint32_t*>(sx + (blk >> 1) * 64 + 16 * (lane & 3)) + (blk & 1);
+  o[0] = w[0];
+  o[2] = w[1];
+  if ((lane & 3) == 0) *reinterpret_cast<float*>(sx + n + 4 * blk) = d;
 }
 
 // x -> rmsnorm -> Q8_K images (Q8_0 images for `q80`) in shared memory (ops.rs:7-18 then quant.rs:248-283).
@@ -773,7 +821,7 @@ __device__ __forceinline__ void phase_norm_quant(bool q80, const LLWord* src, ui
       const float y[8] = {fmul(fmul(v[k][0], r), w0[k].x), fmul(fmul(v[k][1], r), w0[k].y), fmul(fmul(v[k][2], r), w0[k].z),
                           fmul(fmul(v[k][3], r), w0[k].w), fmul(fmul(v[k][4], r), w1[k].x), fmul(fmul(v[k][5], r), w1[k].y),
                           fmul(fmul(v[k][6], r), w1[k].z), fmul(fmul(v[k][7], r), w1[k].w)};
-      if (Q80 && q80) quantize_q80_blocks(y, M.sx + b * (8 * X0_STRIDE));
+      if (Q80 && q80) quantize_q80_blocks(y, M.sx, n, b);
       else warp_quantize_q8k_vals(y, M.sx + b * XK_STRIDE, 1);
     }
   }
@@ -788,7 +836,7 @@ __device__ __forceinline__ void phase_quant(const LLWord* src, uint32_t tag, int
   for (int b = warp; b < n / 256; b += nw) {
     float v[8];
     ll_wait8(src + b * 256 + 8 * lane, tag, v, M.abort, M.err);
-    if (Q80) quantize_q80_blocks(v, M.sx + b * (8 * X0_STRIDE));
+    if (Q80) quantize_q80_blocks(v, M.sx, n, b);
     else warp_quantize_q8k_vals(v, M.sx + b * XK_STRIDE, 1);
   }
   g.sync();
@@ -1344,7 +1392,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
   const int nb_max = (max(max(P.dim, P.hidden), P.n_head * P.head_dim)) / 256;
   uint8_t* stages = smem;
   uint8_t* sx = stages + (size_t)P.n_stages * P.stage_bytes;
-  uint8_t* cur = sx + (size_t)nb_max * (Q80 ? 8 * X0_STRIDE : XK_STRIDE);  // 16-byte aligned: 304 = 19 * 16, 384
+  uint8_t* cur = sx + (size_t)nb_max * XK_STRIDE;  // 16-byte aligned: 304 = 19 * 16
   float* scr = reinterpret_cast<float*>(cur);
   cur += P.scratch_bytes;                          // a multiple of 128
   uint64_t* bars = reinterpret_cast<uint64_t*>(cur);
