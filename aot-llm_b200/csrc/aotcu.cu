@@ -22,6 +22,7 @@
 #include "attention.cuh"
 #include "kmma.cuh"
 #include "mega.cuh"
+#include "q80mma.cuh"
 #include "q80stream.cuh"
 #include "floatmulti.cuh"
 #include "floatstream.cuh"
@@ -450,6 +451,62 @@ static ChunkShape chunk_shape(int quads_per_cta, bool pair, size_t m, int force_
   return s;
 }
 
+// Q4_0 / Q5_0 / Q8_0 products of several activation rows on the tensor-core kernel of q80mma.cuh.
+// Returns 1 when the call does not fit.
+template <int KIND, bool PAIR>
+static int launch_q80_mma_t(aotcu_ctx* c, const Q80MmaParams& P, int grid) {
+  static bool attr_set[64] = {};
+  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(q80_mma_kernel<KIND, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    attr_set[c->device] = true;
+  }
+  return launch(c, q80_mma_kernel<KIND, PAIR>, dim3(grid), dim3(32 * P.wt), (size_t)QmShape<KIND>::unit_bytes(P.wt), P);
+}
+// A warp's chains take the same time whatever the launch holds, so it has to fill the chip, and a
+// batch that leaves part of a warp's 16 tokens or of the fourth warp idle gains nothing (11264x2048:
+// 82 us against 118 at 64 rows, 83 against 90 at 48, 57 against 61 at 32; 2560x2048: 39 against 49,
+// 2048x5632: 125 against 86).
+constexpr size_t Q80_MMA_MIN_ROWS = 8192, Q80_MMA_MIN_BATCH = 49;
+static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
+  if (call.m < Q80_MMA_MIN_BATCH || call.m > (1u << 16) || (call.pair ? 2 : 1) * span < Q80_MMA_MIN_ROWS || call.cols % 256) return 1;
+  for (int s = 0; s < call.nseg; s++)
+    if ((uintptr_t)call.seg[s].w & 15) return 1;
+  if (call.pair && call.seg[0].kind != call.seg[1].kind) return 1;
+  const int nb = (int)(call.cols / 32), ntg = (int)((call.m + 7) / 8);
+  if (const int rc = ctx_workspace(c, (size_t)ntg * nb * X0F_BLOCK)) return rc;
+  if (int rc = launch(c, x0f_kernel, dim3((unsigned)(((size_t)ntg * nb + 7) / 8)), dim3(256), 0, reinterpret_cast<const uint8_t*>(call.x), (int)(call.x_mode == 1),
+                      c->ximg, (int)call.m, nb))
+    return rc;
+  Q80MmaParams P = {};
+  P.cols = (int)call.cols;
+  P.m = (int)call.m;
+  P.epilogue = call.epilogue;
+  P.xf = c->ximg;
+  P.ntg = ntg;
+  const int nw = (ntg + QM_NG - 1) / QM_NG;  // warps that the batch takes: at most four or five share a row unit
+  P.n_tcta = (nw + 4) / 5;
+  P.wt = (nw + P.n_tcta - 1) / P.n_tcta;
+  const int rows = call.pair ? 16 : 16 * QM_RT;
+  for (int kind : {Q4_0, Q5_0, Q8_0}) {
+    P.nseg = P.n_units = 0;
+    for (int s = 0; s < call.nseg; s++) {
+      if (call.seg[s].kind != kind) continue;
+      P.seg[P.nseg] = call.seg[s];
+      P.units_before[P.nseg] = call.pair ? 0 : P.n_units;
+      if (!call.pair || s == 0) P.n_units += (call.seg[s].rows + rows - 1) / rows;
+      P.nseg++;
+    }
+    if (!P.nseg) continue;
+    const int grid = P.n_units * P.n_tcta;
+    int rc;
+    if (kind == Q4_0) rc = call.pair ? launch_q80_mma_t<Q4_0, true>(c, P, grid) : launch_q80_mma_t<Q4_0, false>(c, P, grid);
+    else if (kind == Q5_0) rc = call.pair ? launch_q80_mma_t<Q5_0, true>(c, P, grid) : launch_q80_mma_t<Q5_0, false>(c, P, grid);
+    else rc = call.pair ? launch_q80_mma_t<Q8_0, true>(c, P, grid) : launch_q80_mma_t<Q8_0, false>(c, P, grid);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 static int launch_q80_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   const int kind = call.seg[0].kind;
   const size_t row_bytes = kind_row_bytes(kind, call.cols);
@@ -782,6 +839,8 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
     if (rc <= 0) return rc;  // 1: a conversion buffer would have to grow during a stream capture
   }
   if (act == ACT_Q8_0 && g_q80_chunks) {
+    const int mc = launch_q80_mma(c, call, span);
+    if (mc <= 0) return mc;
     const int rc = launch_q80_stream(c, call, span);
     if (rc <= 0) return rc;  // 1: mixed kinds or a very long activation row, the whole-row kernels take it
   }

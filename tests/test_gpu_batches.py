@@ -51,3 +51,23 @@ def test_float_tile_edges(pkg, ob, ctx, kind, rows, cols):
     for m in (2, 3, 5, 9, 41, 64):                    # 41: a last warp with one row, two CTAs per row tile
         xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
         _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+
+
+@pytest.mark.parametrize("kind", [3, 4, 5])           # Q4_0, Q5_0, Q8_0
+def test_q80_tile_edges(pkg, ob, ctx, kind):
+    for rows, cols, ms in ((8192, 256, (49, 64)), (8205, 768, (50, 81, 129))):   # a partial row tile, half-full warps, two CTAs per tile
+        w = make_weights(pkg, kind, rows, cols, 41 + kind)
+        for m in ms:
+            xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+            _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+
+
+def test_q80_pair_tile_edges(pkg, ob, ctx):
+    rows, cols, m = 4105, 512, 60
+    ws = [make_weights(pkg, 3, rows, cols, 51 + i) for i in range(2)]
+    q = ob.quantize_act(3, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32))
+    outs = [ctx.alloc(m * rows * 4) for _ in ws]
+    ctx.matmul2(3, *outs, *[ctx.to_device(w) for w in ws], ctx.to_device(q.view(np.uint8)), m, rows, cols)
+    for o, w in zip(outs, ws):
+        assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), ob.matmul(ob.Pool(4), ob.detect_table(), 3, w, q, m, rows, cols), "pair")
+    ctx.device_status()
