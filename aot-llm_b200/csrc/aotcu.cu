@@ -1261,8 +1261,8 @@ static int gpu_qk_post(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos0,
 }
 
 // Positions whose scores fit shared memory: two CTAs per SM if that is enough, else one.
-static size_t attn_smem_bytes(int head_dim, size_t max_len) { return ((size_t)attn_fixed(head_dim) + max_len * ATTN_NQ) * sizeof(float); }
-static size_t attn_ctas(size_t m, int n_head, int n_kv_head) { return ((m * (n_head / n_kv_head) + ATTN_NQ - 1) / ATTN_NQ) * n_kv_head; }
+static size_t attn_smem_bytes(int nq, int head_dim, size_t max_len) { return ((size_t)attn_fixed(nq, head_dim) + max_len * nq) * sizeof(float); }
+static size_t attn_ctas(int nq, size_t m, int n_head, int n_kv_head) { return ((m * (n_head / n_kv_head) + nq - 1) / nq) * n_kv_head; }
 
 static int launch_attention(aotcu_ctx* c, float* out, const float* q, const float* kc, const float* vc, float* scratch,
                             const int* pos_ptr, size_t pos0, size_t m, int n_head, int n_kv_head, int head_dim,
@@ -1287,25 +1287,32 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
   ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim must be a multiple of 4, at most 256");
   // Scores in shared memory when the longest row of this call fits, else in `scratch`.
   const size_t max_len = pos_ptr ? n_ctx : std::min(n_ctx, pos0 + m);
-  size_t smem = attn_smem_bytes(head_dim, max_len);
+  // eight queries share a K element best; four, where eight leave SMs idle, halve the score and
+  // exponential phases (7 rows at position 300, 28 or 56 CTAs)
+  const int nq = attn_ctas(ATTN_NQ, m, n_head, n_kv_head) < (size_t)c->n_sm ? ATTN_NQ / 2 : ATTN_NQ;
+  size_t smem = attn_smem_bytes(nq, head_dim, max_len);
   const bool in_smem = smem <= c->max_smem;
   if (!in_smem) {
-    smem = attn_smem_bytes(head_dim, 0);
-    const size_t ctas = attn_ctas(m, n_head, n_kv_head);
+    smem = attn_smem_bytes(nq, head_dim, 0);
+    const size_t ctas = attn_ctas(nq, m, n_head, n_kv_head);
     if (!scratch) {  // the stand-alone entry point: scores in the context's conversion buffer
-      const int rc = ctx_workspace(c, ctas * n_ctx * ATTN_NQ * sizeof(float));
+      const int rc = ctx_workspace(c, ctas * n_ctx * nq * sizeof(float));
       if (rc) return rc < 0 ? rc : fail(AOTCU_ERR_UNSUPPORTED, "attention over %zu positions needs a score buffer, which cannot grow during a stream capture", max_len);
       P.scratch = reinterpret_cast<float*>(c->ximg);
     }
   }
   static bool attr_set[64] = {};
   if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
-    CU_TRY(cudaFuncSetAttribute(attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
-    CU_TRY(cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<true, ATTN_NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<false, ATTN_NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<true, ATTN_NQ / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    CU_TRY(cudaFuncSetAttribute(attention_kernel<false, ATTN_NQ / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
     attr_set[c->device] = true;
   }
-  const unsigned groups = (unsigned)((m * (n_head / n_kv_head) + ATTN_NQ - 1) / ATTN_NQ);
-  return launch(c, in_smem ? attention_kernel<true> : attention_kernel<false>, dim3((unsigned)n_kv_head, groups), dim3(ATTN_THREADS), smem, P);
+  const unsigned groups = (unsigned)(attn_ctas(nq, m, n_head, n_kv_head) / n_kv_head);
+  const auto kernel = nq == ATTN_NQ ? (in_smem ? attention_kernel<true, ATTN_NQ> : attention_kernel<false, ATTN_NQ>)
+                                    : (in_smem ? attention_kernel<true, ATTN_NQ / 2> : attention_kernel<false, ATTN_NQ / 2>);
+  return launch(c, kernel, dim3((unsigned)n_kv_head, groups), dim3(ATTN_THREADS), smem, P);
 }
 
 static int gpu_attention(aotcu_gpu* g, float* out, const float* q, size_t li, const int* pos_ptr, size_t pos0, size_t m,
@@ -2172,8 +2179,8 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   }
   // Attention scores: shared memory when the context fits, else a global scratch.
   {
-    if (attn_smem_bytes(d.head_dim, n_ctx) > c->max_smem)
-      G_TRY(cudaMalloc(&g->attn_scratch, attn_ctas(g->max_batch, d.n_head, d.n_kv_head) * n_ctx * ATTN_NQ * sizeof(float)));
+    if (attn_smem_bytes(ATTN_NQ, d.head_dim, n_ctx) > c->max_smem)
+      G_TRY(cudaMalloc(&g->attn_scratch, attn_ctas(ATTN_NQ, g->max_batch, d.n_head, d.n_kv_head) * n_ctx * ATTN_NQ * sizeof(float)));
   }
   g->history_cap = n_ctx;
   G_TRY(cudaMalloc(&g->d_step, 4 * sizeof(int)));

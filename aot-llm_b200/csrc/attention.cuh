@@ -16,7 +16,9 @@
 //  * the denominators of the eight queries are eight lanes' add chains in one warp.
 // Two CTAs share an SM, so one's chains and barriers run under the other's arithmetic.
 // 32 heads of 64 on 4 KV heads: 64 rows at position 448 took 53 us with one (row, head) pair per
-// CTA and take 40; 7 rows at position 300, where no phase fills the chip, 32.7 and 22.9.
+// CTA and take 40; 7 rows at position 300, where no phase fills the chip, 32.7 and 22.9,
+// and four pairs per CTA (ATTN_NQ / 2, taken where eight leave SMs idle) save 3.7 of those: a prompt
+// of 7 at 300 takes 1577 us instead of 1661.
 #pragma once
 #include "blockmath.cuh"
 #include "device_utils.cuh"
@@ -39,34 +41,36 @@ struct AttnParams {
   float scale, neg_zero; // neg_zero: -0.0f, from the host so that the compiler does not know it
 };
 
-constexpr int ATTN_NQ = 8;                       // queries per CTA
+constexpr int ATTN_NQ = 8;                       // queries per CTA, or half of them where that leaves SMs idle
 constexpr int ATTN_WARPS = 8, ATTN_THREADS = ATTN_WARPS * 32;
-static_assert(ATTN_WARPS == ATTN_NQ, "a warp loads a query");
+static_assert(ATTN_WARPS >= ATTN_NQ, "a warp loads a query");
 constexpr int ATTN_KD = 8;                       // dimensions of a staged K piece
 constexpr int ATTN_KRING = 4;                    // pieces in a warp's ring
 constexpr int ATTN_KPITCH = ATTN_KD + 4;         // floats per position: eight lanes' 16-byte reads fall on different banks
 constexpr int ATTN_KBUF = 32 * ATTN_KPITCH;      // floats of one piece
 constexpr int ATTN_STAGE = ATTN_WARPS * ATTN_KRING * ATTN_KBUF;  // floats of the staging area (K pieces of all warps, then V chunks)
 // floats besides the scores
-__host__ __device__ inline int attn_fixed(int head_dim) { return ATTN_STAGE + ATTN_NQ * head_dim + ATTN_WARPS * ATTN_NQ + ATTN_NQ; }
+__host__ __device__ inline int attn_fixed(int nq, int head_dim) { return ATTN_STAGE + nq * head_dim + ATTN_WARPS * nq + nq; }
 
 // SM: the scores are in shared memory (a pointer that could be either costs generic loads).
-template <bool SM>
+template <bool SM, int NQ>
 __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnParams P) {
+  static_assert(NQ == 4 || NQ == 8, "");
+  constexpr int NH = NQ / 4;  // groups of four queries
   extern __shared__ __align__(16) float sm_f[];
   __shared__ uint64_t exp_tab[32];
   // [staging][queries: dim x 4 pairs][maxima per warp][1 / denominator][scores: position x 8]
   float* const stage = sm_f;
   float* const qp = stage + ATTN_STAGE;
-  float* const red = qp + ATTN_NQ * P.head_dim;
-  float* const inv = red + ATTN_WARPS * ATTN_NQ;
+  float* const red = qp + NQ * P.head_dim;
+  float* const inv = red + ATTN_WARPS * NQ;
   pdl_launch_dependents();
   exp_table_load(exp_tab);
   pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hd = P.head_dim, kv_dim = P.n_kv_head * hd, q_dim = P.n_head * hd, gqa = P.n_head / P.n_kv_head;
-  const int kvh = blockIdx.x, n_query = P.m * gqa, q0 = blockIdx.y * ATTN_NQ, nq = min(ATTN_NQ, n_query - q0);
-  float* const sc = SM ? sm_f + attn_fixed(P.head_dim) : P.scratch + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * P.ctx * ATTN_NQ;
+  const int kvh = blockIdx.x, n_query = P.m * gqa, q0 = blockIdx.y * NQ, nq = min(NQ, n_query - q0);
+  float* const sc = SM ? sm_f + attn_fixed(NQ, P.head_dim) : P.scratch + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * P.ctx * NQ;
   const int base = P.pos_ptr ? *P.pos_ptr : P.pos0;
   const int row_a = q0 / gqa, row_b = (q0 + nq - 1) / gqa;
   // positions [T0, N) are the union of the queries' ranges, [T1, N1) lie in every one of them
@@ -101,26 +105,26 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
 #pragma unroll
   for (int i = 0; i < ATTN_KRING - 1; i++) stage_k();
   // the queries, two by two per dimension (missing ones repeat the last)
-  {
+  if (warp < NQ) {
     const int qi = q0 + min(warp, nq - 1), row = qi / gqa;  // a warp per query
     const float* src = P.q + (size_t)row * q_dim + (kvh * gqa + qi - row * gqa) * hd;
-    for (int d = lane; d < hd; d += 32) qp[d * ATTN_NQ + warp] = src[d];
+    for (int d = lane; d < hd; d += 32) qp[d * NQ + warp] = src[d];
   }
   __syncthreads();
-  float mx[ATTN_NQ];
+  float mx[NQ];
 #pragma unroll
-  for (int q = 0; q < ATTN_NQ; q++) mx[q] = -INFINITY;
+  for (int q = 0; q < NQ; q++) mx[q] = -INFINITY;
   int buf = 0;
   for (int blk = warp; blk < n_block; blk += ATTN_WARPS) {
-    F2 s[ATTN_NQ / 2];
+    F2 s[NQ / 2];
 #pragma unroll
-    for (int p = 0; p < ATTN_NQ / 2; p++) s[p] = 0ull;
+    for (int p = 0; p < NQ / 2; p++) s[p] = 0ull;
     for (int piece = 0; piece < n_piece; piece++) {
       stage_k();
       cp_async_wait<ATTN_KRING - 1>();
       __syncwarp();
       const float* kt = kb + buf * ATTN_KBUF + lane * ATTN_KPITCH;
-      const float4* q4 = reinterpret_cast<const float4*>(qp + piece * ATTN_KD * ATTN_NQ);
+      const float4* q4 = reinterpret_cast<const float4*>(qp + piece * ATTN_KD * NQ);
       const int n4 = min(ATTN_KD, hd - piece * ATTN_KD) >> 2;
 #pragma unroll 2
       for (int j = 0; j < n4; j++) {
@@ -128,12 +132,13 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
         const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          const float4 a = q4[2 * (4 * j + e)], b = q4[2 * (4 * j + e) + 1];
           const F2 k2 = f2_pack(kk[e], kk[e]);
-          s[0] = f2_add(s[0], f2_fma(f2_pack(a.x, a.y), k2, nz));
-          s[1] = f2_add(s[1], f2_fma(f2_pack(a.z, a.w), k2, nz));
-          s[2] = f2_add(s[2], f2_fma(f2_pack(b.x, b.y), k2, nz));
-          s[3] = f2_add(s[3], f2_fma(f2_pack(b.z, b.w), k2, nz));
+#pragma unroll
+          for (int g = 0; g < NH; g++) {
+            const float4 a = q4[NH * (4 * j + e) + g];
+            s[2 * g] = f2_add(s[2 * g], f2_fma(f2_pack(a.x, a.y), k2, nz));
+            s[2 * g + 1] = f2_add(s[2 * g + 1], f2_fma(f2_pack(a.z, a.w), k2, nz));
+          }
         }
       }
       __syncwarp();  // every lane has read the buffer that is filled next
@@ -141,25 +146,25 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
     }
     const int t = blk * 32 + lane;
     if (t < len) {
-      float v[ATTN_NQ];
+      float v[NQ];
 #pragma unroll
-      for (int p = 0; p < ATTN_NQ / 2; p++) f2_unpack(f2_mul(s[p], scale2), v[2 * p], v[2 * p + 1]);
+      for (int p = 0; p < NQ / 2; p++) f2_unpack(f2_mul(s[p], scale2), v[2 * p], v[2 * p + 1]);
       const bool all = T0 + t >= T1 && T0 + t < N1;
 #pragma unroll
-      for (int q = 0; q < ATTN_NQ; q++) {
+      for (int q = 0; q < NQ; q++) {
         if (!all && !in_range(q, T0 + t)) v[q] = -INFINITY;
         mx[q] = fmaxf(mx[q], v[q]);
       }
-      *reinterpret_cast<float4*>(sc + (size_t)t * ATTN_NQ) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4*>(sc + (size_t)t * ATTN_NQ + 4) = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+      for (int g = 0; g < NH; g++) *reinterpret_cast<float4*>(sc + (size_t)t * NQ + 4 * g) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int q = 0; q < ATTN_NQ; q++) {
+  for (int q = 0; q < NQ; q++) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx[q] = fmaxf(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
-    if (lane == 0) red[warp * ATTN_NQ + q] = mx[q];
+    if (lane == 0) red[warp * NQ + q] = mx[q];
   }
   __syncthreads();
   // V rows of positions [c0, c0 + v_chunk) of the union, into one of two buffers
@@ -177,16 +182,16 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
   stage_v(0, 0);
 
   // ---- softmax (ops.rs:98-112): exp, the denominators in position order, the scaled weights ----
-  const int half = tid & 1;  // this thread's four queries
+  const int half = NH == 2 ? tid & 1 : 0;  // this thread's four queries
   {
     float m4[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       m4[q] = red[4 * half + q];
 #pragma unroll
-      for (int w = 1; w < ATTN_WARPS; w++) m4[q] = fmaxf(m4[q], red[w * ATTN_NQ + 4 * half + q]);
+      for (int w = 1; w < ATTN_WARPS; w++) m4[q] = fmaxf(m4[q], red[w * NQ + 4 * half + q]);
     }
-    for (int i = tid; i < 2 * len; i += ATTN_THREADS) {
+    for (int i = tid; i < NH * len; i += ATTN_THREADS) {
       float4 v = reinterpret_cast<float4*>(sc)[i];
       v.x = expf_exact(fsub(v.x, m4[0]), exp_tab);
       v.y = expf_exact(fsub(v.y, m4[1]), exp_tab);
@@ -196,17 +201,17 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
     }
   }
   __syncthreads();
-  if (tid < ATTN_NQ) {
+  if (tid < NQ) {
     // positions outside the query's range are +0; eight terms load under the chain of the eight before
     float s = 0.0f, v[8], w[8];
     const float* p = sc + tid;
     auto load = [&](float (&x)[8], int t) {
       if (t + 8 <= len) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = p[(size_t)(t + j) * ATTN_NQ];
+        for (int j = 0; j < 8; j++) x[j] = p[(size_t)(t + j) * NQ];
       } else {
 #pragma unroll
-        for (int j = 0; j < 8; j++) x[j] = t + j < len ? p[(size_t)(t + j) * ATTN_NQ] : 0.0f;
+        for (int j = 0; j < 8; j++) x[j] = t + j < len ? p[(size_t)(t + j) * NQ] : 0.0f;
       }
     };
     load(v, 0);
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
   __syncthreads();
   {
     const float4 f = reinterpret_cast<const float4*>(inv)[half];
-    for (int i = tid; i < 2 * len; i += ATTN_THREADS) {
+    for (int i = tid; i < NH * len; i += ATTN_THREADS) {
       float4 v = reinterpret_cast<float4*>(sc)[i];
       v.x = fmul(v.x, f.x);
       v.y = fmul(v.y, f.y);
@@ -235,11 +240,15 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
   }
 
   // ---- out[d] = sum_t a_t * v_t[d], t in order (ops.rs:208-214) ----
-  // task = (32 dimensions, four queries); a warp takes tasks warp and warp + 8
-  const int n_task = 2 * ((hd + 31) >> 5);
-  F2 o[2][2];
+  // task = (32 dimensions, half of the queries); a warp takes tasks warp and warp + 8 (tasks of two
+  // queries out of eight keep more warps busy, and cost a full chip 1 % of a prompt)
+  constexpr int NT = 2, NG = 2, QT = NQ / NG, PAIRS = QT / 2;
+  const int n_task = NG * ((hd + 31) >> 5);
+  F2 o[NT][PAIRS];
 #pragma unroll
-  for (int k = 0; k < 2; k++) o[k][0] = o[k][1] = 0ull;
+  for (int k = 0; k < NT; k++)
+#pragma unroll
+    for (int i = 0; i < PAIRS; i++) o[k][i] = 0ull;
   for (int c0 = 0, ci = 0; c0 < len; c0 += vch, ci++) {
     const int cn = min(vch, len - c0);
     if (c0 + vch < len) {
@@ -250,56 +259,66 @@ __global__ void __launch_bounds__(ATTN_THREADS, 2) attention_kernel(const AttnPa
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const int task = warp + k * ATTN_WARPS, d = (task >> 1) * 32 + lane, g4 = task & 1;
+    for (int k = 0; k < NT; k++) {
+      const int task = warp + k * ATTN_WARPS, d = (task >> 1) * 32 + lane, g = task & 1;
       if (task < n_task) {
         const float* v = stage + (ci & 1) * vch * hd + min(d, hd - 1);
-        const float4* a = reinterpret_cast<const float4*>(sc + (size_t)c0 * ATTN_NQ) + g4;
+        const float* a = sc + (size_t)c0 * NQ + g * QT;
+        const float4* a4 = reinterpret_cast<const float4*>(sc + (size_t)c0 * NQ) + g;
+        const float2* a2 = reinterpret_cast<const float2*>(sc + (size_t)c0 * NQ) + g;
         // positions of every query's range (outside it a query adds nothing: a value there may
         // not even be finite)
         const int ta = max(0, min(cn, T1 - T0 - c0)), tb = max(ta, min(cn, N1 - T0 - c0));
         auto edge = [&](int from, int to) {
           for (int t = from; t < to; t++) {
-            const float4 w = a[2 * t];
             const float x = v[t * hd];
-            float r[4];
-            f2_unpack(o[k][0], r[0], r[1]);
-            f2_unpack(o[k][1], r[2], r[3]);
-            const float wq[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-              if (in_range(4 * g4 + q, T0 + c0 + t)) r[q] = fadd(r[q], fmul(wq[q], x));
-            o[k][0] = f2_pack(r[0], r[1]);
-            o[k][1] = f2_pack(r[2], r[3]);
+            for (int i = 0; i < PAIRS; i++) {
+              float r[2];
+              f2_unpack(o[k][i], r[0], r[1]);
+#pragma unroll
+              for (int q = 0; q < 2; q++)
+                if (in_range(g * QT + 2 * i + q, T0 + c0 + t)) r[q] = fadd(r[q], fmul(a[t * NQ + 2 * i + q], x));
+              o[k][i] = f2_pack(r[0], r[1]);
+            }
           }
         };
         edge(0, ta);
-        F2 o0 = o[k][0], o1 = o[k][1];
+        F2 p[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; i++) p[i] = o[k][i];
 #pragma unroll 8
         for (int t = ta; t < tb; t++) {
-          const float4 w = a[2 * t];
-          const F2 x = f2_pack(v[t * hd], v[t * hd]);
-          o0 = f2_add(o0, f2_fma(f2_pack(w.x, w.y), x, nz));
-          o1 = f2_add(o1, f2_fma(f2_pack(w.z, w.w), x, nz));
+          if (QT == 4) {
+            const float4 w = a4[(NQ / 4) * t];
+            const F2 x = f2_pack(v[t * hd], v[t * hd]);
+            p[0] = f2_add(p[0], f2_fma(f2_pack(w.x, w.y), x, nz));
+            p[PAIRS - 1] = f2_add(p[PAIRS - 1], f2_fma(f2_pack(w.z, w.w), x, nz));
+          } else {
+            const float2 w = a2[(NQ / 2) * t];
+            p[0] = f2_add(p[0], f2_fma(f2_pack(w.x, w.y), f2_pack(v[t * hd], v[t * hd]), nz));
+          }
         }
-        o[k][0] = o0;
-        o[k][1] = o1;
+#pragma unroll
+        for (int i = 0; i < PAIRS; i++) o[k][i] = p[i];
         edge(tb, cn);
       }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const int task = warp + k * ATTN_WARPS, d = (task >> 1) * 32 + lane, g4 = task & 1;
+  for (int k = 0; k < NT; k++) {
+    const int task = warp + k * ATTN_WARPS, d = (task >> 1) * 32 + lane, g = task & 1;
     if (task < n_task && d < hd) {
-      float r[4];
-      f2_unpack(o[k][0], r[0], r[1]);
-      f2_unpack(o[k][1], r[2], r[3]);
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int qi = q0 + 4 * g4 + q, row = qi / gqa;
-        if (qi < n_query) P.out[(size_t)row * q_dim + (kvh * gqa + qi - row * gqa) * hd + d] = r[q];
+      for (int i = 0; i < PAIRS; i++) {
+        float r[2];
+        f2_unpack(o[k][i], r[0], r[1]);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const int qi = q0 + g * QT + 2 * i + q, row = qi / gqa;
+          if (qi < n_query) P.out[(size_t)row * q_dim + (kvh * gqa + qi - row * gqa) * hd + d] = r[q];
+        }
       }
     }
   }
