@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
     (6, 2, 20, 700, [(1, 699, 0), (11, 600, 0), (64, 300, 77)]),     # three heads per group, a partial piece
     (1, 1, 256, 300, [(1, 0, 0), (9, 290, 33)]),                      # one query per row, widest heads
     (24, 2, 64, 260, [(3, 0, 0), (5, 255, 0)]),                       # twelve heads per group: two CTAs a row
-    (4, 1, 32, 6200, [(1, 6100, 0), (3, 6190, 0), (2, 6000, 5900)]),  # scores in global memory
+    (4, 1, 32, 6200, [(1, 6100, 0), (3, 6190, 0), (2, 6000, 5900)]),  # few CTAs: four queries each
+    (4, 1, 32, 12000, [(3, 11990, 0)]),                               # the same, scores in global memory
+    (32, 4, 16, 6200, [(64, 6130, 0), (40, 6100, 3000)]),             # eight queries each, scores in global memory
 ])
 def test_attention_paths(pkg, ob, ctx, n_head, n_kv, hd, ctxlen, calls):
     rng = np.random.default_rng(hd)
