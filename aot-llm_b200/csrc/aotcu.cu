@@ -593,7 +593,12 @@ static int launch_float_multi_t(aotcu_ctx* c, const FloatMultiParams& P, int gri
     CU_TRY(cudaFuncSetAttribute(float_multi_kernel<KIND, R, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
     attr_set[c->device] = true;
   }
-  return launch(c, float_multi_kernel<KIND, R, T>, dim3(grid), dim3(32 * P.wt), (size_t)FM_STAGES * FmShape<KIND, R, T>::stage_bytes(P.wt), P);
+  size_t smem = (size_t)FM_STAGES * FmShape<KIND, R, T>::stage_bytes(P.wt);
+  // A grid of one CTA per SM asks for more than half of an SM's shared memory: launched while its
+  // predecessor ends, its first CTAs would otherwise pair up on the SMs that are free by then
+  // (bf16 4096x4096, 37 rows, back to back: 60 us or 81).
+  if (grid <= c->n_sm) smem = std::max(smem, c->max_smem / 2 + 1024);
+  return launch(c, float_multi_kernel<KIND, R, T>, dim3(grid), dim3(32 * P.wt), smem, P);
 }
 template <int KIND, int R>
 static int launch_float_multi_r(aotcu_ctx* c, const FloatMultiParams& P, int t, int grid) {
@@ -618,10 +623,10 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
   P.m = (int)call.m;
   P.epilogue = call.pair ? EPI_STORE : call.epilogue;
   P.x = reinterpret_cast<const float*>(call.x);
-  // Shape: R weight rows and T activation rows per lane, wt warps per CTA. Fitted to 116 timings
-  // over eight matrices and batches of 2 to 64: a step of eight columns takes a scheduler about
-  // 20 + 4 R T cycles per warp that it holds, and 50 + 8 R T if it holds few; the fullest
-  // scheduler's share (a CTA's warps go to schedulers in turn) counts for a quarter.
+  // Shape: R weight rows and T activation rows per lane, wt warps per CTA (all of the batch's up to
+  // eight, or four). Fitted to timings of twelve matrices and batches of 2 to 64 at every shape: a
+  // step of eight columns takes a scheduler about 20 + 3 R T + 4 T cycles per warp that it holds,
+  // and 50 + 6 R T if it holds few; CTAs of three warps leave one scheduler idle.
   int r_best = 2, t_best = 2;
   size_t grid = 0;
   double best = 1e30;
@@ -630,10 +635,10 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
     for (int s = 0; s < call.nseg; s++) tiles += (call.seg[s].rows + 8 * r - 1) / (8 * r);
     for (int t : {2, 4, 5, 8}) {
       const size_t nw = (call.m + t - 1) / t;
-      for (int k = FM_MAX_WARPS; k >= 1; k--) {
-        const size_t nc = (nw + k - 1) / k, wt = (nw + nc - 1) / nc, per_sm = (tiles * nc + c->n_sm - 1) / c->n_sm;
-        const double warps = 0.75 * (double)(tiles * nc * wt) / (4 * c->n_sm) + 0.25 * (double)(per_sm * ((wt + 3) / 4));
-        const double cost = std::max(warps * (20 + 4 * r * t), 50.0 + 8 * r * t);
+      for (int k : {FM_MAX_WARPS, 4}) {
+        const size_t nc = (nw + k - 1) / k, wt = (nw + nc - 1) / nc;
+        const double warps = (double)(tiles * nc * wt) / (4 * c->n_sm) * (wt == 3 ? 1.15 : 1.0);
+        const double cost = std::max(warps * (20 + 3 * r * t + 4 * t), 50.0 + 6 * r * t);
         if (cost < best * 0.999 && tiles * nc < (1u << 30)) {
           best = cost;
           r_best = r;
