@@ -120,11 +120,19 @@ __device__ __forceinline__ void xf_store(uint8_t* o, int g, int lane, uint32_t w
     reinterpret_cast<__half*>(o + XF_BSUMS + (g * 4 + ((lane & 7) >> 1)) * 8)[(lane >> 3) * 2 + (lane & 1)] = __int2half_rn(bsum);
   if (lane == 0) *reinterpret_cast<float*>(o + XF_D + 4 * g) = d;
 }
-// Block b of row `tok` (of nt groups of 8 rows), quantized straight into that order.
-__device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, int tok, int b, int nt) {
+// Block b of row `tok` (of nt groups of 8 rows), quantized straight into that order. `wide`: src is
+// 16-byte aligned (a buffer read at an offset of the caller's need not be).
+__device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, int tok, int b, int nt, bool wide) {
   const int lane = threadIdx.x & 31;
-  const float4 a = reinterpret_cast<const float4*>(src)[2 * lane], c = reinterpret_cast<const float4*>(src)[2 * lane + 1];
-  const float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+  float v[8];
+  if (wide) {
+    const float4 a = reinterpret_cast<const float4*>(src)[2 * lane], c = reinterpret_cast<const float4*>(src)[2 * lane + 1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = src[8 * lane + i];
+  }
   const Q8kLane r = warp_q8k_lane(v);
   const int s2 = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
   const int bs = __shfl_sync(0xffffffffu, s2, (2 * lane) & 31);
@@ -177,7 +185,8 @@ __global__ void quantize_xf_kernel(const float* __restrict__ x, uint8_t* __restr
   pdl_launch_dependents();
   pdl_wait();
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5, nt = (m + 7) >> 3;
-  for (int i = wid; i < m * nb; i += nw) warp_quantize_xf(x + (size_t)i * 256, xf, i / nb, i % nb, nt);
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // blocks lie 1024 bytes apart
+  for (int i = wid; i < m * nb; i += nw) warp_quantize_xf(x + (size_t)i * 256, xf, i / nb, i % nb, nt, wide);
 }
 __global__ void quantize_q80_kernel(const float* __restrict__ x, uint8_t* __restrict__ out, int n_blocks, int image) {
   pdl_launch_dependents();
@@ -250,7 +259,7 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   if (P.q8k_out) {
     int nb = P.n / 256;
     for (int b = warp; b < nb; b += nwarps) {
-      if (P.xf_nt) warp_quantize_xf(row + b * 256, P.q8k_out, blockIdx.x, b, P.xf_nt);
+      if (P.xf_nt) warp_quantize_xf(row + b * 256, P.q8k_out, blockIdx.x, b, P.xf_nt, true);
       else warp_quantize_q8k(row + b * 256, P.q8k_out + ((size_t)blockIdx.x * nb + b) * XIMG_K, 1);
     }
   }

@@ -1,0 +1,41 @@
+"""Operator calls on parts of a buffer: offsets and row lengths that the step itself never uses.
+Bit-exact against the CPU oracle (batched == per-token, crates/aot-kernels/tests/dots.rs:205-266)."""
+import numpy as np
+import pytest
+
+from conftest import assert_bits_equal, make_weights
+
+pytestmark = pytest.mark.gpu
+
+KINDS = [0, 1, 5, 6, 8]  # F32, F16, Q8_0, Q4_K, Q6_K
+
+
+def _model_with(pkg, ctx, mats, n_ctx, max_batch):
+    """A small model whose tensor section also holds `mats` ((kind, rows, cols) each)."""
+    spec = pkg.model.tiny("llama", n_layer=1)
+    parts, off, out = [spec.weights], spec.weights.size, []
+    for kind, rows, cols in mats:
+        w = make_weights(pkg, kind, rows, cols, 61 + kind + cols)
+        pad = -off % 32
+        parts += [np.zeros(pad, dtype=np.uint8), w]
+        out.append((w, pkg.lib.Tensor(kind=kind, present=1, off=off + pad, len=w.size, rows=rows, cols=cols)))
+        off += pad + w.size
+    return pkg.Gpu(ctx, spec.head, spec.layers, np.concatenate(parts), n_ctx, max_batch), out
+
+
+def _want(ob, kind, w, x, m, rows, cols):
+    return ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, ob.quantize_act(kind, x), m, rows, cols)
+
+
+@pytest.mark.parametrize("src_off,dst_off", [(0, 0), (1, 3), (2, 0), (4, 1)])
+def test_matmul_of_a_part_of_a_buffer(pkg, ob, ctx, src_off, dst_off):
+    rows, cols = 48, 512
+    g, mats = _model_with(pkg, ctx, [(k, rows, cols) for k in KINDS], 16, 16)
+    for (w, t), kind in zip(mats, KINDS):
+        for m in (1, 2, 9):
+            x = np.random.default_rng(kind + m).standard_normal(m * cols).astype(np.float32)
+            g.write("Bhb", x, src_off)
+            g.matmul("Bq", t, "Bhb", m, src_off=src_off, dst_off=dst_off)
+            assert_bits_equal(g.read("Bq", m * rows, dst_off).reshape(m, rows), _want(ob, kind, w, x, m, rows, cols), f"kind {kind} m {m} at {src_off}")
+    g.finish()
+    g.close()
