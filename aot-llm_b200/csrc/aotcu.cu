@@ -979,8 +979,9 @@ struct aotcu_gpu {
   size_t buf_len[AOTCU_N_BUFS] = {};
   float* rope_table = nullptr;        // n_ctx x rot_dim
   float* rope_table_local = nullptr;  // swa layers
-  uint8_t* aqk = nullptr;             // Q8_K block images, max_batch rows of max(dim, q_dim, hidden)
+  uint8_t* aqk = nullptr;             // Q8_K block images or fragments, max_batch rows of max(dim, q_dim, hidden)
   uint8_t* aq0 = nullptr;             // Q8_0 block images
+  size_t aqk_bytes = 0, aq0_bytes = 0;
   float* attn_scratch = nullptr;      // scores for contexts that do not fit shared memory
   int* d_step = nullptr;              // {token, pos, n_generated}
   int* d_tokens = nullptr;            // prompt batch ids
@@ -1052,10 +1053,18 @@ static void note_write(aotcu_gpu* g, const float* p) {
   if (p == g->bufs[AOTCU_BUF_LOGITS]) g->h_logits_fresh = false;  // the host copy made by aotcu_forward is stale
 }
 
-// Make sure the block images of `src` (m rows of n floats) exist for `act`.
 // Q8_K activations of several rows are kept in the fragment order of kmma.cuh, those of a single
-// row (and of chunks sent to the tcgen05 kernels) as block images.
-static bool xf_rows(size_t m) { return m >= 2 && g_tc_force <= 0; }
+// row (and of chunks sent to the tcgen05 kernels) as block images. Fragments come in whole groups of
+// eight rows, so a few rows that are longer than any of the model's (operator calls) may fit the
+// buffer as images only.
+static bool xf_rows(const aotcu_gpu* g, size_t n, size_t m) {
+  return m >= 2 && g_tc_force <= 0 && (m + 7) / 8 * (n / 256) * XF_BLOCK <= g->aqk_bytes;
+}
+static bool images_fit(const aotcu_gpu* g, int act, size_t n, size_t m) {
+  return act == ACT_Q8_K ? n / 256 * m * XIMG_K <= g->aqk_bytes : n / 32 * m * XIMG_0 <= g->aq0_bytes;
+}
+
+// Make sure the quantized form of `src` (m rows of n floats) exists for `act`.
 static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, int act) {
   if (act == ACT_F32) return 0;
   aotcu_ctx* c = g->c;
@@ -1066,19 +1075,22 @@ static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, 
     g->qsrc.n = n;
     g->qsrc.m = m;
   }
-  if (act == ACT_Q8_K && (!g->qsrc.q8k || g->qsrc.xf != xf_rows(m))) {
+  const bool xf = act == ACT_Q8_K && xf_rows(g, n, m);
+  if (act == ACT_Q8_K && (!g->qsrc.q8k || g->qsrc.xf != xf)) {
     ARG_CHECK(n % 256 == 0, "row length %zu is not a multiple of 256", n);
+    ARG_CHECK(xf || images_fit(g, act, n, m), "%zu rows of %zu floats exceed the quantized-activation buffer", m, n);
     int nblk = (int)(n * m / 256);
-    if (xf_rows(m)) {
+    if (xf) {
       if (int rc = launch(c, quantize_xf_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, (int)m, (int)(n / 256))) return rc;
     } else {
       if (int rc = launch(c, quantize_q8k_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, nblk, 1)) return rc;
     }
     g->qsrc.q8k = true;
-    g->qsrc.xf = xf_rows(m);
+    g->qsrc.xf = xf;
   }
   if (act == ACT_Q8_0 && !g->qsrc.q80) {
     ARG_CHECK(n % 32 == 0, "row length %zu is not a multiple of 32", n);
+    ARG_CHECK(images_fit(g, act, n, m), "%zu rows of %zu floats exceed the quantized-activation buffer", m, n);
     int nblk = (int)(n * m / 32);
     if (int rc = launch(c, quantize_q80_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aq0, nblk, 1)) return rc;
     g->qsrc.q80 = true;
@@ -1086,7 +1098,8 @@ static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, 
   return 0;
 }
 
-static int act_mode(int act, size_t m) { return act == ACT_Q8_K && xf_rows(m) ? 2 : 1; }
+// How the activations of the last ensure_quantized lie (GemvCall::x_mode).
+static int act_mode(const aotcu_gpu* g, int act) { return act == ACT_Q8_K && g->qsrc.xf ? 2 : 1; }
 static const void* act_images(const aotcu_gpu* g, int act, const float* src) {
   return act == ACT_Q8_K ? (const void*)g->aqk : act == ACT_Q8_0 ? (const void*)g->aq0 : (const void*)src;
 }
@@ -1104,9 +1117,10 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   P.eps = eps;
   P.accumulate = accumulate;
   bool q = quantize && !accumulate && dst_stride == n;
-  P.q8k_out = (q && g->need_q8k && n % 256 == 0) ? g->aqk : nullptr;
-  P.q80_out = (q && g->need_q80 && n % 32 == 0) ? g->aq0 : nullptr;
-  P.xf_nt = P.q8k_out && xf_rows(m) ? (int)((m + 7) / 8) : 0;
+  const bool xf = xf_rows(g, n, m);
+  P.q8k_out = (q && g->need_q8k && n % 256 == 0 && (xf || images_fit(g, ACT_Q8_K, n, m))) ? g->aqk : nullptr;
+  P.q80_out = (q && g->need_q80 && n % 32 == 0 && images_fit(g, ACT_Q8_0, n, m)) ? g->aq0 : nullptr;
+  P.xf_nt = P.q8k_out && xf ? (int)((m + 7) / 8) : 0;
   size_t smem = (2 * n + 12) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "rmsnorm row of %zu floats does not fit shared memory", n);
   note_write(g, dst);
@@ -1170,7 +1184,7 @@ static int gpu_matmul(aotcu_gpu* g, float* dst, const aotcu_tensor& t, const flo
   call.nseg = 1;
   call.cols = t.cols;
   call.x = act_images(g, act, src);
-  call.x_mode = act_mode(act, m);
+  call.x_mode = act_mode(g, act);
   call.m = m;
   call.epilogue = accumulate ? EPI_ACCUM : EPI_STORE;
   call.prep[0] = prep_of(g, t, m);
@@ -1200,7 +1214,7 @@ static int gpu_mv3(aotcu_gpu* g, float* const dst[3], const aotcu_tensor* const 
     if (int rc = ensure_quantized(g, src, t[a]->cols, m, act)) return rc;
     call.cols = t[a]->cols;
     call.x = act_images(g, act, src);
-    call.x_mode = act_mode(act, m);
+    call.x_mode = act_mode(g, act);
     call.m = m;
     if (int rc = launch_gemv(g->c, call)) return rc;
   }
@@ -1221,7 +1235,7 @@ static int gpu_gate_up(aotcu_gpu* g, float* hb, float* hb2, const aotcu_tensor& 
     call.pair = 1;
     call.cols = gate.cols;
     call.x = act_images(g, act, src);
-    call.x_mode = act_mode(act, m);
+    call.x_mode = act_mode(g, act);
     call.m = m;
     call.epilogue = gelu ? EPI_STORE : EPI_SILU_MUL;
     call.prep[0] = prep_of(g, gate, m);
@@ -2178,9 +2192,11 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   {
     size_t widest = xbw > (size_t)d.hidden ? xbw : (size_t)d.hidden;
     size_t rows = g->max_batch;
-    G_TRY(cudaMalloc(&g->aqk, ((rows + 7) / 8) * (widest / 256 + 1) * 8 * XIMG_K));  // whole groups of 8 rows (XF_BLOCK <= 8 * XIMG_K)
-    G_TRY(cudaMemsetAsync(g->aqk, 0, ((rows + 7) / 8) * (widest / 256 + 1) * 8 * XIMG_K, c->stream));
-    G_TRY(cudaMalloc(&g->aq0, rows * (widest / 32 + 1) * XIMG_0));
+    g->aqk_bytes = ((rows + 7) / 8) * (widest / 256 + 1) * 8 * XIMG_K;  // whole groups of 8 rows (XF_BLOCK <= 8 * XIMG_K)
+    g->aq0_bytes = rows * (widest / 32 + 1) * XIMG_0;
+    G_TRY(cudaMalloc(&g->aqk, g->aqk_bytes));
+    G_TRY(cudaMemsetAsync(g->aqk, 0, g->aqk_bytes, c->stream));
+    G_TRY(cudaMalloc(&g->aq0, g->aq0_bytes));
   }
   // Attention scores: shared memory when the context fits, else a global scratch.
   {

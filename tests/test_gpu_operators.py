@@ -39,3 +39,29 @@ def test_matmul_of_a_part_of_a_buffer(pkg, ob, ctx, src_off, dst_off):
             assert_bits_equal(g.read("Bq", m * rows, dst_off).reshape(m, rows), _want(ob, kind, w, x, m, rows, cols), f"kind {kind} m {m} at {src_off}")
     g.finish()
     g.close()
+
+
+def test_rows_longer_than_any_of_the_model(pkg, ob, ctx):
+    """Quantized rows that do not fit the activation buffer in groups of eight, or not at all."""
+    cases = [(6, 48, 4096, 2), (8, 2800, 2560, 3), (6, 48, 768, 9), (5, 48, 4096, 2)]
+    too_long = [(6, 4, 16384), (5, 4, 16384)]
+    g, mats = _model_with(pkg, ctx, [c[:3] for c in cases] + too_long, 256, 16)
+    for (kind, rows, cols, m), (w, t) in zip(cases, mats):
+        x = np.random.default_rng(cols).standard_normal(m * cols).astype(np.float32)
+        g.write("Bhb", x)
+        g.matmul("KCache", t, "Bhb", m)
+        assert_bits_equal(g.read("KCache", m * rows).reshape(m, rows), _want(ob, kind, w, x, m, rows, cols), f"kind {kind} {rows}x{cols} m {m}")
+    for _, t in mats[len(cases):]:
+        with pytest.raises(pkg.AotCudaError) as e:
+            g.matmul("Q", t, "KCache")
+        assert e.value.status == pkg.lib.ERR_BAD_ARG
+    # a norm of such a row is computed, and not quantized
+    n = 16384
+    g2, [(w, t)] = _model_with(pkg, ctx, [(0, 1, n)], 256, 16)
+    x = np.random.default_rng(3).standard_normal(n).astype(np.float32)
+    g2.write("KCache", x)
+    g2.rmsnorm("VCache", "KCache", t, n, 1, 1e-5)
+    assert_bits_equal(g2.read("VCache", n), ob.rmsnorm(x, w.view(np.float32), 1e-5), "norm of a long row")
+    for h in (g, g2):
+        h.finish()
+        h.close()
