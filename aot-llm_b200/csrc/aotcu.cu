@@ -69,6 +69,7 @@ struct aotcu_ctx {
   std::vector<struct aotcu_gpu*> gpus;  // live Gpus of this context (freed with it)
   uint8_t* ximg = nullptr;              // activations converted from reference-layout blocks (ctx_workspace)
   size_t ximg_bytes = 0;
+  size_t ximg_limit = SIZE_MAX;         // option "workspace_mib"
 };
 
 constexpr size_t WEIGHT_PAD = 256;
@@ -276,10 +277,12 @@ static int launch_gemv_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   return 0;
 }
 
-// The context's conversion buffer, at least `need` bytes: kept from call to call, grown on demand
-// (not during a stream capture: 1 then, and the caller takes a path without it).
+// The context's conversion buffer, at least `need` bytes: kept from call to call, grown on demand.
+// 1 where it cannot grow (during a stream capture, above its limit, or when the device's memory is
+// handed out): the caller takes a path without it.
 static int ctx_workspace(aotcu_ctx* c, size_t need) {
   if (need <= c->ximg_bytes) return 0;
+  if (need > c->ximg_limit) return 1;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CU_TRY(cudaStreamIsCapturing(c->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return 1;
@@ -287,14 +290,20 @@ static int ctx_workspace(aotcu_ctx* c, size_t need) {
   if (c->ximg) cudaFree(c->ximg);
   c->ximg = nullptr;
   c->ximg_bytes = 0;
-  CU_TRY(cudaMalloc(&c->ximg, need));
+  const cudaError_t e = cudaMalloc(&c->ximg, need);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    c->ximg = nullptr;
+    return 1;
+  }
+  CU_TRY(e);
   c->ximg_bytes = need;
   return 0;
 }
 
 // K-quant products of several activation rows on the int8 tensor-core kernel of kmma.cuh.
-// Activations that are not in its fragment order are converted first. Returns 1 when the call
-// does not fit.
+// Activations that are not in its fragment order are converted first. Returns 1 when there is no
+// buffer for that.
 template <int KIND, int RT, bool PAIR, int WK>
 static int launch_kmma_t(aotcu_ctx* c, KmmaParams& P, int grid) {
   using S = KmmaShape<KIND, RT, PAIR, WK>;
@@ -841,7 +850,7 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
       if (rc <= 0) return rc;  // 1: a pair or a very long row
     }
     const int rc = launch_kmma(c, call);
-    if (rc <= 0) return rc;  // 1: a conversion buffer would have to grow during a stream capture
+    if (rc <= 0) return rc;  // 1: no conversion buffer
   }
   if (act == ACT_Q8_0 && g_q80_chunks) {
     const int mc = launch_q80_mma(c, call, span);
@@ -1316,7 +1325,7 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
     const size_t ctas = attn_ctas(nq, m, n_head, n_kv_head);
     if (!scratch) {  // the stand-alone entry point: scores in the context's conversion buffer
       const int rc = ctx_workspace(c, ctas * n_ctx * nq * sizeof(float));
-      if (rc) return rc < 0 ? rc : fail(AOTCU_ERR_UNSUPPORTED, "attention over %zu positions needs a score buffer, which cannot grow during a stream capture", max_len);
+      if (rc) return rc < 0 ? rc : fail(AOTCU_ERR_UNSUPPORTED, "attention over %zu positions needs a score buffer, for which there is no memory", max_len);
       P.scratch = reinterpret_cast<float*>(c->ximg);
     }
   }
@@ -2715,6 +2724,19 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
     return 0;
   }
   if (!strcmp(name, "mega_available")) return g->mega_ok ? 1 : 0;
+  if (!strcmp(name, "workspace_mib")) {
+    // bound of the context's conversion buffer (no bound by default); a larger one is given back
+    ARG_CHECK(value >= 0, "workspace_mib must not be negative");
+    aotcu_ctx* const c = g->c;
+    c->ximg_limit = (size_t)value << 20;
+    if (c->ximg_bytes > c->ximg_limit) {
+      CU_TRY(cudaStreamSynchronize(c->stream));
+      CU_TRY(cudaFree(c->ximg));
+      c->ximg = nullptr;
+      c->ximg_bytes = 0;
+    }
+    return 0;
+  }
   if (!strcmp(name, "wide_rows")) {  // process-wide: rows per CTA from which single-row products use one lane per super-block
     ARG_CHECK(value >= 1, "wide_rows must be at least 1");
     g_wide_rows = value;

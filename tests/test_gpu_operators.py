@@ -65,3 +65,30 @@ def test_rows_longer_than_any_of_the_model(pkg, ob, ctx):
     for h in (g, g2):
         h.finish()
         h.close()
+
+
+@pytest.mark.parametrize("kind,rows,cols,ms", [(3, 8192, 256, (2, 64)), (4, 600, 1024, (17,)), (5, 8200, 512, (49,)),
+                                               (6, 2400, 512, (4, 65)), (7, 900, 1280, (12,)), (8, 2400, 768, (9,))])
+def test_products_without_a_conversion_buffer(pkg, ob, ctx, kind, rows, cols, ms):
+    """What a product does when the buffer for its activations cannot be had."""
+    g, _ = _model_with(pkg, ctx, [], 16, 2)  # only to reach the context's option
+    ws = [make_weights(pkg, kind, rows, cols, 71 + kind + i) for i in range(2)]
+    dws = [ctx.to_device(w) for w in ws]
+    try:
+        for limit in (0, 1 << 20):  # 1 << 20 MiB: as good as none
+            g.set_option("workspace_mib", limit)
+            for m in ms:
+                x = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+                q = ob.quantize_act(kind, x)
+                dq = ctx.to_device(q.view(np.uint8))
+                want = [ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols) for w in ws]
+                outs = [ctx.alloc(m * rows * 4) for _ in ws]
+                ctx.matmul(kind, outs[0], dws[0], dq, m, rows, cols)
+                assert_bits_equal(outs[0].download(np.float32, m * rows).reshape(m, rows), want[0], f"kind {kind} m {m} limit {limit}")
+                ctx.matmul2(kind, *outs, *dws, dq, m, rows, cols)
+                for i in range(2):
+                    assert_bits_equal(outs[i].download(np.float32, m * rows).reshape(m, rows), want[i], f"pair, kind {kind} m {m} limit {limit}")
+    finally:
+        g.set_option("workspace_mib", 1 << 20)
+        g.close()
+    ctx.device_status()
