@@ -1056,10 +1056,11 @@ static int tensor_check(const aotcu_gpu* g, const aotcu_tensor& t, const char* n
 static const uint8_t* wptr(const aotcu_gpu* g, const aotcu_tensor& t) { return g->d_weights + t.off; }
 static const float* wf32(const aotcu_gpu* g, const aotcu_tensor& t) { return reinterpret_cast<const float*>(g->d_weights + t.off); }
 
-static void note_write(aotcu_gpu* g, const float* p) {
-  // A write to the buffer whose quantized image is cached invalidates the image.
-  if (g->qsrc.ptr && p == g->qsrc.ptr) g->qsrc = aotcu_gpu::QSrc();
-  if (p == g->bufs[AOTCU_BUF_LOGITS]) g->h_logits_fresh = false;  // the host copy made by aotcu_forward is stale
+// A write of n floats at p: what was derived from them is stale.
+static void note_write(aotcu_gpu* g, const float* p, size_t n) {
+  auto meets = [&](const float* q, size_t len) { return q && p < q + len && q < p + n; };
+  if (meets(g->qsrc.ptr, g->qsrc.n * g->qsrc.m)) g->qsrc = aotcu_gpu::QSrc();  // the quantized form
+  if (meets(g->bufs[AOTCU_BUF_LOGITS], g->buf_len[AOTCU_BUF_LOGITS])) g->h_logits_fresh = false;  // the host copy made by aotcu_forward
 }
 
 // Q8_K activations of several rows are kept in the fragment order of kmma.cuh, those of a single
@@ -1132,7 +1133,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   P.xf_nt = P.q8k_out && xf ? (int)((m + 7) / 8) : 0;
   size_t smem = (2 * n + 12) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "rmsnorm row of %zu floats does not fit shared memory", n);
-  note_write(g, dst);
+  note_write(g, dst, (m - 1) * dst_stride + n);
   if (int rc = launch(c, rmsnorm_kernel, dim3((unsigned)m), dim3(512), smem, P)) return rc;
   if (q) {
     g->qsrc = aotcu_gpu::QSrc();
@@ -1197,7 +1198,7 @@ static int gpu_matmul(aotcu_gpu* g, float* dst, const aotcu_tensor& t, const flo
   call.m = m;
   call.epilogue = accumulate ? EPI_ACCUM : EPI_STORE;
   call.prep[0] = prep_of(g, t, m);
-  note_write(g, dst);
+  note_write(g, dst, m * t.rows);
   return launch_gemv(g->c, call);
 }
 
@@ -1217,7 +1218,7 @@ static int gpu_mv3(aotcu_gpu* g, float* const dst[3], const aotcu_tensor* const 
         call.prep[call.nseg] = prep_of(g, *t[b], m);
         call.seg[call.nseg++] = GemvSeg{wptr(g, *t[b]), dst[b], (int)t[b]->rows, t[b]->kind};
         done[b] = true;
-        note_write(g, dst[b]);
+        note_write(g, dst[b], m * t[b]->rows);
       }
     }
     if (int rc = ensure_quantized(g, src, t[a]->cols, m, act)) return rc;
@@ -1249,8 +1250,8 @@ static int gpu_gate_up(aotcu_gpu* g, float* hb, float* hb2, const aotcu_tensor& 
     call.epilogue = gelu ? EPI_STORE : EPI_SILU_MUL;
     call.prep[0] = prep_of(g, gate, m);
     call.prep[1] = prep_of(g, up, m);
-    note_write(g, hb);
-    note_write(g, hb2);
+    note_write(g, hb, m * gate.rows);
+    note_write(g, hb2, m * up.rows);
     if (int rc = launch_gemv(c, call)) return rc;
     if (!gelu) return 0;
     const size_t n = m * gate.rows;
@@ -1284,7 +1285,7 @@ static int gpu_qk_post(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos0,
   P.rot_dim = d.rot_dim;
   P.neox = d.rope_neox;
   P.eps = d.eps;
-  note_write(g, P.q);
+  note_write(g, P.q, m * d.n_head * d.head_dim);
   return launch(g->c, qk_post_kernel, dim3(d.n_head + d.n_kv_head, (unsigned)m), dim3(128), 0, P);
 }
 
@@ -1347,7 +1348,7 @@ static int gpu_attention(aotcu_gpu* g, float* out, const float* q, size_t li, co
                          size_t window) {
   const aotcu_dims& d = g->head.dims;
   size_t kvd = (size_t)d.n_kv_head * d.head_dim;
-  note_write(g, out);
+  note_write(g, out, m * d.n_head * d.head_dim);
   return launch_attention(g->c, out, q, g->bufs[AOTCU_BUF_KCACHE] + li * g->n_ctx * kvd,
                           g->bufs[AOTCU_BUF_VCACHE] + li * g->n_ctx * kvd, g->attn_scratch, pos_ptr, pos0, m, d.n_head,
                           d.n_kv_head, d.head_dim, g->n_ctx, window);
@@ -1360,7 +1361,7 @@ static int tp_all_reduce(aotcu_gpu* g, float* buf, size_t n) {
   TpState* t = g->tp;
   const int r = t->all_reduce(buf, buf, n, NCCL_FLOAT32, NCCL_SUM, t->comm, g->c->stream);
   if (r != 0) return fail(AOTCU_ERR_CUDA, "ncclAllReduce: %s", t->get_error_string(r));
-  note_write(g, buf);
+  note_write(g, buf, n);
   return 0;
 }
 
@@ -1374,7 +1375,7 @@ static int tp_gather_logits(aotcu_gpu* g) {
 }
 
 static int gpu_add(aotcu_gpu* g, float* x, const float* y, size_t n) {
-  note_write(g, x);
+  note_write(g, x, n);
   return launch(g->c, add_inplace_kernel, dim3(grid_for(g->c, n, 256)), dim3(256), 0, x, y, n);
 }
 
@@ -1443,7 +1444,7 @@ static int layer_forward(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos
 static int embed(aotcu_gpu* g, float* dst, const int* d_tokens, size_t m) {
   const aotcu_dims& d = g->head.dims;
   const aotcu_tensor& e = g->head.token_embd;
-  note_write(g, dst);
+  note_write(g, dst, m * d.dim);
   return launch(g->c, embed_rows_kernel, dim3((d.dim + 255) / 256, (unsigned)m), dim3(256), 0, dst, wptr(g, e), d_tokens,
                 (int)e.kind, (int)d.dim, kind_row_bytes(e.kind, e.cols), sqrtf((float)d.dim), (int)d.embd_scale);
 }
@@ -2282,7 +2283,7 @@ int aotcu_gpu_write(aotcu_gpu* g, int buf, size_t off, const float* src, size_t 
   ARG_CHECK(g && buf >= 0 && buf < AOTCU_N_BUFS && src, "bad argument");
   g->h_logits_fresh = false;  // anything but aotcu_forward may change the logits behind the host copy
   ARG_CHECK(off + n <= g->buf_len[buf], "write of %zu floats at %zu exceeds buffer %d (%zu)", n, off, buf, g->buf_len[buf]);
-  note_write(g, g->bufs[buf]);
+  note_write(g, g->bufs[buf] + off, n);
   return aotcu_h2d(g->c, g->bufs[buf] + off, src, n * sizeof(float));
 }
 

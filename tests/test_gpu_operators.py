@@ -92,3 +92,18 @@ def test_products_without_a_conversion_buffer(pkg, ob, ctx, kind, rows, cols, ms
         g.set_option("workspace_mib", 1 << 20)
         g.close()
     ctx.device_status()
+
+
+def test_a_write_inside_a_quantized_row_is_seen(pkg, ob, ctx):
+    rows, cols, m = 48, 512, 2
+    g, mats = _model_with(pkg, ctx, [(k, rows, cols) for k in (5, 6)], 16, 16)
+    for (w, t), kind in zip(mats, (5, 6)):
+        x = np.random.default_rng(kind).standard_normal(m * cols).astype(np.float32)
+        g.write("Bhb", x)
+        g.matmul("Bq", t, "Bhb", m)
+        x[700:720] = 3.0
+        g.write("Bhb", x[700:720], 700)
+        g.matmul("Bq", t, "Bhb", m)
+        assert_bits_equal(g.read("Bq", m * rows).reshape(m, rows), _want(ob, kind, w, x, m, rows, cols), f"kind {kind}")
+    g.finish()
+    g.close()
