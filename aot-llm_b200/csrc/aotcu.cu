@@ -2071,6 +2071,7 @@ int aotcu_attention(aotcu_ctx* c, float* out, const float* q, const float* k_cac
   ARG_CHECK(n_kv_head > 0 && n_head % n_kv_head == 0, "n_head must be a multiple of n_kv_head");
   ARG_CHECK(head_dim % 4 == 0 && head_dim <= 256, "head_dim %zu must be a multiple of 4, at most 256", head_dim);
   ARG_CHECK(pos0 + m <= ctx_len, "positions exceed the context");
+  ARG_CHECK(((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0, "cached rows must be 16-byte aligned");
   if (m == 0) return 0;
   return launch_attention(c, out, q, k_cache, v_cache, nullptr, nullptr, pos0, m, (int)n_head, (int)n_kv_head,
                           (int)head_dim, ctx_len, window);

@@ -181,7 +181,7 @@ int aotcu_add_inplace(aotcu_ctx* ctx, float* x, const float* y, size_t n); /* op
 int aotcu_add_bias_rows(aotcu_ctx* ctx, float* x, const float* b, size_t n, size_t m); /* ops.rs:90-95 */
 int aotcu_scale_inplace(aotcu_ctx* ctx, float* x, float s, size_t n);      /* ops.rs:137-141 */
 /* attention_rows (ops.rs:517-556; attention of 185-218 is m == 1): caches are
- * the layer's ctx x kv_dim slices. window == 0 attends to everything. */
+ * the layer's ctx x kv_dim slices, 16-byte aligned. window == 0 attends to everything. */
 int aotcu_attention(aotcu_ctx* ctx, float* out, const float* q, const float* k_cache, const float* v_cache,
                     size_t n_head, size_t n_kv_head, size_t head_dim, size_t ctx_len, size_t pos0, size_t m,
                     size_t window);

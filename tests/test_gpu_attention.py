@@ -30,3 +30,13 @@ def test_attention_paths(pkg, ob, ctx, n_head, n_kv, hd, ctxlen, calls):
         assert_bits_equal(dout.download(np.float32, q.size), ob.attention_rows(ob.Pool(4), q, kc, vc, d, ctxlen, 0, pos0, m, window),
                           f"m {m} pos0 {pos0} window {window}")
     ctx.device_status()
+
+
+def test_misaligned_caches_are_refused(pkg, ctx):
+    hd, n = 32, 8
+    dq, dk, dv = ctx.alloc(hd * 4), ctx.alloc((n + 1) * hd * 4), ctx.alloc((n + 1) * hd * 4)
+    for k, v in ((dk.at(4), dv), (dk, dv.at(8))):
+        with pytest.raises(pkg.AotCudaError) as e:
+            ctx.attention(dq, dq, k, v, 1, 1, hd, n, 0, 1, 0)
+        assert e.value.status == pkg.lib.ERR_BAD_ARG
+    ctx.device_status()
