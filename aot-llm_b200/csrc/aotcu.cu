@@ -593,6 +593,84 @@ static int launch_q80_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
   return 0;
 }
 
+// F16 / BF16 / F32 products on the chunk-streaming kernel (floatstream.cuh): matrices of one
+// kind, columns in eights, rows in fours, 16-byte aligned rows and activations. Returns 1
+// when the call does not fit. A single activation row always, several where launch_float_multi says.
+template <int KIND, int NR, int NT>
+static int launch_float_stream_t(aotcu_ctx* c, const FloatStreamParams& P, int grid, size_t smem) {
+  static bool attr_set[64] = {};
+  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(float_stream_kernel<KIND, NR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    attr_set[c->device] = true;
+  }
+  return launch(c, float_stream_kernel<KIND, NR, NT>, dim3(grid), dim3(MEGA_THREADS), smem, P);
+}
+template <int KIND>
+static int launch_float_stream_k(aotcu_ctx* c, const FloatStreamParams& P, int nr, int nt, int grid, size_t smem) {
+  if (nr == 4) return launch_float_stream_t<KIND, 4, 8>(c, P, grid, smem);
+  if (nt == 16) return launch_float_stream_t<KIND, 2, 16>(c, P, grid, smem);
+  if (nt == 8) return nr == 2 ? launch_float_stream_t<KIND, 2, 8>(c, P, grid, smem) : launch_float_stream_t<KIND, 1, 8>(c, P, grid, smem);
+  return nr == 2 ? launch_float_stream_t<KIND, 2, 1>(c, P, grid, smem) : launch_float_stream_t<KIND, 1, 1>(c, P, grid, smem);
+}
+static int g_float_chunks = 1;  // 0: keep float-kind products on gemv_float_kernel (option "float_chunks")
+static int g_float_rows4 = 1;  // 9..16 activation rows, many weight rows per CTA: four weight rows per lane (option "float_rows4")
+static int launch_float_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
+  const int kind = call.seg[0].kind;
+  const size_t row_bytes = kind_row_bytes(kind, call.cols);
+  if (call.cols % 8 || row_bytes % 16 || span % 4 || ((uintptr_t)call.x & 15)) return 1;
+  for (int s = 0; s < call.nseg; s++)
+    if (call.seg[s].kind != kind || call.seg[s].rows % 4 || ((uintptr_t)call.seg[s].w & 15)) return 1;
+  const int cb = fs_chunk_bytes(call.m);
+  FloatStreamParams P = {};
+  for (int s = 0; s < call.nseg; s++) {
+    P.seg[s] = call.seg[s];
+    if (!weight_tensor_map(&P.map[s], call.seg[s].w, (size_t)call.seg[s].rows, row_bytes, cb)) return 1;
+  }
+  P.nseg = call.nseg;
+  P.pair = call.pair;
+  P.cols = (int)call.cols;
+  P.epilogue = call.epilogue;
+  P.err = c->d_err;
+  const size_t quads = span / 4;
+  const int grid = quads < (size_t)c->n_sm ? (int)quads : c->n_sm;
+  P.quad_base = (int)(quads / grid);
+  P.quad_rem = (int)(quads % grid);
+  ChunkShape shape = chunk_shape(P.quad_base + (P.quad_rem ? 1 : 0), call.pair != 0, call.m, 0);
+  if (shape.nt == 16 && !call.pair && g_float_rows4) {
+    // 16 rows as two token groups of 8 with four weight rows per lane: 12 shared-memory loads
+    // per 32 fused multiply-adds instead of 18 (the load/store pipe is what bounds this kernel)
+    shape = ChunkShape{4, 8, MEGA_CONSUMER_WARPS / 2, 2};
+  }
+  if (shape.nt == 16 && call.m <= 8) shape = ChunkShape{2, 8, MEGA_CONSUMER_WARPS, 1};  // a short batch: one token group
+  if (shape.nr == 4 && call.m <= 8) shape = ChunkShape{2, 8, MEGA_CONSUMER_WARPS, 1};
+  P.qw = shape.qw;
+  P.ts = shape.ts;
+  const int chunk_cols = cb / (kind == F32 ? 4 : 2), xrows = call.m == 1 ? 1 : FS_MAX_TOK;
+  const int x_copies = chunk_cols > 256 ? 2 : 1, xbox = chunk_cols / x_copies;  // a box row holds at most 256 elements
+  const size_t stage = (size_t)shape.qw * shape.nr * 4 * cb + x_copies * (((size_t)xrows * xbox * 4 + 127) & ~(size_t)127);
+  const size_t tail = 128 + 16 + 128;
+  int n_stages = (int)((c->max_smem - tail) / stage);
+  n_stages = n_stages > 8 ? 8 : n_stages;
+  if (n_stages < 2) return 1;
+  P.n_stages = n_stages;
+  const size_t smem = (size_t)n_stages * stage + tail;
+  const size_t group = (size_t)shape.ts * shape.nt;
+  const float* x = reinterpret_cast<const float*>(call.x);
+  for (size_t t0 = 0; t0 < call.m; t0 += group) {
+    const size_t mg = std::min(group, call.m - t0);
+    P.m = (int)mg;
+    if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x + t0 * call.cols, call.cols, mg, call.cols * 4, xbox, xrows))
+      return t0 == 0 ? 1 : fail(AOTCU_ERR_CUDA, "tensor map of the activation rows refused");
+    for (int s = 0; s < call.nseg; s++) P.seg[s].out = call.seg[s].out + t0 * (size_t)call.seg[s].rows;
+    int rc;
+    if (kind == F16) rc = launch_float_stream_k<F16>(c, P, shape.nr, shape.nt, grid, smem);
+    else if (kind == BF16) rc = launch_float_stream_k<BF16>(c, P, shape.nr, shape.nt, grid, smem);
+    else rc = launch_float_stream_k<F32>(c, P, shape.nr, shape.nt, grid, smem);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
 // F16 / BF16 / F32 products of several activation rows on the packed kernel of floatmulti.cuh.
 // Returns 1 when the call does not fit.
 template <int KIND, int R, int T>
@@ -620,8 +698,40 @@ template <int KIND>
 static int launch_float_multi_k(aotcu_ctx* c, const FloatMultiParams& P, int r, int t, int grid) {
   return r == 2 ? launch_float_multi_r<KIND, 2>(c, P, t, grid) : launch_float_multi_r<KIND, 4>(c, P, t, grid);
 }
-static int g_float_chunks = 1;  // 0: keep float-kind products on gemv_float_kernel (option "float_chunks")
-static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
+// What a step of eight columns costs an SM that holds `ctas` CTAs of `wt` warps, in cycles: a step's
+// latency (longer where one warp copies all of the weights), the fullest scheduler's issue and the
+// shared memory's traffic, as independent bounds.
+static double float_multi_step(bool f32, int r, int t, int wt, size_t ctas) {
+  const double latency = 6.4 - 1.4 * r * t + 17.7 * (r + t) + (f32 ? 15 : 0) + (wt == 1 ? 7.5 * r * (f32 ? 2 : 1) : 0), warps = ctas * wt / 4.0;
+  const double issue = (0.9 * ceil(warps) + 0.1 * warps) * (15.5 + 3.6 * r * t), shared = ctas * (r * (f32 ? 8.0 : 4.0) + wt * t);
+  return sqrt(latency * latency + issue * issue + shared * shared);
+}
+static double float_multi_us(const aotcu_ctx* c, bool f32, size_t cols, int r, int t, int wt, size_t grid) {
+  const size_t smem = FM_STAGES * ((size_t)8 * r * (FM_COLS + 8) * (f32 ? 4 : 2) + (size_t)wt * t * FM_COLS * 4);
+  const size_t per_sm = std::max<size_t>(1, std::min<size_t>((r == 2 ? 24 : 16) / wt, c->max_smem / smem)), round = per_sm * c->n_sm, rest = grid % round;
+  double cycles = (double)(grid / round) * float_multi_step(f32, r, t, wt, per_sm);
+  if (rest) {  // a last round begins as CTAs of the one before end
+    const double last = float_multi_step(f32, r, t, wt, (rest + c->n_sm - 1) / c->n_sm);
+    cycles += grid < round ? last : 0.7 * last + 0.3 * float_multi_step(f32, r, t, wt, per_sm) * rest / round;
+  }
+  return 2 + cycles * (cols / 8) / 1965;
+}
+// Time of the streaming kernel in launches of 16 activation rows: per pass over the quads that a CTA
+// keeps resident (chunk_shape and what launch_float_stream makes of it), a start and a cost linear in
+// their number; a pair's quads come in twos.
+static double float_stream_us(const aotcu_ctx* c, bool f32, bool pair, size_t cols, size_t span, size_t m) {
+  const int quads = (int)((span / 4 + c->n_sm - 1) / c->n_sm) * (pair ? 2 : 1), half = MEGA_CONSUMER_WARPS / 2;
+  double us = 0.5;
+  if (quads <= 2 * half) {
+    us += 1.5 + (45 + 4.0 * quads + (f32 && quads < 4 ? 8 : 0)) * 1e-3 * (cols / 8);
+  } else {
+    const int cap = m > 8 && !pair ? 4 * half : 2 * MEGA_CONSUMER_WARPS;
+    const double start = m <= 8 ? (f32 ? 55 : 45) : (f32 ? 75 : pair ? 73 : 65), each = m <= 8 ? (f32 ? 3.1 : 2.25) : (f32 ? 3.45 : pair ? 3.1 : 2.8);
+    for (int left = quads; left > 0; left -= cap) us += 1.5 + (start + each * std::min(left, cap)) * 1e-3 * (cols / 8);
+  }
+  return us * ((m + FS_MAX_TOK - 1) / FS_MAX_TOK);
+}
+static int launch_float_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
   const int kind = call.seg[0].kind;
   if (call.cols % 8 || ((uintptr_t)call.x & 15)) return 1;
   for (int s = 0; s < call.nseg; s++)
@@ -633,12 +743,16 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
   P.epilogue = call.pair ? EPI_STORE : call.epilogue;
   P.x = reinterpret_cast<const float*>(call.x);
   // Shape: R weight rows and T activation rows per lane, wt warps per CTA (all of the batch's up to
-  // eight, or four). Fitted to timings of twelve matrices and batches of 2 to 64 at every shape: a
-  // step of eight columns takes a scheduler about 20 + 3 R T + 4 T cycles per warp that it holds,
-  // and 50 + 6 R T if it holds few; CTAs of three warps leave one scheduler idle.
-  int r_best = 2, t_best = 2;
-  size_t grid = 0;
-  double best = 1e30;
+  // eight, or four). A first choice by a rough cost: a step of eight columns takes a scheduler about
+  // 20 + 3 R T + 4 T cycles per warp that it holds, and 50 + 6 R T if it holds few; CTAs of three
+  // warps leave one scheduler idle. Another shape has to look 8 % faster by float_multi_us, which
+  // errs by 7 % over all shapes (fitted to f16 and f32, 18 matrices, batches of 2 to 64).
+  const bool f32 = kind == F32;
+  struct Shape {
+    int r = 0, t = 0, n_tcta = 0, wt = 0;
+    size_t grid = 0;
+    double cost = 1e30, us = 1e30;
+  } first, quickest;
   for (int r : {2, 4}) {
     size_t tiles = 0;
     for (int s = 0; s < call.nseg; s++) tiles += (call.seg[s].rows + 8 * r - 1) / (8 * r);
@@ -646,20 +760,29 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
       const size_t nw = (call.m + t - 1) / t;
       for (int k : {FM_MAX_WARPS, 4}) {
         const size_t nc = (nw + k - 1) / k, wt = (nw + nc - 1) / nc;
+        if (tiles * nc >= (1u << 30)) continue;
         const double warps = (double)(tiles * nc * wt) / (4 * c->n_sm) * (wt == 3 ? 1.15 : 1.0);
-        const double cost = std::max(warps * (20 + 3 * r * t + 4 * t), 50.0 + 6 * r * t);
-        if (cost < best * 0.999 && tiles * nc < (1u << 30)) {
-          best = cost;
-          r_best = r;
-          t_best = t;
-          P.n_tcta = (int)nc;
-          P.wt = (int)wt;
-          grid = tiles * nc;
-        }
+        Shape x{r, t, (int)nc, (int)wt, tiles * nc};
+        x.cost = std::max(warps * (20 + 3 * r * t + 4 * t), 50.0 + 6 * r * t);
+        x.us = float_multi_us(c, f32, call.cols, r, t, (int)wt, x.grid);
+        if (x.cost < first.cost * 0.999) first = x;
+        if (x.us < quickest.us) quickest = x;
       }
     }
   }
-  if (!grid) return 1;
+  const Shape shape = quickest.us < 0.92 * first.us ? quickest : first;
+  if (!shape.grid) return 1;
+  // The streaming kernel with 8 or 16 activation rows per lane is the better one where the tiles of
+  // this one fill the SMs unevenly (16 rows: f32 5632x4096 50 us against 71, f16 14336x4096 74
+  // against 91, and as a pair of 4096x4096 55 against 65).
+  if (float_stream_us(c, f32, call.pair != 0, call.cols, span, call.m) < 0.99 * shape.us) {
+    const int rc = launch_float_stream(c, call, span);
+    if (rc <= 0) return rc;
+  }
+  const int r_best = shape.r, t_best = shape.t;
+  const size_t grid = shape.grid;
+  P.n_tcta = shape.n_tcta;
+  P.wt = shape.wt;
   int tiles = 0;
   for (int s = 0; s < call.nseg; s++) {
     P.seg[s] = call.seg[s];
@@ -673,60 +796,6 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call) {
   if (rc || !call.pair || call.epilogue != EPI_SILU_MUL) return rc;
   const size_t n = call.m * (size_t)call.seg[0].rows;
   return launch(c, silu_mul_kernel, dim3(grid_for(c, n, 256)), dim3(256), 0, call.seg[0].out, (const float*)call.seg[1].out, n);
-}
-
-// F16 / BF16 / F32 products of one activation row on the chunk-streaming kernel (floatstream.cuh): matrices of one
-// kind, columns in eights, rows in fours, 16-byte aligned rows and activations. Returns 1
-// when the call does not fit.
-template <int KIND, int NR>
-static int launch_float_stream_t(aotcu_ctx* c, const FloatStreamParams& P, int grid, size_t smem) {
-  static bool attr_set[64] = {};
-  if (c->device >= 0 && c->device < 64 && !attr_set[c->device]) {
-    CU_TRY(cudaFuncSetAttribute(float_stream_kernel<KIND, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
-    attr_set[c->device] = true;
-  }
-  return launch(c, float_stream_kernel<KIND, NR>, dim3(grid), dim3(MEGA_THREADS), smem, P);
-}
-template <int KIND>
-static int launch_float_stream_k(aotcu_ctx* c, const FloatStreamParams& P, int nr, int grid, size_t smem) {
-  return nr == 2 ? launch_float_stream_t<KIND, 2>(c, P, grid, smem) : launch_float_stream_t<KIND, 1>(c, P, grid, smem);
-}
-static int launch_float_stream(aotcu_ctx* c, const GemvCall& call, size_t span) {
-  const int kind = call.seg[0].kind;
-  const size_t row_bytes = kind_row_bytes(kind, call.cols);
-  if (call.cols % 8 || row_bytes % 16 || span % 4 || ((uintptr_t)call.x & 15)) return 1;
-  for (int s = 0; s < call.nseg; s++)
-    if (call.seg[s].kind != kind || call.seg[s].rows % 4 || ((uintptr_t)call.seg[s].w & 15)) return 1;
-  const int cb = FS_CB;
-  FloatStreamParams P = {};
-  for (int s = 0; s < call.nseg; s++) {
-    P.seg[s] = call.seg[s];
-    if (!weight_tensor_map(&P.map[s], call.seg[s].w, (size_t)call.seg[s].rows, row_bytes, cb)) return 1;
-  }
-  P.nseg = call.nseg;
-  P.pair = call.pair;
-  P.cols = (int)call.cols;
-  P.epilogue = call.epilogue;
-  P.err = c->d_err;
-  const size_t quads = span / 4;
-  const int grid = quads < (size_t)c->n_sm ? (int)quads : c->n_sm;
-  P.quad_base = (int)(quads / grid);
-  P.quad_rem = (int)(quads % grid);
-  const ChunkShape shape = chunk_shape(P.quad_base + (P.quad_rem ? 1 : 0), call.pair != 0, 1, 0);
-  P.qw = shape.qw;
-  const int chunk_cols = cb / (kind == F32 ? 4 : 2);
-  const int x_copies = chunk_cols > 256 ? 2 : 1, xbox = chunk_cols / x_copies;  // a box row holds at most 256 elements
-  const size_t stage = (size_t)shape.qw * shape.nr * 4 * cb + x_copies * (((size_t)xbox * 4 + 127) & ~(size_t)127);
-  const size_t tail = 128 + 16 + 128;
-  int n_stages = (int)((c->max_smem - tail) / stage);
-  n_stages = n_stages > 8 ? 8 : n_stages;
-  if (n_stages < 2) return 1;
-  P.n_stages = n_stages;
-  const size_t smem = (size_t)n_stages * stage + tail;
-  if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, call.x, call.cols, 1, call.cols * 4, xbox, 1)) return 1;
-  if (kind == F16) return launch_float_stream_k<F16>(c, P, shape.nr, grid, smem);
-  if (kind == BF16) return launch_float_stream_k<BF16>(c, P, shape.nr, grid, smem);
-  return launch_float_stream_k<F32>(c, P, shape.nr, grid, smem);
 }
 
 // K-quant products of the smallest batches (see launch_gemv): gemv_stream_kernel<3>, one lane per super-block, grid = (row
@@ -829,7 +898,7 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
     ARG_CHECK(((uintptr_t)call.x % 4) == 0, "activations must be 4-byte aligned");
     if (g_float_chunks) {
       // 1: a shape that the 16-byte (tensor) copies do not take, the plain kernel does
-      const int rc = call.m >= 2 ? launch_float_multi(c, call) : launch_float_stream(c, call, span);
+      const int rc = call.m >= 2 ? launch_float_multi(c, call, span) : launch_float_stream(c, call, span);
       if (rc <= 0) return rc;
     }
     int rows_per_block = 32;
@@ -2755,6 +2824,10 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
   }
   if (!strcmp(name, "wide_multi")) {  // process-wide: K-quant prompt chunks of few tiles (and Q6_K) on gemv_stream_kernel<3> (1, default)
     g_wide_multi = value != 0;
+    return 0;
+  }
+  if (!strcmp(name, "float_rows4")) {  // process-wide: four weight rows per lane in the float chunk kernel at 9..16 activation rows (1, default)
+    g_float_rows4 = value != 0;
     return 0;
   }
   if (!strcmp(name, "float_chunks")) {  // process-wide: F16 / BF16 / F32 products on the chunk-streaming kernel (1, default)

@@ -9,7 +9,9 @@
 // memory and the conversion of 4 weight pairs per 4 T packed operations, against one load per
 // operation when a lane owned one chain. A warp covers 32 rows, its eight row groups lie 16 bytes
 // apart modulo the banks, and an activation pair is read by eight lanes at once.
-// bf16 4096x4096, 37 rows: 119 us with a chain per lane, 59 us now; f16 32768x4096, 2 rows: 107 and 51.
+// bf16 4096x4096, 37 rows: 119 us with a chain per lane (float_stream_kernel), 59 us now; f16 32768x4096, 2
+// rows: 107 and 51. Its weak spot is a batch that just fills 16 rows on a matrix whose tiles fall
+// unevenly on the SMs: launch_float_multi sends that to float_stream_kernel, by estimates of both.
 #pragma once
 #include "mmautils.cuh"
 #include "rowdot.cuh"

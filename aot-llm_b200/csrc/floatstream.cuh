@@ -2,13 +2,19 @@
 // (simd_avx2.rs:433-493: eight AVX2 lane accumulators per row, acc_k = fma(w[8j+k], x[8j+k],
 // acc_k) for j in order, then the horizontal sum of simd_avx2.rs:29-34).
 //
-// The structure of q80stream.cuh for one activation row: a group of 60 or 120 rows stays resident
-// as 544-byte column chunks, one 2-D tensor copy per four rows ("quad") and chunk, and lane (g, k)
-// of a consumer warp owns chain k of row g of the warp's quad(s) from the first chunk to the last.
-// The activation row is f32 in global memory, so its chunk travels with the stage as one more
-// tensor copy, and no length of row has to fit in shared memory. Columns in eights only (the
-// scalar tail of an odd length is left to gemv_float_kernel). Several activation rows are
-// floatmulti.cuh's.
+// The structure of q80stream.cuh: a group of 60 or 120 rows stays resident as 288- or 544-byte
+// column chunks, one 2-D tensor copy per four rows ("quad") and chunk, and lane (g, k) of a
+// consumer warp owns chain k of row g of the warp's quad(s) from the first chunk to the
+// last. The activation rows are f32 in global memory, so their chunk travels with the
+// stage as one more tensor copy (box: chunk columns by 1 or 16 rows; rows past the launch's
+// last are filled with zeros and their results dropped), and no length of row or number of
+// rows has to fit in shared memory. Columns in eights only (the scalar tail of an odd
+// length is left to gemv_float_kernel).
+//
+// What bounds it: a single row streams at 92 % of the copy bandwidth (f16 128256x4096); several are
+// bound by shared-memory loads, one per multiply-add of a lane's chain and row, less what a lane's
+// rows share. It is then the slower of the two several-row kernels but for batches that just fill
+// its 8 or 16 rows (see launch_float_multi).
 #pragma once
 #include <cuda.h>
 
@@ -17,23 +23,28 @@
 
 namespace aot {
 
-// bytes of a chunk row (32 modulo 128); large copies: the copy engine's rate of requests is what
-// limits a pure stream
-constexpr int FS_CB = 544;
+// bytes of a chunk row (32 modulo 128): 544 for a single activation row (larger copies: the copy
+// engine's rate of requests is what limits a pure stream), 288 for several (the stage also holds
+// 16 rows of activations, and the arithmetic sets the pace)
+constexpr int FS_CB_ONE = 544, FS_CB_MANY = 288;
+inline int fs_chunk_bytes(size_t m) { return m == 1 ? FS_CB_ONE : FS_CB_MANY; }
+constexpr int FS_MAX_TOK = 16;   // activation rows per launch
 
 struct FloatStreamParams {
   alignas(64) CUtensorMap map[3];  // per matrix: u32 elements, [rows][row_bytes / 4], box [4][chunk bytes / 4]
-  alignas(64) CUtensorMap xmap;    // activations: f32 [1][cols], box [1][136]
+  alignas(64) CUtensorMap xmap;    // activations: f32 [m][cols], box [1 or 16][chunk columns, at most 136]
   GemvSeg seg[3];
   int nseg, pair, cols, epilogue;
   int quad_base, quad_rem;  // quads (four rows of the row space; pair rows in pair mode) split over the grid
-  int qw;                   // consumer warps that own NR quads of a stage each
+  int m;                    // activation rows of this launch
+  int qw, ts;               // consumer warps per token group (each owns NR quads of a stage), token groups
   int n_stages;
   int* err;
 };
 
-template <int KIND, int NR>
+template <int KIND, int NR, int NT>
 __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __grid_constant__ FloatStreamParams P) {
+  constexpr int FS_CB = NT == 1 ? FS_CB_ONE : FS_CB_MANY;
   constexpr int ES = KIND == F32 ? 4 : 2;       // bytes per weight
   constexpr int CCOLS = FS_CB / ES;             // columns per chunk
   constexpr int CSTEPS = CCOLS / 8;             // AVX2 steps per chunk
@@ -41,7 +52,9 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
   constexpr int XROW = CCOLS * 4;               // bytes of an activation row's chunk
   // a tensor box holds at most 256 elements per row: the 272-column chunk of a single row comes as two copies
   constexpr int NXC = CCOLS > 256 ? 2 : 1, XBOX = CCOLS / NXC;
-  constexpr int XCOPY = (XBOX * 4 + 127) & ~127;
+  constexpr int XROWS = NT == 1 ? 1 : FS_MAX_TOK;   // rows of the activation box
+  static_assert(NXC == 1 || XROWS == 1, "split activation boxes are single rows");
+  constexpr int XCOPY = (XROWS * XBOX * 4 + 127) & ~127;
   const int SLOTS = P.qw * NR;                  // quads per stage
   const int WBYTES = SLOTS * QUAD;
   const int STAGE = WBYTES + NXC * XCOPY;
@@ -100,7 +113,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
     for (int grp = 0; grp < n_groups; grp++) {
       int sg = 0, lr = 0;
       const bool mine = lane < SLOTS && (NR == 2 || !P.pair) && slot_quad(q0 + grp * qpg, lane, sg, lr);
-      const uint32_t total = __popc(__ballot_sync(0xffffffffu, mine)) * (uint32_t)QUAD + (uint32_t)XROW;
+      const uint32_t total = __popc(__ballot_sync(0xffffffffu, mine)) * (uint32_t)QUAD + (uint32_t)(XROWS * XROW);
 #pragma unroll 1
       for (int c = 0; c < n_chunks; c++) {
         int ok = 1;
@@ -123,6 +136,8 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
   }
   pdl_wait();  // residual adds read what the previous kernel wrote
   const int k = lane & 7, g = lane >> 3;
+  // token group tg (activation rows tok0 .. tok0 + NT - 1), quads wq * NR .. of every stage
+  const int tg = warp / P.qw, wq = warp - tg * P.qw, tok0 = tg * NT;
   RingPos cp{0, 0u};
 #pragma unroll 1
   for (int grp = 0; grp < n_groups; grp++) {
@@ -133,21 +148,23 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
     for (int nr = 0; nr < NR; nr++) {
       sgi[nr] = 0;
       lri[nr] = 0;
-      live[nr] = warp < P.qw && (NR == 2 || !P.pair) && slot_quad(q0 + grp * qpg, warp * NR + nr, sgi[nr], lri[nr]);
+      live[nr] = tg < P.ts && (NR == 2 || !P.pair) && slot_quad(q0 + grp * qpg, wq * NR + nr, sgi[nr], lri[nr]);
       lri[nr] += g;
       any_live = any_live || live[nr];
     }
-    float acc[NR];
+    float acc[NR][NT];
 #pragma unroll
-    for (int nr = 0; nr < NR; nr++) acc[nr] = 0.0f;
+    for (int nr = 0; nr < NR; nr++)
+#pragma unroll
+      for (int t = 0; t < NT; t++) acc[nr][t] = 0.0f;
 #pragma unroll 1
     for (int c = 0; c < n_chunks; c++) {
       if (!ring_wait(R, &R.full[cp.st], cp.parity)) return;
       const uint32_t stage = smem_addr(stages + (size_t)cp.st * STAGE);
-      const uint32_t wrow0 = stage + (uint32_t)(warp * NR) * QUAD + (uint32_t)g * FS_CB + (uint32_t)k * ES;
-      const uint32_t xrow0 = stage + (uint32_t)WBYTES + (uint32_t)k * 4;
+      const uint32_t wrow0 = stage + (uint32_t)(wq * NR) * QUAD + (uint32_t)g * FS_CB + (uint32_t)k * ES;
+      const uint32_t xrow0 = stage + (uint32_t)WBYTES + (uint32_t)tok0 * XROW + (uint32_t)k * 4;
       const int nsteps = any_live ? min(CSTEPS, (P.cols - c * CCOLS) >> 3) : 0;  // a warp without rows only keeps the ring turning
-#pragma unroll 6
+#pragma unroll(NT == 1 ? 6 : 1)
       for (int j = 0; j < nsteps; j++) {
         float w[NR];
 #pragma unroll
@@ -162,35 +179,43 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
             w[nr] = KIND == F16 ? half_bits_hw(h) : __uint_as_float(h << 16);
           }
         }
-        const float x = __uint_as_float(rd_lds32(xrow0 + (uint32_t)j * 32 + (NXC == 2 && j >= CSTEPS / 2 ? XCOPY - XBOX * 4 : 0)));
 #pragma unroll
-        for (int nr = 0; nr < NR; nr++) acc[nr] = ffma(w[nr], x, acc[nr]);
+        for (int t = 0; t < NT; t++) {
+          const float x = __uint_as_float(rd_lds32(xrow0 + (uint32_t)t * XROW + (uint32_t)j * 32 + (NXC == 2 && j >= CSTEPS / 2 ? XCOPY - XBOX * 4 : 0)));
+#pragma unroll
+          for (int nr = 0; nr < NR; nr++) acc[nr][t] = ffma(w[nr], x, acc[nr][t]);
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&R.empty[cp.st]);
       cp.advance(R.n_stages);
     }
     // ((a0+a4)+(a2+a6)) + ((a1+a5)+(a3+a7)) over a row's eight lanes, then the epilogue
-    float v[NR];
 #pragma unroll
-    for (int nr = 0; nr < NR; nr++) {
-      float a = acc[nr];
-      a = fadd(a, __shfl_xor_sync(0xffffffffu, a, 4));
-      a = fadd(a, __shfl_xor_sync(0xffffffffu, a, 2));
-      v[nr] = fadd(a, __shfl_xor_sync(0xffffffffu, a, 1));
-    }
-    if (k != 0) continue;
-    if (NR == 2 && P.pair) {
-      if (live[0]) {
-        P.seg[0].out[lri[0]] = P.epilogue == EPI_SILU_MUL ? silu_mul_exact(v[0], v[NR - 1]) : v[0];
-        P.seg[1].out[lri[0]] = v[NR - 1];
-      }
-    } else {
+    for (int t = 0; t < NT; t++) {
+      float v[NR];
 #pragma unroll
       for (int nr = 0; nr < NR; nr++) {
-        if (live[nr]) {
-          float* o = P.seg[sgi[nr]].out + lri[nr];
-          *o = P.epilogue == EPI_ACCUM ? fadd(__ldcg(o), v[nr]) : v[nr];
+        float a = acc[nr][t];
+        a = fadd(a, __shfl_xor_sync(0xffffffffu, a, 4));
+        a = fadd(a, __shfl_xor_sync(0xffffffffu, a, 2));
+        v[nr] = fadd(a, __shfl_xor_sync(0xffffffffu, a, 1));
+      }
+      if (k == 0 && tok0 + t < P.m) {
+        if (NR == 2 && P.pair) {
+          if (live[0]) {
+            const size_t r = (size_t)(tok0 + t) * P.seg[0].rows + lri[0];
+            P.seg[0].out[r] = P.epilogue == EPI_SILU_MUL ? silu_mul_exact(v[0], v[NR - 1]) : v[0];
+            P.seg[1].out[r] = v[NR - 1];
+          }
+        } else {
+#pragma unroll
+          for (int nr = 0; nr < NR; nr++) {
+            if (live[nr]) {
+              float* o = P.seg[sgi[nr]].out + (size_t)(tok0 + t) * P.seg[sgi[nr]].rows + lri[nr];
+              *o = P.epilogue == EPI_ACCUM ? fadd(__ldcg(o), v[nr]) : v[nr];
+            }
+          }
         }
       }
     }

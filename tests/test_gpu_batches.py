@@ -53,6 +53,38 @@ def test_float_tile_edges(pkg, ob, ctx, kind, rows, cols):
         _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
 
 
+# Batches for which the streaming kernel's estimate is the lower one, in each of its forms: rows of a
+# CTA in one or two quads per lane, two token groups of eight with four rows per lane (or, by option,
+# sixteen tokens per lane), up to eight tokens, pairs; 28 rows are two launches of it.
+@pytest.mark.parametrize("kind,rows,pair,ms", [(1, 5632, False, (13,)), (2, 14336, False, (8, 16, 28)), (0, 2560, False, (9, 14)),
+                                               (0, 11264, False, (16,)), (1, 4096, True, (16,)), (2, 5632, True, (7, 15)), (0, 5632, True, (13,))])
+def test_float_batches_on_the_streaming_kernel(pkg, ob, ctx, kind, rows, pair, ms):
+    cols = 520
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)  # for the option and the count of launches
+    ws = [make_weights(pkg, kind, rows, cols, 33 + i) for i in range(1 + pair)]
+    dws = [ctx.to_device(w) for w in ws]
+    try:
+        for rows4 in (0, 1):
+            g.set_option("float_rows4", rows4)
+            for m in ms:
+                x = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+                dx, outs = ctx.to_device(x), [ctx.alloc(m * rows * 4) for _ in ws]
+                before = g.dispatches()
+                if pair:
+                    ctx.matmul2(kind, *outs, *dws, dx, m, rows, cols)
+                else:
+                    ctx.matmul(kind, outs[0], dws[0], dx, m, rows, cols)
+                assert g.dispatches() - before == (m + 15) // 16
+                for o, w in zip(outs, ws):
+                    assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, x, m, rows, cols),
+                                      f"kind {kind} {rows}x{cols} m {m} rows4 {rows4}")
+    finally:
+        g.set_option("float_rows4", 1)
+        g.close()
+    ctx.device_status()
+
+
 @pytest.mark.parametrize("kind", [3, 4, 5])           # Q4_0, Q5_0, Q8_0
 def test_q80_tile_edges(pkg, ob, ctx, kind):
     for rows, cols, ms in ((8192, 256, (49, 64)), (8205, 768, (50, 81, 129))):   # a partial row tile, half-full warps, two CTAs per tile
