@@ -471,31 +471,63 @@ static int launch_q80_mma_t(aotcu_ctx* c, const Q80MmaParams& P, int grid) {
   }
   return launch(c, q80_mma_kernel<KIND, PAIR>, dim3(grid), dim3(32 * P.wt), (size_t)QmShape<KIND>::unit_bytes(P.wt), P);
 }
-// A warp's chains take the same time whatever the launch holds, so it has to fill the chip, and a
-// batch that leaves part of a warp's 16 tokens or of the fourth warp idle gains nothing (11264x2048:
-// 82 us against 118 at 64 rows, 83 against 90 at 48, 57 against 61 at 32; 2560x2048: 39 against 49,
-// 2048x5632: 125 against 86).
-constexpr size_t Q80_MMA_MIN_ROWS = 8192, Q80_MMA_MIN_BATCH = 49;
+// Estimates of both kernels for a product of m rows, in microseconds (fitted to 22 matrices, three
+// kinds and batches of 2 to 256 rows: errors of 8 and 11 %).
+// q80_mma_kernel: a warp's chains take the same time however many run beside it until an SM's
+// schedulers are full, so a launch is rounds of as many CTAs as the registers (256 a thread) hold. Per
+// 32 columns a full round takes `full`, one that leaves SMs with fewer CTAs than the schedulers can
+// hide takes less, down to `light`.
+static double q80_mma_us(const aotcu_ctx* c, int kind, size_t cols, int wt, size_t ctas) {
+  static const struct {
+    int per_sm;
+    double full, light, from, over;  // CTAs per SM from which, and over which, `light` becomes `full`
+  } shape[6] = {{}, {7, 0.95, 0.65, 3, 4}, {4, 0.76, 0.53, 1, 0.5}, {2, 0.69, 0.48, 0.3, 0.4}, {2, 0.69, 0.46, 0.3, 0.4}, {1, 0.645, 0.645, 0, 1}};
+  const auto& s = shape[wt];
+  const size_t round = (size_t)s.per_sm * c->n_sm, rest = ctas % round;
+  double t = (double)(ctas / round) * s.full;
+  if (rest) t += s.light + (s.full - s.light) * std::min(1.0, std::max(0.0, ((double)rest / c->n_sm - s.from) / s.over));
+  return 3 + (cols / 32) * t * (kind == Q4_0 ? 1 : kind == Q5_0 ? 1.07 : 1.09);
+}
+// q80_stream_kernel: a launch for every 16 rows, each linear in the quads of a CTA.
+static double q80_stream_us(const aotcu_ctx* c, int kind, size_t cols, size_t rows, size_t m) {
+  const double quads = (double)((rows / 4 + c->n_sm - 1) / c->n_sm);
+  const double block = quads <= 14 ? std::max(0.09, 0.06 + 0.016 * quads) : 0.055 + 0.0175 * quads;
+  return 0.5 + ((m + 15) / 16) * (1.5 + (cols / 32) * block * (kind == Q4_0 ? 1 : kind == Q5_0 ? 1.1 : 0.95));
+}
+// Taken where the estimate is lower (both measured, us, this kernel first): Q4_0 11264x2048 76 and 116
+// at 64 rows, 77 and 88 at 48, 53 and 59 at 32; 5632x2048 48 and 66 at 64 rows, 39 and 34 at 32;
+// 2048x5632 123 and 83 at 64 rows, 124 and 165 at 128; Q8_0 14336x4096 193 and 242 at 64 rows, 195 and
+// 182 at 48. Up to 16 rows the streaming kernel is a single launch and the faster one nearly everywhere.
+// Matrices that it does not take (rows not in fours, mixed kinds) would go to the whole-row kernel,
+// whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows, 14337x4096 103 and 784.
+constexpr size_t Q80_MMA_MIN_BATCH = 17, Q80_MMA_MIN_BATCH_ODD = 32;
 static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
-  if (call.m < Q80_MMA_MIN_BATCH || call.m > (1u << 16) || (call.pair ? 2 : 1) * span < Q80_MMA_MIN_ROWS || call.cols % 256) return 1;
+  if (call.m < Q80_MMA_MIN_BATCH || call.m > (1u << 16) || call.cols % 256) return 1;
   for (int s = 0; s < call.nseg; s++)
     if ((uintptr_t)call.seg[s].w & 15) return 1;
   if (call.pair && call.seg[0].kind != call.seg[1].kind) return 1;
   const int nb = (int)(call.cols / 32), ntg = (int)((call.m + 7) / 8);
-  if (const int rc = ctx_workspace(c, (size_t)ntg * nb * X0F_BLOCK)) return rc;
-  if (int rc = launch(c, x0f_kernel, dim3((unsigned)(((size_t)ntg * nb + 7) / 8)), dim3(256), 0, reinterpret_cast<const uint8_t*>(call.x), (int)(call.x_mode == 1),
-                      c->ximg, (int)call.m, nb))
-    return rc;
   Q80MmaParams P = {};
   P.cols = (int)call.cols;
   P.m = (int)call.m;
   P.epilogue = call.epilogue;
-  P.xf = c->ximg;
   P.ntg = ntg;
-  const int nw = (ntg + QM_NG - 1) / QM_NG;  // warps that the batch takes: at most four or five share a row unit
+  const int nw = (ntg + QM_NG - 1) / QM_NG;  // warps that the batch takes: at most five share a row unit
   P.n_tcta = (nw + 4) / 5;
   P.wt = (nw + P.n_tcta - 1) / P.n_tcta;
   const int rows = call.pair ? 16 : 16 * QM_RT;
+  size_t units = 0;
+  for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) units += (call.seg[s].rows + rows - 1) / rows;
+  bool streams = true;  // what launch_q80_stream asks of the matrices
+  for (int s = 0; s < call.nseg; s++) streams = streams && call.seg[s].rows % 4 == 0 && call.seg[s].kind == call.seg[0].kind;
+  if (streams ? q80_mma_us(c, call.seg[0].kind, call.cols, P.wt, units * P.n_tcta) > 0.98 * q80_stream_us(c, call.seg[0].kind, call.cols, (call.pair ? 2 : 1) * span, call.m)
+              : call.m < Q80_MMA_MIN_BATCH_ODD)
+    return 1;
+  if (const int rc = ctx_workspace(c, (size_t)ntg * nb * X0F_BLOCK)) return rc;
+  if (int rc = launch(c, x0f_kernel, dim3((unsigned)(((size_t)ntg * nb + 7) / 8)), dim3(256), 0, reinterpret_cast<const uint8_t*>(call.x), (int)(call.x_mode == 1),
+                      c->ximg, (int)call.m, nb))
+    return rc;
+  P.xf = c->ximg;
   for (int kind : {Q4_0, Q5_0, Q8_0}) {
     P.nseg = P.n_units = 0;
     for (int s = 0; s < call.nseg; s++) {

@@ -18,7 +18,9 @@
 //    to the last.
 // Q8_0 14336x4096, 64 rows: 242 us on q80_stream_kernel, 192 here (about 9.7 instructions per matrix
 // instruction; a bare loop of loads, products and sums runs with 4.7 at 14 cycles each, 88 us).
-// Smaller tiles (one row tile, 8 tokens) fill small launches better but lose what the reuse gains.
+// Smaller tiles (one row tile, 8 tokens) fill small launches better but lose what the reuse gains. A
+// launch takes 0.7 us per 32 columns and round of two CTAs of four warps per SM, also where the round is
+// not full; where that is more than the streaming kernel takes, launch_q80_mma leaves the product to it.
 #pragma once
 #include <cuda_fp16.h>
 

@@ -94,6 +94,22 @@ def test_q80_tile_edges(pkg, ob, ctx, kind):
             _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
 
 
+# Both sides of the choice between the streaming and the matrix-instruction kernel: few rows and
+# many tokens, two and three warps per CTA, five with one CTA per SM, rows not in fours; and products
+# just before it.
+@pytest.mark.parametrize("kind,rows,cols,m,mma", [(3, 300, 512, 128, True), (4, 260, 256, 112, True), (5, 4100, 512, 81, True), (3, 11264, 256, 32, True),
+                                                  (5, 8192, 256, 48, True), (4, 12000, 512, 17, True), (3, 16400, 256, 80, True),
+                                                  (3, 301, 512, 32, True), (3, 300, 512, 32, False), (5, 2048, 512, 48, False), (4, 8192, 256, 16, False)])
+def test_q80_sizes_around_the_choice_of_kernel(pkg, ob, ctx, kind, rows, cols, m, mma):
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)  # for the count of launches
+    w = make_weights(pkg, kind, rows, cols, 43 + kind)
+    before = g.dispatches()
+    _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+    assert g.dispatches() - before == (2 if mma else 1 + (m + 15) // 16)
+    g.close()
+
+
 def test_q80_pair_tile_edges(pkg, ob, ctx):
     rows, cols, m = 4105, 512, 60
     ws = [make_weights(pkg, 3, rows, cols, 51 + i) for i in range(2)]
