@@ -502,7 +502,7 @@ static double q80_stream_us(const aotcu_ctx* c, int kind, size_t cols, size_t ro
 // whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows, 14337x4096 103 and 784.
 constexpr size_t Q80_MMA_MIN_BATCH = 17, Q80_MMA_MIN_BATCH_ODD = 32;
 static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
-  if (call.m < Q80_MMA_MIN_BATCH || call.m > (1u << 16) || call.cols % 256) return 1;
+  if (call.m < Q80_MMA_MIN_BATCH || call.cols % 256) return 1;
   for (int s = 0; s < call.nseg; s++)
     if ((uintptr_t)call.seg[s].w & 15) return 1;
   if (call.pair && call.seg[0].kind != call.seg[1].kind) return 1;
@@ -889,6 +889,7 @@ static int launch_gemv_stream_multi(aotcu_ctx* c, const GemvCall& call, size_t s
   return launch(c, gemv_stream_kernel<3>, dim3(n_ranges, n_tg), dim3(MEGA_THREADS), smem, P);
 }
 
+constexpr size_t BATCH_PART = 4096;  // activation rows of one pass through the launchers
 static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
   ARG_CHECK(call.nseg >= 1 && call.nseg <= 3, "1..3 matrices per launch");
   const int act = kind_act(call.seg[0].kind);
@@ -913,6 +914,20 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
     span = (size_t)call.seg[0].rows;
   }
   ARG_CHECK(span < (1u << 30) && call.cols < (1u << 24), "matrix too large");
+
+  // Long batches go in parts: the conversion buffer is sized for one of them, and the kernels' 32-bit
+  // counts of (row, block) pairs hold it for every length of row.
+  if (call.m > BATCH_PART && call.x_mode != 2) {
+    const size_t x_bytes = act == ACT_F32 ? call.cols * 4 : act == ACT_Q8_K ? call.cols / 256 * (call.x_mode == 1 ? XK_STRIDE : 292) : call.cols / 32 * (call.x_mode == 1 ? X0_STRIDE : 36);
+    for (size_t t0 = 0; t0 < call.m; t0 += BATCH_PART) {
+      GemvCall part = call;
+      part.m = std::min(BATCH_PART, call.m - t0);
+      part.x = reinterpret_cast<const uint8_t*>(call.x) + t0 * x_bytes;
+      for (int s = 0; s < call.nseg; s++) part.seg[s].out = call.seg[s].out + t0 * (size_t)call.seg[s].rows;
+      if (int rc = launch_gemv(c, part)) return rc;
+    }
+    return 0;
+  }
 
   GemvParams P = {};
   for (int s = 0; s < call.nseg; s++) P.seg[s] = call.seg[s];

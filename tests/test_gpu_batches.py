@@ -110,6 +110,13 @@ def test_q80_sizes_around_the_choice_of_kernel(pkg, ob, ctx, kind, rows, cols, m
     g.close()
 
 
+@pytest.mark.parametrize("kind,rows,cols", [(0, 20, 64), (1, 37, 20), (3, 301, 256), (5, 64, 96), (6, 40, 256), (8, 3, 512)])
+def test_batches_longer_than_a_pass(pkg, ob, ctx, kind, rows, cols):
+    m = 4096 + 9 if cols % 32 == 0 else 8192 + 3
+    w = make_weights(pkg, kind, rows, cols, 47 + kind)
+    _run(pkg, ob, ctx, kind, w, np.random.default_rng(kind).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+
+
 def test_q80_pair_tile_edges(pkg, ob, ctx):
     rows, cols, m = 4105, 512, 60
     ws = [make_weights(pkg, 3, rows, cols, 51 + i) for i in range(2)]
