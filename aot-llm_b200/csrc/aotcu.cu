@@ -830,11 +830,22 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
   return launch(c, silu_mul_kernel, dim3(grid_for(c, n, 256)), dim3(256), 0, call.seg[0].out, (const float*)call.seg[1].out, n);
 }
 
-// K-quant products of the smallest batches (see launch_gemv): gemv_stream_kernel<3>, one lane per super-block, grid = (row
+// K-quant products of two or three rows: gemv_stream_kernel<3>, one lane per super-block, grid = (row
 // ranges) x (groups of activation rows). Returns 1 when the call does not fit.
-static int g_wide_multi = 1;          // option "wide_multi": 0 sends these products to kmma.cuh as well
-static int g_wide_multi_work = 8192;  // option "wide_multi_work": weight rows x activation rows up to which three rows or more take it
-static bool takes_kmma(size_t m, size_t work) { return !g_wide_multi || (m > 2 && work > (size_t)g_wide_multi_work); }
+static int g_wide_multi = 1;       // option "wide_multi": 0 sends these products to kmma.cuh as well
+static int g_wide_multi_work = 0;  // option "wide_multi_work": weight rows x activation rows up to which every batch takes it
+// Its time grows with the batch where kmma_kernel's hardly depends on it (us, this kernel first; Q4_K
+// 2048x2048: 3.7 and 4.5 at 2 rows, 4.6 and 4.5 at 3, 8.0 and 4.5 at 8; 14336x4096: 14.3 and 19.4, 20.1
+// and 19.5, 43 and 20). Two rows take it unless they are long (4096x12288 16.1 and 14.5; Q6_K 21.1 and
+// 23.2), three on large Q6_K matrices (14336x4096 27.4 and 30.0) and where the product is so small that
+// kmma_kernel's second launch, for the activations, is what takes the time.
+static bool takes_one_lane(const GemvCall& call, size_t span) {
+  if (!g_wide_multi) return false;
+  if (call.m * span <= (size_t)g_wide_multi_work) return true;
+  const bool q6 = call.seg[0].kind == Q6_K;
+  if (call.m == 2) return q6 || call.cols <= 5120 || span < 2048;
+  return call.m == 3 && ((q6 && span >= 8192 && call.cols <= 4096) || span <= 2730);
+}
 static int launch_gemv_stream_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
   if (call.pair || g_dbg_sumi || call.cols % 256) return 1;
   StreamGemvParams P = {};
@@ -956,12 +967,13 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
   }
   ARG_CHECK(((uintptr_t)call.x % (P.x_image ? 16 : 4)) == 0, "activation blocks are misaligned");
 
-  // K-quant products of several activation rows: the tensor-core kernel of kmma.cuh, but for two
-  // rows and the smallest products one lane per super-block against every row, whose time grows
-  // with rows x batch (2048 x 2048: 4.1 us at 2 rows and 8.3 at 8 against 6.8 at either).
+  // K-quant products of several activation rows: the tensor-core kernel of kmma.cuh, but for the
+  // smallest batches one lane per super-block against every row. A Gpu keeps its activations in
+  // kmma's order (xf_rows) whatever the batch: half of a layer's products are pairs or mixed kinds,
+  // which the one-lane kernel does not take, and a prompt of two costs what one of three does.
   if (act == ACT_Q8_K && call.m >= 2) {
     if (takes_tc(call)) return launch_gemm_tc(c, call);
-    if (!takes_kmma(call.m, call.m * span) && call.x_mode != 2) {
+    if (call.x_mode != 2 && takes_one_lane(call, span)) {
       const int rc = launch_gemv_stream_multi(c, call, span);
       if (rc <= 0) return rc;  // 1: a pair or a very long row
     }
@@ -2864,12 +2876,12 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
     g_q80_chunks = value != 0;
     return 0;
   }
-  if (!strcmp(name, "wide_multi_work")) {  // process-wide: see launch_gemv
+  if (!strcmp(name, "wide_multi_work")) {  // process-wide: see takes_one_lane
     ARG_CHECK(value >= 0, "wide_multi_work must not be negative");
     g_wide_multi_work = value;
     return 0;
   }
-  if (!strcmp(name, "wide_multi")) {  // process-wide: K-quant prompt chunks of few tiles (and Q6_K) on gemv_stream_kernel<3> (1, default)
+  if (!strcmp(name, "wide_multi")) {  // process-wide: see takes_one_lane
     g_wide_multi = value != 0;
     return 0;
   }

@@ -30,6 +30,21 @@ def test_k_quant_tile_edges(pkg, ob, ctx, kind, rows, cols):
         _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
 
 
+# Which kernel a small batch takes, by launches: the one-lane kernel is one, kmma_kernel has its
+# activations converted first. The two tests around this one rely on kmma_kernel from four rows on.
+@pytest.mark.parametrize("kind,rows,cols,m,one_lane", [(Q4_K, 300, 512, 2, True), (Q5_K, 2048, 5376, 2, False), (Q6_K, 2048, 5376, 2, True), (Q4_K, 40, 5376, 2, True),
+                                                       (Q6_K, 8200, 256, 3, True), (Q5_K, 8200, 256, 3, False), (Q4_K, 2730, 256, 3, True), (Q6_K, 2731, 256, 3, False), (Q6_K, 1, 256, 4, False),
+                                                       (Q4_K, 17, 768, 4, False), (Q6_K, 48, 1024, 12, False)])
+def test_k_quant_small_batches(pkg, ob, ctx, kind, rows, cols, m, one_lane):
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)  # for the count of launches
+    w = make_weights(pkg, kind, rows, cols, 23 + kind, "uniform")
+    before = g.dispatches()
+    _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+    assert g.dispatches() - before == (1 if one_lane else 2)
+    g.close()
+
+
 @pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
 def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, kind):
     rows, cols, m = 48, 1024, 12
