@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
   pdl_wait();  // residual adds read what the previous kernel wrote
   const int k = lane & 7, g = lane >> 3;
   // token group tg (activation rows tok0 .. tok0 + NT - 1), quads wq * NR .. of every stage
-  const int tg = warp / P.qw, wq = warp - tg * P.qw, tok0 = tg * NT;
+  const int tg = NT == 1 ? 0 : warp / P.qw, wq = warp - tg * P.qw, tok0 = tg * NT;
   RingPos cp{0, 0u};
 #pragma unroll 1
   for (int grp = 0; grp < n_groups; grp++) {
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
     for (int nr = 0; nr < NR; nr++) {
       sgi[nr] = 0;
       lri[nr] = 0;
-      live[nr] = tg < P.ts && (NR == 2 || !P.pair) && slot_quad(q0 + grp * qpg, wq * NR + nr, sgi[nr], lri[nr]);
+      live[nr] = (NT == 1 ? warp < P.qw : tg < P.ts) && (NR == 2 || !P.pair) && slot_quad(q0 + grp * qpg, wq * NR + nr, sgi[nr], lri[nr]);
       lri[nr] += g;
       any_live = any_live || live[nr];
     }
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) float_stream_kernel(const __g
         a = fadd(a, __shfl_xor_sync(0xffffffffu, a, 2));
         v[nr] = fadd(a, __shfl_xor_sync(0xffffffffu, a, 1));
       }
-      if (k == 0 && tok0 + t < P.m) {
+      if (k == 0 && (NT == 1 || tok0 + t < P.m)) {
         if (NR == 2 && P.pair) {
           if (live[0]) {
             const size_t r = (size_t)(tok0 + t) * P.seg[0].rows + lri[0];
