@@ -183,7 +183,8 @@ static int launch_gemm_tc(aotcu_ctx* c, const GemvCall& call) {
 // 1: prompt chunks of Q4_K / Q5_K matrices go to the tcgen05 kernels (option "tc_gemm" 2). Not the
 // default: their tiles of 128 rows pay about 1.6 K cycles of mbarrier hand-overs per super-block
 // and up to 2.7 K instructions per 64-weight chunk for the digits; kmma.cuh is 1.6x (14336 x
-// 4096 x 64: 48 against 77 us) to 5x (4096 x 14336 x 64: 43 against 230 us) faster.
+// 4096 x 64: 48 against 77 us) to 5x (4096 x 14336 x 64: 43 against 230 us) faster, and no size was
+// measured where it is not. They stay as a second implementation to compare results with.
 static int g_tc_force = 0;
 static bool takes_tc(const GemvCall& call) {
   bool k4 = g_use_tc && g_tc_force > 0 && call.m >= 8 && call.m <= (size_t)TC_TOK;

@@ -23,7 +23,8 @@
 namespace aot {
 
 // 512 threads (15 consumer warps and the producer warp) leave 128 registers per thread:
-// measured faster than 640 or 768 threads, whose register budgets spill in the row products.
+// measured faster than 640 or 768 threads, whose register budgets spill in the row products (here 16
+// bytes of a thread spill, 52 in the sharded variant, none in the long-context ones of one GPU).
 #ifndef MEGA_THREADS_N
 #define MEGA_THREADS_N 512
 #endif

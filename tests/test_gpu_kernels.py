@@ -435,7 +435,7 @@ def test_bad_arguments_are_reported_not_fatal(pkg, ctx):
     ctx.device_status()  # the context is still usable
 
 
-# north_star: "integer per-block dot products are bit-exact" -- checked on the integers the
+# Integer per-block dot products are bit-exact: checked on the integers the
 # production kernels themselves form (the streaming single-row product and the tcgen05 prompt
 # product write them out while they compute), not on a separate checker kernel.
 @pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])

@@ -229,7 +229,7 @@ def test_prepared_tensor_core_operands_bit_exact(pkg, ob, ctx):
     g1.forward_batch(toks, pos, True)
     om.forward_batch(toks, pos, True)
     assert_bits_equal(g1.logits(), om.logits(), "after switching prepared operands off")
-    g1.set_option("tc_gemm", 1)      # back to the default: by size
+    g1.set_option("tc_gemm", 1)      # back to the default kernel
     g1.close()
     g0.close()
     ctx.device_status()
