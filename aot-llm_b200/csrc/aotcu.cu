@@ -779,13 +779,16 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
   // eight, or four). A first choice by a rough cost: a step of eight columns takes a scheduler about
   // 20 + 3 R T + 4 T cycles per warp that it holds, and 50 + 6 R T if it holds few; CTAs of three
   // warps leave one scheduler idle. Another shape has to look 8 % faster by float_multi_us, which
-  // errs by 7 % over all shapes (fitted to f16 and f32, 18 matrices, batches of 2 to 64).
+  // errs by 7 % over all shapes (fitted to f16 and f32, 18 matrices, batches of 2 to 64). Products of
+  // a microsecond or two keep the first choice: the estimates take the host 0.3 us, and the launch
+  // itself is what bounds those (f16 256x256, 4 rows: 4.5 us, 4.9 with estimates).
   const bool f32 = kind == F32;
   struct Shape {
     int r = 0, t = 0, n_tcta = 0, wt = 0;
     size_t grid = 0;
     double cost = 1e30, us = 1e30;
-  } first, quickest;
+  } shape, all[16];
+  int n_shapes = 0;
   for (int r : {2, 4}) {
     size_t tiles = 0;
     for (int s = 0; s < call.nseg; s++) tiles += (call.seg[s].rows + 8 * r - 1) / (8 * r);
@@ -793,24 +796,31 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
       const size_t nw = (call.m + t - 1) / t;
       for (int k : {FM_MAX_WARPS, 4}) {
         const size_t nc = (nw + k - 1) / k, wt = (nw + nc - 1) / nc;
-        if (tiles * nc >= (1u << 30)) continue;
+        if (tiles * nc >= (1u << 30) || (k == 4 && nw <= 4)) continue;
         const double warps = (double)(tiles * nc * wt) / (4 * c->n_sm) * (wt == 3 ? 1.15 : 1.0);
-        Shape x{r, t, (int)nc, (int)wt, tiles * nc};
+        Shape& x = all[n_shapes++];
+        x = Shape{r, t, (int)nc, (int)wt, tiles * nc};
         x.cost = std::max(warps * (20 + 3 * r * t + 4 * t), 50.0 + 6 * r * t);
-        x.us = float_multi_us(c, f32, call.cols, r, t, (int)wt, x.grid);
-        if (x.cost < first.cost * 0.999) first = x;
-        if (x.us < quickest.us) quickest = x;
+        if (x.cost < shape.cost * 0.999) shape = x;
       }
     }
   }
-  const Shape shape = quickest.us < 0.92 * first.us ? quickest : first;
   if (!shape.grid) return 1;
-  // The streaming kernel with 8 or 16 activation rows per lane is the better one where the tiles of
-  // this one fill the SMs unevenly (16 rows: f32 5632x4096 50 us against 71, f16 14336x4096 74
-  // against 91, and as a pair of 4096x4096 55 against 65).
-  if (float_stream_us(c, f32, call.pair != 0, call.cols, span, call.m) < 0.99 * shape.us) {
-    const int rc = launch_float_stream(c, call, span);
-    if (rc <= 0) return rc;
+  if (shape.cost * (call.cols / 8) > 2 * 1965) {
+    const Shape* quickest = all;
+    for (int i = 0; i < n_shapes; i++) {
+      all[i].us = float_multi_us(c, f32, call.cols, all[i].r, all[i].t, all[i].wt, all[i].grid);
+      if (all[i].us < quickest->us) quickest = all + i;
+    }
+    shape.us = float_multi_us(c, f32, call.cols, shape.r, shape.t, shape.wt, shape.grid);
+    if (quickest->us < 0.92 * shape.us) shape = *quickest;
+    // The streaming kernel with 8 or 16 activation rows per lane is the better one where the tiles of
+    // this one fill the SMs unevenly (16 rows: f32 5632x4096 50 us against 71, f16 14336x4096 74
+    // against 91, and as a pair of 4096x4096 55 against 65).
+    if (float_stream_us(c, f32, call.pair != 0, call.cols, span, call.m) < 0.99 * shape.us) {
+      const int rc = launch_float_stream(c, call, span);
+      if (rc <= 0) return rc;
+    }
   }
   const int r_best = shape.r, t_best = shape.t;
   const size_t grid = shape.grid;
