@@ -21,6 +21,7 @@
 #include "gemm_tc.cuh"
 #include "attention.cuh"
 #include "kmma.cuh"
+#include "ktensor.cuh"
 #include "mega.cuh"
 #include "q80mma.cuh"
 #include "q80stream.cuh"
@@ -112,7 +113,8 @@ struct GemvCall {
   int pair = 0;
   size_t cols = 0;
   const void* x = nullptr;
-  int x_mode = 0;  // 0 reference-layout blocks (or f32 for float kinds), 1 block images, 2 fragments (Q8_K, kmma.cuh)
+  const uint8_t* xt = nullptr;  // x_mode 2: the second array of xf_store, if there
+  int x_mode = 0;  // 0 reference-layout blocks (or f32 for float kinds), 1 block images, 2 the orders of xf_store (Q8_K)
   size_t m = 1;
   int epilogue = EPI_STORE;
   const uint8_t* prep[3] = {nullptr, nullptr, nullptr};  // prepared tensor-core operands of each matrix, if any
@@ -302,9 +304,28 @@ static int ctx_workspace(aotcu_ctx* c, size_t need) {
   return 0;
 }
 
-// K-quant products of several activation rows on the int8 tensor-core kernel of kmma.cuh.
-// Activations that are not in its fragment order are converted first. Returns 1 when there is no
-// buffer for that.
+// 2-D tensor map over 32-bit elements: [dim1][dim0] with rows `stride_bytes` apart, box
+// [box1][box0]. cuTensorMapEncodeTiled comes from the driver through the runtime (no link
+// against libcuda). Returns false when the driver refuses the map.
+static bool tensor_map_2d(CUtensorMap* out, CUtensorMapDataType dtype, const void* base, size_t dim0, size_t dim1, size_t stride_bytes,
+                          int box0, int box1) {
+  using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static EncodeFn encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<EncodeFn>(fn);
+  }();
+  if (!encode) return false;
+  const cuuint64_t gdim[2] = {dim0, dim1}, gstride[1] = {stride_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)box0, (cuuint32_t)box1}, estride[2] = {1, 1};
+  return encode(out, dtype, 2, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// K-quant products of several activation rows on the int8 warp-level kernel of kmma.cuh.
 template <int KIND, int RT, bool PAIR, int WK>
 static int launch_kmma_t(aotcu_ctx* c, KmmaParams& P, int grid) {
   using S = KmmaShape<KIND, RT, PAIR, WK>;
@@ -322,12 +343,10 @@ static int launch_kmma_k(aotcu_ctx* c, KmmaParams& P, int rt, bool pair, int wk,
   if (rt == 2) return wk == 8 ? launch_kmma_t<KIND, 2, false, 8>(c, P, grid) : launch_kmma_t<KIND, 2, false, 4>(c, P, grid);
   return wk == 8 ? launch_kmma_t<KIND, 1, false, 8>(c, P, grid) : launch_kmma_t<KIND, 1, false, 4>(c, P, grid);
 }
-// The matrices of one kind of `call` (all of them have it), activations in fragment order.
-static int launch_kmma_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xf, int xf_nt) {
-  const int nb = (int)(call.cols / 256), kind = call.seg[0].kind;
-  // Shape: a CTA's tile costs ceil(nb / WK) stages; two row tiles per warp instead of one cost
-  // about 1.5 times as much.
-  int rt = 2, wk = 8;
+// Shape: a CTA's tile costs ceil(nb / WK) stages; two row tiles per warp instead of one cost
+// about 1.5 times as much. Returns the stages.
+static double kmma_shape(const aotcu_ctx* c, const GemvCall& call, int* rt, int* wk) {
+  const int nb = (int)(call.cols / 256);
   double best = 1e30;
   for (int k : {8, 4})
     for (int r = call.pair ? 2 : 1; r <= 2; r++) {
@@ -337,10 +356,17 @@ static int launch_kmma_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xf
       const double t = (double)((tiles + c->n_sm - 1) / c->n_sm) * ((nb + k - 1) / k) * (r == 2 ? 1.5 : 1.0);
       if (t < best * 0.999) {
         best = t;
-        rt = r;
-        wk = k;
+        *rt = r;
+        *wk = k;
       }
     }
+  return best;
+}
+// The matrices of one kind of `call` (all of them have it), activations in fragment order.
+static int launch_kmma_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xf, int xf_nt) {
+  const int kind = call.seg[0].kind;
+  int rt, wk;
+  kmma_shape(c, call, &rt, &wk);
   const int rows = 16 * (call.pair ? 1 : rt) * (KM_WARPS / wk);
   KmmaParams P = {};
   int tiles = 0;
@@ -367,23 +393,184 @@ static int launch_kmma_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xf
   }
   return 0;
 }
-static int launch_kmma(aotcu_ctx* c, const GemvCall& call) {
-  const int nb = (int)(call.cols / 256), nt = (int)((call.m + 7) / 8);
-  const uint8_t* xf = reinterpret_cast<const uint8_t*>(call.x);
-  if (call.x_mode != 2) {
-    if (const int rc = ctx_workspace(c, (size_t)nt * nb * XF_BLOCK)) return rc;
-    if (int rc = launch(c, xf_kernel, dim3((unsigned)nt * nb), dim3(256), 0, xf, call.x_mode, c->ximg, (int)call.m, nb)) return rc;
-    xf = c->ximg;
+// K-quant products of several activation rows on the tensor-core kernel of ktensor.cuh.
+// Activations that are not in its order are converted first. Returns 1 when there is no buffer
+// for that.
+template <int KIND, int C>
+static size_t kt_smem(const KtParams& P) {
+  return 2 * (size_t)KT_TERMS + (size_t)P.n_b * ((P.nt + 1) / 2 * 2) * XT_BLOCK + (size_t)P.n_raw * KtKind<KIND>::RAW +
+         KT_SIDE_SLOTS * KT_ROWS * sizeof(float2) + (KT_BARS + 2) * 8 + (P.pair ? KT_ROWS * KT_XCH<C> * sizeof(float) : 0);
+}
+static void kt_config(aotcu_ctx* c, cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[2], int cluster, int ctas, size_t smem) {
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(KT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->pdl ? 2 : 1;
+}
+// Clusters of C CTAs that run at once: the dies and their SM groups do not divide evenly.
+template <int KIND, int C>
+static int kt_clusters(aotcu_ctx* c, int* out) {
+  static int known[64] = {};
+  if (c->device < 0 || c->device >= 64 || !known[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(kt_kernel<KIND, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    kt_config(c, cfg, attr, C, C, c->max_smem);
+    cfg.numAttrs = 1;
+    int n = 0;
+    CU_TRY(cudaOccupancyMaxActiveClusters(&n, kt_kernel<KIND, C>, &cfg));
+    if (c->device < 0 || c->device >= 64) return *out = n, 0;
+    known[c->device] = n;
   }
-  if (call.pair) return launch_kmma_one(c, call, xf, nt);
+  *out = known[c->device];
+  return 0;
+}
+template <int KIND, int C>
+static int launch_kt_c(aotcu_ctx* c, KtParams& P, int clusters) {
+  using K = KtKind<KIND>;
+  P.n_raw = P.n_b = 2;
+  for (bool grown = true; grown;) {
+    grown = false;
+    if (P.n_b < KT_MAX_SLOTS && (P.n_b++, kt_smem<KIND, C>(P) > c->max_smem ? (P.n_b--, false) : true)) grown = true;
+    if (P.n_raw < KT_MAX_SLOTS && (P.n_raw++, kt_smem<KIND, C>(P) > c->max_smem ? (P.n_raw--, false) : true)) grown = true;
+  }
+  const size_t row_bytes = (size_t)(P.cols / 256) * K::BS;
+  P.tma = 1;
+  for (int s = 0; s < P.nseg && P.tma; s++)
+    P.tma = row_bytes % 16 == 0 && ((uintptr_t)P.seg[s].w & 15) == 0 &&
+            tensor_map_2d(&P.map[s], CU_TENSOR_MAP_DATA_TYPE_UINT32, P.seg[s].w, row_bytes / 4, P.seg[s].rows, row_bytes, K::PITCH / 4,
+                          P.pair ? KT_ROWS / 2 : KT_ROWS);
+  P.err = c->d_err;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  kt_config(c, cfg, attr, C, C * std::min(clusters, P.n_tiles), kt_smem<KIND, C>(P));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kt_kernel<KIND, C>, P);
+  if (e != cudaSuccess) return fail(AOTCU_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
+  c->launches++;
+  return 0;
+}
+static int g_kt_cluster = 0;  // 0: by shape; else forced (option "kt_cluster")
+static int kt_tiles(const GemvCall& call) {
+  const int rows = call.pair ? KT_ROWS / 2 : KT_ROWS;
+  int tiles = 0;
+  for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) tiles += (call.seg[s].rows + rows - 1) / rows;
+  return tiles;
+}
+// Cluster size: a product's time is its stages, rounds of tiles over the clusters times a tile's
+// super-blocks per CTA; at equal counts clusters of four (24576 x 4096 x 64: 44.3 us, 45.7 with two,
+// 47.8 with eight). Returns the stages.
+template <int KIND>
+static int kt_shape(aotcu_ctx* c, int tiles, int nb, int* cluster, int* clusters, long* stages) {
+  *stages = 0;
+  for (int size : {4, 2, 8}) {
+    if (g_kt_cluster && g_kt_cluster != size) continue;
+    int n = 0;
+    if (int rc = size == 2 ? kt_clusters<KIND, 2>(c, &n) : size == 4 ? kt_clusters<KIND, 4>(c, &n) : kt_clusters<KIND, 8>(c, &n)) return rc;
+    if (!n) continue;
+    const long t = (long)((tiles + n - 1) / n) * ((nb + size - 1) / size);
+    if (!*stages || t < *stages) *stages = t, *cluster = size, *clusters = n;
+  }
+  return 0;
+}
+template <int KIND>
+static int launch_kt_k(aotcu_ctx* c, KtParams& P) {
+  int size = 0, n = 0;
+  long stages;
+  if (int rc = kt_shape<KIND>(c, P.n_tiles, P.cols / 256, &size, &n, &stages)) return rc;
+  return size == 2 ? launch_kt_c<KIND, 2>(c, P, n) : size == 4 ? launch_kt_c<KIND, 4>(c, P, n) : launch_kt_c<KIND, 8>(c, P, n);
+}
+// The matrices of one kind of `call` (all of them have it), activations in the kernel's order.
+static int launch_kt_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xt, int xf_nt) {
+  const int kind = call.seg[0].kind, rows = call.pair ? KT_ROWS / 2 : KT_ROWS;
+  KtParams P = {};
+  for (int s = 0; s < call.nseg; s++) {
+    P.seg[s] = call.seg[s];
+    P.tiles_before[s] = call.pair ? 0 : P.n_tiles;
+    if (!call.pair || s == 0) P.n_tiles += (call.seg[s].rows + rows - 1) / rows;
+  }
+  P.nseg = call.nseg;
+  P.pair = call.pair;
+  P.cols = (int)call.cols;
+  P.epilogue = call.epilogue;
+  P.xf_nt = xf_nt;
+  for (size_t t0 = 0; t0 < call.m; t0 += KT_MAX_M) {
+    P.m = (int)std::min<size_t>(KT_MAX_M, call.m - t0);
+    P.nt = (P.m + 7) / 8;
+    P.xf = xt + (t0 / 8) * XT_BLOCK;
+    for (int s = 0; s < call.nseg; s++) P.seg[s].out = call.seg[s].out + t0 * (size_t)call.seg[s].rows;
+    const int rc = kind == Q4_K ? launch_kt_k<Q4_K>(c, P) : kind == Q5_K ? launch_kt_k<Q5_K>(c, P) : launch_kt_k<Q6_K>(c, P);
+    if (rc) return rc;
+  }
+  return 0;
+}
+// Which of the two: 0 by estimates, 1 kmma.cuh, 2 ktensor.cuh (option "k_tensor").
+// Estimates in microseconds, fitted to 1620 timings (20 matrices of each kind, 2 to 64 rows): a
+// launch, and per stage a part that does not depend on the batch (bringing and unpacking weights) and
+// one that does. On these the choice is 1.2 % from the better kernel on average. kmma.cuh has the
+// small products, where the shorter start counts (4096 x 4096 x 8 Q4_K: 8.9 against 10.4), and from
+// 16 to 24 rows on almost everything is ktensor.cuh's (24576 x 4096 x 64 Q4_K 44 against 74, Q6_K 48
+// against 100).
+static int g_k_tensor = 0;
+static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
+  struct Cost {
+    double launch, stage, rows;
+  };
+  static const Cost mma[3] = {{5.87, 0.826, 0.374}, {5.54, 1.026, 0.381}, {4.82, 1.488, 0.454}};  // rows: a group of 8
+  static const Cost tensor[3] = {{7.50, 0.633, 0.252}, {7.37, 0.674, 0.257}, {6.78, 1.029, 0.193}};  // rows: a group of 16
+  const bool can = call.x_mode != 2 || call.xt;
+  *yes = can && g_k_tensor == 2;
+  if (!can || g_k_tensor) return 0;
+  const int kind = call.seg[0].kind, k = kind == Q4_K ? 0 : kind == Q5_K ? 1 : 2, tiles = kt_tiles(call), nb = (int)(call.cols / 256);
+  int rt, wk, size = 0, n = 0;
+  long stages;
+  const double s_mma = kmma_shape(c, call, &rt, &wk);
+  if (int rc = kind == Q4_K ? kt_shape<Q4_K>(c, tiles, nb, &size, &n, &stages)
+               : kind == Q5_K ? kt_shape<Q5_K>(c, tiles, nb, &size, &n, &stages) : kt_shape<Q6_K>(c, tiles, nb, &size, &n, &stages))
+    return rc;
+  double t_mma = 0.0, t_tensor = 0.0;
+  for (size_t t0 = 0; t0 < call.m; t0 += KT_MAX_M) {
+    const size_t m = std::min<size_t>(KT_MAX_M, call.m - t0);
+    t_mma += mma[k].launch + s_mma * (mma[k].stage + mma[k].rows * (double)((m + 7) / 8));
+    t_tensor += tensor[k].launch + (double)stages * (tensor[k].stage + tensor[k].rows * (double)((m + 15) / 16));
+  }
+  *yes = stages != 0 && t_tensor < t_mma;
+  return 0;
+}
+static int launch_k_batch(aotcu_ctx* c, const GemvCall& call) {
+  const int nb = (int)(call.cols / 256), nt = (int)((call.m + 7) / 8);
+  // the matrices kind by kind (a pair has one kind), and which kernel takes them
+  GemvCall part[3];
+  bool tensor[3];
+  int n = 0;
+  bool any[2] = {false, false};
   for (int kind : {Q4_K, Q5_K, Q6_K}) {
-    GemvCall one = call;
+    GemvCall& one = part[n];
+    one = call;
     one.nseg = 0;
     for (int s = 0; s < call.nseg; s++)
       if (call.seg[s].kind == kind) one.seg[one.nseg++] = call.seg[s];
-    if (one.nseg)
-      if (int rc = launch_kmma_one(c, one, xf, nt)) return rc;
+    if (!one.nseg) continue;
+    if (int rc = takes_kt(c, one, &tensor[n])) return rc;
+    any[tensor[n++]] = true;
   }
+  const uint8_t *xf = reinterpret_cast<const uint8_t*>(call.x), *xt = call.xt;
+  if (call.x_mode != 2) {
+    const size_t xf_bytes = any[0] ? (size_t)nt * nb * XF_BLOCK : 0, xt_bytes = any[1] ? (size_t)nt * nb * XT_BLOCK : 0;
+    if (const int rc = ctx_workspace(c, xf_bytes + xt_bytes)) return rc;
+    uint8_t *f = any[0] ? c->ximg : nullptr, *t = any[1] ? c->ximg + xf_bytes : nullptr;
+    if (int rc = launch(c, xf_kernel, dim3((unsigned)nt * nb), dim3(256), 0, xf, call.x_mode, f, t, (int)call.m, nb)) return rc;
+    xf = f;
+    xt = t;
+  }
+  for (int i = 0; i < n; i++)
+    if (int rc = tensor[i] ? launch_kt_one(c, part[i], xt, nt) : launch_kmma_one(c, part[i], xf, nt)) return rc;
   return 0;
 }
 
@@ -406,27 +593,6 @@ static int launch_q80_stream_k(aotcu_ctx* c, const Q80StreamParams& P, int nr, i
   if (nt == 16) return launch_q80_stream_t<KIND, 2, 16>(c, P, grid, smem);
   if (nt == 8) return nr == 2 ? launch_q80_stream_t<KIND, 2, 8>(c, P, grid, smem) : launch_q80_stream_t<KIND, 1, 8>(c, P, grid, smem);
   return nr == 2 ? launch_q80_stream_t<KIND, 2, 1>(c, P, grid, smem) : launch_q80_stream_t<KIND, 1, 1>(c, P, grid, smem);
-}
-// 2-D tensor map over 32-bit elements: [dim1][dim0] with rows `stride_bytes` apart, box
-// [box1][box0]. cuTensorMapEncodeTiled comes from the driver through the runtime (no link
-// against libcuda). Returns false when the driver refuses the map.
-static bool tensor_map_2d(CUtensorMap* out, CUtensorMapDataType dtype, const void* base, size_t dim0, size_t dim1, size_t stride_bytes,
-                          int box0, int box1) {
-  using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult st;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &st) != cudaSuccess || st != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
-  if (!encode) return false;
-  const cuuint64_t gdim[2] = {dim0, dim1}, gstride[1] = {stride_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)box0, (cuuint32_t)box1}, estride[2] = {1, 1};
-  return encode(out, dtype, 2, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // A weight matrix as rows of u32 words, box of four rows by one chunk.
 static bool weight_tensor_map(CUtensorMap* out, const uint8_t* w, size_t rows, size_t row_bytes, int chunk_bytes) {
@@ -843,7 +1009,7 @@ static int launch_float_multi(aotcu_ctx* c, const GemvCall& call, size_t span) {
 
 // K-quant products of two or three rows: gemv_stream_kernel<3>, one lane per super-block, grid = (row
 // ranges) x (groups of activation rows). Returns 1 when the call does not fit.
-static int g_wide_multi = 1;       // option "wide_multi": 0 sends these products to kmma.cuh as well
+static int g_wide_multi = 1;       // option "wide_multi": 0 sends these products to kmma.cuh or ktensor.cuh as well
 static int g_wide_multi_work = 0;  // option "wide_multi_work": weight rows x activation rows up to which every batch takes it
 // Its time grows with the batch where kmma_kernel's hardly depends on it (us, this kernel first; Q4_K
 // 2048x2048: 3.7 and 4.5 at 2 rows, 4.6 and 4.5 at 3, 8.0 and 4.5 at 8; 14336x4096: 14.3 and 19.4, 20.1
@@ -978,9 +1144,9 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
   }
   ARG_CHECK(((uintptr_t)call.x % (P.x_image ? 16 : 4)) == 0, "activation blocks are misaligned");
 
-  // K-quant products of several activation rows: the tensor-core kernel of kmma.cuh, but for the
+  // K-quant products of several activation rows: the kernels of kmma.cuh and ktensor.cuh, but for the
   // smallest batches one lane per super-block against every row. A Gpu keeps its activations in
-  // kmma's order (xf_rows) whatever the batch: half of a layer's products are pairs or mixed kinds,
+  // their orders (xf_rows) whatever the batch: half of a layer's products are pairs or mixed kinds,
   // which the one-lane kernel does not take, and a prompt of two costs what one of three does.
   if (act == ACT_Q8_K && call.m >= 2) {
     if (takes_tc(call)) return launch_gemm_tc(c, call);
@@ -988,7 +1154,7 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
       const int rc = launch_gemv_stream_multi(c, call, span);
       if (rc <= 0) return rc;  // 1: a pair or a very long row
     }
-    const int rc = launch_kmma(c, call);
+    const int rc = launch_k_batch(c, call);
     if (rc <= 0) return rc;  // 1: no conversion buffer
   }
   if (act == ACT_Q8_0 && g_q80_chunks) {
@@ -1127,7 +1293,8 @@ struct aotcu_gpu {
   size_t buf_len[AOTCU_N_BUFS] = {};
   float* rope_table = nullptr;        // n_ctx x rot_dim
   float* rope_table_local = nullptr;  // swa layers
-  uint8_t* aqk = nullptr;             // Q8_K block images or fragments, max_batch rows of max(dim, q_dim, hidden)
+  uint8_t* aqk = nullptr;             // Q8_K block images or the first array of xf_store, max_batch rows of max(dim, q_dim, hidden)
+  uint8_t* axt = nullptr;             // the second array (as many blocks)
   uint8_t* aq0 = nullptr;             // Q8_0 block images
   size_t aqk_bytes = 0, aq0_bytes = 0;
   float* attn_scratch = nullptr;      // scores for contexts that do not fit shared memory
@@ -1202,10 +1369,12 @@ static void note_write(aotcu_gpu* g, const float* p, size_t n) {
   if (meets(g->bufs[AOTCU_BUF_LOGITS], g->buf_len[AOTCU_BUF_LOGITS])) g->h_logits_fresh = false;  // the host copy made by aotcu_forward
 }
 
-// Q8_K activations of several rows are kept in the fragment order of kmma.cuh, those of a single
+// Q8_K activations of several rows are kept in the orders of xf_store, those of a single
 // row (and of chunks sent to the tcgen05 kernels) as block images. Fragments come in whole groups of
 // eight rows, so a few rows that are longer than any of the model's (operator calls) may fit the
 // buffer as images only.
+// The second array of xf_store: a single token group is read by kmma.cuh alone.
+static uint8_t* xt_of(const aotcu_gpu* g, size_t m) { return m > 8 ? g->axt : nullptr; }
 static bool xf_rows(const aotcu_gpu* g, size_t n, size_t m) {
   return m >= 2 && g_tc_force <= 0 && (m + 7) / 8 * (n / 256) * XF_BLOCK <= g->aqk_bytes;
 }
@@ -1230,7 +1399,7 @@ static int ensure_quantized(aotcu_gpu* g, const float* src, size_t n, size_t m, 
     ARG_CHECK(xf || images_fit(g, act, n, m), "%zu rows of %zu floats exceed the quantized-activation buffer", m, n);
     int nblk = (int)(n * m / 256);
     if (xf) {
-      if (int rc = launch(c, quantize_xf_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, (int)m, (int)(n / 256))) return rc;
+      if (int rc = launch(c, quantize_xf_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, xt_of(g, m), (int)m, (int)(n / 256))) return rc;
     } else {
       if (int rc = launch(c, quantize_q8k_kernel, dim3(grid_for(c, nblk, 8)), dim3(256), 0, src, g->aqk, nblk, 1)) return rc;
     }
@@ -1270,6 +1439,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   P.q8k_out = (q && g->need_q8k && n % 256 == 0 && (xf || images_fit(g, ACT_Q8_K, n, m))) ? g->aqk : nullptr;
   P.q80_out = (q && g->need_q80 && n % 32 == 0 && images_fit(g, ACT_Q8_0, n, m)) ? g->aq0 : nullptr;
   P.xf_nt = P.q8k_out && xf ? (int)((m + 7) / 8) : 0;
+  P.xt_out = xt_of(g, m);
   size_t smem = (2 * n + 12) * sizeof(float);
   ARG_CHECK(smem <= c->max_smem, "rmsnorm row of %zu floats does not fit shared memory", n);
   note_write(g, dst, (m - 1) * dst_stride + n);
@@ -1334,6 +1504,7 @@ static int gpu_matmul(aotcu_gpu* g, float* dst, const aotcu_tensor& t, const flo
   call.cols = t.cols;
   call.x = act_images(g, act, src);
   call.x_mode = act_mode(g, act);
+  call.xt = xt_of(g, m);
   call.m = m;
   call.epilogue = accumulate ? EPI_ACCUM : EPI_STORE;
   call.prep[0] = prep_of(g, t, m);
@@ -1364,6 +1535,7 @@ static int gpu_mv3(aotcu_gpu* g, float* const dst[3], const aotcu_tensor* const 
     call.cols = t[a]->cols;
     call.x = act_images(g, act, src);
     call.x_mode = act_mode(g, act);
+    call.xt = xt_of(g, m);
     call.m = m;
     if (int rc = launch_gemv(g->c, call)) return rc;
   }
@@ -1385,6 +1557,7 @@ static int gpu_gate_up(aotcu_gpu* g, float* hb, float* hb2, const aotcu_tensor& 
     call.cols = gate.cols;
     call.x = act_images(g, act, src);
     call.x_mode = act_mode(g, act);
+    call.xt = xt_of(g, m);
     call.m = m;
     call.epilogue = gelu ? EPI_STORE : EPI_SILU_MUL;
     call.prep[0] = prep_of(g, gate, m);
@@ -2362,8 +2535,11 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   G_TRY(cudaMallocHost(&g->h_pinned, (g->max_batch + 8) * sizeof(int)));
   G_TRY(cudaMallocHost(&g->h_logits, (size_t)d.vocab * sizeof(float)));
   G_TRY(cudaStreamSynchronize(c->stream));
-#undef G_TRY
   if (int rc = mega_setup(g)) return bail(rc);
+  // (last: what the one-kernel step exchanges between CTAs keeps its place in memory, which its time
+  // depends on by up to 3 %)
+  G_TRY(cudaMalloc(&g->axt, (g->aqk_bytes + XF_BLOCK - 1) / XF_BLOCK * XT_BLOCK));
+#undef G_TRY
   *out = g;
   return 0;
 }
@@ -2382,6 +2558,7 @@ void aotcu_gpu_free(aotcu_gpu* g) {
   cudaFree(g->rope_table);
   cudaFree(g->rope_table_local);
   cudaFree(g->aqk);
+  cudaFree(g->axt);
   cudaFree(g->aq0);
   cudaFree(g->attn_scratch);
   cudaFree(g->d_step);
@@ -2885,6 +3062,16 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
   }
   if (!strcmp(name, "q80_chunks")) {  // process-wide: Q4_0 / Q5_0 / Q8_0 products on the chunk-streaming kernel (1, default)
     g_q80_chunks = value != 0;
+    return 0;
+  }
+  if (!strcmp(name, "k_tensor")) {  // process-wide: see takes_kt
+    ARG_CHECK(value >= 0 && value <= 2, "k_tensor is 0, 1 or 2");
+    g_k_tensor = value;
+    return 0;
+  }
+  if (!strcmp(name, "kt_cluster")) {  // process-wide: cluster size of the K-quant batch kernel, 0 by shape
+    ARG_CHECK(value == 0 || value == 2 || value == 4 || value == 8, "kt_cluster is 0, 2, 4 or 8");
+    g_kt_cluster = value;
     return 0;
   }
   if (!strcmp(name, "wide_multi_work")) {  // process-wide: see takes_one_lane

@@ -19,17 +19,18 @@ __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait_at(smem_addr(bar), parity); }
 // Wait for phase `parity` with an iteration limit. On expiry the error word is
 // set and false is returned; the caller leaves its loop and the kernel returns
 // normally (its copies in flight are bounded by the barrier's own transaction
@@ -49,6 +50,13 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                    smem_addr(dst)),
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
+}
+
+// After a wait gave up: whatever phase the barrier is in, leave it the time that its copies need.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar) {
+  for (uint32_t parity = 0; parity < 2; parity++)
+    for (uint32_t it = 0; it < (1u << 10); ++it)
+      if (mbar_try_wait(bar, parity)) break;
 }
 
 // Copy the byte range [src, src+len) so that it lands at `slot + (src & 15)`:

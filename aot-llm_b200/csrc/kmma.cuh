@@ -1,5 +1,6 @@
 // Q4_K / Q5_K / Q6_K matrices against 2..64 activation rows on warp-level int8 tensor-core
-// tiles (matmul_rows of crates/aot-kernels/src/matvec.rs:479-522).
+// tiles (matmul_rows of crates/aot-kernels/src/matvec.rs:479-522): the batches and matrices that are
+// too small for ktensor.cuh.
 //
 // What bounds it. A product costs, per 16 weight rows x 64 tokens x 256 weights, 64 (Q6_K: 128)
 // MMAs of 8 issue cycles and four integer multiply-adds per MMA and lane for the sub-block
@@ -44,9 +45,9 @@ constexpr int KM_MAX_M = 64;
 constexpr int KM_PARK = 2;       // token groups whose terms are parked at a time
 constexpr int KM_B_SLOTS = 3;    // token groups in a ring
 
-// Reference-layout BlockQ8_K (292 bytes) or block images (304 bytes) -> fragments; a warp per
-// (token slot, super-block), slots past the last token zeroed.
-__global__ void __launch_bounds__(256) xf_kernel(const uint8_t* __restrict__ x, int x_image, uint8_t* __restrict__ out, int m, int nb) {
+// Reference-layout BlockQ8_K (292 bytes) or block images (304 bytes) -> the orders of xf_store; a warp
+// per (token slot, super-block), slots past the last token zeroed.
+__global__ void __launch_bounds__(256) xf_kernel(const uint8_t* __restrict__ x, int x_image, uint8_t* __restrict__ xf, uint8_t* __restrict__ xt, int m, int nb) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nt = (m + 7) >> 3;
@@ -63,8 +64,7 @@ __global__ void __launch_bounds__(256) xf_kernel(const uint8_t* __restrict__ x, 
     if (lane < 16) bs = reinterpret_cast<const int16_t*>(p + (x_image ? XK_BSUMS : 260))[lane];
     d = *reinterpret_cast<const float*>(p + (x_image ? XK_D : 0));
   }
-  uint8_t* o = out + ((size_t)b * nt + (tok >> 3)) * XF_BLOCK;
-  xf_store(o, tok & 7, lane, w0, w1, bs, d);
+  xf_store(xf, xt, tok, b, nt, lane, w0, w1, bs, d);
 }
 
 struct KmmaParams {
@@ -88,12 +88,6 @@ __device__ __forceinline__ void mma_s8s8_k16(int (&c)[4], uint32_t a0, uint32_t 
   asm volatile("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
                : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                : "r"(a0), "r"(a1), "r"(b0), "r"(0));
-}
-// Byte i of w, sign-extended: a permute whose upper selectors replicate the byte's sign.
-__device__ __forceinline__ int sext_byte(uint32_t w, int i) {
-  int r;
-  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"(i | (i | 8) << 4 | (i | 8) << 8 | (i | 8) << 12));
-  return r;
 }
 __device__ __forceinline__ uint32_t half2_of_int(int v) {  // (v, v), |v| <= 2048
   const uint32_t h = __half_as_ushort(__int2half_rn(v));

@@ -25,6 +25,16 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+// Byte i of w, sign-extended: a permute whose upper selectors replicate the byte's sign.
+__device__ __forceinline__ int sext_byte(uint32_t w, int i) {
+  return (int)prmt(w, 0, i | (i | 8) << 4 | (i | 8) << 8 | (i | 8) << 12);
+}
+
 // Two f32 values in one register pair: one instruction for two round-to-nearest operations.
 typedef unsigned long long F2;
 __device__ __forceinline__ F2 f2_pack(float a, float b) {

@@ -105,24 +105,38 @@ __device__ __forceinline__ void warp_quantize_q8k_vals(const float (&v)[8], uint
   if (lane == 0) *dptr = r.d;
 }
 
-// Activations of several rows in the order the tensor-core products read them ("XF", see
-// kmma.cuh): [super-block][token group of 8], XF_BLOCK bytes each. Lane l of the warp holds the
-// quants 8l .. 8l+7 of token `g` of the group; lanes 0..15 the sums of the 16-element groups.
-constexpr int XF_BLOCK = 2336;
-constexpr int XF_BSUMS = 2048;
-constexpr int XF_D = 2304;
-__device__ __forceinline__ void xf_store(uint8_t* o, int g, int lane, uint32_t w0, uint32_t w1, int bsum, float d) {
-  const int s = lane >> 1, h = lane & 1;
-  uint32_t* q = reinterpret_cast<uint32_t*>(o + ((s >> 2) * 32 + g * 4 + 2 * h) * 16 + (s & 3) * 4);
-  q[0] = w0;
-  q[4] = w1;
-  if (lane < 16)
-    reinterpret_cast<__half*>(o + XF_BSUMS + (g * 4 + ((lane & 7) >> 1)) * 8)[(lane >> 3) * 2 + (lane & 1)] = __int2half_rn(bsum);
-  if (lane == 0) *reinterpret_cast<float*>(o + XF_D + 4 * g) = d;
+// Activations of several rows in the orders in which the tensor-core products read them: two arrays of
+// blocks, [super-block][token group of 8], XF_BLOCK bytes each for kmma.cuh and XT_BLOCK bytes each for
+// ktensor.cuh.
+constexpr int XF_BLOCK = 2336, XF_BSUMS = 2048, XF_D = 2304;
+constexpr int XT_BLOCK = 2368, XT_BSUMS = 2048, XT_D = 2304, XT_SUMS = 2336;
+// Token tok of nt groups, super-block b; either array may be absent. Lane l of the warp holds the quants
+// 8l .. 8l+7; lanes 0..15 the sums of the 16-element groups.
+__device__ __forceinline__ void xf_store(uint8_t* xf, uint8_t* xt, int tok, int b, int nt, int lane, uint32_t w0, uint32_t w1, int bsum, float d) {
+  const int g = tok & 7, s = lane >> 1, h = lane & 1;
+  const size_t at = (size_t)b * nt + (tok >> 3);
+  const __half bs = __int2half_rn(bsum);
+  if (xf) {
+    uint8_t* const o = xf + at * XF_BLOCK;
+    uint32_t* q = reinterpret_cast<uint32_t*>(o + ((s >> 2) * 32 + g * 4 + 2 * h) * 16 + (s & 3) * 4);
+    q[0] = w0;
+    q[4] = w1;
+    if (lane < 16) reinterpret_cast<__half*>(o + XF_BSUMS + (g * 4 + ((lane & 7) >> 1)) * 8)[(lane >> 3) * 2 + (lane & 1)] = bs;
+    if (lane == 0) *reinterpret_cast<float*>(o + XF_D + 4 * g) = d;
+  }
+  if (xt) {
+    uint8_t* const o = xt + at * XT_BLOCK;
+    *reinterpret_cast<uint2*>(o + s * 128 + g * 16 + h * 8) = make_uint2(w0, w1);
+    if (lane < 16) reinterpret_cast<__half*>(o + XT_BSUMS + (lane >> 3) * 128 + g * 16)[lane & 7] = bs;
+    int sum = lane < 16 ? bsum : 0;
+#pragma unroll
+    for (int i = 8; i > 0; i >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, i);
+    if (lane < 2) *reinterpret_cast<uint32_t*>(o + (lane ? XT_SUMS : XT_D) + 4 * g) = lane ? (uint32_t)(-4096 * sum) : __float_as_uint(d);
+  }
 }
 // Block b of row `tok` (of nt groups of 8 rows), quantized straight into that order. `wide`: src is
 // 16-byte aligned (a buffer read at an offset of the caller's need not be).
-__device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, int tok, int b, int nt, bool wide) {
+__device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, uint8_t* xt, int tok, int b, int nt, bool wide) {
   const int lane = threadIdx.x & 31;
   float v[8];
   if (wide) {
@@ -136,7 +150,7 @@ __device__ __forceinline__ void warp_quantize_xf(const float* src, uint8_t* xf, 
   const Q8kLane r = warp_q8k_lane(v);
   const int s2 = r.s + __shfl_xor_sync(0xffffffffu, r.s, 1);
   const int bs = __shfl_sync(0xffffffffu, s2, (2 * lane) & 31);
-  xf_store(xf + ((size_t)b * nt + (tok >> 3)) * XF_BLOCK, tok & 7, lane, r.w0, r.w1, bs, r.d);
+  xf_store(xf, xt, tok, b, nt, lane, r.w0, r.w1, bs, r.d);
 }
 
 template <bool CG = false>
@@ -181,12 +195,12 @@ __global__ void quantize_q8k_kernel(const float* __restrict__ x, uint8_t* __rest
   for (int b = wid; b < n_blocks; b += nw) warp_quantize_q8k(x + (size_t)b * 256, out + (size_t)b * (image ? XIMG_K : 292), image);
 }
 // m rows of nb blocks into the fragment order.
-__global__ void quantize_xf_kernel(const float* __restrict__ x, uint8_t* __restrict__ xf, int m, int nb) {
+__global__ void quantize_xf_kernel(const float* __restrict__ x, uint8_t* __restrict__ xf, uint8_t* __restrict__ xt, int m, int nb) {
   pdl_launch_dependents();
   pdl_wait();
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5, nt = (m + 7) >> 3;
   const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // blocks lie 1024 bytes apart
-  for (int i = wid; i < m * nb; i += nw) warp_quantize_xf(x + (size_t)i * 256, xf, i / nb, i % nb, nt, wide);
+  for (int i = wid; i < m * nb; i += nw) warp_quantize_xf(x + (size_t)i * 256, xf, xt, i / nb, i % nb, nt, wide);
 }
 __global__ void quantize_q80_kernel(const float* __restrict__ x, uint8_t* __restrict__ out, int n_blocks, int image) {
   pdl_launch_dependents();
@@ -228,7 +242,8 @@ struct RmsnormParams {
   float eps;
   int accumulate;    // out[i] = out[i] + y[i] (Gemma post-norm residual join)
   uint8_t* q8k_out;  // images, n/256 per row
-  int xf_nt;         // > 0: q8k_out in fragment order instead, this many groups of 8 rows
+  int xf_nt;         // > 0: q8k_out and xt_out (if not null) in the orders of xf_store instead, this many groups of 8 rows
+  uint8_t* xt_out;
   uint8_t* q80_out;  // images, n/32 per row
 };
 
@@ -259,7 +274,7 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   if (P.q8k_out) {
     int nb = P.n / 256;
     for (int b = warp; b < nb; b += nwarps) {
-      if (P.xf_nt) warp_quantize_xf(row + b * 256, P.q8k_out, blockIdx.x, b, P.xf_nt, true);
+      if (P.xf_nt) warp_quantize_xf(row + b * 256, P.q8k_out, P.xt_out, blockIdx.x, b, P.xf_nt, true);
       else warp_quantize_q8k(row + b * 256, P.q8k_out + ((size_t)blockIdx.x * nb + b) * XIMG_K, 1);
     }
   }

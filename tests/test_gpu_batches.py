@@ -59,6 +59,72 @@ def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, kind):
     _run(pkg, ob, ctx, kind, w.reshape(-1), xs, m, rows, cols, f"kind {kind} at the bounds")
 
 
+@pytest.fixture
+def cluster_kernel(pkg, ctx):
+    """K-quant batches on the tcgen05 kernel of clusters whatever their size."""
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)
+    g.set_option("k_tensor", 2)
+    g.set_option("wide_multi", 0)
+    yield g
+    for name, value in (("k_tensor", 0), ("wide_multi", 1), ("kt_cluster", 0)):
+        g.set_option(name, value)
+    g.close()
+
+
+# Fewer super-blocks than CTAs in a cluster, a last stage with some of them, rows that tensor copies
+# cannot take (Q6_K: 768 and 2304 columns), a partial row tile, several tiles per cluster, token groups
+# of every parity and a second launch.
+@pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("cluster", [2, 4, 8])
+def test_k_quant_clusters(pkg, ob, ctx, cluster_kernel, kind, cluster):
+    cluster_kernel.set_option("kt_cluster", cluster)
+    for rows, cols, ms in ((1, 256, (2, 64)), (129, 2048, (8, 17, 33, 48)), (300, 768, (25, 65)), (9700, 2304, (64,))):
+        w = make_weights(pkg, kind, rows, cols, 25 + kind + rows, "uniform")
+        for m in ms:
+            _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m} clusters of {cluster}")
+
+
+@pytest.mark.parametrize("kind", [Q4_K, Q6_K])
+def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel, kind):
+    rows, cols, m = 70, 2048, 40                       # a pair: 64 rows of each per tile
+    ws = [make_weights(pkg, kind, rows, cols, 27 + i, "uniform") for i in range(2)]
+    b = ws[0].reshape(rows * cols // 256, -1)
+    if kind == Q6_K:                                   # quants 31 or -32 times -128, and the largest of Q4_K
+        b[:, :192], b[:, 192:208] = np.where(np.arange(b.shape[0])[:, None] % 2, 0xFF, 0x00), 0x80
+    else:
+        b[:, 4:] = 0xFF
+    xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+    xs[:cols], xs[cols:2 * cols] = 1.0, -1.0
+    q = ob.quantize_act(kind, xs)
+    dq, outs = ctx.to_device(q.view(np.uint8)), [ctx.alloc(m * rows * 4) for _ in ws]
+    want = [ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols) for w in ws]
+    ctx.matmul2(kind, *outs, *[ctx.to_device(w) for w in ws], dq, m, rows, cols)
+    for o, x in zip(outs, want):
+        assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), x, "pair")
+    off = 2 if kind == Q6_K else 16                    # a base that tensor copies cannot take, or can
+    d = ctx.to_device(np.concatenate([np.zeros(off, np.uint8), ws[0].reshape(-1), np.zeros(256, np.uint8)]))
+    ctx.matmul(kind, outs[0], d.ptr + off, dq, m, rows, cols)
+    assert_bits_equal(outs[0].download(np.float32, m * rows).reshape(m, rows), want[0], f"offset {off}")
+    ctx.device_status()
+
+
+def test_k_quant_clusters_in_a_model(pkg, ob, ctx, cluster_kernel):
+    """q/k/v of mixed kinds, gated pairs and products onto the residual, chunk after chunk."""
+    spec = pkg.model.tiny("llama", n_layer=2, kinds=lambda layer, tensor: Q6_K if tensor in ("wv", "down", "output") else Q4_K, dim=512, hidden=768, vocab=600)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 160, 64)
+    om = ob.model_from_spec(spec, 160, 64, n_threads=4)
+    pos = 0
+    for n in (64, 21, 9):
+        toks = np.random.default_rng(n).integers(0, 600, n).tolist()
+        g.forward_batch(toks, pos, True)
+        om.forward_batch(toks, pos, True)
+        assert_bits_equal(g.logits(), om.logits(), f"logits after a chunk of {n} at {pos}")
+        pos += n
+    g.close()
+    ctx.device_status()
+
+
 @pytest.mark.parametrize("kind", [0, 1, 2])           # F32, F16, BF16
 @pytest.mark.parametrize("rows,cols", [(1, 8), (33, 72), (600, 1016), (5000, 128)])
 def test_float_tile_edges(pkg, ob, ctx, kind, rows, cols):
