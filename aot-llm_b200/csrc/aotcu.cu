@@ -25,6 +25,7 @@
 #include "mega.cuh"
 #include "q80mma.cuh"
 #include "q80stream.cuh"
+#include "q80tensor.cuh"
 #include "floatmulti.cuh"
 #include "floatstream.cuh"
 #include "ops.cuh"
@@ -668,6 +669,16 @@ static double q80_stream_us(const aotcu_ctx* c, int kind, size_t cols, size_t ro
 // Matrices that it does not take (rows not in fours, mixed kinds) would go to the whole-row kernel,
 // whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows, 14337x4096 103 and 784.
 constexpr size_t Q80_MMA_MIN_BATCH = 17, Q80_MMA_MIN_BATCH_ODD = 32;
+// CTAs of a product, `*wt` warps each: at most five share a row unit.
+static size_t q80_mma_ctas(const GemvCall& call, int* wt, int* n_tcta = nullptr) {
+  const int ntg = (int)((call.m + 7) / 8), nw = (ntg + QM_NG - 1) / QM_NG, parts = (nw + 4) / 5;
+  *wt = (nw + parts - 1) / parts;
+  if (n_tcta) *n_tcta = parts;
+  const int rows = call.pair ? 16 : 16 * QM_RT;
+  size_t units = 0;
+  for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) units += (call.seg[s].rows + rows - 1) / rows;
+  return units * parts;
+}
 static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
   if (call.m < Q80_MMA_MIN_BATCH || call.cols % 256) return 1;
   for (int s = 0; s < call.nseg; s++)
@@ -679,15 +690,11 @@ static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
   P.m = (int)call.m;
   P.epilogue = call.epilogue;
   P.ntg = ntg;
-  const int nw = (ntg + QM_NG - 1) / QM_NG;  // warps that the batch takes: at most five share a row unit
-  P.n_tcta = (nw + 4) / 5;
-  P.wt = (nw + P.n_tcta - 1) / P.n_tcta;
+  const size_t ctas = q80_mma_ctas(call, &P.wt, &P.n_tcta);
   const int rows = call.pair ? 16 : 16 * QM_RT;
-  size_t units = 0;
-  for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) units += (call.seg[s].rows + rows - 1) / rows;
   bool streams = true;  // what launch_q80_stream asks of the matrices
   for (int s = 0; s < call.nseg; s++) streams = streams && call.seg[s].rows % 4 == 0 && call.seg[s].kind == call.seg[0].kind;
-  if (streams ? q80_mma_us(c, call.seg[0].kind, call.cols, P.wt, units * P.n_tcta) > 0.98 * q80_stream_us(c, call.seg[0].kind, call.cols, (call.pair ? 2 : 1) * span, call.m)
+  if (streams ? q80_mma_us(c, call.seg[0].kind, call.cols, P.wt, ctas) > 0.98 * q80_stream_us(c, call.seg[0].kind, call.cols, (call.pair ? 2 : 1) * span, call.m)
               : call.m < Q80_MMA_MIN_BATCH_ODD)
     return 1;
   if (const int rc = ctx_workspace(c, (size_t)ntg * nb * X0F_BLOCK)) return rc;
@@ -710,6 +717,107 @@ static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
     if (kind == Q4_0) rc = call.pair ? launch_q80_mma_t<Q4_0, true>(c, P, grid) : launch_q80_mma_t<Q4_0, false>(c, P, grid);
     else if (kind == Q5_0) rc = call.pair ? launch_q80_mma_t<Q5_0, true>(c, P, grid) : launch_q80_mma_t<Q5_0, false>(c, P, grid);
     else rc = call.pair ? launch_q80_mma_t<Q8_0, true>(c, P, grid) : launch_q80_mma_t<Q8_0, false>(c, P, grid);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+// Q4_0 / Q5_0 / Q8_0 products of several activation rows on the tcgen05 kernel of q80tensor.cuh.
+// Returns 1 when the call does not fit.
+static int g_q80_tensor = 0;  // 0: by estimates; 1: never; 2: wherever it can (option "q80_tensor")
+static int g_q80_tensor_rows = 0;  // tokens per CTA, 0 by estimates (option "q80_tensor_rows")
+template <int KIND, int TPW>
+static int launch_qt_t(aotcu_ctx* c, QtParams& P) {
+  static bool attr_set[64] = {};
+  if (c->device < 0 || c->device >= 64 || !attr_set[c->device]) {
+    CU_TRY(cudaFuncSetAttribute(qt_kernel<KIND, TPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->max_smem));
+    if (c->device >= 0 && c->device < 64) attr_set[c->device] = true;
+  }
+  P.n_raw = QT_MAX_RAW;
+  while (P.n_raw > 1 && qt_smem<KIND, TPW>(P.n_raw, P.pair != 0) > c->max_smem) P.n_raw--;
+  return launch(c, qt_kernel<KIND, TPW>, dim3(std::min(c->n_sm, P.n_tiles * P.n_groups)), dim3(QT_THREADS), qt_smem<KIND, TPW>(P.n_raw, P.pair != 0), P);
+}
+template <int KIND>
+static int launch_qt_k(aotcu_ctx* c, QtParams& P, int tpw) {
+  return tpw == 4 ? launch_qt_t<KIND, 4>(c, P) : tpw == 6 ? launch_qt_t<KIND, 6>(c, P) : launch_qt_t<KIND, 8>(c, P);
+}
+// Microseconds by estimate (fitted to 14336 x 4096 and 2048 x 2048, three kinds, 17 to 64 rows: within
+// 4 %): rounds of CTAs, each the same time per block; the fewest for 16, 24 or 32 tokens per CTA.
+static double q80_tensor_us(const aotcu_ctx* c, int kind, size_t cols, size_t tiles, size_t m, int* tpw) {
+  static const struct {
+    int tpw;
+    double block;
+  } shape[3] = {{4, 0.343}, {6, 0.405}, {8, 0.475}};
+  double best = 1e30;
+  for (const auto& s : shape) {
+    if (g_q80_tensor_rows && g_q80_tensor_rows != 4 * s.tpw) continue;
+    const size_t items = tiles * ((m + 4 * s.tpw - 1) / (4 * s.tpw));
+    const double us = 7 + (double)((items + c->n_sm - 1) / c->n_sm) * (cols / 32) * s.block * (kind == Q5_0 ? 1.025 : 1.0);
+    if (us < best) best = us, *tpw = s.tpw;
+  }
+  return best;
+}
+static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
+  if (g_q80_tensor == 1 || call.m < 2 || call.cols % 256) return 1;
+  for (int s = 0; s < call.nseg; s++)
+    if ((uintptr_t)call.seg[s].w & 15) return 1;
+  if (call.pair && call.seg[0].kind != call.seg[1].kind) return 1;
+  const int nb = (int)(call.cols / 32), box = call.pair ? KT_ROWS / 2 : KT_ROWS;
+  int tiles = 0;
+  for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) tiles += (call.seg[s].rows + box - 1) / box;
+  int tpw = 8;
+  const double us = q80_tensor_us(c, call.seg[0].kind, call.cols, tiles, call.m, &tpw);
+  if (!g_q80_tensor) {
+    // Taken where its estimate is below those of the kernels after it (us, this kernel first: Q8_0 14336 x
+    // 4096 129 and, on q80_mma_kernel, 196 at 64 rows, 59 and 114 at 20; Q4_0 4096 x 4096 51 and, on
+    // q80_stream_kernel, 78 at 40 rows, 50 and 29 at 16; 24576 x 4096 94 and 59 at 8). Up to 8 rows the
+    // streaming kernel is nowhere the slower one. Of 576 timings (16 matrices, three kinds, 4 to 64 rows) those
+    // from 9 rows on gain a third on average; none loses more than 6 %.
+    bool streams = true;
+    for (int s = 0; s < call.nseg; s++) streams = streams && call.seg[s].rows % 4 == 0 && call.seg[s].kind == call.seg[0].kind;
+    if (streams && call.m <= 8) return 1;
+    double other = 1e30;
+    if (streams) other = q80_stream_us(c, call.seg[0].kind, call.cols, (call.pair ? 2 : 1) * span, call.m);
+    if (call.m >= Q80_MMA_MIN_BATCH) {
+      int wt = 0;
+      const size_t ctas = q80_mma_ctas(call, &wt);
+      other = std::min(other, q80_mma_us(c, call.seg[0].kind, call.cols, wt, ctas));
+    } else if (!streams) {  // the whole-row kernel, linear in the batch (9001 x 1536: 3.6 us a row, Q5_0 5.2)
+      other = 3 + (double)call.m * (call.pair ? 2 : 1) * span * call.cols * (call.seg[0].kind == Q5_0 ? 3.7e-7 : 2.6e-7);
+    }
+    if (us > 0.97 * other) return 1;
+  }
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(call.x);
+  if (call.x_mode != 1) {
+    if (const int rc = ctx_workspace(c, call.m * nb * X0_STRIDE)) return rc;
+    const int n_blocks = (int)(call.m * nb);
+    if (int rc = launch(c, q80_to_image_kernel, dim3(grid_for(c, (size_t)n_blocks * 9, 256)), dim3(256), 0, x, c->ximg, n_blocks)) return rc;
+    x = c->ximg;
+  }
+  if ((uintptr_t)x & 15) return 1;
+  QtParams P = {};
+  P.cols = (int)call.cols;
+  P.m = (int)call.m;
+  P.pair = call.pair;
+  P.epilogue = call.epilogue;
+  P.n_groups = (int)((call.m + 4 * tpw - 1) / (4 * tpw));
+  P.err = c->d_err;
+  if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, x, (size_t)nb * (X0_STRIDE / 4), call.m, (size_t)nb * X0_STRIDE, QT_CHUNK * (X0_STRIDE / 4), 4 * tpw))
+    return 1;
+  for (int kind : {Q4_0, Q5_0, Q8_0}) {
+    P.nseg = P.n_tiles = 0;
+    const size_t row_bytes = kind_row_bytes(kind, call.cols);
+    for (int s = 0; s < call.nseg; s++) {
+      if (call.seg[s].kind != kind) continue;
+      if (!tensor_map_2d(&P.map[P.nseg], CU_TENSOR_MAP_DATA_TYPE_UINT32, call.seg[s].w, row_bytes / 4, call.seg[s].rows, row_bytes, (int)(row_bytes / nb * QT_CHUNK / 4), box))
+        return fail(AOTCU_ERR_CUDA, "tensor map of a weight matrix refused");
+      P.tiles_before[P.nseg] = P.n_tiles;
+      P.seg[P.nseg++] = call.seg[s];
+      if (!call.pair || P.nseg == 1) P.n_tiles += (call.seg[s].rows + box - 1) / box;
+    }
+    if (call.pair) P.tiles_before[1] = 0;
+    if (!P.nseg) continue;
+    const int rc = kind == Q4_0 ? launch_qt_k<Q4_0>(c, P, tpw) : kind == Q5_0 ? launch_qt_k<Q5_0>(c, P, tpw) : launch_qt_k<Q8_0>(c, P, tpw);
     if (rc) return rc;
   }
   return 0;
@@ -1158,6 +1266,8 @@ static int launch_gemv(aotcu_ctx* c, const GemvCall& call) {
     if (rc <= 0) return rc;  // 1: no conversion buffer
   }
   if (act == ACT_Q8_0 && g_q80_chunks) {
+    const int tc = launch_q80_tensor(c, call, span);
+    if (tc <= 0) return tc;
     const int mc = launch_q80_mma(c, call, span);
     if (mc <= 0) return mc;
     const int rc = launch_q80_stream(c, call, span);
@@ -3067,6 +3177,16 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
   if (!strcmp(name, "k_tensor")) {  // process-wide: see takes_kt
     ARG_CHECK(value >= 0 && value <= 2, "k_tensor is 0, 1 or 2");
     g_k_tensor = value;
+    return 0;
+  }
+  if (!strcmp(name, "q80_tensor")) {  // process-wide: see launch_q80_tensor
+    ARG_CHECK(value >= 0 && value <= 2, "q80_tensor is 0, 1 or 2");
+    g_q80_tensor = value;
+    return 0;
+  }
+  if (!strcmp(name, "q80_tensor_rows")) {
+    ARG_CHECK(value == 0 || value == 16 || value == 24 || value == 32, "q80_tensor_rows is 0, 16, 24 or 32");
+    g_q80_tensor_rows = value;
     return 0;
   }
   if (!strcmp(name, "kt_cluster")) {  // process-wide: cluster size of the K-quant batch kernel, 0 by shape

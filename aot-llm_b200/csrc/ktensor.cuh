@@ -136,6 +136,12 @@ __device__ __forceinline__ bool kt_wait(const Ring& R, uint64_t* bar, uint32_t p
   return kt_wait_slow(smem_addr(bar), parity, R.abort, R.err);
 }
 
+// The same with the loop in line, after the first test: for warps whose registers leave no room for a call.
+__device__ __forceinline__ bool kt_wait_inline(const Ring& R, uint64_t* bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return ring_wait(R, bar, parity);
+}
+
 // ---- tensor memory ------------------------------------------------------------------------
 __device__ __forceinline__ void kt_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(

@@ -191,6 +191,58 @@ def test_q80_sizes_around_the_choice_of_kernel(pkg, ob, ctx, kind, rows, cols, m
     g.close()
 
 
+@pytest.fixture
+def q80_tensor(pkg, ctx):
+    """Q8_0-family batches on the tcgen05 kernel whatever their size."""
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)
+    g.set_option("q80_tensor", 2)
+    yield g
+    g.set_option("q80_tensor", 0)
+    g.set_option("q80_tensor_rows", 0)
+    g.close()
+
+
+# One row, a partial row tile, several tiles per CTA, one to three stages; every number of tokens per CTA
+# with a partial group; pairs; all products of one sign with zeros, whose sums must not become -0.
+@pytest.mark.parametrize("kind", [3, 4, 5])           # Q4_0, Q5_0, Q8_0
+@pytest.mark.parametrize("tokens", [16, 24, 32])
+def test_q80_on_tcgen05(pkg, ob, ctx, q80_tensor, kind, tokens):
+    q80_tensor.set_option("q80_tensor_rows", tokens)
+    for rows, cols, ms in ((1, 256, (2, 65)), (301, 768, (17, 33, 64)), (19100, 256, (40,))):
+        w = make_weights(pkg, kind, rows, cols, 45 + kind + rows)
+        for m in ms:
+            _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}, {tokens} per CTA")
+    rows, cols, m = 70, 512, 37
+    ws = [make_weights(pkg, kind, rows, cols, 53 + i) for i in range(2)]
+    b = ws[1].reshape(rows * cols // 32, -1)
+    b[:, 2:] = 0x80 if kind == 5 else 0x00            # the lowest quants
+    xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+    xs[:cols] = 0.0
+    q = ob.quantize_act(kind, xs)
+    outs = [ctx.alloc(m * rows * 4) for _ in ws]
+    ctx.matmul2(kind, *outs, *[ctx.to_device(w) for w in ws], ctx.to_device(q.view(np.uint8)), m, rows, cols)
+    for o, w in zip(outs, ws):
+        assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols), "pair")
+    ctx.device_status()
+
+
+def test_q80_on_tcgen05_in_a_model(pkg, ob, ctx, q80_tensor):
+    """Gated pairs and products onto the residual, chunk after chunk."""
+    spec = pkg.model.tiny("llama", n_layer=2, kinds=lambda layer, tensor: 3 if tensor in ("gate", "up", "wq") else 5, dim=512, hidden=768, vocab=600)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 160, 64)
+    om = ob.model_from_spec(spec, 160, 64, n_threads=4)
+    pos = 0
+    for n in (64, 21, 9):
+        toks = np.random.default_rng(n).integers(0, 600, n).tolist()
+        g.forward_batch(toks, pos, True)
+        om.forward_batch(toks, pos, True)
+        assert_bits_equal(g.logits(), om.logits(), f"logits after a chunk of {n} at {pos}")
+        pos += n
+    g.close()
+    ctx.device_status()
+
+
 @pytest.mark.parametrize("kind,rows,cols", [(0, 20, 64), (1, 37, 20), (3, 301, 256), (5, 64, 96), (6, 40, 256), (8, 3, 512)])
 def test_batches_longer_than_a_pass(pkg, ob, ctx, kind, rows, cols):
     m = 4096 + 9 if cols % 32 == 0 else 8192 + 3
