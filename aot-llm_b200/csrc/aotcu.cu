@@ -1715,9 +1715,14 @@ static int gpu_qk_post(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos0,
 static size_t attn_smem_bytes(int nq, int head_dim, size_t max_len) { return ((size_t)attn_fixed(nq, head_dim) + max_len * nq) * sizeof(float); }
 static size_t attn_ctas(int nq, size_t m, int n_head, int n_kv_head) { return ((m * (n_head / n_kv_head) + nq - 1) / nq) * n_kv_head; }
 
+// Where a launch of attention shall leave its output's quantized form; whether it will.
+struct AttnQuant {
+  uint8_t *xf = nullptr, *xt = nullptr, *q80 = nullptr;
+  bool done = false;
+};
 static int launch_attention(aotcu_ctx* c, float* out, const float* q, const float* kc, const float* vc, float* scratch,
                             const int* pos_ptr, size_t pos0, size_t m, int n_head, int n_kv_head, int head_dim,
-                            size_t n_ctx, size_t window) {
+                            size_t n_ctx, size_t window, AttnQuant* quant = nullptr) {
   AttnParams P = {};
   P.out = out;
   P.q = q;
@@ -1741,6 +1746,15 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
   // eight queries share a K element best; four, where eight leave SMs idle, halve the score and
   // exponential phases (7 rows at position 300, 28 or 56 CTAs)
   const int nq = attn_ctas(ATTN_NQ, m, n_head, n_kv_head) < (size_t)c->n_sm ? ATTN_NQ / 2 : ATTN_NQ;
+  if (quant) {
+    quant->done = quant->xf ? attn_quantizes(nq, head_dim, n_head / n_kv_head) : head_dim % 32 == 0;
+    if (quant->done) {
+      P.xf = quant->xf;
+      P.xt = quant->xt;
+      P.xf_nt = (int)((m + 7) / 8);
+      P.q80 = quant->q80;
+    }
+  }
   size_t smem = attn_smem_bytes(nq, head_dim, max_len);
   const bool in_smem = smem <= c->max_smem;
   if (!in_smem) {
@@ -1766,14 +1780,31 @@ static int launch_attention(aotcu_ctx* c, float* out, const float* q, const floa
   return launch(c, kernel, dim3((unsigned)n_kv_head, groups), dim3(ATTN_THREADS), smem, P);
 }
 
+// next: the matrix whose product reads the output, if it is known; the output's quantized form is made on
+// the way where that fits.
 static int gpu_attention(aotcu_gpu* g, float* out, const float* q, size_t li, const int* pos_ptr, size_t pos0, size_t m,
-                         size_t window) {
+                         size_t window, const aotcu_tensor* next = nullptr) {
   const aotcu_dims& d = g->head.dims;
-  size_t kvd = (size_t)d.n_kv_head * d.head_dim;
-  note_write(g, out, m * d.n_head * d.head_dim);
-  return launch_attention(g->c, out, q, g->bufs[AOTCU_BUF_KCACHE] + li * g->n_ctx * kvd,
-                          g->bufs[AOTCU_BUF_VCACHE] + li * g->n_ctx * kvd, g->attn_scratch, pos_ptr, pos0, m, d.n_head,
-                          d.n_kv_head, d.head_dim, g->n_ctx, window);
+  const size_t kvd = (size_t)d.n_kv_head * d.head_dim, qd = (size_t)d.n_head * d.head_dim;
+  note_write(g, out, m * qd);
+  const int act = next ? kind_act((int)next->kind) : ACT_F32;
+  AttnQuant quant;
+  if (m >= 2 && act == ACT_Q8_K && qd % 256 == 0 && xf_rows(g, qd, m)) quant.xf = g->aqk, quant.xt = xt_of(g, m);
+  if (m >= 2 && act == ACT_Q8_0 && images_fit(g, act, qd, m)) quant.q80 = g->aq0;
+  const bool want = quant.xf || quant.q80;
+  if (int rc = launch_attention(g->c, out, q, g->bufs[AOTCU_BUF_KCACHE] + li * g->n_ctx * kvd,
+                                g->bufs[AOTCU_BUF_VCACHE] + li * g->n_ctx * kvd, g->attn_scratch, pos_ptr, pos0, m, d.n_head,
+                                d.n_kv_head, d.head_dim, g->n_ctx, window, want ? &quant : nullptr))
+    return rc;
+  if (quant.done) {
+    g->qsrc = aotcu_gpu::QSrc();
+    g->qsrc.ptr = out;
+    g->qsrc.n = qd;
+    g->qsrc.m = m;
+    g->qsrc.q8k = g->qsrc.xf = quant.xf != nullptr;
+    g->qsrc.q80 = quant.q80 != nullptr;
+  }
+  return 0;
 }
 
 // ---- the generated forward pass, interpreted (emit.rs) -----------------------------------------------
@@ -1829,7 +1860,7 @@ static int layer_forward(aotcu_gpu* g, size_t li, const int* pos_ptr, size_t pos
   // emit.rs:278-286: q/k norm, rope, store_kv
   if (int rc = gpu_qk_post(g, li, pos_ptr, pos0, m, batch)) return rc;
   // emit.rs:287
-  if (int rc = gpu_attention(g, xb, q, li, pos_ptr, pos0, m, window)) return rc;
+  if (int rc = gpu_attention(g, xb, q, li, pos_ptr, pos0, m, window, &l.wo)) return rc;
   // emit.rs:288-295
   const bool tp = g->tp && g->tp->world > 1;
   if (d.post_norms) {

@@ -40,3 +40,22 @@ def test_misaligned_caches_are_refused(pkg, ctx):
             ctx.attention(dq, dq, k, v, 1, 1, hd, n, 0, 1, 0)
         assert e.value.status == pkg.lib.ERR_BAD_ARG
     ctx.device_status()
+
+
+# Heads whose outputs make whole blocks of 256 in a CTA of four or eight queries (one or two rows of a
+# group of heads), heads that do not, and 32-value blocks; few rows and many.
+@pytest.mark.parametrize("kind", [5, 6])              # Q8_0, Q4_K
+@pytest.mark.parametrize("n_head,n_kv,head_dim", [(8, 2, 64), (8, 1, 64), (4, 1, 128), (2, 2, 128), (8, 2, 32), (1, 1, 256)])
+def test_attention_output_quantized_on_the_way(pkg, ob, ctx, kind, n_head, n_kv, head_dim):
+    spec = pkg.model.build("attn", dim=512, hidden=512, n_layer=2, n_head=n_head, n_kv_head=n_kv, head_dim=head_dim, vocab=300, seed=5,
+                           kinds=lambda layer, tensor: 6 if tensor in ("token_embd", "output") else kind, n_ctx_train=512, rope_base=1e4, eps=1e-5)
+    g, om = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 96, 64), ob.model_from_spec(spec, 96, 64, n_threads=4)
+    pos = 0
+    for n in (64, 3, 9):
+        toks = np.random.default_rng(n).integers(0, 300, n).tolist()
+        g.forward_batch(toks, pos, True)
+        om.forward_batch(toks, pos, True)
+        assert_bits_equal(g.logits(), om.logits(), f"logits after a chunk of {n} at {pos}")
+        pos += n
+    g.close()
+    ctx.device_status()
