@@ -1538,6 +1538,7 @@ static int gpu_rmsnorm(aotcu_gpu* g, float* dst, size_t dst_stride, const float*
   RmsnormParams P = {};
   P.x = src;
   P.w = w;
+  P.w_constant = 1;
   P.out = dst;
   P.n = (int)n;
   P.x_stride = (int)src_stride;

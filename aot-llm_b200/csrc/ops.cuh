@@ -245,6 +245,7 @@ struct RmsnormParams {
   int xf_nt;         // > 0: q8k_out and xt_out (if not null) in the orders of xf_store instead, this many groups of 8 rows
   uint8_t* xt_out;
   uint8_t* q80_out;  // images, n/32 per row
+  int w_constant;    // w is a model's: no kernel before this one writes it
 };
 
 __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
@@ -253,7 +254,19 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   float* sq = sm_f + ((P.n + 3) & ~3);  // n, 16-byte aligned, zero-filled to a multiple of eight
   __shared__ SeqSumScratch ssc;
   pdl_launch_dependents();
+  // The weights are asked for first: behind the sum they cost a trip to L2 of their own.
+  constexpr int NW = 8;
+  float w[NW];
+  auto weights = [&]() {
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+      const int i = threadIdx.x + k * 512;
+      w[k] = i < P.n ? P.w[i] : 0.0f;
+    }
+  };
+  if (P.w_constant) weights();
   pdl_wait();
+  if (!P.w_constant) weights();
   const float* x = P.x + (size_t)blockIdx.x * P.x_stride;
   float* out = P.out + (size_t)blockIdx.x * P.out_stride;
   for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
@@ -264,11 +277,15 @@ __global__ void __launch_bounds__(512) rmsnorm_kernel(const RmsnormParams P) {
   if (P.n + (int)threadIdx.x < ((P.n + 7) & ~7)) sq[P.n + threadIdx.x] = 0.0f;
   float ss = group_seq_sum(sq, P.n, &ssc, CtaGroup{(int)threadIdx.x, (int)blockDim.x, 0});
   float r = fdiv(1.0f, fsqrt(fadd(fdiv(ss, (float)P.n), P.eps)));
-  for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
-    float y = fmul(fmul(row[i], r), P.w[i]);
+  auto scale = [&](int i, float wi) {
+    float y = fmul(fmul(row[i], r), wi);
     row[i] = y;
     if (P.out) out[i] = P.accumulate ? fadd(out[i], y) : y;
-  }
+  };
+#pragma unroll
+  for (int k = 0; k < NW; k++)
+    if ((int)threadIdx.x + k * 512 < P.n) scale(threadIdx.x + k * 512, w[k]);
+  for (int i = threadIdx.x + NW * 512; i < P.n; i += 512) scale(i, P.w[i]);
   __syncthreads();
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   if (P.q8k_out) {
