@@ -330,41 +330,68 @@ __global__ void __launch_bounds__(128) qk_post_kernel(const QkPostParams P) {
   __shared__ float sq[256];
   __shared__ float slot;
   pdl_launch_dependents();
-  pdl_wait();
-  const int hs = blockIdx.x, tok = blockIdx.y;
-  const int pos = (P.pos_ptr ? *P.pos_ptr : P.pos0) + tok;
-  const int hd = P.head_dim;
+  // Nothing here but loads and a few operations, so what is needed is asked for together: the model's tables
+  // before the previous kernel ends, the value row beside the head.
+  const int hs = blockIdx.x, tok = blockIdx.y, t = threadIdx.x;
+  const int hd = P.head_dim, half = P.rot_dim / 2;  // at most 256: two elements and one pair per thread
   const bool is_q = hs < P.n_head;
   const int kvh = hs - P.n_head;
   const int q_dim = P.n_head * hd, kv_dim = P.n_kv_head * hd;
   const float* src = is_q ? P.q + (size_t)tok * q_dim + hs * hd : P.k + (size_t)tok * kv_dim + kvh * hd;
+  const float* vs = is_q ? nullptr : P.v + (size_t)tok * kv_dim + kvh * hd;
   const float* nw = is_q ? P.q_norm : P.k_norm;
-  for (int i = threadIdx.x; i < hd; i += blockDim.x) {
-    float a = src[i];
-    h[i] = a;
-    sq[i] = fmul(a, a);
+  float w[2] = {0.0f, 0.0f}, a[2], v[2] = {0.0f, 0.0f}, c = 0.0f, s = 0.0f;
+  if (nw) {
+    if (t < hd) w[0] = nw[t];
+    if (t + 128 < hd) w[1] = nw[t + 128];
+  }
+  auto angles = [&](int pos) {
+    if (t < half) {
+      c = P.rope_table[(size_t)pos * P.rot_dim + 2 * t];
+      s = P.rope_table[(size_t)pos * P.rot_dim + 2 * t + 1];
+    }
+  };
+  if (!P.pos_ptr) angles(P.pos0 + tok);
+  pdl_wait();
+  const int pos = (P.pos_ptr ? *P.pos_ptr : P.pos0) + tok;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int i = t + 128 * k;
+    if (i < hd) {
+      a[k] = src[i];
+      if (vs) v[k] = vs[i];
+    }
+  }
+  if (P.pos_ptr) angles(pos);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int i = t + 128 * k;
+    if (i < hd) {
+      h[i] = a[k];
+      sq[i] = fmul(a[k], a[k]);
+    }
   }
   if (nw) {
-    float ss = block_seq_sum(sq, hd, &slot);
-    float r = fdiv(1.0f, fsqrt(fadd(fdiv(ss, (float)hd), P.eps)));
-    for (int i = threadIdx.x; i < hd; i += blockDim.x) h[i] = fmul(fmul(h[i], r), nw[i]);
+    const float ss = block_seq_sum(sq, hd, &slot);
+    const float r = fdiv(1.0f, fsqrt(fadd(fdiv(ss, (float)hd), P.eps)));
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (t + 128 * k < hd) h[t + 128 * k] = fmul(fmul(a[k], r), w[k]);
   }
   __syncthreads();
-  const float* cs = P.rope_table + (size_t)pos * P.rot_dim;
-  const int half = P.rot_dim / 2;
   float* dst = is_q ? P.q + (size_t)tok * q_dim + hs * hd : P.k_cache + (size_t)pos * kv_dim + kvh * hd;
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    int i0 = P.neox ? i : 2 * i, i1 = P.neox ? i + half : 2 * i + 1;
-    float c = cs[2 * i], s = cs[2 * i + 1];
-    float x0 = h[i0], x1 = h[i1];
+  if (t < half) {
+    const int i0 = P.neox ? t : 2 * t, i1 = P.neox ? t + half : 2 * t + 1;
+    const float x0 = h[i0], x1 = h[i1];
     dst[i0] = fsub(fmul(x0, c), fmul(x1, s));
     dst[i1] = fadd(fmul(x0, s), fmul(x1, c));
   }
-  for (int i = P.rot_dim + threadIdx.x; i < hd; i += blockDim.x) dst[i] = h[i];
-  if (!is_q) {
-    const float* vs = P.v + (size_t)tok * kv_dim + kvh * hd;
-    float* vd = P.v_cache + (size_t)pos * kv_dim + kvh * hd;
-    for (int i = threadIdx.x; i < hd; i += blockDim.x) vd[i] = vs[i];
+  float* vd = is_q ? nullptr : P.v_cache + (size_t)pos * kv_dim + kvh * hd;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int i = t + 128 * k;
+    if (i >= P.rot_dim && i < hd) dst[i] = h[i];
+    if (vd && i < hd) vd[i] = v[k];
   }
 }
 
