@@ -111,9 +111,9 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void cluster_arrive(uint32_t mapped_bar) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_sync_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 // 16 bytes into a CTA of the cluster; its barrier counts them when they are there.
 __device__ __forceinline__ void cluster_st128(uint32_t mapped, uint32_t mapped_bar, const float (&v)[4]) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(mapped), "f"(v[0]),
@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
   // stage times the quads it owns
   const int my_quads = (4 * nt16 - rank + C - 1) / C;
   auto t_expect = [&](int stage, uint64_t* bar) { mbar_expect_tx(bar, (uint32_t)((min(C, nb - stage % n_st * C) - (stage % n_st * C + rank < nb ? 1 : 0)) * my_quads * KT_ROWS * 16)); };
+  if (warp == 2 && P.tma && lane < P.nseg) prefetch_map(&P.map[lane]);
   if (tid < KT_BARS) {  // a thread per barrier
     constexpr int S4 = KT_MAX_SLOTS;
     const int i = tid;
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  cluster_sync();  // every CTA's barriers are set up before anyone arrives on them
+  cluster_sync_arrive();  // every CTA's barriers are set up before another CTA writes there: the warps that do wait for it
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
   // matrix and first row of a tile
@@ -511,6 +512,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
     }
   } else if (warp < 20) {
     // ---- terms ----
+    cluster_sync_wait();
     const int row = (tid - 384) & 127, e16 = (warp - 12) >> 2;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t owner[4];  // terms ring of the CTAs that own this thread's quads 4 * e16 + qd (+ 8h); the barriers lie t_bar after it
@@ -602,6 +604,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
     }
   } else {
     // ---- sums in block order, and what is done with them ----
+    cluster_sync_wait();
     const int row = tid - 640;
     const uint32_t empty_at = cluster_map(smem_addr(t_empty), lane & (C - 1));
     KtPos pt;
@@ -702,9 +705,11 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
     }
   }
   __syncwarp();
+  if (warp < 12) cluster_sync_wait();
   tc_fence_before();
   __syncthreads();
-  cluster_sync();  // nobody writes into a CTA that has left
+  cluster_sync_arrive();  // nobody writes into a CTA that has left
+  cluster_sync_wait();
   if (warp == 1) tc_dealloc(tmem, 512);
 }
 

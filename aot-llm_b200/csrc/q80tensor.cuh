@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
   float* const exchange = reinterpret_cast<float*>(raw_full + (QT_BARS + 3) / 2 * 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = P.cols >> 5, n_chunk = nb / QT_CHUNK, n_items = P.n_tiles * P.n_groups, trows = P.pair ? KT_ROWS / 2 : KT_ROWS;
+  if (warp == 0 && lane < 4 && (lane < P.nseg || lane == 3)) prefetch_map(lane == 3 ? &P.xmap : &P.map[lane]);
   if (tid < QT_BARS) {  // a thread per barrier
     const int i = tid;
     mbar_init(raw_full + i, i < QT_MAX_RAW ? 1 : i < 2 * QT_MAX_RAW ? 6 : i < 2 * QT_MAX_RAW + QT_SLOTS ? 5 : i < 2 * QT_MAX_RAW + 2 * QT_SLOTS ? 17
