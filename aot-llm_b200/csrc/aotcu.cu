@@ -72,6 +72,11 @@ struct aotcu_ctx {
   uint8_t* ximg = nullptr;              // activations converted from reference-layout blocks (ctx_workspace)
   size_t ximg_bytes = 0;
   size_t ximg_limit = SIZE_MAX;         // option "workspace_mib"
+  // Kernels of batched products (options of the same names):
+  int k_tensor = 0;                     // 0: by estimates; 1: never; 2: wherever it can
+  int kt_cluster = 0;                   // CTAs of a cluster, 0 by shape
+  int q80_tensor = 0;                   // as k_tensor
+  int q80_tensor_rows = 0;              // tokens per CTA, 0 by estimates
 };
 
 constexpr size_t WEIGHT_PAD = 256;
@@ -457,7 +462,6 @@ static int launch_kt_c(aotcu_ctx* c, KtParams& P, int clusters) {
   c->launches++;
   return 0;
 }
-static int g_kt_cluster = 0;  // 0: by shape; else forced (option "kt_cluster")
 static int kt_tiles(const GemvCall& call) {
   const int rows = call.pair ? KT_ROWS / 2 : KT_ROWS;
   int tiles = 0;
@@ -471,7 +475,7 @@ template <int KIND>
 static int kt_shape(aotcu_ctx* c, int tiles, int nb, int* cluster, int* clusters, long* stages) {
   *stages = 0;
   for (int size : {4, 2, 8}) {
-    if (g_kt_cluster && g_kt_cluster != size) continue;
+    if (c->kt_cluster && c->kt_cluster != size) continue;
     int n = 0;
     if (int rc = size == 2 ? kt_clusters<KIND, 2>(c, &n) : size == 4 ? kt_clusters<KIND, 4>(c, &n) : kt_clusters<KIND, 8>(c, &n)) return rc;
     if (!n) continue;
@@ -518,7 +522,6 @@ static int launch_kt_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xt, 
 // small products, where the shorter start counts (4096 x 4096 x 8 Q4_K: 8.9 against 10.4), and from
 // 16 to 24 rows on almost everything is ktensor.cuh's (24576 x 4096 x 64 Q4_K 44 against 74, Q6_K 48
 // against 100).
-static int g_k_tensor = 0;
 static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
   struct Cost {
     double launch, stage, rows;
@@ -526,8 +529,8 @@ static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
   static const Cost mma[3] = {{5.87, 0.826, 0.374}, {5.54, 1.026, 0.381}, {4.82, 1.488, 0.454}};  // rows: a group of 8
   static const Cost tensor[3] = {{7.50, 0.633, 0.252}, {7.37, 0.674, 0.257}, {6.78, 1.029, 0.193}};  // rows: a group of 16
   const bool can = call.x_mode != 2 || call.xt;
-  *yes = can && g_k_tensor == 2;
-  if (!can || g_k_tensor) return 0;
+  *yes = can && c->k_tensor == 2;
+  if (!can || c->k_tensor) return 0;
   const int kind = call.seg[0].kind, k = kind == Q4_K ? 0 : kind == Q5_K ? 1 : 2, tiles = kt_tiles(call), nb = (int)(call.cols / 256);
   int rt, wk, size = 0, n = 0;
   long stages;
@@ -724,8 +727,6 @@ static int launch_q80_mma(aotcu_ctx* c, const GemvCall& call, size_t span) {
 
 // Q4_0 / Q5_0 / Q8_0 products of several activation rows on the tcgen05 kernel of q80tensor.cuh.
 // Returns 1 when the call does not fit.
-static int g_q80_tensor = 0;  // 0: by estimates; 1: never; 2: wherever it can (option "q80_tensor")
-static int g_q80_tensor_rows = 0;  // tokens per CTA, 0 by estimates (option "q80_tensor_rows")
 template <int KIND, int TPW>
 static int launch_qt_t(aotcu_ctx* c, QtParams& P) {
   static bool attr_set[64] = {};
@@ -750,7 +751,7 @@ static double q80_tensor_us(const aotcu_ctx* c, int kind, size_t cols, size_t ti
   } shape[3] = {{4, 0.343}, {6, 0.405}, {8, 0.475}};
   double best = 1e30;
   for (const auto& s : shape) {
-    if (g_q80_tensor_rows && g_q80_tensor_rows != 4 * s.tpw) continue;
+    if (c->q80_tensor_rows && c->q80_tensor_rows != 4 * s.tpw) continue;
     const size_t items = tiles * ((m + 4 * s.tpw - 1) / (4 * s.tpw));
     const double us = 7 + (double)((items + c->n_sm - 1) / c->n_sm) * (cols / 32) * s.block * (kind == Q5_0 ? 1.025 : 1.0);
     if (us < best) best = us, *tpw = s.tpw;
@@ -758,7 +759,7 @@ static double q80_tensor_us(const aotcu_ctx* c, int kind, size_t cols, size_t ti
   return best;
 }
 static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
-  if (g_q80_tensor == 1 || call.m < 2 || call.cols % 256) return 1;
+  if (c->q80_tensor == 1 || call.m < 2 || call.cols % 256) return 1;
   for (int s = 0; s < call.nseg; s++)
     if ((uintptr_t)call.seg[s].w & 15) return 1;
   if (call.pair && call.seg[0].kind != call.seg[1].kind) return 1;
@@ -767,7 +768,7 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
   for (int s = 0; s < (call.pair ? 1 : call.nseg); s++) tiles += (call.seg[s].rows + box - 1) / box;
   int tpw = 8;
   const double us = q80_tensor_us(c, call.seg[0].kind, call.cols, tiles, call.m, &tpw);
-  if (!g_q80_tensor) {
+  if (!c->q80_tensor) {
     // Taken where its estimate is below those of the kernels after it (us, this kernel first: Q8_0 14336 x
     // 4096 129 and, on q80_mma_kernel, 196 at 64 rows, 59 and 114 at 20; Q4_0 4096 x 4096 51 and, on
     // q80_stream_kernel, 78 at 40 rows, 50 and 29 at 16; 24576 x 4096 94 and 59 at 8). Up to 8 rows the
@@ -3206,24 +3207,24 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
     g_q80_chunks = value != 0;
     return 0;
   }
-  if (!strcmp(name, "k_tensor")) {  // process-wide: see takes_kt
+  if (!strcmp(name, "k_tensor")) {  // of the context: see takes_kt
     ARG_CHECK(value >= 0 && value <= 2, "k_tensor is 0, 1 or 2");
-    g_k_tensor = value;
+    g->c->k_tensor = value;
     return 0;
   }
-  if (!strcmp(name, "q80_tensor")) {  // process-wide: see launch_q80_tensor
+  if (!strcmp(name, "q80_tensor")) {  // of the context: see launch_q80_tensor
     ARG_CHECK(value >= 0 && value <= 2, "q80_tensor is 0, 1 or 2");
-    g_q80_tensor = value;
+    g->c->q80_tensor = value;
     return 0;
   }
-  if (!strcmp(name, "q80_tensor_rows")) {
+  if (!strcmp(name, "q80_tensor_rows")) {  // of the context: tokens per CTA
     ARG_CHECK(value == 0 || value == 16 || value == 24 || value == 32, "q80_tensor_rows is 0, 16, 24 or 32");
-    g_q80_tensor_rows = value;
+    g->c->q80_tensor_rows = value;
     return 0;
   }
-  if (!strcmp(name, "kt_cluster")) {  // process-wide: cluster size of the K-quant batch kernel, 0 by shape
+  if (!strcmp(name, "kt_cluster")) {  // of the context: cluster size of the K-quant batch kernel, 0 by shape
     ARG_CHECK(value == 0 || value == 2 || value == 4 || value == 8, "kt_cluster is 0, 2, 4 or 8");
-    g_kt_cluster = value;
+    g->c->kt_cluster = value;
     return 0;
   }
   if (!strcmp(name, "wide_multi_work")) {  // process-wide: see takes_one_lane
