@@ -1992,15 +1992,9 @@ static int mega_setup(aotcu_gpu* g) {
   if (per_sm < 1) return 0;
 
   auto seg = [&](const aotcu_tensor& t, float* out) { return GemvSeg{wptr(g, t), out, (int)t.rows, t.kind}; };
-  // Tagged vectors, two copies: residual, q, k, v, attention output, activated hidden; then the scores of split
-  // heads. Zeroed once: tag 0 is never waited for.
-  const size_t ll_copy = ((size_t)d.dim + qd + 2 * kvd + qd + (size_t)d.hidden + 15) / 16 * 16;
-  const size_t ll_words = 2 * ll_copy + (size_t)d.n_head * g->n_ctx;
-  CU_TRY(cudaMalloc(&g->d_ll, ll_words * sizeof(LLWord)));
-  CU_TRY(cudaMemset(g->d_ll, 0, ll_words * sizeof(LLWord)));
   auto make_op = [&](std::initializer_list<GemvSeg> segs, int pair, int cols, int epilogue, int ll) {
     MegaOp op = {};
-    op.ll = ll ? (int)ll_copy : 0;
+    op.ll = ll;
     size_t max_rb = 1;
     int span = 0, i = 0;
     for (const GemvSeg& sg : segs) {
@@ -2023,13 +2017,18 @@ static int mega_setup(aotcu_gpu* g) {
     megaop_derive(op);
     return op;
   };
+  // Tagged vectors: residual, q, k, v, attention output, activated hidden. Zeroed once:
+  // tag 0 is never waited for.
+  const size_t ll_words = (size_t)d.dim + qd + 2 * kvd + qd + (size_t)d.hidden + (size_t)d.n_head * g->n_ctx;
+  CU_TRY(cudaMalloc(&g->d_ll, ll_words * sizeof(LLWord)));
+  CU_TRY(cudaMemset(g->d_ll, 0, ll_words * sizeof(LLWord)));
   LLWord* const xl = reinterpret_cast<LLWord*>(g->d_ll);
   LLWord* const ql = xl + d.dim;
   LLWord* const kl = ql + qd;
   LLWord* const vl = kl + kvd;
   LLWord* const attl = vl + kvd;
   LLWord* const hbl = attl + qd;
-  LLWord* const scl = xl + 2 * ll_copy;
+  LLWord* const scl = hbl + d.hidden;
   auto as_out = [](LLWord* p) { return reinterpret_cast<float*>(p); };
   std::vector<StepLayer> hl(d.n_layer + 1);
   for (int i = 0; i < d.n_layer; i++) {
@@ -2060,7 +2059,7 @@ static int mega_setup(aotcu_gpu* g) {
   P.token_embd = wptr(g, g->head.token_embd);
   P.embd_kind = g->head.token_embd.kind;
   P.embd_row_bytes = kind_row_bytes(g->head.token_embd.kind, g->head.token_embd.cols);
-  P.xl = xl; P.ql = ql; P.kl = kl; P.vl = vl; P.attl = attl; P.hbl = hbl; P.scl = scl; P.ll_copy = (int)ll_copy;
+  P.xl = xl; P.ql = ql; P.kl = kl; P.vl = vl; P.attl = attl; P.hbl = hbl; P.scl = scl;
   P.x = g->bufs[AOTCU_BUF_X];
   P.logits = g->bufs[AOTCU_BUF_LOGITS]; P.k_cache = g->bufs[AOTCU_BUF_KCACHE]; P.v_cache = g->bufs[AOTCU_BUF_VCACHE];
   P.epoch = g->d_grid_bar + 1;

@@ -57,15 +57,6 @@ __device__ __forceinline__ void ll_store(LLWord* p, float v, uint32_t tag) {
   const LLWord w = ((LLWord)tag << 32) | (LLWord)__float_as_uint(v);
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
 }
-// The words that every CTA reads lie twice, `copy` words apart; even CTAs poll the first and odd ones the
-// second, so half as many polls meet at a vector's lines. A writer reads back its own first copy. With one
-// copy a step's time depends on where the words lie (TinyLlama shape at position 160: 760 to 808 us at eight
-// places, mean 785; with two 764 to 797, mean 781). 16 tokens with 1 / 2 copies: Q4_0 13019 / 12578 us, position
-// 1700 20136 / 19980, the 8B shape at 545 55991 / 55796.
-__device__ __forceinline__ void ll_store_both(LLWord* p, int copy, float v, uint32_t tag) {
-  ll_store(p, v, tag);
-  ll_store(p + copy, v, tag);
-}
 __device__ __forceinline__ LLWord ll_load(const LLWord* p) {
   LLWord w;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
@@ -184,7 +175,7 @@ struct MegaOp {
   GemvSeg seg[3];
   uint32_t row_bytes[3];
   int nseg, pair, cols, span_rows, rows_per_cta, tile_rows, epilogue;
-  int ll;  // not 0: outputs are tagged words (seg[].out points at LLWord), not plain floats, their copy that many words on
+  int ll;  // outputs are tagged words (seg[].out points at LLWord), not plain floats
   int cta_base, cta_rem;  // span_rows / grid and span_rows % grid: CTA b owns cta_base (+1 when b < cta_rem) rows
   // derived by the host so that no consumer warp divides: blocks per row, stride of a row's
   // terms in the warp's strip, units a strip holds, tiles of a CTA with cta_base / cta_base + 1 rows
@@ -213,7 +204,6 @@ struct StepParams {
   int embd_kind;
   size_t embd_row_bytes;
   LLWord *xl, *ql, *kl, *vl, *attl, *hbl;  // tagged activation vectors (residual, q, k, v, attention out, hidden)
-  int ll_copy;                             // words to their second copy
   float *x;                                // plain copy of the final residual stream, for readers outside the kernel
   float *logits, *k_cache, *v_cache;
   unsigned* epoch;                         // launch count; bumped by CTA 0 when the kernel ends
@@ -424,7 +414,7 @@ __device__ __forceinline__ void warp_flush(const MegaOp& op, const float* wterms
     if (lane < pend) {
       const float hv = op.epilogue == EPI_SILU_MUL ? silu_mul_call(v, up) : v;
       if (op.ll) {
-        ll_store_both(reinterpret_cast<LLWord*>(my_out), op.ll, hv, tag);
+        ll_store(reinterpret_cast<LLWord*>(my_out), hv, tag);
       } else {
         *my_out = hv;
         op.seg[1].out[my_out - op.seg[0].out] = up;
@@ -439,7 +429,7 @@ __device__ __forceinline__ void warp_flush(const MegaOp& op, const float* wterms
       part[(int)(reinterpret_cast<LLWord*>(my_out) - reinterpret_cast<LLWord*>(op.seg[0].out)) - part_row0] = v;
     } else if (op.ll) {
       // a residual row is only ever written by its owner, so its old value needs no tag check
-      ll_store_both(reinterpret_cast<LLWord*>(my_out), op.ll, op.epilogue == EPI_ACCUM ? fadd(my_old, v) : v, tag);
+      ll_store(reinterpret_cast<LLWord*>(my_out), op.epilogue == EPI_ACCUM ? fadd(my_old, v) : v, tag);
     } else {
       *my_out = op.epilogue == EPI_ACCUM ? fadd(__ldcg(my_out), v) : v;
     }
@@ -660,7 +650,7 @@ __device__ __forceinline__ void consume_step_q80(const MegaOp& op, const Ring& R
         for (int o = 4; o > 0; o >>= 1) v[i] = fadd(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
       if (writer) {
         const float r = op.pair ? silu_mul_call(v[0], v[1]) : accum ? fadd(old, v[0]) : v[0];
-        if (op.ll) ll_store_both(ll, op.ll, r, tag);
+        if (op.ll) ll_store(ll, r, tag);
         else *U.out = r;  // the output head
       }
     }
@@ -1043,7 +1033,7 @@ __device__ __forceinline__ void attention_chunked(const StepParams& P, int li, i
     if (md >= 0) o = value_mix(o, sc + c0, cur_buf + md, hd, cn);
     g.sync();
   }
-  if (md >= 0) ll_store_both(P.attl + h * hd + md, P.ll_copy, o, tag_out);
+  if (md >= 0) ll_store(P.attl + h * hd + md, o, tag_out);
 }
 
 // How `S` CTAs share one head when its cached rows do not fit one CTA's staging area.
@@ -1094,7 +1084,6 @@ __device__ __noinline__ void attn_split_prefetch(const float* k_cache, const flo
 struct AttnSplitArgs {
   int li, h, s, pos, tid, T;
   int head_dim, n_head, n_kv_head, n_ctx, small_floats, v_chunk, fast;
-  int ll_copy;
   uint32_t tag_out;
   float *k_cache, *v_cache;
   LLWord *scl, *attl;
@@ -1175,7 +1164,7 @@ __device__ __forceinline__ void attention_split(const AttnSplitArgs A) {
     pf.mark(27);
     g.sync();
   }
-  if (md >= 0) ll_store_both(A.attl + A.h * hd + d0 + md, A.ll_copy, o, A.tag_out);
+  if (md >= 0) ll_store(A.attl + A.h * hd + d0 + md, o, A.tag_out);
   pf.mark(24);
 }
 
@@ -1265,7 +1254,7 @@ __device__ __forceinline__ void phase_attention(const StepParams& P, int li, int
   pf.mark(20);
   if (SPLIT) {
     attention_split(AttnSplitArgs{li, h, split_s, pos, tid, T, P.head_dim, P.n_head, P.n_kv_head, P.n_ctx, P.small_floats, P.v_chunk,
-                                  P.fast, P.ll_copy, tag_out, P.k_cache, P.v_cache, P.scl, P.attl, M.scr, M.red, M.ss, M.abort, M.err, prof});
+                                  P.fast, tag_out, P.k_cache, P.v_cache, P.scl, P.attl, M.scr, M.red, M.ss, M.abort, M.err, prof});
     return;
   }
   if (!staged) {
@@ -1301,7 +1290,7 @@ __device__ __forceinline__ void phase_attention(const StepParams& P, int li, int
   // value mix, positions in order (ops.rs:208-214)
   {
     const int md = mix_dim(tid, T, hd);
-    if (md >= 0) ll_store_both(P.attl + h * hd + md, P.ll_copy, value_mix(0.0f, sc, vbuf + md, hd, n), tag_out);
+    if (md >= 0) ll_store(P.attl + h * hd + md, value_mix(0.0f, sc, vbuf + md, hd, n), tag_out);
   }
   pf.mark(24);
 }
@@ -1550,18 +1539,17 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
         }
       }
     }
-    const int ll_mine = (blockIdx.x & 1) ? P.ll_copy : 0;
     if ((ph & 1) == 0) {
       // attention norm -> q/k/v, ffn norm -> gate/up + SiLU, output norm -> logits
       const float* w = head ? P.output_norm : (ph == 0 ? L.attn_norm : L.ffn_norm);
       const uint32_t tin = ph == 0 ? tl : tl + 3u;  // residual after the previous layer's down / this layer's wo
-      phase_norm_quant<Q80>(!head || head_q80, P.xl + ll_mine, tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
+      phase_norm_quant<Q80>(!head || head_q80, P.xl, tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
                        SubProf{prof_on && ph == 0 && !head ? P.prof : nullptr, 0},
                        P.prof && (int)blockIdx.x == P.prof_cta && ph == 0 && !head && g.tid == (MEGA_CONSUMER_WARPS - 1) * 32 ? P.prof : nullptr);
     } else {
       // attention output -> wo, activated hidden -> down; both join the residual stream
-      if (ph == 1) phase_quant<Q80>(P.attl + ll_mine, tl + 2u, qd, M, g);
-      else phase_quant<Q80>(P.hbl + ll_mine, tl + 4u, P.hidden, M, g);
+      if (ph == 1) phase_quant<Q80>(P.attl, tl + 2u, qd, M, g);
+      else phase_quant<Q80>(P.hbl, tl + 4u, P.hidden, M, g);
     }
     if (!head) MEGA_PROF(slot);
     // q/k/v: tl+1, wo: tl+3, gate/up: tl+4, down: tl+5 (the head writes plain floats)
@@ -1603,7 +1591,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
             const float t = __shfl_sync(0xffffffffu, v, base + src);
             if (src < P.tp.world) sum = fadd(sum, t);
           }
-          if (i < r1 && sub == 0) ll_store_both(P.xl + i, P.ll_copy, fadd(ll_value(P.xl + i), sum), tag_out);
+          if (i < r1 && sub == 0) ll_store(P.xl + i, fadd(ll_value(P.xl + i), sum), tag_out);
         }
       }
     }
