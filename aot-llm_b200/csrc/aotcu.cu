@@ -1992,6 +1992,14 @@ static int mega_setup(aotcu_gpu* g) {
   if (per_sm < 1) return 0;
 
   auto seg = [&](const aotcu_tensor& t, float* out) { return GemvSeg{wptr(g, t), out, (int)t.rows, t.kind}; };
+  // Tagged vectors: residual, q, k, v, attention output, activated hidden; a second copy of the three that every
+  // CTA reads; the scores of split heads. Zeroed once: tag 0 is never waited for.
+  const size_t ll_copy = ((size_t)d.dim + qd + 2 * kvd + qd + (size_t)d.hidden + 15) / 16 * 16;
+  const size_t ll_words = 2 * ll_copy + (size_t)d.n_head * g->n_ctx;
+  CU_TRY(cudaMalloc(&g->d_ll, ll_words * sizeof(LLWord)));
+  CU_TRY(cudaMemset(g->d_ll, 0, ll_words * sizeof(LLWord)));
+  constexpr int PLAIN = 0, ONCE = -1;
+  const int twice = (int)ll_copy;
   auto make_op = [&](std::initializer_list<GemvSeg> segs, int pair, int cols, int epilogue, int ll) {
     MegaOp op = {};
     op.ll = ll;
@@ -2017,18 +2025,13 @@ static int mega_setup(aotcu_gpu* g) {
     megaop_derive(op);
     return op;
   };
-  // Tagged vectors: residual, q, k, v, attention output, activated hidden. Zeroed once:
-  // tag 0 is never waited for.
-  const size_t ll_words = (size_t)d.dim + qd + 2 * kvd + qd + (size_t)d.hidden + (size_t)d.n_head * g->n_ctx;
-  CU_TRY(cudaMalloc(&g->d_ll, ll_words * sizeof(LLWord)));
-  CU_TRY(cudaMemset(g->d_ll, 0, ll_words * sizeof(LLWord)));
   LLWord* const xl = reinterpret_cast<LLWord*>(g->d_ll);
   LLWord* const ql = xl + d.dim;
   LLWord* const kl = ql + qd;
   LLWord* const vl = kl + kvd;
   LLWord* const attl = vl + kvd;
   LLWord* const hbl = attl + qd;
-  LLWord* const scl = hbl + d.hidden;
+  LLWord* const scl = xl + 2 * ll_copy;
   auto as_out = [](LLWord* p) { return reinterpret_cast<float*>(p); };
   std::vector<StepLayer> hl(d.n_layer + 1);
   for (int i = 0; i < d.n_layer; i++) {
@@ -2037,14 +2040,14 @@ static int mega_setup(aotcu_gpu* g) {
     hl[i].ffn_norm = wf32(g, l.ffn_norm);
     hl[i].q_norm = d.qk_norm ? wf32(g, l.q_norm) : nullptr;
     hl[i].k_norm = d.qk_norm ? wf32(g, l.k_norm) : nullptr;
-    hl[i].qkv = make_op({seg(l.wq, as_out(ql)), seg(l.wk, as_out(kl)), seg(l.wv, as_out(vl))}, 0, d.dim, EPI_STORE, 1);
-    hl[i].wo = make_op({seg(l.wo, as_out(xl))}, 0, (int)qd, EPI_ACCUM, 1);
-    hl[i].gu = make_op({seg(l.gate, as_out(hbl)), seg(l.up, nullptr)}, 1, d.dim, EPI_SILU_MUL, 1);
-    hl[i].down = make_op({seg(l.down, as_out(xl))}, 0, d.hidden, EPI_ACCUM, 1);
+    hl[i].qkv = make_op({seg(l.wq, as_out(ql)), seg(l.wk, as_out(kl)), seg(l.wv, as_out(vl))}, 0, d.dim, EPI_STORE, ONCE);
+    hl[i].wo = make_op({seg(l.wo, as_out(xl))}, 0, (int)qd, EPI_ACCUM, twice);
+    hl[i].gu = make_op({seg(l.gate, as_out(hbl)), seg(l.up, nullptr)}, 1, d.dim, EPI_SILU_MUL, twice);
+    hl[i].down = make_op({seg(l.down, as_out(xl))}, 0, d.hidden, EPI_ACCUM, twice);
   }
   // The output head rides in the slot after the last layer (only its qkv field is used).
   hl[d.n_layer] = StepLayer{};
-  hl[d.n_layer].qkv = make_op({seg(out_t, g->bufs[AOTCU_BUF_LOGITS])}, 0, d.dim, EPI_STORE, 0);
+  hl[d.n_layer].qkv = make_op({seg(out_t, g->bufs[AOTCU_BUF_LOGITS])}, 0, d.dim, EPI_STORE, PLAIN);
   CU_TRY(cudaMalloc(&g->d_step_layers, hl.size() * sizeof(StepLayer) + 16));
   CU_TRY(cudaMemcpy(g->d_step_layers, hl.data(), hl.size() * sizeof(StepLayer), cudaMemcpyHostToDevice));
   CU_TRY(cudaMalloc(&g->d_grid_bar, 2 * sizeof(unsigned)));
@@ -2059,7 +2062,8 @@ static int mega_setup(aotcu_gpu* g) {
   P.token_embd = wptr(g, g->head.token_embd);
   P.embd_kind = g->head.token_embd.kind;
   P.embd_row_bytes = kind_row_bytes(g->head.token_embd.kind, g->head.token_embd.cols);
-  P.xl = xl; P.ql = ql; P.kl = kl; P.vl = vl; P.attl = attl; P.hbl = hbl; P.scl = scl;
+  P.xl = xl; P.ql = ql; P.kl = kl; P.vl = vl; P.attl = attl; P.hbl = hbl; P.scl = scl; P.ll_copy = twice;
+  for (int i : {0, 1}) P.xl_in[i] = xl + i * ll_copy, P.attl_in[i] = attl + i * ll_copy, P.hbl_in[i] = hbl + i * ll_copy;
   P.x = g->bufs[AOTCU_BUF_X];
   P.logits = g->bufs[AOTCU_BUF_LOGITS]; P.k_cache = g->bufs[AOTCU_BUF_KCACHE]; P.v_cache = g->bufs[AOTCU_BUF_VCACHE];
   P.epoch = g->d_grid_bar + 1;

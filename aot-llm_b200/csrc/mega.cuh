@@ -57,6 +57,17 @@ __device__ __forceinline__ void ll_store(LLWord* p, float v, uint32_t tag) {
   const LLWord w = ((LLWord)tag << 32) | (LLWord)__float_as_uint(v);
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
 }
+// The words that every CTA reads (residual, attention output, hidden) lie twice, `copy` words apart (copy <= 0:
+// once); even CTAs poll the first and odd ones the second, so half as many polls meet at a vector's lines. A
+// writer reads back its own first copy. A step's time depends on where the words lie, so both forms were timed
+// at 40 random places (24 and 20 in the second two), us a token, mean and standard deviation, once / twice:
+// TinyLlama shape Q4_K_M at position 160 802, 23 / 765, 11; at 1700 1235, 25 / 1194, 13; Q4_0 at 160 804, 9 / 799, 3;
+// the 8B shape at 545 3464, 28 / 3435, 24. (Copies of q, k and v, which nobody read, and one offset to the copy held
+// in a register instead of a second set of pointers made the 8B shape slower than one copy: 3500 against 3456.)
+__device__ __forceinline__ void ll_store_both(LLWord* p, int copy, float v, uint32_t tag) {
+  ll_store(p, v, tag);
+  if (copy > 0) ll_store(p + copy, v, tag);
+}
 __device__ __forceinline__ LLWord ll_load(const LLWord* p) {
   LLWord w;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
@@ -175,7 +186,7 @@ struct MegaOp {
   GemvSeg seg[3];
   uint32_t row_bytes[3];
   int nseg, pair, cols, span_rows, rows_per_cta, tile_rows, epilogue;
-  int ll;  // outputs are tagged words (seg[].out points at LLWord), not plain floats
+  int ll;  // not 0: outputs are tagged words (seg[].out points at LLWord), not plain floats; > 0: their copy that many words on
   int cta_base, cta_rem;  // span_rows / grid and span_rows % grid: CTA b owns cta_base (+1 when b < cta_rem) rows
   // derived by the host so that no consumer warp divides: blocks per row, stride of a row's
   // terms in the warp's strip, units a strip holds, tiles of a CTA with cta_base / cta_base + 1 rows
@@ -204,6 +215,8 @@ struct StepParams {
   int embd_kind;
   size_t embd_row_bytes;
   LLWord *xl, *ql, *kl, *vl, *attl, *hbl;  // tagged activation vectors (residual, q, k, v, attention out, hidden)
+  const LLWord *xl_in[2], *attl_in[2], *hbl_in[2];  // both copies of those that every CTA reads
+  int ll_copy;                             // words between them
   float *x;                                // plain copy of the final residual stream, for readers outside the kernel
   float *logits, *k_cache, *v_cache;
   unsigned* epoch;                         // launch count; bumped by CTA 0 when the kernel ends
@@ -414,7 +427,7 @@ __device__ __forceinline__ void warp_flush(const MegaOp& op, const float* wterms
     if (lane < pend) {
       const float hv = op.epilogue == EPI_SILU_MUL ? silu_mul_call(v, up) : v;
       if (op.ll) {
-        ll_store(reinterpret_cast<LLWord*>(my_out), hv, tag);
+        ll_store_both(reinterpret_cast<LLWord*>(my_out), op.ll, hv, tag);
       } else {
         *my_out = hv;
         op.seg[1].out[my_out - op.seg[0].out] = up;
@@ -429,7 +442,7 @@ __device__ __forceinline__ void warp_flush(const MegaOp& op, const float* wterms
       part[(int)(reinterpret_cast<LLWord*>(my_out) - reinterpret_cast<LLWord*>(op.seg[0].out)) - part_row0] = v;
     } else if (op.ll) {
       // a residual row is only ever written by its owner, so its old value needs no tag check
-      ll_store(reinterpret_cast<LLWord*>(my_out), op.epilogue == EPI_ACCUM ? fadd(my_old, v) : v, tag);
+      ll_store_both(reinterpret_cast<LLWord*>(my_out), op.ll, op.epilogue == EPI_ACCUM ? fadd(my_old, v) : v, tag);
     } else {
       *my_out = op.epilogue == EPI_ACCUM ? fadd(__ldcg(my_out), v) : v;
     }
@@ -650,7 +663,7 @@ __device__ __forceinline__ void consume_step_q80(const MegaOp& op, const Ring& R
         for (int o = 4; o > 0; o >>= 1) v[i] = fadd(v[i], __shfl_xor_sync(0xffffffffu, v[i], o));
       if (writer) {
         const float r = op.pair ? silu_mul_call(v[0], v[1]) : accum ? fadd(old, v[0]) : v[0];
-        if (op.ll) ll_store(ll, r, tag);
+        if (op.ll) ll_store_both(ll, op.ll, r, tag);
         else *U.out = r;  // the output head
       }
     }
@@ -1033,7 +1046,7 @@ __device__ __forceinline__ void attention_chunked(const StepParams& P, int li, i
     if (md >= 0) o = value_mix(o, sc + c0, cur_buf + md, hd, cn);
     g.sync();
   }
-  if (md >= 0) ll_store(P.attl + h * hd + md, o, tag_out);
+  if (md >= 0) ll_store_both(P.attl + h * hd + md, P.ll_copy, o, tag_out);
 }
 
 // How `S` CTAs share one head when its cached rows do not fit one CTA's staging area.
@@ -1084,6 +1097,7 @@ __device__ __noinline__ void attn_split_prefetch(const float* k_cache, const flo
 struct AttnSplitArgs {
   int li, h, s, pos, tid, T;
   int head_dim, n_head, n_kv_head, n_ctx, small_floats, v_chunk, fast;
+  int ll_copy;
   uint32_t tag_out;
   float *k_cache, *v_cache;
   LLWord *scl, *attl;
@@ -1164,7 +1178,7 @@ __device__ __forceinline__ void attention_split(const AttnSplitArgs A) {
     pf.mark(27);
     g.sync();
   }
-  if (md >= 0) ll_store(A.attl + A.h * hd + d0 + md, o, A.tag_out);
+  if (md >= 0) ll_store_both(A.attl + A.h * hd + d0 + md, A.ll_copy, o, A.tag_out);
   pf.mark(24);
 }
 
@@ -1254,7 +1268,7 @@ __device__ __forceinline__ void phase_attention(const StepParams& P, int li, int
   pf.mark(20);
   if (SPLIT) {
     attention_split(AttnSplitArgs{li, h, split_s, pos, tid, T, P.head_dim, P.n_head, P.n_kv_head, P.n_ctx, P.small_floats, P.v_chunk,
-                                  P.fast, tag_out, P.k_cache, P.v_cache, P.scl, P.attl, M.scr, M.red, M.ss, M.abort, M.err, prof});
+                                  P.fast, P.ll_copy, tag_out, P.k_cache, P.v_cache, P.scl, P.attl, M.scr, M.red, M.ss, M.abort, M.err, prof});
     return;
   }
   if (!staged) {
@@ -1290,7 +1304,7 @@ __device__ __forceinline__ void phase_attention(const StepParams& P, int li, int
   // value mix, positions in order (ops.rs:208-214)
   {
     const int md = mix_dim(tid, T, hd);
-    if (md >= 0) ll_store(P.attl + h * hd + md, value_mix(0.0f, sc, vbuf + md, hd, n), tag_out);
+    if (md >= 0) ll_store_both(P.attl + h * hd + md, P.ll_copy, value_mix(0.0f, sc, vbuf + md, hd, n), tag_out);
   }
   pf.mark(24);
 }
@@ -1539,17 +1553,18 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
         }
       }
     }
+    const int mine = blockIdx.x & 1;
     if ((ph & 1) == 0) {
       // attention norm -> q/k/v, ffn norm -> gate/up + SiLU, output norm -> logits
       const float* w = head ? P.output_norm : (ph == 0 ? L.attn_norm : L.ffn_norm);
       const uint32_t tin = ph == 0 ? tl : tl + 3u;  // residual after the previous layer's down / this layer's wo
-      phase_norm_quant<Q80>(!head || head_q80, P.xl, tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
+      phase_norm_quant<Q80>(!head || head_q80, P.xl_in[mine], tin, st == 0, head && blockIdx.x == 0 ? P.x : nullptr, w, P.dim, P.eps, P.fast, M, g,
                        SubProf{prof_on && ph == 0 && !head ? P.prof : nullptr, 0},
                        P.prof && (int)blockIdx.x == P.prof_cta && ph == 0 && !head && g.tid == (MEGA_CONSUMER_WARPS - 1) * 32 ? P.prof : nullptr);
     } else {
       // attention output -> wo, activated hidden -> down; both join the residual stream
-      if (ph == 1) phase_quant<Q80>(P.attl, tl + 2u, qd, M, g);
-      else phase_quant<Q80>(P.hbl, tl + 4u, P.hidden, M, g);
+      if (ph == 1) phase_quant<Q80>(P.attl_in[mine], tl + 2u, qd, M, g);
+      else phase_quant<Q80>(P.hbl_in[mine], tl + 4u, P.hidden, M, g);
     }
     if (!head) MEGA_PROF(slot);
     // q/k/v: tl+1, wo: tl+3, gate/up: tl+4, down: tl+5 (the head writes plain floats)
@@ -1591,7 +1606,7 @@ __global__ void __launch_bounds__(MEGA_THREADS, 1) decode_step_kernel(const Step
             const float t = __shfl_sync(0xffffffffu, v, base + src);
             if (src < P.tp.world) sum = fadd(sum, t);
           }
-          if (i < r1 && sub == 0) ll_store(P.xl + i, fadd(ll_value(P.xl + i), sum), tag_out);
+          if (i < r1 && sub == 0) ll_store_both(P.xl + i, P.ll_copy, fadd(ll_value(P.xl + i), sum), tag_out);
         }
       }
     }
