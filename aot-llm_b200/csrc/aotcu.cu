@@ -2666,6 +2666,7 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
     g->aq0_bytes = rows * (widest / 32 + 1) * XIMG_0;
     G_TRY(cudaMalloc(&g->aqk, g->aqk_bytes));
     G_TRY(cudaMemsetAsync(g->aqk, 0, g->aqk_bytes, c->stream));
+    G_TRY(cudaMalloc(&g->axt, (g->aqk_bytes + XF_BLOCK - 1) / XF_BLOCK * XT_BLOCK));
     G_TRY(cudaMalloc(&g->aq0, g->aq0_bytes));
   }
   // Attention scores: shared memory when the context fits, else a global scratch.
@@ -2682,11 +2683,8 @@ int aotcu_gpu_new(aotcu_ctx* c, const aotcu_model_head* head, const aotcu_layer*
   G_TRY(cudaMallocHost(&g->h_pinned, (g->max_batch + 8) * sizeof(int)));
   G_TRY(cudaMallocHost(&g->h_logits, (size_t)d.vocab * sizeof(float)));
   G_TRY(cudaStreamSynchronize(c->stream));
-  if (int rc = mega_setup(g)) return bail(rc);
-  // (last: what the one-kernel step exchanges between CTAs keeps its place in memory, which its time
-  // depends on by up to 3 %)
-  G_TRY(cudaMalloc(&g->axt, (g->aqk_bytes + XF_BLOCK - 1) / XF_BLOCK * XT_BLOCK));
 #undef G_TRY
+  if (int rc = mega_setup(g)) return bail(rc);
   *out = g;
   return 0;
 }
