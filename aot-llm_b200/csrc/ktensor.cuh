@@ -107,9 +107,12 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
-// Nothing but "I have read it": a release at cluster scope would cost 1000 to 2000 cycles a time.
+// "I have read it": the loads of this warp come before the arrive that lets their slot be overwritten, so it is a
+// release (by default, for the CTA), which costs nothing here: 24576 x 4096 x 64 Q4_K 44.3 us and 44.3 with a
+// relaxed arrive, Q6_K 48.5 and 48.5. A release at cluster scope, which also waits for what the warp has stored, is
+// 50.7 and 55.6.
 __device__ __forceinline__ void cluster_arrive(uint32_t mapped_bar) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
