@@ -551,7 +551,7 @@ static int launch_k_batch(aotcu_ctx* c, const GemvCall& call) {
   const int nb = (int)(call.cols / 256), nt = (int)((call.m + 7) / 8);
   // the matrices kind by kind (a pair has one kind), and which kernel takes them
   GemvCall part[3];
-  bool tensor[3];
+  bool tensor[3] = {false, false, false};
   int n = 0;
   bool any[2] = {false, false};
   for (int kind : {Q4_K, Q5_K, Q6_K}) {
@@ -566,8 +566,15 @@ static int launch_k_batch(aotcu_ctx* c, const GemvCall& call) {
   }
   const uint8_t *xf = reinterpret_cast<const uint8_t*>(call.x), *xt = call.xt;
   if (call.x_mode != 2) {
-    const size_t xf_bytes = any[0] ? (size_t)nt * nb * XF_BLOCK : 0, xt_bytes = any[1] ? (size_t)nt * nb * XT_BLOCK : 0;
-    if (const int rc = ctx_workspace(c, xf_bytes + xt_bytes)) return rc;
+    size_t xf_bytes = any[0] ? (size_t)nt * nb * XF_BLOCK : 0, xt_bytes = any[1] ? (size_t)nt * nb * XT_BLOCK : 0;
+    int rc = ctx_workspace(c, xf_bytes + xt_bytes);
+    if (rc == 1 && any[1]) {  // kmma.cuh takes every kind, and its order alone is the smallest
+      any[0] = true;
+      any[1] = tensor[0] = tensor[1] = tensor[2] = false;
+      xf_bytes = (size_t)nt * nb * XF_BLOCK;
+      rc = ctx_workspace(c, xf_bytes);
+    }
+    if (rc) return rc;
     uint8_t *f = any[0] ? c->ximg : nullptr, *t = any[1] ? c->ximg + xf_bytes : nullptr;
     if (int rc = launch(c, xf_kernel, dim3((unsigned)nt * nb), dim3(256), 0, xf, call.x_mode, f, t, (int)call.m, nb)) return rc;
     xf = f;

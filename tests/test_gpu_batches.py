@@ -109,6 +109,22 @@ def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel,
     ctx.device_status()
 
 
+@pytest.mark.parametrize("kind", [Q4_K, Q6_K])
+def test_k_quant_batch_where_one_order_of_the_activations_fits(pkg, ob, ctx, cluster_kernel, kind):
+    """8 token groups x 56 super-blocks: 448 blocks of 2336 bytes (mma.sync kernel) are below 1 MiB, of 2368 (clusters)
+    above it. A conversion and a product all the same, not the per-token kernel."""
+    rows, cols, m = 130, 56 * 256, 64
+    w = make_weights(pkg, kind, rows, cols, 29 + kind, "uniform")
+    cluster_kernel.set_option("workspace_mib", 0)      # gives back a larger buffer
+    cluster_kernel.set_option("workspace_mib", 1)
+    before = cluster_kernel.dispatches()
+    try:
+        _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} under a bound")
+    finally:
+        cluster_kernel.set_option("workspace_mib", 1 << 20)
+    assert cluster_kernel.dispatches() - before == 2
+
+
 def test_k_quant_clusters_in_a_model(pkg, ob, ctx, cluster_kernel):
     """q/k/v of mixed kinds, gated pairs and products onto the residual, chunk after chunk."""
     spec = pkg.model.tiny("llama", n_layer=2, kinds=lambda layer, tensor: Q6_K if tensor in ("wv", "down", "output") else Q4_K, dim=512, hidden=768, vocab=600)
