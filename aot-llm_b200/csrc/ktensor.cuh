@@ -713,7 +713,13 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
   __syncthreads();
   cluster_sync_arrive();  // nobody writes into a CTA that has left
   cluster_sync_wait();
-  if (warp == 1) tc_dealloc(tmem, 512);
+  if (warp == 1) {
+    // The cluster barrier does not wait for what was sent asynchronously. Who has done all its stages has all its
+    // terms; after a wait that gave up some may be on their way still.
+    if (*R.abort)
+      for (int i = 0; i < 2; i++) mbar_drain(&t_full[i]);
+    tc_dealloc(tmem, 512);
+  }
 }
 
 }  // namespace aot
