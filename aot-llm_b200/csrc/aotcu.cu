@@ -77,6 +77,7 @@ struct aotcu_ctx {
   int kt_cluster = 0;                   // CTAs of a cluster, 0 by shape
   int q80_tensor = 0;                   // as k_tensor
   int q80_tensor_rows = 0;              // tokens per CTA, 0 by estimates
+  int give_up = 0;                      // their kernels' give_up: what a wait that runs out does, for tests
 };
 
 constexpr size_t WEIGHT_PAD = 256;
@@ -505,6 +506,7 @@ static int launch_kt_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xt, 
   P.cols = (int)call.cols;
   P.epilogue = call.epilogue;
   P.xf_nt = xf_nt;
+  P.give_up = c->give_up;
   for (size_t t0 = 0; t0 < call.m; t0 += KT_MAX_M) {
     P.m = (int)std::min<size_t>(KT_MAX_M, call.m - t0);
     P.nt = (P.m + 7) / 8;
@@ -809,6 +811,7 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
   P.pair = call.pair;
   P.epilogue = call.epilogue;
   P.n_groups = (int)((call.m + 4 * tpw - 1) / (4 * tpw));
+  P.give_up = c->give_up;
   P.err = c->d_err;
   if (!tensor_map_2d(&P.xmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, x, (size_t)nb * (X0_STRIDE / 4), call.m, (size_t)nb * X0_STRIDE, QT_CHUNK * (X0_STRIDE / 4), 4 * tpw))
     return 1;
@@ -3229,6 +3232,11 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
   if (!strcmp(name, "q80_tensor_rows")) {  // of the context: tokens per CTA
     ARG_CHECK(value == 0 || value == 16 || value == 24 || value == 32, "q80_tensor_rows is 0, 16, 24 or 32");
     g->c->q80_tensor_rows = value;
+    return 0;
+  }
+  if (!strcmp(name, "give_up")) {  // of the context: batch kernels on tcgen05 act as if a wait ran out after that many requests
+    ARG_CHECK(value >= 0, "give_up must not be negative");
+    g->c->give_up = value;
     return 0;
   }
   if (!strcmp(name, "kt_cluster")) {  // of the context: cluster size of the K-quant batch kernel, 0 by shape

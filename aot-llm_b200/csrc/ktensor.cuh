@@ -81,6 +81,7 @@ struct KtParams {
   int tiles_before[4];                    // first tile of each matrix (pair: one list, 64 rows of both per tile)
   int n_tiles;
   int tma, n_raw, n_b;                    // slots of the raw and the activation ring
+  int give_up;                            // requests of activations after which the CTA's waits end (0: never)
   int* err;
 };
 
@@ -123,26 +124,34 @@ __device__ __forceinline__ void cluster_st128(uint32_t mapped, uint32_t mapped_b
                "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(mapped_bar)
                : "memory");
 }
-// ring_wait whose loop is out of line: inline, around a phase that has already ended, it cost 100 to 180
-// cycles where the first test costs 40.
-__device__ __noinline__ bool kt_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort, int* err) {
+// Waits of whole warps, as bounded as ring_wait. The lanes decide together: where some saw the phase end and others
+// that a wait had run out, the warp would go on in two parts, over instructions that all of it has to execute.
+// The loop is out of line: inline, around a phase that has already ended, it cost 100 to 180 cycles where the first
+// test costs 40.
+__device__ __forceinline__ bool kt_try_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_try_wait_at(bar, parity)); }
+__device__ __forceinline__ bool kt_wait_loop(uint32_t bar, uint32_t parity, volatile int* abort, int* err) {
   for (uint32_t it = 0; it < (1u << 22); ++it) {
-    if (mbar_try_wait_at(bar, parity)) return true;
-    if (*abort) return false;
+    if (kt_try_wait(bar, parity)) return true;
+    if (__any_sync(0xffffffffu, *abort)) return false;
   }
   *abort = 1;
   if (err) atomicOr(err, DEVERR_MBAR_TIMEOUT);
   return false;
 }
+__device__ __noinline__ bool kt_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort, int* err) { return kt_wait_loop(bar, parity, abort, err); }
 __device__ __forceinline__ bool kt_wait(const Ring& R, uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (kt_try_wait(smem_addr(bar), parity)) return true;
   return kt_wait_slow(smem_addr(bar), parity, R.abort, R.err);
 }
-
 // The same with the loop in line, after the first test: for warps whose registers leave no room for a call.
 __device__ __forceinline__ bool kt_wait_inline(const Ring& R, uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return ring_wait(R, bar, parity);
+  if (kt_try_wait(smem_addr(bar), parity)) return true;
+  return kt_wait_loop(smem_addr(bar), parity, R.abort, R.err);
+}
+// What a wait that runs out does, brought about by the option "give_up": after that many requests of a CTA.
+__device__ __forceinline__ void kt_give_up(const Ring& R) {
+  *R.abort = 1;
+  if (R.err) atomicOr(R.err, DEVERR_MBAR_TIMEOUT);
 }
 
 // ---- tensor memory ------------------------------------------------------------------------
@@ -373,6 +382,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
     // ---- activations ----
     KtPos pb;
     bool ok = true;
+    int left = P.give_up;
     pdl_wait();
 #pragma unroll 1
     for (int tile = cl; tile < P.n_tiles && ok; tile += n_cl) {
@@ -383,6 +393,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         if (elect_one()) {
           mbar_expect_tx(&b_full[pb.slot], (uint32_t)(nt * XT_BLOCK));
           bulk_g2s(b_ring + pb.slot * b_bytes, P.xf + (size_t)sb * P.xf_nt * XT_BLOCK, (uint32_t)(nt * XT_BLOCK), &b_full[pb.slot]);
+          if (left && --left == 0) kt_give_up(R);
         }
         __syncwarp();
         pb.advance(P.n_b);

@@ -48,6 +48,7 @@ struct QtParams {
   int tiles_before[4];             // first row tile of each matrix (pair: one list, 64 rows of both per tile)
   int n_tiles, n_groups;           // row tiles, groups of T tokens
   int n_raw;
+  int give_up;                     // stages requested after which the CTA's waits end (0: never)
   int* err;
 };
 
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
       // ---- requests ----
       KtPos pr;
       bool ok = true;
+      int left = P.give_up;
       pdl_wait();  // (the weights alone do not depend on the previous kernel; they share their barrier with the activations)
 #pragma unroll 1
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -215,6 +217,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
             tma_load_2d(dst, &P.map[sg], c * (K::PITCH / 4), r0, &raw_full[pr.slot]);
             if (P.pair) tma_load_2d(dst + K::RAW / 2, &P.map[1], c * (K::PITCH / 4), r0, &raw_full[pr.slot]);
             tma_load_2d(dst + K::RAW, &P.xmap, c * (QT_CHUNK * X0_STRIDE / 4), t0, &raw_full[pr.slot]);
+            if (left && --left == 0) kt_give_up(R);
           }
           __syncwarp();
           pr.advance(P.n_raw);

@@ -109,6 +109,26 @@ def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel,
     ctx.device_status()
 
 
+# What follows a wait that runs out: the kernel ends, the status says so, and the next product is right. No CTA may wait
+# for one that has left: every CTA of a cluster makes that many requests, before it needs anything of its peers.
+# Copied by tensor copies or not (Q6_K, 768 columns), one stage per tile, several.
+@pytest.mark.parametrize("kind,cluster,cols,after", [(Q4_K, 4, 1024, 1), (Q4_K, 4, 1024, 2), (Q4_K, 2, 1024, 3), (Q6_K, 8, 2048, 2), (Q6_K, 2, 768, 1)])
+def test_k_quant_clusters_after_a_wait_that_gave_up(pkg, ob, ctx, cluster_kernel, kind, cluster, cols, after):
+    cluster_kernel.set_option("kt_cluster", cluster)
+    rows, m = 3 * 148 * 128, 40                        # at least three tiles per cluster
+    dw, dout = ctx.alloc(rows * cols // 256 * (144 if kind == Q4_K else 210)), ctx.alloc(m * rows * 4)
+    dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
+    cluster_kernel.set_option("give_up", after)
+    try:
+        ctx.matmul(kind, dout, dw, dq, m, rows, cols)
+        with pytest.raises(pkg.AotCudaError, match="wait expired"):
+            ctx.device_status()
+    finally:
+        cluster_kernel.set_option("give_up", 0)
+    w = make_weights(pkg, kind, 129, cols, 35 + kind, "uniform")
+    _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, 129, cols, f"kind {kind} after a wait that gave up")
+
+
 @pytest.mark.parametrize("kind", [Q4_K, Q6_K])
 def test_k_quant_batch_where_one_order_of_the_activations_fits(pkg, ob, ctx, cluster_kernel, kind):
     """8 token groups x 56 super-blocks: 448 blocks of 2336 bytes (mma.sync kernel) are below 1 MiB, of 2368 (clusters)
@@ -241,6 +261,22 @@ def test_q80_on_tcgen05(pkg, ob, ctx, q80_tensor, kind, tokens):
     for o, w in zip(outs, ws):
         assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols), "pair")
     ctx.device_status()
+
+
+@pytest.mark.parametrize("kind,after", [(3, 1), (4, 3), (5, 6)])
+def test_q80_on_tcgen05_after_a_wait_that_gave_up(pkg, ob, ctx, q80_tensor, kind, after):
+    rows, cols, m = 2 * 148 * 128, 1024, 40
+    dw, dout = ctx.alloc(rows * cols // 32 * {3: 18, 4: 22, 5: 34}[kind]), ctx.alloc(m * rows * 4)
+    dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
+    q80_tensor.set_option("give_up", after)
+    try:
+        ctx.matmul(kind, dout, dw, dq, m, rows, cols)
+        with pytest.raises(pkg.AotCudaError, match="wait expired"):
+            ctx.device_status()
+    finally:
+        q80_tensor.set_option("give_up", 0)
+    w = make_weights(pkg, kind, 129, cols, 37 + kind)
+    _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, 129, cols, f"kind {kind} after a wait that gave up")
 
 
 def test_q80_on_tcgen05_in_a_model(pkg, ob, ctx, q80_tensor):
