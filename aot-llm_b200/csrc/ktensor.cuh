@@ -154,6 +154,21 @@ __device__ __forceinline__ void kt_give_up(const Ring& R) {
   if (R.err) atomicOr(R.err, DEVERR_MBAR_TIMEOUT);
 }
 
+// The exchange of a pair: 128 threads meet at barrier `bar`, and leave together: a warp whose wait gave up would
+// leave the others waiting at the next meeting.
+__device__ __forceinline__ bool kt_meet(int bar, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %2, 0;\n\t"
+      "barrier.cta.red.and.pred.aligned q, %1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(bar), "r"((uint32_t)ok)
+      : "memory");
+  return all != 0;
+}
+
 // ---- tensor memory ------------------------------------------------------------------------
 __device__ __forceinline__ void kt_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
@@ -669,7 +684,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         if (lane < C) cluster_arrive(empty_at + 8 * pt.slot);
         pt.advance(2);
       }
-      if (!ok) break;
+      if (!ok && !P.pair) break;
       float out[OQ][4];
 #pragma unroll
       for (int i = 0; i < OQ; i++) {
@@ -688,7 +703,8 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         for (int i = 0; i < HQ; i++)
           *reinterpret_cast<float4*>(xch + 4 * i) = up ? make_float4(out[2 * i][0], out[2 * i][1], out[2 * i][2], out[2 * i][3])
                                                        : make_float4(out[2 * i + 1][0], out[2 * i + 1][1], out[2 * i + 1][2], out[2 * i + 1][3]);
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        ok = kt_meet(1, ok);
+        if (!ok) break;
         const float* const other = exchange + (row ^ 64) * KT_XCH<C>;
 #pragma unroll
         for (int i = 0; i < HQ; i++) {

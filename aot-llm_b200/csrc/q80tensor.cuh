@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
         if (++set == S::SETS) set = 0;
         pi.advance(QT_SLOTS);
       }
-      if (!ok) break;
+      if (!ok && !P.pair) break;
       // ((a0+a4)+(a2+a6)) + ((a1+a5)+(a3+a7)), then what is done with it
       float out[TPW];
 #pragma unroll
@@ -419,7 +419,8 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
         float* const mine = exchange + (wg * 128 + row) * H;
 #pragma unroll
         for (int i = 0; i < H; i++) mine[i] = up ? out[2 * i] : out[2 * i + 1];
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
+        ok = kt_meet(1 + wg, ok);
+        if (!ok) break;
         const float* const other = exchange + (wg * 128 + (row ^ 64)) * H;
         const int gr = r0 + (row & 63);
 #pragma unroll

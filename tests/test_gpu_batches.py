@@ -111,16 +111,20 @@ def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel,
 
 # What follows a wait that runs out: the kernel ends, the status says so, and the next product is right. No CTA may wait
 # for one that has left: every CTA of a cluster makes that many requests, before it needs anything of its peers.
-# Copied by tensor copies or not (Q6_K, 768 columns), one stage per tile, several.
+# Copied by tensor copies or not (Q6_K, 768 columns), one stage per tile, several; pairs, whose warps meet at every tile.
+@pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("kind,cluster,cols,after", [(Q4_K, 4, 1024, 1), (Q4_K, 4, 1024, 2), (Q4_K, 2, 1024, 3), (Q6_K, 8, 2048, 2), (Q6_K, 2, 768, 1)])
-def test_k_quant_clusters_after_a_wait_that_gave_up(pkg, ob, ctx, cluster_kernel, kind, cluster, cols, after):
+def test_k_quant_clusters_after_a_wait_that_gave_up(pkg, ob, ctx, cluster_kernel, kind, cluster, cols, after, pair):
     cluster_kernel.set_option("kt_cluster", cluster)
     rows, m = 3 * 148 * 128, 40                        # at least three tiles per cluster
-    dw, dout = ctx.alloc(rows * cols // 256 * (144 if kind == Q4_K else 210)), ctx.alloc(m * rows * 4)
+    dw, dout, dout2 = ctx.alloc(rows * cols // 256 * (144 if kind == Q4_K else 210)), ctx.alloc(m * rows * 4), ctx.alloc(m * rows * 4)
     dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
     cluster_kernel.set_option("give_up", after)
     try:
-        ctx.matmul(kind, dout, dw, dq, m, rows, cols)
+        if pair:
+            ctx.matmul2(kind, dout, dout2, dw, dw, dq, m, rows, cols)
+        else:
+            ctx.matmul(kind, dout, dw, dq, m, rows, cols)
         with pytest.raises(pkg.AotCudaError, match="wait expired"):
             ctx.device_status()
     finally:
@@ -263,14 +267,18 @@ def test_q80_on_tcgen05(pkg, ob, ctx, q80_tensor, kind, tokens):
     ctx.device_status()
 
 
+@pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("kind,after", [(3, 1), (4, 3), (5, 6)])
-def test_q80_on_tcgen05_after_a_wait_that_gave_up(pkg, ob, ctx, q80_tensor, kind, after):
+def test_q80_on_tcgen05_after_a_wait_that_gave_up(pkg, ob, ctx, q80_tensor, kind, after, pair):
     rows, cols, m = 2 * 148 * 128, 1024, 40
-    dw, dout = ctx.alloc(rows * cols // 32 * {3: 18, 4: 22, 5: 34}[kind]), ctx.alloc(m * rows * 4)
+    dw, dout, dout2 = ctx.alloc(rows * cols // 32 * {3: 18, 4: 22, 5: 34}[kind]), ctx.alloc(m * rows * 4), ctx.alloc(m * rows * 4)
     dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
     q80_tensor.set_option("give_up", after)
     try:
-        ctx.matmul(kind, dout, dw, dq, m, rows, cols)
+        if pair:
+            ctx.matmul2(kind, dout, dout2, dw, dw, dq, m, rows, cols)
+        else:
+            ctx.matmul(kind, dout, dw, dq, m, rows, cols)
         with pytest.raises(pkg.AotCudaError, match="wait expired"):
             ctx.device_status()
     finally:
