@@ -414,8 +414,6 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         pb.advance(P.n_b);
       }
     }
-    if (!ok)  // copies in flight land before the CTA's shared memory goes
-      for (int i = 0; i < KT_MAX_SLOTS; i++) mbar_drain(&b_full[i]);
   } else if (warp == 1) {
     // ---- MMAs ----
     const uint32_t idesc = (2u << 4) | (1u << 10) | ((KT_ROWS >> 4) << 24), fdesc = (1u << 4) | ((KT_ROWS >> 4) << 24);
@@ -501,8 +499,6 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (!ok && P.tma)
-      for (int i = 0; i < KT_MAX_SLOTS; i++) mbar_drain(&raw_full[i]);
   } else if (warp < 12) {
     // ---- unpack ----
     const int row = (tid - 128) & 127, u = (warp - 4) >> 2;
@@ -741,10 +737,14 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
   cluster_sync_arrive();  // nobody writes into a CTA that has left
   cluster_sync_wait();
   if (warp == 1) {
-    // The cluster barrier does not wait for what was sent asynchronously. Who has done all its stages has all its
-    // terms; after a wait that gave up some may be on their way still.
-    if (*R.abort)
+    // Nothing is written into a CTA that has left. Who has done all its stages has all that was requested and all its
+    // terms; after a wait that gave up, whichever warp's, some may be on their way still, and the cluster barrier does
+    // not wait for what was sent asynchronously.
+    if (*R.abort) {
+      for (int i = 0; i < P.n_b; i++) mbar_drain(&b_full[i]);
+      for (int i = 0; i < P.n_raw && P.tma; i++) mbar_drain(&raw_full[i]);
       for (int i = 0; i < 2; i++) mbar_drain(&t_full[i]);
+    }
     tc_dealloc(tmem, 512);
   }
 }

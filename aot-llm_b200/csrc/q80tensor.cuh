@@ -223,8 +223,6 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
           pr.advance(P.n_raw);
         }
       }
-      if (!ok)  // copies in flight land before the CTA's shared memory goes
-        for (int i = 0; i < P.n_raw; i++) mbar_drain(&raw_full[i]);
     } else if (warp == 1) {
       // ---- MMAs ----
       constexpr uint32_t idesc = (1u << 4) | ((S::N >> 3) << 17) | ((KT_ROWS >> 4) << 24);
@@ -448,7 +446,11 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tc_dealloc(tmem, 512);
+  if (warp == 1) {
+    if (*R.abort)  // whichever warp gave up, the copies in flight land before the CTA's shared memory goes
+      for (int i = 0; i < P.n_raw; i++) mbar_drain(&raw_full[i]);
+    tc_dealloc(tmem, 512);
+  }
 }
 
 }  // namespace aot
