@@ -680,7 +680,10 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         if (lane < C) cluster_arrive(empty_at + 8 * pt.slot);
         pt.advance(2);
       }
-      if (!ok && !P.pair) break;
+      if (!ok) {
+        if (P.pair) kt_meet(1, false);
+        break;
+      }
       float out[OQ][4];
 #pragma unroll
       for (int i = 0; i < OQ; i++) {
@@ -699,7 +702,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
         for (int i = 0; i < HQ; i++)
           *reinterpret_cast<float4*>(xch + 4 * i) = up ? make_float4(out[2 * i][0], out[2 * i][1], out[2 * i][2], out[2 * i][3])
                                                        : make_float4(out[2 * i + 1][0], out[2 * i + 1][1], out[2 * i + 1][2], out[2 * i + 1][3]);
-        ok = kt_meet(1, ok);
+        ok = kt_meet(1, true);
         if (!ok) break;
         const float* const other = exchange + (row ^ 64) * KT_XCH<C>;
 #pragma unroll

@@ -396,7 +396,10 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
         if (++set == S::SETS) set = 0;
         pi.advance(QT_SLOTS);
       }
-      if (!ok && !P.pair) break;
+      if (!ok) {  // (not carried to the meeting below: sums that outlive a wait's failure made a product a third slower)
+        if (P.pair) kt_meet(1 + wg, false);
+        break;
+      }
       // ((a0+a4)+(a2+a6)) + ((a1+a5)+(a3+a7)), then what is done with it
       float out[TPW];
 #pragma unroll
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(QT_THREADS, 1) qt_kernel(const __grid_constant
         float* const mine = exchange + (wg * 128 + row) * H;
 #pragma unroll
         for (int i = 0; i < H; i++) mine[i] = up ? out[2 * i] : out[2 * i + 1];
-        ok = kt_meet(1 + wg, ok);
+        ok = kt_meet(1 + wg, true);
         if (!ok) break;
         const float* const other = exchange + (wg * 128 + (row ^ 64)) * H;
         const int gr = r0 + (row & 63);
