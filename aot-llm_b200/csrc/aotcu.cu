@@ -67,6 +67,7 @@ struct aotcu_ctx {
   int* d_err = nullptr;
   bool pdl = true;  // programmatic dependent launch between the kernels of a stream
   uint64_t launches = 0;
+  uint64_t kt_launches = 0, qt_launches = 0;  // those of ktensor.cuh and q80tensor.cuh among them (queries of the same names)
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   std::vector<struct aotcu_gpu*> gpus;  // live Gpus of this context (freed with it)
   uint8_t* ximg = nullptr;              // activations converted from reference-layout blocks (ctx_workspace)
@@ -461,6 +462,7 @@ static int launch_kt_c(aotcu_ctx* c, KtParams& P, int clusters) {
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kt_kernel<KIND, C>, P);
   if (e != cudaSuccess) return fail(AOTCU_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
   c->launches++;
+  c->kt_launches++;
   return 0;
 }
 static int kt_tiles(const GemvCall& call) {
@@ -830,6 +832,7 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
     if (!P.nseg) continue;
     const int rc = kind == Q4_0 ? launch_qt_k<Q4_0>(c, P, tpw) : kind == Q5_0 ? launch_qt_k<Q5_0>(c, P, tpw) : launch_qt_k<Q8_0>(c, P, tpw);
     if (rc) return rc;
+    c->qt_launches++;
   }
   return 0;
 }
@@ -3197,6 +3200,9 @@ int aotcu_gpu_set_option(aotcu_gpu* g, const char* name, int value) {
     return 0;
   }
   if (!strcmp(name, "mega_available")) return g->mega_ok ? 1 : 0;
+  // queries: launches of the batch kernels on tcgen05 by this context
+  if (!strcmp(name, "kt_launches")) return (int)(g->c->kt_launches & 0x7FFFFFFF);
+  if (!strcmp(name, "qt_launches")) return (int)(g->c->qt_launches & 0x7FFFFFFF);
   if (!strcmp(name, "workspace_mib")) {
     // bound of the context's conversion buffer (no bound by default); a larger one is given back
     ARG_CHECK(value >= 0, "workspace_mib must not be negative");

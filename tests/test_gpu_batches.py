@@ -21,9 +21,31 @@ def _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, what):
     ctx.device_status()
 
 
+# All kernels give the same bits, so what ran is asked of the context: launches of the tcgen05 batch kernels.
+def _launches(g):
+    return g.set_option("kt_launches", 0), g.set_option("qt_launches", 0)
+
+
+@pytest.fixture(params=["by estimates", "warp level"])
+def batch_kernels(pkg, ctx, request):
+    """The kernels that a batch gets, and those of mma.sync and of streaming alone."""
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)
+    alone = request.param == "warp level"
+    for name in ("k_tensor", "q80_tensor"):
+        g.set_option(name, int(alone))
+    before = _launches(g)
+    yield g
+    if alone:
+        assert _launches(g) == before
+    for name in ("k_tensor", "q80_tensor"):
+        g.set_option(name, 0)
+    g.close()
+
+
 @pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
 @pytest.mark.parametrize("rows,cols", [(1, 256), (17, 768), (2400, 2304), (4735, 1280)])
-def test_k_quant_tile_edges(pkg, ob, ctx, kind, rows, cols):
+def test_k_quant_tile_edges(pkg, ob, ctx, batch_kernels, kind, rows, cols):
     w = make_weights(pkg, kind, rows, cols, 21 + kind + rows, "uniform")
     for m in (3, 8, 9, 17, 64, 65):
         xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
@@ -46,7 +68,7 @@ def test_k_quant_small_batches(pkg, ob, ctx, kind, rows, cols, m, one_lane):
 
 
 @pytest.mark.parametrize("kind", [Q4_K, Q5_K, Q6_K])
-def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, kind):
+def test_k_quant_integers_at_their_bounds(pkg, ob, ctx, batch_kernels, kind):
     rows, cols, m = 48, 1024, 12
     w = make_weights(pkg, kind, rows, cols, 5, "uniform").reshape(rows * cols // 256, -1)
     w[:, 4:] = 0xFF                                   # largest quants, scales and mins (Q4_K, Q5_K)
@@ -82,7 +104,9 @@ def test_k_quant_clusters(pkg, ob, ctx, cluster_kernel, kind, cluster):
     for rows, cols, ms in ((1, 256, (2, 64)), (129, 2048, (8, 17, 33, 48)), (300, 768, (25, 65)), (9700, 2304, (64,))):
         w = make_weights(pkg, kind, rows, cols, 25 + kind + rows, "uniform")
         for m in ms:
+            before = _launches(cluster_kernel)[0]
             _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m} clusters of {cluster}")
+            assert _launches(cluster_kernel)[0] - before == (m + 63) // 64
 
 
 @pytest.mark.parametrize("kind", [Q4_K, Q6_K])
@@ -99,6 +123,7 @@ def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel,
     q = ob.quantize_act(kind, xs)
     dq, outs = ctx.to_device(q.view(np.uint8)), [ctx.alloc(m * rows * 4) for _ in ws]
     want = [ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols) for w in ws]
+    before = _launches(cluster_kernel)[0]
     ctx.matmul2(kind, *outs, *[ctx.to_device(w) for w in ws], dq, m, rows, cols)
     for o, x in zip(outs, want):
         assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), x, "pair")
@@ -106,6 +131,7 @@ def test_k_quant_clusters_pairs_bounds_and_offsets(pkg, ob, ctx, cluster_kernel,
     d = ctx.to_device(np.concatenate([np.zeros(off, np.uint8), ws[0].reshape(-1), np.zeros(256, np.uint8)]))
     ctx.matmul(kind, outs[0], d.ptr + off, dq, m, rows, cols)
     assert_bits_equal(outs[0].download(np.float32, m * rows).reshape(m, rows), want[0], f"offset {off}")
+    assert _launches(cluster_kernel)[0] - before == 2
     ctx.device_status()
 
 
@@ -119,6 +145,7 @@ def test_k_quant_clusters_after_a_wait_that_gave_up(pkg, ob, ctx, cluster_kernel
     rows, m = 3 * 148 * 128, 40                        # at least three tiles per cluster
     dw, dout, dout2 = ctx.alloc(rows * cols // 256 * (144 if kind == Q4_K else 210)), ctx.alloc(m * rows * 4), ctx.alloc(m * rows * 4)
     dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
+    before = _launches(cluster_kernel)[0]
     cluster_kernel.set_option("give_up", after)
     try:
         if pair:
@@ -131,6 +158,7 @@ def test_k_quant_clusters_after_a_wait_that_gave_up(pkg, ob, ctx, cluster_kernel
         cluster_kernel.set_option("give_up", 0)
     w = make_weights(pkg, kind, 129, cols, 35 + kind, "uniform")
     _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, 129, cols, f"kind {kind} after a wait that gave up")
+    assert _launches(cluster_kernel)[0] - before == 2
 
 
 @pytest.mark.parametrize("kind", [Q4_K, Q6_K])
@@ -141,12 +169,12 @@ def test_k_quant_batch_where_one_order_of_the_activations_fits(pkg, ob, ctx, clu
     w = make_weights(pkg, kind, rows, cols, 29 + kind, "uniform")
     cluster_kernel.set_option("workspace_mib", 0)      # gives back a larger buffer
     cluster_kernel.set_option("workspace_mib", 1)
-    before = cluster_kernel.dispatches()
+    before, kt = cluster_kernel.dispatches(), _launches(cluster_kernel)[0]
     try:
         _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} under a bound")
     finally:
         cluster_kernel.set_option("workspace_mib", 1 << 20)
-    assert cluster_kernel.dispatches() - before == 2
+    assert cluster_kernel.dispatches() - before == 2 and _launches(cluster_kernel)[0] == kt
 
 
 def test_k_quant_clusters_in_a_model(pkg, ob, ctx, cluster_kernel):
@@ -155,11 +183,14 @@ def test_k_quant_clusters_in_a_model(pkg, ob, ctx, cluster_kernel):
     g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 160, 64)
     om = ob.model_from_spec(spec, 160, 64, n_threads=4)
     pos = 0
-    for n in (64, 21, 9):
+    for n in (64, 21, 9, 8):
+        before = _launches(g)[0]
         toks = np.random.default_rng(n).integers(0, 600, n).tolist()
         g.forward_batch(toks, pos, True)
         om.forward_batch(toks, pos, True)
         assert_bits_equal(g.logits(), om.logits(), f"logits after a chunk of {n} at {pos}")
+        # per layer q/k of one kind and v of another, wo, gate/up, down; up to eight rows lie in the other kernel's order only
+        assert _launches(g)[0] - before == (10 if n > 8 else 0)
         pos += n
     g.close()
     ctx.device_status()
@@ -207,7 +238,7 @@ def test_float_batches_on_the_streaming_kernel(pkg, ob, ctx, kind, rows, pair, m
 
 
 @pytest.mark.parametrize("kind", [3, 4, 5])           # Q4_0, Q5_0, Q8_0
-def test_q80_tile_edges(pkg, ob, ctx, kind):
+def test_q80_tile_edges(pkg, ob, ctx, batch_kernels, kind):
     for rows, cols, ms in ((8192, 256, (49, 64)), (8205, 768, (50, 81, 129))):   # a partial row tile, half-full warps, two CTAs per tile
         w = make_weights(pkg, kind, rows, cols, 41 + kind)
         for m in ms:
@@ -222,12 +253,23 @@ def test_q80_tile_edges(pkg, ob, ctx, kind):
                                                   (5, 8192, 256, 48, True), (4, 12000, 512, 17, True), (3, 16400, 256, 80, True),
                                                   (3, 301, 512, 32, True), (3, 300, 512, 32, False), (5, 2048, 512, 48, False), (4, 8192, 256, 16, False)])
 def test_q80_sizes_around_the_choice_of_kernel(pkg, ob, ctx, kind, rows, cols, m, mma):
+    """On the kernels of warp-level instructions alone, whose choice this is; then as products get them."""
     spec = pkg.model.tiny("llama", n_layer=1)
     g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)  # for the count of launches
     w = make_weights(pkg, kind, rows, cols, 43 + kind)
+    xs = np.random.default_rng(m).standard_normal(m * cols).astype(np.float32)
+    qt = _launches(g)[1]
+    g.set_option("q80_tensor", 1)
     before = g.dispatches()
-    _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+    try:
+        _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
+    finally:
+        g.set_option("q80_tensor", 0)
     assert g.dispatches() - before == (2 if mma else 1 + (m + 15) // 16)
+    assert _launches(g)[1] == qt
+    before = g.dispatches()
+    _run(pkg, ob, ctx, kind, w, xs, m, rows, cols, f"kind {kind} {rows}x{cols} m {m} by estimates")
+    assert g.dispatches() - before == (2 if mma or _launches(g)[1] != qt else 1 + (m + 15) // 16)
     g.close()
 
 
@@ -249,6 +291,7 @@ def q80_tensor(pkg, ctx):
 @pytest.mark.parametrize("tokens", [16, 24, 32])
 def test_q80_on_tcgen05(pkg, ob, ctx, q80_tensor, kind, tokens):
     q80_tensor.set_option("q80_tensor_rows", tokens)
+    before = _launches(q80_tensor)[1]
     for rows, cols, ms in ((1, 256, (2, 65)), (301, 768, (17, 33, 64)), (19100, 256, (40,))):
         w = make_weights(pkg, kind, rows, cols, 45 + kind + rows)
         for m in ms:
@@ -264,6 +307,7 @@ def test_q80_on_tcgen05(pkg, ob, ctx, q80_tensor, kind, tokens):
     ctx.matmul2(kind, *outs, *[ctx.to_device(w) for w in ws], ctx.to_device(q.view(np.uint8)), m, rows, cols)
     for o, w in zip(outs, ws):
         assert_bits_equal(o.download(np.float32, m * rows).reshape(m, rows), ob.matmul(ob.Pool(4), ob.detect_table(), kind, w, q, m, rows, cols), "pair")
+    assert _launches(q80_tensor)[1] - before == 7
     ctx.device_status()
 
 
@@ -273,6 +317,7 @@ def test_q80_on_tcgen05_after_a_wait_that_gave_up(pkg, ob, ctx, q80_tensor, kind
     rows, cols, m = 2 * 148 * 128, 1024, 40
     dw, dout, dout2 = ctx.alloc(rows * cols // 32 * {3: 18, 4: 22, 5: 34}[kind]), ctx.alloc(m * rows * 4), ctx.alloc(m * rows * 4)
     dq = ctx.to_device(ob.quantize_act(kind, np.ones(m * cols, np.float32)).view(np.uint8))
+    before = _launches(q80_tensor)[1]
     q80_tensor.set_option("give_up", after)
     try:
         if pair:
@@ -285,6 +330,7 @@ def test_q80_on_tcgen05_after_a_wait_that_gave_up(pkg, ob, ctx, q80_tensor, kind
         q80_tensor.set_option("give_up", 0)
     w = make_weights(pkg, kind, 129, cols, 37 + kind)
     _run(pkg, ob, ctx, kind, w, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, 129, cols, f"kind {kind} after a wait that gave up")
+    assert _launches(q80_tensor)[1] - before == 2
 
 
 def test_q80_on_tcgen05_in_a_model(pkg, ob, ctx, q80_tensor):
@@ -293,12 +339,14 @@ def test_q80_on_tcgen05_in_a_model(pkg, ob, ctx, q80_tensor):
     g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 160, 64)
     om = ob.model_from_spec(spec, 160, 64, n_threads=4)
     pos = 0
+    before = _launches(g)[1]
     for n in (64, 21, 9):
         toks = np.random.default_rng(n).integers(0, 600, n).tolist()
         g.forward_batch(toks, pos, True)
         om.forward_batch(toks, pos, True)
         assert_bits_equal(g.logits(), om.logits(), f"logits after a chunk of {n} at {pos}")
         pos += n
+    assert _launches(g)[1] - before == 3 * 10          # per layer wq, wk and wv, wo, gate/up, down
     g.close()
     ctx.device_status()
 
@@ -310,7 +358,7 @@ def test_batches_longer_than_a_pass(pkg, ob, ctx, kind, rows, cols):
     _run(pkg, ob, ctx, kind, w, np.random.default_rng(kind).standard_normal(m * cols).astype(np.float32), m, rows, cols, f"kind {kind} {rows}x{cols} m {m}")
 
 
-def test_q80_pair_tile_edges(pkg, ob, ctx):
+def test_q80_pair_tile_edges(pkg, ob, ctx, batch_kernels):
     rows, cols, m = 4105, 512, 60
     ws = [make_weights(pkg, 3, rows, cols, 51 + i) for i in range(2)]
     q = ob.quantize_act(3, np.random.default_rng(m).standard_normal(m * cols).astype(np.float32))
