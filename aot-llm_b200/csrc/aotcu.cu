@@ -533,22 +533,24 @@ static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
   static const Cost mma[3] = {{5.87, 0.826, 0.374}, {5.54, 1.026, 0.381}, {4.82, 1.488, 0.454}};  // rows: a group of 8
   static const Cost tensor[3] = {{7.50, 0.633, 0.252}, {7.37, 0.674, 0.257}, {6.78, 1.029, 0.193}};  // rows: a group of 16
   const bool can = call.x_mode != 2 || call.xt;
-  *yes = can && c->k_tensor == 2;
-  if (!can || c->k_tensor) return 0;
+  *yes = false;
+  if (!can || c->k_tensor == 1) return 0;
   const int kind = call.seg[0].kind, k = kind == Q4_K ? 0 : kind == Q5_K ? 1 : 2, tiles = kt_tiles(call), nb = (int)(call.cols / 256);
   int rt, wk, size = 0, n = 0;
   long stages;
-  const double s_mma = kmma_shape(c, call, &rt, &wk);
   if (int rc = kind == Q4_K ? kt_shape<Q4_K>(c, tiles, nb, &size, &n, &stages)
                : kind == Q5_K ? kt_shape<Q5_K>(c, tiles, nb, &size, &n, &stages) : kt_shape<Q6_K>(c, tiles, nb, &size, &n, &stages))
     return rc;
+  if (!stages) return 0;  // no cluster of a size that it may have fits the GPU
+  if (c->k_tensor == 2) return *yes = true, 0;
+  const double s_mma = kmma_shape(c, call, &rt, &wk);
   double t_mma = 0.0, t_tensor = 0.0;
   for (size_t t0 = 0; t0 < call.m; t0 += KT_MAX_M) {
     const size_t m = std::min<size_t>(KT_MAX_M, call.m - t0);
     t_mma += mma[k].launch + s_mma * (mma[k].stage + mma[k].rows * (double)((m + 7) / 8));
     t_tensor += tensor[k].launch + (double)stages * (tensor[k].stage + tensor[k].rows * (double)((m + 15) / 16));
   }
-  *yes = stages != 0 && t_tensor < t_mma;
+  *yes = t_tensor < t_mma;
   return 0;
 }
 static int launch_k_batch(aotcu_ctx* c, const GemvCall& call) {
