@@ -801,6 +801,13 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
     }
     if (us > 0.97 * other) return 1;
   }
+  CUtensorMap map[3];
+  // all of them before the first launch: a call that cannot have its maps goes to the next kernel untouched
+  for (int s = 0; s < call.nseg; s++) {
+    const size_t row_bytes = kind_row_bytes(call.seg[s].kind, call.cols);
+    if (!tensor_map_2d(&map[s], CU_TENSOR_MAP_DATA_TYPE_UINT32, call.seg[s].w, row_bytes / 4, call.seg[s].rows, row_bytes, (int)(row_bytes / nb * QT_CHUNK / 4), box))
+      return 1;
+  }
   const uint8_t* x = reinterpret_cast<const uint8_t*>(call.x);
   if (call.x_mode != 1) {
     if (const int rc = ctx_workspace(c, call.m * nb * X0_STRIDE)) return rc;
@@ -821,11 +828,9 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
     return 1;
   for (int kind : {Q4_0, Q5_0, Q8_0}) {
     P.nseg = P.n_tiles = 0;
-    const size_t row_bytes = kind_row_bytes(kind, call.cols);
     for (int s = 0; s < call.nseg; s++) {
       if (call.seg[s].kind != kind) continue;
-      if (!tensor_map_2d(&P.map[P.nseg], CU_TENSOR_MAP_DATA_TYPE_UINT32, call.seg[s].w, row_bytes / 4, call.seg[s].rows, row_bytes, (int)(row_bytes / nb * QT_CHUNK / 4), box))
-        return fail(AOTCU_ERR_CUDA, "tensor map of a weight matrix refused");
+      P.map[P.nseg] = map[s];
       P.tiles_before[P.nseg] = P.n_tiles;
       P.seg[P.nseg++] = call.seg[s];
       if (!call.pair || P.nseg == 1) P.n_tiles += (call.seg[s].rows + box - 1) / box;
