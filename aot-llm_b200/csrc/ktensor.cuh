@@ -128,25 +128,44 @@ __device__ __forceinline__ void cluster_st128(uint32_t mapped, uint32_t mapped_b
 // that a wait had run out, the warp would go on in two parts, over instructions that all of it has to execute.
 // The loop is out of line: inline, around a phase that has already ended, it cost 100 to 180 cycles where the first
 // test costs 40.
-__device__ __forceinline__ bool kt_try_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_try_wait_at(bar, parity)); }
+// CLUSTER: what the phase stands for was written, or read, by other CTAs of the cluster.
+template <bool CLUSTER>
+__device__ __forceinline__ bool kt_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if (CLUSTER) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } else {
+    ok = mbar_try_wait_at(bar, parity);
+  }
+  return __all_sync(0xffffffffu, ok);
+}
+template <bool CLUSTER>
 __device__ __forceinline__ bool kt_wait_loop(uint32_t bar, uint32_t parity, volatile int* abort, int* err) {
   for (uint32_t it = 0; it < (1u << 22); ++it) {
-    if (kt_try_wait(bar, parity)) return true;
+    if (kt_try_wait<CLUSTER>(bar, parity)) return true;
     if (__any_sync(0xffffffffu, *abort)) return false;
   }
   *abort = 1;
   if (err) atomicOr(err, DEVERR_MBAR_TIMEOUT);
   return false;
 }
-__device__ __noinline__ bool kt_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort, int* err) { return kt_wait_loop(bar, parity, abort, err); }
+template <bool CLUSTER>
+__device__ __noinline__ bool kt_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort, int* err) { return kt_wait_loop<CLUSTER>(bar, parity, abort, err); }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool kt_wait(const Ring& R, uint64_t* bar, uint32_t parity) {
-  if (kt_try_wait(smem_addr(bar), parity)) return true;
-  return kt_wait_slow(smem_addr(bar), parity, R.abort, R.err);
+  if (kt_try_wait<CLUSTER>(smem_addr(bar), parity)) return true;
+  return kt_wait_slow<CLUSTER>(smem_addr(bar), parity, R.abort, R.err);
 }
 // The same with the loop in line, after the first test: for warps whose registers leave no room for a call.
 __device__ __forceinline__ bool kt_wait_inline(const Ring& R, uint64_t* bar, uint32_t parity) {
-  if (kt_try_wait(smem_addr(bar), parity)) return true;
-  return kt_wait_loop(smem_addr(bar), parity, R.abort, R.err);
+  if (kt_try_wait<false>(smem_addr(bar), parity)) return true;
+  return kt_wait_loop<false>(smem_addr(bar), parity, R.abort, R.err);
 }
 // What a wait that runs out does, brought about by the option "give_up": after that many requests of a CTA.
 __device__ __forceinline__ void kt_give_up(const Ring& R) {
@@ -558,7 +577,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
           d = side[ps.slot * KT_ROWS + row];
         }
         const F2 dd = f2_pack(d.x, d.x), dm = f2_pack(d.y, d.y), minus1 = f2_pack(-1.0f, -1.0f);
-        ok = kt_wait(R, &t_empty[pt.slot], pt.par ^ 1u);
+        ok = kt_wait<true>(R, &t_empty[pt.slot], pt.par ^ 1u);
         if (!ok) break;
         if (mine) {
           const uint32_t tb = pt.slot * KT_TERMS + (rank * OQ * KT_ROWS + row) * 16, fb = t_bar + 8 * pt.slot, own = smem_addr(terms) + tb;
@@ -646,7 +665,7 @@ __global__ void __launch_bounds__(KT_THREADS, 1) kt_kernel(const __grid_constant
       for (int i = 0; i < OQ; i++) acc[i][0] = acc[i][1] = f2_pack(0.0f, 0.0f);
 #pragma unroll 1
       for (int s = 0; s < n_st; s++) {
-        ok = kt_wait(R, &t_full[pt.slot], pt.par);
+        ok = kt_wait<true>(R, &t_full[pt.slot], pt.par);
         if (!ok) break;
         // (the other three warps' phase cannot end again before they have said that they read this one)
         if (warp == 20 && stage + 2 < stages) {
