@@ -678,12 +678,11 @@ static double q80_stream_us(const aotcu_ctx* c, int kind, size_t cols, size_t ro
   const double block = quads <= 14 ? std::max(0.09, 0.06 + 0.016 * quads) : 0.055 + 0.0175 * quads;
   return 0.5 + ((m + 15) / 16) * (1.5 + (cols / 32) * block * (kind == Q4_0 ? 1 : kind == Q5_0 ? 1.1 : 0.95));
 }
-// Taken where the estimate is lower (both measured, us, this kernel first): Q4_0 11264x2048 76 and 116
-// at 64 rows, 77 and 88 at 48, 53 and 59 at 32; 5632x2048 48 and 66 at 64 rows, 39 and 34 at 32;
-// 2048x5632 123 and 83 at 64 rows, 124 and 165 at 128; Q8_0 14336x4096 193 and 242 at 64 rows, 195 and
-// 182 at 48. Up to 16 rows the streaming kernel is a single launch and the faster one nearly everywhere.
-// Matrices that it does not take (rows not in fours, mixed kinds) would go to the whole-row kernel,
-// whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows, 14337x4096 103 and 784.
+// Taken, of what launch_q80_tensor leaves (rows of up to about 1000 columns), where the estimate is lower than the
+// streaming kernel's. Fitted to timings of both, with q80_tensor at 1 (us, this kernel first): Q4_0 11264x2048 76 and 116 at 64 rows, 77 and 88 at 48, 53 and 59 at 32; 5632x2048 48 and 66 at 64
+// rows, 39 and 34 at 32; 2048x5632 123 and 83 at 64 rows, 124 and 165 at 128. Up to 16 rows the streaming kernel is a
+// single launch and the faster one nearly everywhere. Matrices that it does not take (rows not in fours, mixed kinds)
+// would go to the whole-row kernel, whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows.
 constexpr size_t Q80_MMA_MIN_BATCH = 17, Q80_MMA_MIN_BATCH_ODD = 32;
 // CTAs of a product, `*wt` warps each: at most five share a row unit.
 static size_t q80_mma_ctas(const GemvCall& call, int* wt, int* n_tcta = nullptr) {
@@ -755,8 +754,10 @@ template <int KIND>
 static int launch_qt_k(aotcu_ctx* c, QtParams& P, int tpw) {
   return tpw == 4 ? launch_qt_t<KIND, 4>(c, P) : tpw == 6 ? launch_qt_t<KIND, 6>(c, P) : launch_qt_t<KIND, 8>(c, P);
 }
-// Microseconds by estimate (fitted to 14336 x 4096 and 2048 x 2048, three kinds, 17 to 64 rows: within
-// 4 %): rounds of CTAs, each the same time per block; the fewest for 16, 24 or 32 tokens per CTA.
+// Microseconds by estimate: rounds of CTAs, each the same time per block; the fewest for 16, 24 or 32 tokens per CTA.
+// Fitted to 14336 x 4096 and 2048 x 2048 (three kinds, 17 to 64 rows: within 4 %). For shorter products the start is
+// less than its 7 us, so small matrices stay with the other kernels where this one is faster (Q8_0 1024 x 1024 x 64 24
+// and here 16, 1024 x 4096 60 and 48; Q4_0 2560 x 256 7.7 and 7.3): see the timings at launch_q80_tensor.
 static double q80_tensor_us(const aotcu_ctx* c, int kind, size_t cols, size_t tiles, size_t m, int* tpw) {
   static const struct {
     int tpw;
@@ -783,10 +784,12 @@ static int launch_q80_tensor(aotcu_ctx* c, const GemvCall& call, size_t span) {
   const double us = q80_tensor_us(c, call.seg[0].kind, call.cols, tiles, call.m, &tpw);
   if (!c->q80_tensor) {
     // Taken where its estimate is below those of the kernels after it (us, this kernel first: Q8_0 14336 x
-    // 4096 129 and, on q80_mma_kernel, 196 at 64 rows, 59 and 114 at 20; Q4_0 4096 x 4096 51 and, on
+    // 4096 131 and, on q80_mma_kernel, 196 at 64 rows, 59 and 114 at 20; Q4_0 4096 x 4096 51 and, on
     // q80_stream_kernel, 78 at 40 rows, 50 and 29 at 16; 24576 x 4096 94 and 59 at 8). Up to 8 rows the
-    // streaming kernel is nowhere the slower one. Of 576 timings (16 matrices, three kinds, 4 to 64 rows) those
-    // from 9 rows on gain a third on average; none loses more than 6 %.
+    // streaming kernel is nowhere the slower one. Of 672 timings (16 matrices of 256 x 2048 to 24576 x 4096, three kinds,
+    // 4 to 64 rows) those from 9 rows on are 1.29 times as fast with this kernel among the choices; none loses more than
+    // 5 % (Q4_0 2048 x 5632 x 48 65.9, 62.8 without), and the choice is 1 % from the faster kernel on average, 53 % at
+    // worst (Q8_0 1024 x 1024 x 56, which is left to the streaming kernel).
     bool streams = true;
     for (int s = 0; s < call.nseg; s++) streams = streams && call.seg[s].rows % 4 == 0 && call.seg[s].kind == call.seg[0].kind;
     if (streams && call.m <= 8) return 1;

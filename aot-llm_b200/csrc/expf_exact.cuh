@@ -6,9 +6,9 @@
 // a degree-3 polynomial for 2^(r/32) evaluated in double precision and one final
 // rounding to f32. Restated here in fp64 device arithmetic, with the reduction
 // r = fma(32/ln2, x, -k) that the FMA build of the library performs, it returns
-// the same bits as the library on every one of the 2^32 inputs (checked
-// exhaustively on the CPU by tests/test_expf.py through a host copy of this
-// function).
+// the same bits as the library on every one of the 2^32 inputs but NaN (compared on
+// the CPU; tests/test_host_logic.py repeats it for every 61st input and for all of
+// the softmax's core, through a host build of this function).
 //
 // The table holds bits(2^(i/32)) - (i << 47) for i in 0..31, each 2^(i/32)
 // correctly rounded to double (generated with 80-digit decimal arithmetic; the

@@ -2,10 +2,10 @@
 // kind::i8, weights as the operand in tensor memory (matmul_rows of
 // crates/aot-kernels/src/matvec.rs:479-522).
 //
-// A weight times the scale of its sub-block is an integer of at most 13 bits. It is held as two
+// A weight times the scale of its sub-block is an integer of at most 14 bits. It is held as two
 // unsigned bytes (digits), so that one int32 accumulator per digit takes a whole super-block:
 //   Q4_K, Q5_K: sc = 8 * s1 + s0; digits q * s0 and q * s1 (at most 31 * 7), sumi = 8 * acc1 + acc0
-//   Q6_K:       v = sc * (q - 32) + 4096, 0..8160; its low and high byte,
+//   Q6_K:       v = sc * (q - 32) + 4096, 32..8192 (sc -128..127, q 0..63); its low and high byte (at most 32),
 //               sumi = 256 * acc1 + acc0 - 4096 * (sum of the block's activations)
 // The mins' sum_j m_j * (bsums[2j] + bsums[2j+1]) is one kind::f16 MMA per block (mins <= 63 and
 // 16-element sums <= 2048 are exact in f16, their products and sums in f32). Accumulators are read
@@ -22,10 +22,10 @@
 //   warps 12..19   terms: thread = weight row and every other 16 tokens; accumulators -> f32 terms -> the owners
 //   warps 20..23   sums: thread = weight row; adds the stage's C terms of its quads, in order; outputs
 //
-// What bounds it: a stage (a super-block per CTA) of 64 tokens takes about 1.3 us. Its MMAs are 0.28 us;
-// the rest is about 6000 warp instructions of unpacking, terms and sums at 1.9 per cycle, waiting for
-// one another's barriers and for distributed shared memory (32 KB of terms per stage at about 19 bytes
-// per cycle). The start of a product, from its first instruction to the first terms, is 4.5 us.
+// What bounds it: a stage (a super-block per CTA) of 64 tokens takes 1.64 us of Q4_K, 1.70 of Q5_K, 1.80 of Q6_K
+// (the fits of takes_kt in aotcu.cu). Its MMAs are 0.28 us; the rest is unpacking, terms and sums (Q6_K 8500 warp
+// instructions per stage and CTA at 2.3 per cycle) that wait for one another's barriers and for distributed shared
+// memory (32 KB of terms per stage). The start of a product, from its first instruction to the first terms, is 4.5 us.
 // Measured with the conversion of the activations (us; kmma.cuh, which unpacks into registers and has
 // its MMAs wait on the same warps, in brackets): 4096 x 14336 x 64 Q4_K 31 (46), Q6_K 33 (61); 24576 x
 // 4096 x 64 Q4_K 44 (74), Q6_K 48 (100); 2048 x 5632 x 64 Q6_K 17 (20). Tried: weights as f16 operands
@@ -110,8 +110,9 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
 }
 // "I have read it": the loads of this warp come before the arrive that lets their slot be overwritten, so it is a
 // release (by default, for the CTA), which costs nothing here: 24576 x 4096 x 64 Q4_K 44.3 us and 44.3 with a
-// relaxed arrive, Q6_K 48.5 and 48.5. A release at cluster scope, which also waits for what the warp has stored, is
-// 50.7 and 55.6.
+// relaxed arrive, Q6_K 48.5 and 48.5. A release at cluster scope, which the peers' acquire would ask for, also waits
+// for what the warp has stored, which nobody reads, and is 50.7 and 55.6; what has to come first here is loads alone,
+// and a load that has returned its value has been performed for every thread.
 __device__ __forceinline__ void cluster_arrive(uint32_t mapped_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }

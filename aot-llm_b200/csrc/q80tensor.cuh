@@ -12,7 +12,7 @@
 // What bounds it: instructions of the warps that run the chains. A block of 128 rows x 32 tokens needs
 // 390 cycles of their packed multiply-adds and scales and takes 930 (24 tokens 780, 16 tokens 680), its
 // MMAs 128. Measured with the conversion of the activations (us; the faster of the kernels before in
-// brackets): Q8_0 14336 x 4096, 64 rows 129 (196), 33 rows 110 (181), 17 rows 58 (114); Q4_0 6144 x 4096,
+// brackets): Q8_0 14336 x 4096, 64 rows 131 (196; 129 before the lanes of a warp voted on their waits), 33 rows 110 (181), 17 rows 58 (114); Q4_0 6144 x 4096,
 // 40 rows 51 (95). Tried: a wait and a release per step instead of per block 187; scalar multiply-adds, no
 // faster in their pipe, 1265 cycles against 1410 at 32 tokens but 940 against 830 at 16; the weights in
 // tensor memory, which leaves room for fewer results.
