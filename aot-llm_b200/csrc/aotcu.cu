@@ -679,10 +679,11 @@ static double q80_stream_us(const aotcu_ctx* c, int kind, size_t cols, size_t ro
   return 0.5 + ((m + 15) / 16) * (1.5 + (cols / 32) * block * (kind == Q4_0 ? 1 : kind == Q5_0 ? 1.1 : 0.95));
 }
 // Taken, of what launch_q80_tensor leaves (rows of up to about 1000 columns), where the estimate is lower than the
-// streaming kernel's. Fitted to timings of both, with q80_tensor at 1 (us, this kernel first): Q4_0 11264x2048 76 and 116 at 64 rows, 77 and 88 at 48, 53 and 59 at 32; 5632x2048 48 and 66 at 64
-// rows, 39 and 34 at 32; 2048x5632 123 and 83 at 64 rows, 124 and 165 at 128. Up to 16 rows the streaming kernel is a
-// single launch and the faster one nearly everywhere. Matrices that it does not take (rows not in fours, mixed kinds)
-// would go to the whole-row kernel, whose time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows.
+// streaming kernel's. Fitted to timings of both, with q80_tensor at 1 (us, this kernel first): Q4_0 11264x2048 76 and
+// 116 at 64 rows, 77 and 88 at 48, 53 and 59 at 32; 5632x2048 48 and 66 at 64 rows, 39 and 34 at 32; 2048x5632 123 and
+// 83 at 64 rows, 124 and 165 at 128. Up to 16 rows the streaming kernel is a single launch and the faster one nearly
+// everywhere. Matrices that it does not take (rows not in fours, mixed kinds) would go to the whole-row kernel, whose
+// time is linear in the batch: Q4_0 2049x5632 97 and 119 at 32 rows.
 constexpr size_t Q80_MMA_MIN_BATCH = 17, Q80_MMA_MIN_BATCH_ODD = 32;
 // CTAs of a product, `*wt` warps each: at most five share a row unit.
 static size_t q80_mma_ctas(const GemvCall& call, int* wt, int* n_tcta = nullptr) {
