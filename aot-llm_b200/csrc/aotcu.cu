@@ -520,18 +520,21 @@ static int launch_kt_one(aotcu_ctx* c, const GemvCall& call, const uint8_t* xt, 
   return 0;
 }
 // Which of the two: 0 by estimates, 1 kmma.cuh, 2 ktensor.cuh (option "k_tensor").
-// Estimates in microseconds, fitted to 1620 timings (20 matrices of each kind, 2 to 64 rows): a
-// launch, and per stage a part that does not depend on the batch (bringing and unpacking weights) and
-// one that does. On these the choice is 1.2 % from the better kernel on average. kmma.cuh has the
-// small products, where the shorter start counts (4096 x 4096 x 8 Q4_K: 8.9 against 10.4), and from
-// 16 to 24 rows on almost everything is ktensor.cuh's (24576 x 4096 x 64 Q4_K 44 against 74, Q6_K 48
-// against 100).
+// What each costs, a launch and per stage a part that does not depend on the batch (bringing and unpacking weights) and
+// one that does, with constants for which the choice itself is best on 1551 timings (45 matrices of 256 x 256 to 32768 x
+// 14336 and 12 pairs of each kind, 4 to 64 rows, weights not in L2; they are not microseconds): 0.3 % from the better
+// kernel on average, and at worst 7 % above kmma.cuh (11 % on 24 other matrices). (Constants fitted to times took ktensor.cuh too early: on 232 of
+// these more than 3 % above kmma.cuh, up to 40; Q6_K 5632 x 2048 x 8 9.6 us and 7.2.) kmma.cuh has the small products,
+// where the shorter start counts, and ktensor.cuh the large ones from 16 to 24 rows on (24576 x 4096 x 64 Q4_K 44 us
+// against 74, Q6_K 48 against 100). Pairs cost kmma.cuh more than their stages say, most with SiLU (a prompt of 20 rows of
+// the TinyLlama shape 1534 us where its Q4_K pairs are kmma.cuh's, 1507 where they are not; of 16 rows 1395 and 1409).
 static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
   struct Cost {
     double launch, stage, rows;
   };
-  static const Cost mma[3] = {{5.87, 0.826, 0.374}, {5.54, 1.026, 0.381}, {4.82, 1.488, 0.454}};  // rows: a group of 8
-  static const Cost tensor[3] = {{7.50, 0.633, 0.252}, {7.37, 0.674, 0.257}, {6.78, 1.029, 0.193}};  // rows: a group of 16
+  static const Cost mma[3] = {{2.034, 0.634, 0.413}, {1.474, 0.762, 0.591}, {1.185, 2.779, 0.396}};  // rows: a group of 8
+  static const Cost tensor[3] = {{6.024, 0.364, 0.240}, {7.461, 0.211, 0.367}, {9.178, 1.455, 0.120}};  // rows: a group of 16
+  static const double pair[3] = {1.08, 1.08, 1.35};
   const bool can = call.x_mode != 2 || call.xt;
   *yes = false;
   if (!can || c->k_tensor == 1) return 0;
@@ -543,7 +546,7 @@ static int takes_kt(aotcu_ctx* c, const GemvCall& call, bool* yes) {
     return rc;
   if (!stages) return 0;  // no cluster of a size that it may have fits the GPU
   if (c->k_tensor == 2) return *yes = true, 0;
-  const double s_mma = kmma_shape(c, call, &rt, &wk);
+  const double s_mma = kmma_shape(c, call, &rt, &wk) * (call.pair ? pair[k] : 1.0);
   double t_mma = 0.0, t_tensor = 0.0;
   for (size_t t0 = 0; t0 < call.m; t0 += KT_MAX_M) {
     const size_t m = std::min<size_t>(KT_MAX_M, call.m - t0);

@@ -22,8 +22,8 @@
 //   warps 12..19   terms: thread = weight row and every other 16 tokens; accumulators -> f32 terms -> the owners
 //   warps 20..23   sums: thread = weight row; adds the stage's C terms of its quads, in order; outputs
 //
-// What bounds it: a stage (a super-block per CTA) of 64 tokens takes 1.64 us of Q4_K, 1.70 of Q5_K, 1.80 of Q6_K
-// (the fits of takes_kt in aotcu.cu). Its MMAs are 0.28 us; the rest is unpacking, terms and sums (Q6_K 8500 warp
+// What bounds it: a stage (a super-block per CTA) of 64 tokens takes 1.65 us of Q4_K, 1.69 of Q5_K, 1.96 of Q6_K, and all
+// the rest of a product 5 (fits to 1755 timings, within 9 %). Its MMAs are 0.28 us; the rest is unpacking, terms and sums (Q6_K 8500 warp
 // instructions per stage and CTA at 2.3 per cycle) that wait for one another's barriers and for distributed shared
 // memory (32 KB of terms per stage). The start of a product, from its first instruction to the first terms, is 4.5 us.
 // Measured with the conversion of the activations (us; kmma.cuh, which unpacks into registers and has

@@ -94,6 +94,19 @@ def cluster_kernel(pkg, ctx):
     g.close()
 
 
+# Which of the two batch kernels is taken: measured, one is 10 % to twice as fast.
+@pytest.mark.parametrize("kind,rows,cols,m,cluster", [(Q6_K, 5632, 2048, 8, False), (Q6_K, 2048, 256, 40, False), (Q5_K, 1024, 1024, 48, False), (Q4_K, 300, 14336, 4, False),
+                                                      (Q6_K, 2049, 5632, 48, False), (Q4_K, 24576, 4096, 64, True), (Q5_K, 4096, 14336, 64, True), (Q6_K, 4096, 14336, 64, True)])
+def test_k_quant_choice_of_kernel(pkg, ob, ctx, kind, rows, cols, m, cluster):
+    spec = pkg.model.tiny("llama", n_layer=1)
+    g = pkg.Gpu(ctx, spec.head, spec.layers, spec.weights, 16, 2)
+    before = _launches(g)[0]
+    _run(pkg, ob, ctx, kind, make_weights(pkg, kind, rows, cols, 39 + kind, "uniform"), np.random.default_rng(m).standard_normal(m * cols).astype(np.float32), m, rows, cols,
+         f"kind {kind} {rows}x{cols} m {m}")
+    assert _launches(g)[0] - before == int(cluster)
+    g.close()
+
+
 # Fewer super-blocks than CTAs in a cluster, a last stage with some of them, rows that tensor copies
 # cannot take (Q6_K: 768 and 2304 columns), a partial row tile, several tiles per cluster, token groups
 # of every parity and a second launch.
